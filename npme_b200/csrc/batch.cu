@@ -42,7 +42,8 @@ struct BatchSys {
   float *grid;    // real N1 N2 N3 (real kernels) or complex (Helmholtz)
   float2 *kgrid;  // R2C half spectrum (real kernels)
   const float *G;
-  long N1, N2, N3;
+  long N1, N2, N3;  // FFT box
+  long g1, g2, g3;  // dimensions the grid is stored with
   float c1, c2, c3;
   const double4 *gpos, *spos;
   const int4 *groups;
@@ -94,7 +95,7 @@ __global__ void __launch_bounds__(256) batch_spread_kernel(const BatchSys *__res
   const int s = find_sys(off, count, u);
   const BatchSys &S = sys[s];
   spread_brick_fixed<P, CPLX>(S.brick_list[u - off[s]], S.brick_start, S.bpts, S.qb, S.grid,
-                              S.nb2, S.nb3, S.N1, S.N2, S.N3, reinterpret_cast<int *>(smem_raw));
+                              S.nb2, S.nb3, S.g1, S.g2, S.g3, reinterpret_cast<int *>(smem_raw));
 }
 
 // one warp per spectrum row of one system (units: rows)
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(256) batch_interp_kernel(const BatchSys *__res
   const int s = find_sys(off, count, u);
   const BatchSys &S = sys[s];
   interp_brick_body<float, P, CPLX>(S.brick_list[u - off[s]], S.brick_start, S.bpts, S.grid, S.V,
-                                    S.nb2, S.nb3, S.N1, S.N2, S.N3, S.c1, S.c2, S.c3,
+                                    S.nb2, S.nb3, S.g1, S.g2, S.g3, S.c1, S.c2, S.c3,
                                     reinterpret_cast<float *>(smem_raw),
                                     S.fold ? (void *)S.vsrc : nullptr, S.vs, S.gs);
 }
@@ -208,6 +209,15 @@ struct Class {
   std::vector<int> members;  // indices into the batch's FP32 handle list
   std::vector<long long> off;   // prefix of the class's work units
   size_t desc_at = 0, off_at = 0;  // byte offsets in the descriptor block
+};
+
+// The members whose transforms the library's own kernels run.
+struct FftClass {
+  std::vector<int> members;
+  std::vector<long long> off;  // CTA prefixes of x, y and z
+  long units[3] = {0, 0, 0};
+  size_t smem[3] = {0, 0, 0};
+  size_t desc_at = 0, off_at = 0;
 };
 
 size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
@@ -326,6 +336,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     S.kgrid = (float2 *)h->d_kgrid;
     S.G = (const float *)h->d_G;
     S.N1 = h->grid.N[0], S.N2 = h->grid.N[1], S.N3 = h->grid.N[2];
+    S.g1 = h->gd[0], S.g2 = h->gd[1], S.g3 = h->gd[2];
     S.c1 = (float)(h->grid.N[0] / h->box[6]);
     S.c2 = (float)(h->grid.N[1] / h->box[7]);
     S.c3 = (float)(h->grid.N[2] / h->box[8]);
@@ -351,7 +362,8 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   }
 
   // launch classes
-  std::map<int, Class> gath, mult;                           // key: complex
+  std::map<int, Class> gath, mult;                           // key: complex (mult: cuFFT members)
+  std::map<int, FftClass> own;                               // key: complex
   std::map<std::pair<int, int>, Class> spr;                  // (order, complex)
   typedef std::tuple<int, int, int, int, double, double, double, double, double> DKey;
   std::map<DKey, Class> dir;  // direct sums
@@ -359,7 +371,8 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     const npme_handle *h = hs[f32[k]];
     const int cx = h->complex_kernel ? 1 : 0;
     gath[cx].members.push_back(k);
-    mult[cx].members.push_back(k);
+    if (h->own_fft) own[cx].members.push_back(k);
+    else mult[cx].members.push_back(k);
     spr[{h->grid.order, cx}].members.push_back(k);
     const DKey key(pairs_once(h) ? 1 : 0, h->p.funcType, h->p.EwaldSplit, h->p.nDeriv,
                    h->p.Rdir, h->p.alpha, h->p.k0_r, h->p.k0_i, h->beta);
@@ -392,6 +405,26 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   for (auto &kv : mult) lay(kv.second, units_mult);
   for (auto &kv : spr) lay(kv.second, units_spread);  // spread and interpolation: bricks
   for (auto &kv : dir) lay(kv.second, units_dir);
+  for (auto &kv : own) {  // transform descriptors, then the CTA prefixes of x, y and z
+    FftClass &c = kv.second;
+    const size_t n = c.members.size();
+    c.off.assign(3 * (n + 1), 0);
+    for (int a = 0; a < 3; a++) {
+      long long *o = c.off.data() + a * (n + 1);
+      c.smem[a] = 0;
+      for (size_t t = 0; t < n; t++) {
+        const FftJob &j = hs[f32[c.members[t]]]->fft;
+        o[t + 1] = o[t] + (a == 0 ? j.ux : a == 1 ? j.uy : j.uz);
+        c.smem[a] = std::max(c.smem[a], own_fft_smem(j, a, sizeof(float2)));
+      }
+      c.units[a] = o[n];
+      if (c.units[a] >= (1LL << 31)) return bfail(b, NPME_EINVAL, "batch too large");
+    }
+    c.desc_at = bytes;
+    bytes = align16(bytes + sizeof(FftJob) * n);
+    c.off_at = bytes;
+    bytes = align16(bytes + sizeof(long long) * c.off.size());
+  }
 
   // the pinned staging buffer is reused: wait for the previous batch's copy
   if (b->pending) {
@@ -423,6 +456,12 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     BatchSys *dd = (BatchSys *)(b->h_pinned + c->desc_at);
     for (size_t t = 0; t < c->members.size(); t++) dd[t] = desc[c->members[t]];
     memcpy(b->h_pinned + c->off_at, c->off.data(), sizeof(long long) * c->off.size());
+  }
+  for (auto &kv : own) {
+    FftClass &c = kv.second;
+    FftJob *dj = (FftJob *)(b->h_pinned + c.desc_at);
+    for (size_t t = 0; t < c.members.size(); t++) dj[t] = hs[f32[c.members[t]]]->fft;
+    memcpy(b->h_pinned + c.off_at, c.off.data(), sizeof(long long) * c.off.size());
   }
   cudaMemcpyAsync(b->d_block, b->h_pinned, bytes, cudaMemcpyHostToDevice, s);
   auto D = [&](const Class &c) { return (const BatchSys *)(b->d_block + c.desc_at); };
@@ -527,10 +566,19 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return bfail(b, NPME_ECUDA, std::string("batch: ") + cudaGetErrorString(e));
   }
-  // 4. forward transforms
+  // 4. transforms and kernel multiply of the members with the library's own
+  // transforms: five launches for all of one kind
+  for (auto &kv : own) {
+    FftClass &c = kv.second;
+    own_convolve_batch((const FftJob *)(b->d_block + c.desc_at),
+                       (const long long *)(b->d_block + c.off_at), (int)c.members.size(),
+                       kv.first != 0, c.units, c.smem, s);
+    b->launches += 5;
+  }
+  // the others: forward transforms
   for (int k = 0; k < m; k++) {
     npme_handle *h = hs[f32[k]];
-    if (fft_forward(h, s)) return bfail(b, NPME_ECUDA, "batch: " + h->err);
+    if (!h->own_fft && fft_forward(h, s)) return bfail(b, NPME_ECUDA, "batch: " + h->err);
   }
   // 5. kernel multiply
   for (auto &kv : mult) {
@@ -547,7 +595,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   // 6. inverse transforms
   for (int k = 0; k < m; k++) {
     npme_handle *h = hs[f32[k]];
-    if (fft_inverse(h, s)) return bfail(b, NPME_ECUDA, "batch: " + h->err);
+    if (!h->own_fft && fft_inverse(h, s)) return bfail(b, NPME_ECUDA, "batch: " + h->err);
   }
   // 7. interpolation after the direct sums
   cudaStreamWaitEvent(s, b->ev_join, 0);

@@ -1,5 +1,6 @@
 // The reciprocal sum's transforms with cuFFT, pruned to the charge octant,
-// and the plans they share across handles.
+// and the plans they share across handles: the path of boxes with an FFT
+// length that has a prime factor above 5 (fft_own.cuh takes the others).
 //
 // The spread grid is the zero-padded box N1 x N2 x N3 whose charges all lie
 // in the octant [0, N1/2) x [0, N2/2) x [0, N3/2), and the interpolation
@@ -124,6 +125,13 @@ static size_t cplx_bytes(const npme_handle *h) { return h->fp32 ? 8 : 16; }
 
 int grid_clear(npme_handle *h, cudaStream_t s) {
   const long *N = h->grid.N;
+  if (h->own_fft) {  // the octant
+    const size_t b = (h->fp32 ? 4 : 8) * (h->complex_kernel ? 2 : 1);
+    return cudaMemsetAsync(h->d_grid, 0, b * (size_t)h->gd[0] * h->gd[1] * h->gd[2], s) ==
+                   cudaSuccess
+               ? NPME_OK
+               : NPME_ECUDA;
+  }
   // real kernels: only the slabs x < N1/2 feed the transform; complex
   // kernels: the whole grid (the upper slabs hold the last inverse pass)
   const size_t bytes = h->complex_kernel ? cplx_bytes(h) * (size_t)N[0] * N[1] * N[2]
@@ -176,6 +184,7 @@ int fft_inverse(npme_handle *h, cudaStream_t s) {
 
 // Looks up the handle's plans and sizes its work buffer.
 int prepare_plans(npme_handle *h) {
+  if (h->own_fft) return own_fft_prepare(h);
   const long *N = h->grid.N;
   int tf, ti, tx;
   long slab_points;

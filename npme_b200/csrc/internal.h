@@ -63,6 +63,28 @@ struct FFTPlan {
   std::mutex mu;    // guards stream / work-area binding + enqueue
 };
 
+// A transform by the library's own kernels (fft_own.cuh): the passes of one
+// axis, and what the launches of one system need.
+struct FftPass {
+  int R, Ns;       // radix, product of the radices before it
+  unsigned magic;  // ceil(2^32 / Ns): j / Ns by a high multiply
+  int step;        // twiddle table stride of this pass
+};
+struct FftAxis {
+  int N, np, lb;   // length, passes, log2 of the lines per CTA
+  int twlen;
+  const void *tw;  // exp(-2 pi i m / twlen), the bulk precision
+  FftPass p[8];
+};
+struct FftJob {
+  void *grid, *spec;
+  const void *G;
+  int H[3], N[3];
+  int K, KP;       // values per spectrum row, and its pitch
+  FftAxis x, xi, y, z;  // xi: x with the passes in reverse order
+  long ux, uy, uz; // CTAs of each pass
+};
+
 }  // namespace npme
 
 struct npme_handle {
@@ -93,6 +115,9 @@ struct npme_handle {
   // and the transforms along x (fft.cu)
   npme::FFTPlan *pf = nullptr, *pi = nullptr, *px = nullptr;
   void *d_work = nullptr;                        // this handle's cuFFT work area
+  bool own_fft = false;  // transforms by the library's kernels (fft_own.cuh), not cuFFT
+  npme::FftJob fft = {}; // their description
+  long gd[3] = {0, 0, 0};  // dimensions the grid is stored with: the octant, or (cuFFT) the box
   cudaMemPool_t pool = nullptr;                  // device memory pool (shared, not owned)
 
   // device buffers (all allocated in setup; calcv allocates nothing)
@@ -222,6 +247,18 @@ int prepare_plans(npme_handle *h);
 int grid_clear(npme_handle *h, cudaStream_t s);
 int fft_forward(npme_handle *h, cudaStream_t s);
 int fft_inverse(npme_handle *h, cudaStream_t s);
+// fftk.cu: whether the handle's box has lengths the library's own transforms
+// take, the description of its transforms, and the convolution of the spread
+// grid with the kernel transform (five launches, whole batches in the same
+// five)
+bool own_fft_lengths(const long N[3]);
+int own_fft_prepare(npme_handle *h);
+// part 0: forward along z and y; 1: forward along x, kernel multiply, inverse
+// along x; 2: inverse along y and z
+void own_convolve(npme_handle *h, int part, cudaStream_t s);
+void own_convolve_batch(const FftJob *jobs, const long long *offs, int count, bool cplx,
+                        const long units[3], const size_t smem[3], cudaStream_t s);
+size_t own_fft_smem(const FftJob &j, int axis, size_t cbytes);
 
 // recsum.cu
 int build_kernel_transform(npme_handle *h);  // F-hat, lambda^2 -> d_G

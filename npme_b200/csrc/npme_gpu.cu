@@ -425,6 +425,8 @@ static int setup_prepare(npme_handle *h, size_t n, const double *coord) {
     h->grid.nb[d] = (Ns[d] / 2 + npme::kBrick - 1) / npme::kBrick;
   }
   h->grid.order = p.BnOrder;
+  h->own_fft = npme::own_fft_lengths(Ns);
+  for (int d = 0; d < 3; d++) h->gd[d] = h->own_fft ? h->grid.H[d] : Ns[d];
   // the reference's cells of edge >= Rdir / nNeigh (reported by
   // npme_gpu_get_info; the direct sum walks warp groups instead)
   const double target = p.Rdir / p.nNeigh;
@@ -647,12 +649,21 @@ static int enqueue_calcv(npme_handle *h, double *d_V, const double *d_charge, cu
   npme::launch_spread(h, s);
   CK(cudaGetLastError());
   tmark(h, 2, s);
-  if ((frc = npme::fft_forward(h, s))) return frc;
-  tmark(h, 3, s);
-  npme::launch_multiply(h, s);
-  CK(cudaGetLastError());
-  tmark(h, 4, s);
-  if ((frc = npme::fft_inverse(h, s))) return frc;
+  if (h->own_fft) {
+    npme::own_convolve(h, 0, s);
+    tmark(h, 3, s);
+    npme::own_convolve(h, 1, s);
+    tmark(h, 4, s);
+    npme::own_convolve(h, 2, s);
+    CK(cudaGetLastError());
+  } else {
+    if ((frc = npme::fft_forward(h, s))) return frc;
+    tmark(h, 3, s);
+    npme::launch_multiply(h, s);
+    CK(cudaGetLastError());
+    tmark(h, 4, s);
+    if ((frc = npme::fft_inverse(h, s))) return frc;
+  }
   tmark(h, 5, s);
   if (serial && (frc = fork_direct())) return frc;
   CK(cudaStreamWaitEvent(s, h->ev_join, 0));

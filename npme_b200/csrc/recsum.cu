@@ -924,8 +924,8 @@ static void spread_dispatch(npme_handle *h, cudaStream_t s) {
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   kern<<<(unsigned)h->n_nonempty, 256, smem, s>>>(
       h->d_brick_list, h->d_brick_start, (const BrickPoint<T> *)h->d_bpts,
-      (const T *)h->d_qb, (T *)h->d_grid, (int)h->grid.nb[1], (int)h->grid.nb[2],
-      h->grid.N[0], h->grid.N[1], h->grid.N[2]);
+      (const T *)h->d_qb, (T *)h->d_grid, (int)h->grid.nb[1], (int)h->grid.nb[2], h->gd[0],
+      h->gd[1], h->gd[2]);
 }
 
 template <typename T, bool CPLX>
@@ -1035,7 +1035,7 @@ static void interp_dispatch(npme_handle *h, double *d_V, cudaStream_t s) {
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   kern<<<(unsigned)h->n_nonempty, 256, smem, s>>>(
       h->d_brick_list, h->d_brick_start, (const BrickPoint<T> *)h->d_bpts, (const T *)h->d_grid,
-      d_V, (int)h->grid.nb[1], (int)h->grid.nb[2], h->grid.N[0], h->grid.N[1], h->grid.N[2],
+      d_V, (int)h->grid.nb[1], (int)h->grid.nb[2], h->gd[0], h->gd[1], h->gd[2],
       (T)(h->grid.N[0] / L[0]), (T)(h->grid.N[1] / L[1]), (T)(h->grid.N[2] / L[2]),
       h->merge_pending ? (h->fp32 ? (void *)h->d_vsrc : (void *)h->d_vsrc64) : nullptr,
       h->merge_vs, h->merge_gs);

@@ -788,7 +788,14 @@ int describe(npme_handle *h, SysDesc &D) {
   const long *N = gr.N;
   const size_t Ntot = (size_t)N[0] * N[1] * N[2];
   const size_t Mtot = (size_t)(N[0] / 2 + 1) * (N[1] / 2 + 1) * (N[2] / 2 + 1);
-  if (h->complex_kernel) {
+  if (h->own_fft) {  // the octant, and half the box of spectrum rows
+    const size_t K = h->complex_kernel ? N[2] : N[2] / 2 + 1;
+    if ((rc = handle_buffer(h, &h->d_grid, sizeof(T) * C * (Ntot / 8))) ||
+        (rc = handle_buffer(h, &h->d_kgrid,
+                            sizeof(T) * 2 * (size_t)(N[0] / 2) * N[1] * ((K + 3) & ~size_t(3)))) ||
+        (rc = handle_buffer(h, &h->d_G, sizeof(T) * C * Mtot)))
+      return rc;
+  } else if (h->complex_kernel) {
     if ((rc = handle_buffer(h, &h->d_grid, sizeof(T) * 2 * Ntot)) ||
         (rc = handle_buffer(h, &h->d_G, sizeof(T) * 2 * Mtot)))
       return rc;
