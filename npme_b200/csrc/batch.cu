@@ -151,9 +151,8 @@ __global__ void __launch_bounds__(32 * kGroupWarps, kGroupMinBlocks) batch_direc
                                            sp[wid], slo[wid], lane);
 }
 
-// Pair-once direct sums of a batch (direct_group_sym and its complex and
-// scalar forms): KIND 0 the packed real DM body, 1 Helmholtz DM, 2 the scalar
-// body of the original Ewald split.
+// Pair-once direct sums of a batch: KIND 0 the packed real body
+// (direct_group_sym), 1 Helmholtz DM.
 template <int KIND, int FUNC, int ND>
 __global__ void __launch_bounds__(32 * kGroupWarps) batch_sym_kernel(
     PairCoef<float> k, const BatchSys *__restrict__ sys, const long long *__restrict__ off,
@@ -166,18 +165,17 @@ __global__ void __launch_bounds__(32 * kGroupWarps) batch_sym_kernel(
   const int s = find_sys(off, count, u);
   const BatchSys &S = sys[s];
   const long g = (long)(u - off[s]);
-  if constexpr (KIND == 0)
-    direct_group_sym<FUNC, ND>(k, S.gpos, S.spos, S.qc, S.q, S.hgroups[g], S.hcen[g], S.hsegs,
-                               S.cperm, S.refine2, S.fself_r, S.V, S.vsrc, ta[wid], tb[wid],
-                               lane);
-  else if constexpr (KIND == 1)
+  if constexpr (KIND == 0) {
+    double acc[4] = {0, 0, 0, 0};
+    const int4 G = S.hgroups[g];
+    direct_group_sym<FUNC, ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.cperm,
+                               S.refine2, S.vsrc, ta[wid], tb[wid], lane, 0, 1, acc);
+    sym_store(k, G, S.cperm, S.q, S.fself_r, S.V, lane, acc);
+  } else {
     direct_group_sym_helm<ND>(k, S.gpos, S.spos, S.qc, S.q, S.hgroups[g], S.hcen[g], S.hsegs,
                               S.cperm, S.refine2, S.fself_r, S.fself_i, S.V, S.vsrc, ta[wid],
                               tb[wid], lane);
-  else
-    direct_group_sym_scalar<0, 1, 0>(k, S.gpos, S.spos, S.qc, S.q, S.hgroups[g], S.hcen[g],
-                                     S.hsegs, S.cperm, S.refine2, S.fself_r, S.V, S.vsrc,
-                                     ta[wid], tb[wid], lane);
+  }
 }
 
 }  // namespace npme
@@ -355,7 +353,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     S.fself_i = h->fself_i;
     S.fold = pairs_once(h) ? 1 : 0;
     const bool scaled =
-        h->p.funcType != NPME_FUNC_HELMHOLTZ && h->p.EwaldSplit != NPME_SPLIT_LAPLACE_ORIG;
+        h->p.funcType != NPME_FUNC_HELMHOLTZ;
     const PairCoef<float> pc = make_pair_coef<float>(h);
     S.vs = scaled ? pc.vscale : 1.0;
     S.gs = scaled ? pc.gscale : 1.0;
@@ -489,7 +487,9 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     if (ng == 0) continue;
     const unsigned g = (unsigned)((ng + kGroupWarps - 1) / kGroupWarps);
     const int cnt = (int)c.members.size();
-    const int f = h0->p.funcType, sp = h0->p.EwaldSplit, nd = sp == 1 ? 0 : h0->p.nDeriv;
+    const int f = h0->p.funcType, sp = h0->p.EwaldSplit;
+    // fixed-order instances: see dm_eval2 for alpha
+    const int nd = sp == 1 || (f == NPME_FUNC_RALPHA && h0->p.alpha >= 0) ? 0 : h0->p.nDeriv;
     if (std::get<0>(kv.first)) {  // pair-once walk, then the source-side sums
 #define NPME_BSYM(KD, FN, ND) \
   batch_sym_kernel<KD, FN, ND><<<g, 32 * kGroupWarps, 0, b->stream2>>>(k, D(c), O(c), cnt)
@@ -501,7 +501,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     default: NPME_BSYM(KD, FN, 0); break;   \
   }
       if (f == NPME_FUNC_HELMHOLTZ) { NPME_BSYM_ND(1, 2); }
-      else if (sp == NPME_SPLIT_LAPLACE_ORIG) { NPME_BSYM(2, 0, 0); }
+      else if (sp == NPME_SPLIT_LAPLACE_ORIG) { NPME_BSYM(0, 2, 0); }
       else if (f == NPME_FUNC_RALPHA) { NPME_BSYM_ND(0, 1); }
       else { NPME_BSYM_ND(0, 0); }
 #undef NPME_BSYM_ND

@@ -426,69 +426,118 @@ __device__ __forceinline__ void interp_brick_body(int brick, const int *__restri
 constexpr int kPackedBlock = NPME_PACKED_BLOCK;
 
 // Real DM pair kernel in the scaled frame (coordinates in units of Rdir,
-// s = r^2): f0 = Rdir^(-alpha)... scaled f_SR and t = -(scaled f1) for two
-// squared distances at once.  1/r: f0 = 1/r - P(s), t = 1/r^3 + D(s);
-// r^alpha: f0 = s^(alpha/2) - P(s), t = -alpha s^(alpha/2) / s + D(s), with
-// P, D the DM polynomials (src/KernelFunctionLaplace.cpp:394-436,
+// s = r^2 <= 1) for two squared distances at once: f0 = scaled f_SR = s^a - P
+// and t = (scaled f1) / alpha, a = alpha / 2, from the Taylor form of the
+// derivative match in u = 1 - s (PairCoef; src/KernelFunctionLaplace.cpp:394-436,
 // src/KernelFunctionRalpha.cpp:342-384).
-// ND > 0: the derivative-match order as a compile-time constant (the
-// polynomials fully unrolled); ND = 0: any order up to kMaxDeriv, evaluated
-// as the polynomials of degree kMaxDeriv whose coefficients above the order
-// are zero (make_pair_coef), so Horner's leading steps give exactly 0 and
-// the result is bit for bit that of the exact degree, at the cost of the
-// extra steps but with every coefficient at a fixed offset of the parameter
-// bank (a loop over a run-time degree indexes it dynamically and is ~2x
-// slower still).
+// ND > 0: the derivative-match order as a compile-time constant and alpha < 0:
+// P by Horner, t = (f0 + K u^ND) / s, which needs no second polynomial (1/r,
+// order 6: 6 multiply-adds for t against 7; order 8: 6 against 9) and has no
+// cancellation, both terms being positive.  ND = 0: any order up to
+// kMaxDeriv and any alpha (for alpha >= 0 the two terms of that t cancel at
+// small s), both polynomials evaluated at degree kMaxDeriv with zero
+// coefficients above the order, so that every coefficient sits at a fixed
+// offset of the parameter bank (a loop over a run-time degree indexes it
+// dynamically and is ~2x slower still).
+// At s = 1 the result is exactly zero in f0 and t: a miss is a pair with its
+// s clamped to 1.
+// FUNC 2: the original Ewald split, f0 = erfc(b sqrt(s))/sqrt(s) with b = beta
+// Rdir (src/PotentialLaplace.cpp:614-719), about 20 operations like the DM
+// kernel; erfcf and expf take about twice that.
 template <int ND>
 constexpr int dm_degree() {
   return ND > 0 ? ND : kMaxDeriv;
 }
 
-template <int FUNC, int ND>
-__device__ __forceinline__ void dm_eval2(const PairCoef<float> &k, float2 sv, float2 &f0,
+// 1/x and 2^x by the special-function unit (1 and 2 ulp)
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+template <bool FTZ>
+__device__ __forceinline__ float2 rsqrt2(float2 s) {
+  if (!FTZ) return make_float2(rsqrtf(s.x), rsqrtf(s.y));
+  float2 r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(s.x));
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(s.y));
+  return r;
+}
+
+// u^N, N > 0 known at compile time
+template <int N>
+__device__ __forceinline__ float2 pow2_n(float2 u) {
+  if constexpr (N == 1) {
+    return u;
+  } else {
+    const float2 h = pow2_n<N / 2>(u), h2 = __fmul2_rn(h, h);
+    if constexpr (N % 2) return __fmul2_rn(h2, u);
+    else return h2;
+  }
+}
+
+// FTZ: s is a normal number (no pair of a sweep is close), so the
+// special-function unit's rsqrt is taken as it is; rsqrtf adds four
+// instructions per value for subnormal arguments.
+template <int FUNC, int ND, bool FTZ = false>
+__device__ __forceinline__ void dm_eval2(const PairCoef<float> &k, float2 s, float2 &f0,
                                          float2 &t) {
   constexpr int nd = dm_degree<ND>();
-  float2 np = k.nar2[nd];  // -Rdir^(-alpha) f_LR polynomial
+  const float2 one = make_float2(1.f, 1.f), mone = make_float2(-1.f, -1.f);
+  if constexpr (FUNC == 2) {  // original Ewald split: not zero at s = 1
+    // erfc(x) = exp(-x^2) erfcx(x), x = beta r; erfcx a polynomial in tau = (x
+    // - 3)/(x + 3) over x + 3, so that the exponential serves f0 and t
+    const float2 ri = rsqrt2<FTZ>(s);
+    const float2 x = __fmul2_rn(__fmul2_rn(s, k.nq2[0]), ri);
+    const float2 d = __fadd2_rn(x, make_float2(3.f, 3.f));
+    const float2 w = make_float2(rcp_approx(d.x), rcp_approx(d.y));
+    const float2 tau = __ffma2_rn(w, make_float2(-6.f, -6.f), one);
+    float2 h = k.nc2[9];
 #pragma unroll
-  for (int n = nd - 1; n >= 0; n--) np = __ffma2_rn(np, sv, k.nar2[n]);
-  float2 d = k.br2[nd - 1];  // Rdir^(2-alpha) (1/r) d f_LR / dr polynomial
+    for (int n = 8; n >= 0; n--) h = __ffma2_rn(h, tau, k.nc2[n]);
+    const float2 a = __fmul2_rn(s, k.nq2[1]);
+    const float2 e = make_float2(ex2_approx(a.x), ex2_approx(a.y));
+    f0 = __fmul2_rn(__fmul2_rn(__fmul2_rn(h, w), e), ri);
+    t = __fmul2_rn(__ffma2_rn(e, k.kn2, f0), __fmul2_rn(ri, ri));
+    return;
+  }
+  const float2 u = __ffma2_rn(s, mone, one);
+  float2 h = k.nc2[nd];
 #pragma unroll
-  for (int n = nd - 2; n >= 0; n--) d = __ffma2_rn(d, sv, k.br2[n]);
-  if (FUNC == 0) {
-    const float2 ri = make_float2(rsqrtf(sv.x), rsqrtf(sv.y));
-    f0 = __fadd2_rn(ri, np);                    // Rdir (1/r - f_LR)
-    t = __ffma2_rn(__fmul2_rn(ri, ri), ri, d);  // -Rdir^3 f1
+  for (int n = nd - 1; n >= 1; n--) h = __ffma2_rn(h, u, k.nc2[n]);
+  const float2 ri = rsqrt2<FTZ>(s);
+  // 1/r: s^a = rsqrt(s); r^alpha: 2^(a log2 s) on the special-function unit
+  float2 e0 = ri;
+  if (FUNC == 1)
+    e0 = FTZ ? make_float2(ex2_approx(k.half_alpha * __log2f(s.x)),
+                           ex2_approx(k.half_alpha * __log2f(s.y)))
+             : make_float2(exp2f(k.half_alpha * __log2f(s.x)),
+                           exp2f(k.half_alpha * __log2f(s.y)));
+  f0 = __ffma2_rn(h, u, __fadd2_rn(e0, mone));
+  const float2 ri2 = __fmul2_rn(ri, ri);
+  if constexpr (ND > 0) {
+    t = __fmul2_rn(__ffma2_rn(pow2_n<ND>(u), k.kn2, f0), ri2);
   } else {
-    // s^(alpha/2) = 2^((alpha/2) log2 s) on the special-function unit;
-    // 1/s = rsqrt(s)^2
-    const float2 e0 = make_float2(exp2f(k.half_alpha * __log2f(sv.x)),
-                                  exp2f(k.half_alpha * __log2f(sv.y)));
-    const float2 ri = make_float2(rsqrtf(sv.x), rsqrtf(sv.y));
-    f0 = __fadd2_rn(e0, np);
-    t = __ffma2_rn(__fmul2_rn(e0, make_float2(-k.alpha, -k.alpha)), __fmul2_rn(ri, ri), d);
+    float2 d = k.nq2[nd - 1];
+#pragma unroll
+    for (int n = nd - 2; n >= 0; n--) d = __ffma2_rn(d, u, k.nq2[n]);
+    t = __ffma2_rn(e0, ri2, d);
   }
 }
 
 // The same pair kernel for one squared distance.
 template <int FUNC, int ND>
-__device__ __forceinline__ void dm_eval1(const PairCoef<float> &k, float sv, float &f0,
-                                         float &t) {
-  constexpr int nd = dm_degree<ND>();
-  float np = k.nar2[nd].x;
-#pragma unroll
-  for (int n = nd - 1; n >= 0; n--) np = fmaf(np, sv, k.nar2[n].x);
-  float d = k.br2[nd - 1].x;
-#pragma unroll
-  for (int n = nd - 2; n >= 0; n--) d = fmaf(d, sv, k.br2[n].x);
-  const float ri = rsqrtf(sv);
-  if (FUNC == 0) {
-    f0 = ri + np;
-    t = fmaf(ri * ri, ri, d);
-  } else {
-    const float e0 = exp2f(k.half_alpha * __log2f(sv));
-    f0 = e0 + np;
-    t = fmaf(e0 * -k.alpha, ri * ri, d);
-  }
+__device__ __forceinline__ void dm_eval1(const PairCoef<float> &k, float s, float &f0, float &t) {
+  float2 f, g;
+  dm_eval2<FUNC, ND>(k, make_float2(s, s), f, g);
+  f0 = f.x;
+  t = g.x;
 }
 
 template <int FUNC, int ND, bool REFINE>
@@ -673,150 +722,172 @@ __device__ __forceinline__ void direct_group_packed(
   }
 }
 
-// One block of steps of the Newton's-third-law sweep (below):
-// lane l holds the source pair (a, b) of a 64-source chunk in registers and
-// meets target (l + k) mod 32 of the group at step k, read from the group's
-// target tile in shared memory.  Every pair is evaluated once and gives both
-// sides: the target-side sums (aV, aX, aY, aZ) travel with their target,
-// one lane down per step (__shfl_sync from lane + 1), and the source-side
-// sums (SV, SX, SY, SZ, packed for a and b) stay in the lane.  Source
-// coordinates are held negated (sx2 = -x_s) as in the staged layout of the
-// one-sided body; misses get r^2 = 1 (Rdir^2) and charge 0 on both sides.
-#ifndef NPME_SYM_BLOCK
-#define NPME_SYM_BLOCK 0
-#endif
-// steps per block of the pair-once sweep (measured: 2 for 1/r, 4 for r^alpha)
-template <int FUNC>
-constexpr int sym_block_steps() {
-  return NPME_SYM_BLOCK > 0 ? NPME_SYM_BLOCK : (FUNC == 1 ? 4 : 2);
-}
+// The two sources of a lane in the pair-once sweep: coordinates relative to
+// the group centre, negated (so that t + (-s) gives t - s exactly), and the
+// residuals of their rounding, each as the pair (v, v) that meets two
+// targets at once.
+struct SymSource {
+  float2 x, y, z, q, lx, ly, lz;
+};
 
-template <int FUNC, int ND, bool REFINE>
-__device__ __forceinline__ void sym_block(
-    const PairCoef<float> &k, const float4 *tsm, const float4 *tlo, int lane, int k0,
-    float2 sx2, float2 sy2, float2 sz2, float2 q2, float2 lx2, float2 ly2, float2 lz2,
-    float refine2, float &aV, float &aX, float &aY, float &aZ, float2 &SV, float2 &SX,
-    float2 &SY, float2 &SZ) {
-  constexpr int U = sym_block_steps<FUNC>();
-  const unsigned FULL = 0xffffffffu;
-  const unsigned rb = __float_as_uint(1.f);
-  float2 x[U], y[U], z[U], rr[U], qm[U], qt[U];
-  int tt[U];
-  float rmin = 3.0e38f;
-  bool any = false;
+// One step of the Newton's-third-law sweep (below): the lane's two sources
+// against one pair of targets (A = x0 x1 y0 y1, B = z0 z1 q0 q1; LA, LB the
+// residuals), four pairs, every one evaluated once for both of its points:
+// target sums aV.. (packed over the two targets) and source sums S[i].
+// CHECKED = false: no pair of the chunk is closer than the refinement radius
+// and all charges are finite, so a miss needs nothing but s clamped to 1,
+// where the pair kernel is exactly zero.  CHECKED = true: close pairs are
+// recomputed from heads and residuals, coincident points are no pair, and
+// misses also get charge 0 (a non-finite charge stays out of their sums).
+template <int FUNC, int ND, bool CHECKED>
+__device__ __forceinline__ void sym_step(const PairCoef<float> &k, const float4 A, const float4 B,
+                                         const float4 *la, const float4 *lb,
+                                         const SymSource (&src)[2], float refine2, float2 &aV,
+                                         float2 &aX, float2 &aY, float2 &aZ, float2 (&S)[2][4]) {
+  float2 x[2], y[2], z[2], s[2], qs[2], qt[2];
 #pragma unroll
-  for (int u = 0; u < U; u++) {
-    tt[u] = (lane + k0 + u) & 31;
-    const float4 T = tsm[tt[u]];
-    x[u] = __fadd2_rn(make_float2(T.x, T.x), sx2);
-    y[u] = __fadd2_rn(make_float2(T.y, T.y), sy2);
-    z[u] = __fadd2_rn(make_float2(T.z, T.z), sz2);
-    const float2 r2 = __ffma2_rn(x[u], x[u], __ffma2_rn(y[u], y[u], __fmul2_rn(z[u], z[u])));
-    const bool h0 = __float_as_uint(r2.x) - 1u < rb, h1 = __float_as_uint(r2.y) - 1u < rb;
-    rr[u] = make_float2(h0 ? r2.x : 1.f, h1 ? r2.y : 1.f);
-    qm[u] = make_float2(h0 ? q2.x : 0.f, h1 ? q2.y : 0.f);
-    qt[u] = make_float2(h0 ? T.w : 0.f, h1 ? T.w : 0.f);
-    if (REFINE) rmin = fminf(rmin, fminf(rr[u].x, rr[u].y));
-    any |= h0 | h1;
-  }
-  if (!__any_sync(FULL, any)) {  // no pair of the block inside the cutoff
-    const int src = (lane + U) & 31;
-    aV = __shfl_sync(FULL, aV, src);
-    aX = __shfl_sync(FULL, aX, src);
-    aY = __shfl_sync(FULL, aY, src);
-    aZ = __shfl_sync(FULL, aZ, src);
-    return;
-  }
-  if (REFINE && rmin < refine2) {  // close pair: exact difference from head + residual
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      if (fminf(rr[u].x, rr[u].y) < refine2) {
-        const float4 L = tlo[tt[u]];
-        x[u] = __fadd2_rn(x[u], __fadd2_rn(make_float2(L.x, L.x), lx2));
-        y[u] = __fadd2_rn(y[u], __fadd2_rn(make_float2(L.y, L.y), ly2));
-        z[u] = __fadd2_rn(z[u], __fadd2_rn(make_float2(L.z, L.z), lz2));
-        const float2 rn = __ffma2_rn(x[u], x[u], __ffma2_rn(y[u], y[u], __fmul2_rn(z[u], z[u])));
-        // the hit decision stays that of the unrefined distance
-        rr[u].x = rr[u].x < 1.f ? rn.x : rr[u].x;
-        rr[u].y = rr[u].y < 1.f ? rn.y : rr[u].y;
+  for (int i = 0; i < 2; i++) {
+    x[i] = __fadd2_rn(make_float2(A.x, A.y), src[i].x);
+    y[i] = __fadd2_rn(make_float2(A.z, A.w), src[i].y);
+    z[i] = __fadd2_rn(make_float2(B.x, B.y), src[i].z);
+    float2 r2 = __ffma2_rn(x[i], x[i], __ffma2_rn(y[i], y[i], __fmul2_rn(z[i], z[i])));
+    qs[i] = src[i].q;
+    qt[i] = make_float2(B.z, B.w);
+    if (CHECKED) {
+      if (fminf(r2.x, r2.y) < refine2) {  // exact differences from head + residual
+        const float4 LA = *la, LB = *lb;
+        x[i] = __fadd2_rn(x[i], __fadd2_rn(make_float2(LA.x, LA.y), src[i].lx));
+        y[i] = __fadd2_rn(y[i], __fadd2_rn(make_float2(LA.z, LA.w), src[i].ly));
+        z[i] = __fadd2_rn(z[i], __fadd2_rn(make_float2(LB.x, LB.y), src[i].lz));
+        r2 = __ffma2_rn(x[i], x[i], __ffma2_rn(y[i], y[i], __fmul2_rn(z[i], z[i])));
+      }
+      // a pair is inside iff 0 < r^2 <= 1, i.e. bits(r^2) - 1 < bits(1) as
+      // unsigned integers (r^2 >= 0)
+      const unsigned one = __float_as_uint(1.f);
+      const bool h0 = __float_as_uint(r2.x) - 1u < one, h1 = __float_as_uint(r2.y) - 1u < one;
+      s[i] = make_float2(h0 ? r2.x : 1.f, h1 ? r2.y : 1.f);
+      qs[i] = make_float2(h0 ? qs[i].x : 0.f, h1 ? qs[i].y : 0.f);
+      qt[i] = make_float2(h0 ? qt[i].x : 0.f, h1 ? qt[i].y : 0.f);
+    } else {
+      s[i] = make_float2(fminf(r2.x, 1.f), fminf(r2.y, 1.f));
+      if (FUNC == 2) {  // the Ewald kernel is not zero at Rdir: misses get charge 0
+        const bool h0 = r2.x <= 1.f, h1 = r2.y <= 1.f;
+        qs[i] = make_float2(h0 ? qs[i].x : 0.f, h1 ? qs[i].y : 0.f);
+        qt[i] = make_float2(h0 ? qt[i].x : 0.f, h1 ? qt[i].y : 0.f);
       }
     }
   }
-  const int src = (lane + 1) & 31;
 #pragma unroll
-  for (int u = 0; u < U; u++) {
+  for (int i = 0; i < 2; i++) {
     float2 f0, t;  // t = -f1
-    dm_eval2<FUNC, ND>(k, rr[u], f0, t);
-    const float2 gq = __fmul2_rn(t, qm[u]), gs = __fmul2_rn(t, qt[u]);
-    aV = fmaf(f0.x, qm[u].x, fmaf(f0.y, qm[u].y, aV));
-    aX = fmaf(gq.x, x[u].x, fmaf(gq.y, x[u].y, aX));
-    aY = fmaf(gq.x, y[u].x, fmaf(gq.y, y[u].y, aY));
-    aZ = fmaf(gq.x, z[u].x, fmaf(gq.y, z[u].y, aZ));
-    SV = __ffma2_rn(f0, qt[u], SV);
-    SX = __ffma2_rn(gs, x[u], SX);
-    SY = __ffma2_rn(gs, y[u], SY);
-    SZ = __ffma2_rn(gs, z[u], SZ);
-    aV = __shfl_sync(FULL, aV, src);
-    aX = __shfl_sync(FULL, aX, src);
-    aY = __shfl_sync(FULL, aY, src);
-    aZ = __shfl_sync(FULL, aZ, src);
+    dm_eval2<FUNC, ND, !CHECKED>(k, s[i], f0, t);
+    const float2 gs = __fmul2_rn(t, qs[i]), gt = __fmul2_rn(t, qt[i]);
+    aV = __ffma2_rn(f0, qs[i], aV);
+    aX = __ffma2_rn(gs, x[i], aX);
+    aY = __ffma2_rn(gs, y[i], aY);
+    aZ = __ffma2_rn(gs, z[i], aZ);
+    S[i][0] = __ffma2_rn(f0, qt[i], S[i][0]);
+    S[i][1] = __ffma2_rn(gt, x[i], S[i][1]);
+    S[i][2] = __ffma2_rn(gt, y[i], S[i][2]);
+    S[i][3] = __ffma2_rn(gt, z[i], S[i][3]);
   }
 }
 
-// Real derivative-match kernels (1/r, r^alpha) of the FP32 direct sum with
-// every unordered pair evaluated once (Newton's third law, as the
+// v of lane (lane + 1) mod 32, both halves
+__device__ __forceinline__ float2 rotate2(float2 v, int src) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+
+// The 16 steps of one chunk; target sums rotate after each.
+template <int FUNC, int ND, bool CHECKED>
+__device__ __forceinline__ void sym_sweep(const PairCoef<float> &k, const float4 *tsm,
+                                          const float4 *tlo, const SymSource (&src)[2],
+                                          float refine2, int lane, float2 &aV, float2 &aX,
+                                          float2 &aY, float2 &aZ, float2 (&S)[2][4]) {
+  constexpr int kUnroll = CHECKED ? 1 : 8;
+  const int next = (lane + 1) & 31;
+#pragma unroll kUnroll
+  for (int kk = 0; kk < 16; kk++) {
+    const int j = (lane + kk) & 15;
+    sym_step<FUNC, ND, CHECKED>(k, tsm[j], tsm[16 + j], tlo + j, tlo + 16 + j, src, refine2, aV,
+                                aX, aY, aZ, S);
+    aV = rotate2(aV, next), aX = rotate2(aX, next);
+    aY = rotate2(aY, next), aZ = rotate2(aZ, next);
+  }
+}
+
+// Real derivative-match kernels (1/r, r^alpha) and the original Ewald split of
+// the FP32 direct sum with every unordered pair evaluated once (Newton's third law, as the
 // reference's own cell-pair loops do: src/PotentialLaplace.cpp:145-197,
 // :3447-3610).  The group walks its half-shell source segments: sources
 // whose point lies in a later coarse column, or later in the group's own
 // column, than the group's targets (set-up, setup.cu); the pairs inside the
 // group are the first phase, from both sides with target-side sums only.
+// The group's targets sit in shared memory as 16 pairs; a lane holds two
+// sources of a 64-source chunk in registers and meets target pair (lane + k)
+// mod 16 at step k, four pairs of points per step in packed FP32.  The
+// target sums of a pair travel with it, one lane down per step; after 16
+// steps lanes l and l + 16 hold the two halves of the sums of pair l mod 16,
+// and lane l keeps target 2 (l mod 16) + l / 16.  Packing over targets (the
+// former sweep packed the lane's two sources) leaves no scalar arithmetic in
+// the target sums, makes the operands of every packed instruction register
+// pairs as loaded, and reads two lanes' targets with one shared wavefront.
 // Target-side sums accumulate per chunk in FP32 and across chunks in FP64,
 // as in the one-sided body; the source-side sums of a chunk are added to
 // vsrc (FP32, scaled frame; slot = the source's brick-order position, from
 // spos[j].w) with one vector atomic per source, and folded into V by the
 // interpolation (CalcV) or by merge_source_kernel.
+// The group's work is shared by nsplit warps of the CTA, warp `part` taking
+// chunks part, part + nsplit, ... (and every nsplit-th source of the pairs
+// inside the group); the caller adds their acc.
 template <int FUNC, int ND>
 __device__ __forceinline__ void direct_group_sym(
     const PairCoef<float> &k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const float *__restrict__ qs, const double *__restrict__ qcaller, const int4 G,
     const double4 c, const int2 *__restrict__ segs, const uint32_t *__restrict__ perm,
-    float refine2, double fself_r, double *__restrict__ V, float4 *__restrict__ vsrc,
-    float4 *tsm, float4 *tlo, int lane) {
+    float refine2, float4 *__restrict__ vsrc, float4 *tsm, float4 *tlo, int lane, int part,
+    int nsplit, double (&acc)[4]) {
   const unsigned FULL = 0xffffffffu;
-  const int ti = G.x + lane;
-  const bool active = lane < G.y;
-  // idle lanes sit far outside the cutoff with charge 0
+  const int tid = 2 * (lane & 15) + (lane >> 4);  // the lane's target in the group
+  // absent targets sit far outside the cutoff with charge 0
   float tx = 1e18f, ty = 1e18f, tz = 1e18f, tlx = 0.f, tly = 0.f, tlz = 0.f, tq = 0.f;
   const double ir = k.invR;  // coordinates in units of Rdir
-  long o = 0;
-  if (active) {
-    const double4 p = gpos[ti];
-    o = perm[ti];
+  if (tid < G.y) {
+    const double4 p = gpos[G.x + tid];
     const double dx = (p.x - c.x) * ir, dy = (p.y - c.y) * ir, dz = (p.z - c.z) * ir;
     tx = (float)dx, ty = (float)dy, tz = (float)dz;
     tlx = (float)(dx - (double)tx), tly = (float)(dy - (double)ty), tlz = (float)(dz - (double)tz);
-    tq = (float)qcaller[o];
+    tq = (float)qcaller[perm[G.x + tid]];
   }
-  tsm[lane] = make_float4(tx, ty, tz, tq);
-  tlo[lane] = make_float4(tlx, tly, tlz, 0.f);
+  // tsm[j] = (x0 x1 y0 y1), tsm[16 + j] = (z0 z1 q0 q1) of target pair j; tlo
+  // the residuals
+  {
+    float *ts = reinterpret_cast<float *>(tsm), *tl = reinterpret_cast<float *>(tlo);
+    const int at = 4 * (lane & 15) + (lane >> 4);
+    ts[at] = tx, ts[at + 2] = ty, ts[at + 64] = tz, ts[at + 66] = tq;
+    tl[at] = tlx, tl[at + 2] = tly, tl[at + 64] = tlz, tl[at + 66] = 0.f;
+  }
   __syncwarp();
   refine2 = (float)((double)refine2 * ir * ir);
-  const unsigned rb = __float_as_uint(1.f);
-  double acc[4] = {0, 0, 0, 0};
+  // a non-finite charge in the group: every chunk takes the checked steps
+  const bool odd_group = __any_sync(FULL, !(fabsf(tq) <= 3.402823466e38f));
 
   // pairs inside the group, from both sides; the differences are always
   // refined (head difference + residual difference)
   {
+    const float *ts = reinterpret_cast<const float *>(tsm),
+                *tl = reinterpret_cast<const float *>(tlo);
+    const unsigned rb = __float_as_uint(1.f);
     float aV = 0.f, aX = 0.f, aY = 0.f, aZ = 0.f;
-    for (int s = 0; s < G.y; s++) {
-      const float4 S = tsm[s], L = tlo[s];
-      const float x = (tx - S.x) + (tlx - L.x), y = (ty - S.y) + (tly - L.y),
-                  z = (tz - S.z) + (tlz - L.z);
+    for (int s = part; s < G.y; s += nsplit) {
+      const int at = 4 * (s >> 1) + (s & 1);
+      const float x = (tx - ts[at]) + (tlx - tl[at]), y = (ty - ts[at + 2]) + (tly - tl[at + 2]),
+                  z = (tz - ts[at + 64]) + (tlz - tl[at + 64]);
       const float r2 = fmaf(x, x, fmaf(y, y, z * z));
       const bool hit = __float_as_uint(r2) - 1u < rb;  // 0 < r^2 <= 1, not the target itself
       float f0, t;
       dm_eval1<FUNC, ND>(k, hit ? r2 : 1.f, f0, t);
-      const float q = hit ? S.w : 0.f, g = t * q;
+      const float q = hit ? ts[at + 66] : 0.f, g = t * q;
       aV = fmaf(f0, q, aV);
       aX = fmaf(g, x, aX);
       aY = fmaf(g, y, aY);
@@ -832,77 +903,112 @@ __device__ __forceinline__ void direct_group_sym(
   // and l + 32 of the chunk (register prefetch of the next chunk)
   const double rfs = sqrt((double)refine2) + c.w * ir;
   const double near2 = rfs * rfs;
-  SrcCursor ca{G.z, lane};
-  ca.normalize(segs, G.w);
-  SrcCursor cb{ca.seg, ca.off + 32};
-  cb.normalize(segs, G.w);
-  bool va = ca.seg < G.w, vb = cb.seg < G.w;
-  long ja = -1, jb = -1;
-  double4 pa = make_double4(0, 0, 0, 0), pb = pa;
-  float qa = 0.f, qb = 0.f;
-  if (va) ja = (long)segs[ca.seg].x + ca.off, pa = spos[ja], qa = qs[ja];
-  if (vb) jb = (long)segs[cb.seg].x + cb.off, pb = spos[jb], qb = qs[jb];
-  while (__any_sync(FULL, va)) {
+  const int stride = 64 * nsplit;
+  SrcCursor cur[2];
+  cur[0] = SrcCursor{G.z, lane + 64 * part};
+  cur[0].normalize(segs, G.w);
+  cur[1] = SrcCursor{cur[0].seg, cur[0].off + 32};
+  cur[1].normalize(segs, G.w);
+  bool v[2];
+  double4 p[2];
+  float q[2];
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    v[i] = cur[i].seg < G.w;
+    p[i] = make_double4(0, 0, 0, 0);
+    q[i] = 0.f;
+    if (v[i]) {
+      const long j = (long)segs[cur[i].seg].x + cur[i].off;
+      p[i] = spos[j], q[i] = qs[j];
+    }
+  }
+  while (__any_sync(FULL, v[0])) {
     // this chunk's sources, relative to the group centre; empty slots far
-    // away (on the other side from idle targets) with charge 0
-    float hxa = -1e18f, hya = -1e18f, hza = -1e18f, lxa = 0.f, lya = 0.f, lza = 0.f;
-    float hxb = -1e18f, hyb = -1e18f, hzb = -1e18f, lxb = 0.f, lyb = 0.f, lzb = 0.f;
-    bool near = false;
-    // source-side slots: the sources' brick-order positions
-    const long ka = va ? (long)pa.w : -1, kb = vb ? (long)pb.w : -1;
-    float q0 = 0.f, q1 = 0.f;
-    if (va) {
-      const double dx = (pa.x - c.x) * ir, dy = (pa.y - c.y) * ir, dz = (pa.z - c.z) * ir;
-      hxa = (float)dx, hya = (float)dy, hza = (float)dz;
-      lxa = (float)(dx - (double)hxa), lya = (float)(dy - (double)hya), lza = (float)(dz - (double)hza);
-      q0 = qa;
-      near = dx * dx + dy * dy + dz * dz < near2;
+    // away (on the other side from absent targets) with charge 0
+    SymSource src[2];
+    int slot[2];  // source-side slots: the sources' brick-order positions
+    bool checked = odd_group;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      float hx = -1e18f, hy = -1e18f, hz = -1e18f, lx = 0.f, ly = 0.f, lz = 0.f, qv = 0.f;
+      slot[i] = -1;
+      if (v[i]) {
+        const double dx = (p[i].x - c.x) * ir, dy = (p[i].y - c.y) * ir,
+                     dz = (p[i].z - c.z) * ir;
+        hx = (float)dx, hy = (float)dy, hz = (float)dz;
+        lx = (float)(dx - (double)hx), ly = (float)(dy - (double)hy),
+        lz = (float)(dz - (double)hz);
+        qv = q[i];
+        slot[i] = (int)p[i].w;
+        checked = checked || dx * dx + dy * dy + dz * dz < near2 ||
+                  !(fabsf(qv) <= 3.402823466e38f);
+      }
+      src[i].x = make_float2(-hx, -hx), src[i].y = make_float2(-hy, -hy);
+      src[i].z = make_float2(-hz, -hz), src[i].q = make_float2(qv, qv);
+      src[i].lx = make_float2(-lx, -lx), src[i].ly = make_float2(-ly, -ly);
+      src[i].lz = make_float2(-lz, -lz);
+      // prefetch the next chunk
+      cur[i].off += stride;
+      cur[i].normalize(segs, G.w);
+      v[i] = cur[i].seg < G.w;
+      if (v[i]) {
+        const long j = (long)segs[cur[i].seg].x + cur[i].off;
+        p[i] = spos[j], q[i] = qs[j];
+      }
     }
-    if (vb) {
-      const double dx = (pb.x - c.x) * ir, dy = (pb.y - c.y) * ir, dz = (pb.z - c.z) * ir;
-      hxb = (float)dx, hyb = (float)dy, hzb = (float)dz;
-      lxb = (float)(dx - (double)hxb), lyb = (float)(dy - (double)hyb), lzb = (float)(dz - (double)hzb);
-      q1 = qb;
-      near = near || dx * dx + dy * dy + dz * dz < near2;
-    }
-    const float2 sx2 = make_float2(-hxa, -hxb), sy2 = make_float2(-hya, -hyb),
-                 sz2 = make_float2(-hza, -hzb), q2 = make_float2(q0, q1);
-    const float2 lx2 = make_float2(-lxa, -lxb), ly2 = make_float2(-lya, -lyb),
-                 lz2 = make_float2(-lza, -lzb);
-    // prefetch the next chunk
-    ca.off += 64;
-    ca.normalize(segs, G.w);
-    cb.off += 64;
-    cb.normalize(segs, G.w);
-    va = ca.seg < G.w, vb = cb.seg < G.w;
-    if (va) ja = (long)segs[ca.seg].x + ca.off, pa = spos[ja], qa = qs[ja];
-    if (vb) jb = (long)segs[cb.seg].x + cb.off, pb = spos[jb], qb = qs[jb];
+    float2 aV = make_float2(0.f, 0.f), aX = aV, aY = aV, aZ = aV;
+    float2 S[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; i++) S[i][0] = S[i][1] = S[i][2] = S[i][3] = make_float2(0.f, 0.f);
+    if (__any_sync(FULL, checked))
+      sym_sweep<FUNC, ND, true>(k, tsm, tlo, src, refine2, lane, aV, aX, aY, aZ, S);
+    else
+      sym_sweep<FUNC, ND, false>(k, tsm, tlo, src, refine2, lane, aV, aX, aY, aZ, S);
+    // lanes l and l + 16 hold half of the sums of target pair l mod 16 each
+    const bool hi = lane >= 16;
+    auto total = [&](float2 a) {
+      const float give = hi ? a.x : a.y, keep = hi ? a.y : a.x;
+      return keep + __shfl_xor_sync(FULL, give, 16);
+    };
+    acc[0] += (double)total(aV);
+    acc[1] -= (double)total(aX);
+    acc[2] -= (double)total(aY);
+    acc[3] -= (double)total(aZ);
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      if (slot[i] >= 0)
+        atomicAdd(vsrc + slot[i], make_float4(S[i][0].x + S[i][0].y, S[i][1].x + S[i][1].y,
+                                              S[i][2].x + S[i][2].y, S[i][3].x + S[i][3].y));
+  }
+}
 
-    float aV = 0.f, aX = 0.f, aY = 0.f, aZ = 0.f;
-    float2 SV = make_float2(0.f, 0.f), SX = SV, SY = SV, SZ = SV;
-    if (__any_sync(FULL, near)) {
-      for (int k0 = 0; k0 < 32; k0 += sym_block_steps<FUNC>())
-        sym_block<FUNC, ND, true>(k, tsm, tlo, lane, k0, sx2, sy2, sz2, q2, lx2, ly2, lz2,
-                                  refine2, aV, aX, aY, aZ, SV, SX, SY, SZ);
-    } else {
-      for (int k0 = 0; k0 < 32; k0 += sym_block_steps<FUNC>())
-        sym_block<FUNC, ND, false>(k, tsm, tlo, lane, k0, sx2, sy2, sz2, q2, lx2, ly2, lz2,
-                                   refine2, aV, aX, aY, aZ, SV, SX, SY, SZ);
-    }
-    // after 32 steps every target's sums are back in its own lane
-    acc[0] += (double)aV;
-    acc[1] -= (double)aX;
-    acc[2] -= (double)aY;
-    acc[3] -= (double)aZ;
-    if (ka >= 0) atomicAdd(vsrc + ka, make_float4(SV.x, SX.x, SY.x, SZ.x));
-    if (kb >= 0) atomicAdd(vsrc + kb, make_float4(SV.y, SX.y, SY.y, SZ.y));
-  }
-  if (active) {
-    const double vs = k.vscale, gs = k.gscale;
-    // V -= f_LR(0) q (src/Interface.cpp:2061-2062)
-    reinterpret_cast<double4 *>(V)[o] =
-        make_double4(vs * acc[0] - fself_r * qcaller[o], gs * acc[1], gs * acc[2], gs * acc[3]);
-  }
+// Sum over the nsplit warps of a CTA that share one group: acc of every part
+// into that of part 0 (same lane, same target).  red: [nsplit][32][4].
+__device__ __forceinline__ void reduce_parts(double (&acc)[4], double (*red)[32][4], int part,
+                                             int nsplit, int lane) {
+  if (part > 0)
+#pragma unroll
+    for (int m = 0; m < 4; m++) red[part][lane][m] = acc[m];
+  __syncthreads();
+  if (part == 0)
+    for (int w = 1; w < nsplit; w++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) acc[m] += red[w][lane][m];
+}
+
+// The target sums of direct_group_sym to V, less the self term f_LR(0) q
+// (src/Interface.cpp:2061-2062).
+__device__ __forceinline__ void sym_store(const PairCoef<float> &k, const int4 G,
+                                          const uint32_t *__restrict__ perm,
+                                          const double *__restrict__ qcaller, double fself_r,
+                                          double *__restrict__ V, int lane,
+                                          const double (&acc)[4]) {
+  const int tid = 2 * (lane & 15) + (lane >> 4);
+  if (tid >= G.y) return;
+  const long o = perm[G.x + tid];
+  const double vs = k.vscale, gs = k.gscale;
+  reinterpret_cast<double4 *>(V)[o] =
+      make_double4(vs * acc[0] - fself_r * qcaller[o], gs * acc[1], gs * acc[2], gs * acc[3]);
 }
 
 // sin and cos of x on the special-function unit after a Cody-Waite
@@ -1392,8 +1498,7 @@ __device__ __forceinline__ void direct_group_fp64(
 }
 
 // FP32 direct sum of one warp group with every unordered pair evaluated once,
-// for the real kernels without a packed body (the original Ewald split and
-// caller-defined kernels): the pair-once walk of direct_group_sym with the
+// for real caller-defined kernels: the pair-once walk of direct_group_sym with the
 // scalar pair kernel (pair_sr) of the one-sided body.  Coordinates are
 // unscaled FP32 offsets from the group centre (heads in th with the target
 // charge, residuals in tl), close pairs refined from the residuals; the

@@ -31,15 +31,21 @@ struct PairCoef {
   T k0r, k0i;
   T ar[kMaxDeriv + 1], ai[kMaxDeriv + 1];
   T br[kMaxDeriv + 1], bi[kMaxDeriv + 1];
-  // Packed (two pairs per instruction) evaluation of the real kernels
-  // works in coordinates scaled by 1/Rdir, so r^2 is s itself.  With
-  // alpha = -1 for 1/r it accumulates
-  //   f0' = s^(alpha/2) - Rdir^(-alpha) f_LR  = Rdir^(-alpha) f0,
-  //   t'  = Rdir^(2-alpha) d - alpha s^(alpha/2) / s = -Rdir^(2-alpha) f1,
-  // so V = vscale sum q f0' and grad V = -gscale sum q t' x' with
-  // vscale = Rdir^alpha, gscale = Rdir^(alpha-1).  Coefficient pairs:
-  // nar2[n] = -Rdir^(-alpha) ar[n], br2[n] = Rdir^(2-alpha) br[n].
-  typename Vec2<T>::type nar2[kMaxDeriv + 1], br2[kMaxDeriv + 1];
+  // Packed (two pairs per instruction) evaluation of the real kernels s^a,
+  // a = alpha / 2 (1/r: alpha = -1), in coordinates scaled by 1/Rdir, so r^2
+  // is s itself.  The derivative match at Rdir is the Taylor polynomial of
+  // s^a about s = 1: with u = 1 - s,
+  //   P(u) = sum_{n <= N} c_n u^n,  c_0 = 1, c_{n+1} = c_n (n - a) / (n + 1),
+  //   f0 = s^a - P = Rdir^(-alpha) f_SR,
+  //   t = (1/(alpha r)) d f0 / dr = s^(a-1) - (dP/ds) / a = (f0 + K u^N) / s
+  // with K = (1 - N / a) c_N (from s dP/ds = a P + (N - a) c_N u^N).  So
+  // V = vscale sum q f0 and grad V = -gscale sum q t x with vscale =
+  // Rdir^alpha, gscale = -alpha Rdir^(alpha-1).  Coefficient pairs: nc2[n] =
+  // -c_n, nq2[n] = (n + 1) c_{n+1} / a (those of -(dP/ds) / a), kn2 = K.  At s
+  // = 1 both f0 and t are exactly zero, and the coefficients of 1/r are exact
+  // in FP32.  (alpha = 0, a constant kernel with no short range: t as for a ->
+  // 0 and gscale = 0.)
+  typename Vec2<T>::type nc2[kMaxDeriv + 1], nq2[kMaxDeriv + 1], kn2;
   double invR, vscale, gscale;
   // Helmholtz packed evaluation: (re, im) pairs of -ar/-ai and -br/-bi
   typename Vec2<T>::type nac2[kMaxDeriv + 1], nbc2[kMaxDeriv + 1];

@@ -14,12 +14,24 @@
 // of those atomic additions.  The one-sided walk uses no atomics.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
+#include <complex>
+#include <cstdlib>
 
 #include "bodies.cuh"
 #include "internal.h"
 
 namespace npme {
+
+// Original Ewald split in FP32: erfcx(x) (x + 3) = sum_n e_n tau^n with tau =
+// (x - 3)/(x + 3), a relative-error fit of degree 9 over 0 <= x <= 12 (error
+// 5e-09, below FP32 rounding; beyond x = 10.2 exp(-x^2) is zero in FP32).
+constexpr double kErfcxFit[10] = {
+    1.0740069096e+00, -8.8339451071e-01, 5.9022814413e-01, 
+    -3.1046536357e-01, 1.1953133388e-01, -2.6843410022e-02, 
+    -1.2380858249e-03, 3.0828154886e-03, -4.6349936557e-04, 
+    -3.1471575889e-04};
 
 template <typename T>
 PairCoef<T> make_pair_coef(const npme_handle *h) {
@@ -44,11 +56,8 @@ PairCoef<T> make_pair_coef(const npme_handle *h) {
     k.ai[i] = (T)(h->a_i[i] * s);
     k.br[i] = (T)(h->b_r[i] * s);
     k.bi[i] = (T)(h->b_i[i] * s);
-    const double al = h->p.funcType == NPME_FUNC_RALPHA ? h->p.alpha : -1.0;
     k.nac2[i].x = (T)(-h->a_r[i] * s), k.nac2[i].y = (T)(-h->a_i[i] * s);
     k.nbc2[i].x = (T)(-h->b_r[i] * s), k.nbc2[i].y = (T)(-h->b_i[i] * s);
-    k.nar2[i].x = k.nar2[i].y = (T)(-h->a_r[i] * s * std::pow(R, -al));
-    k.br2[i].x = k.br2[i].y = (T)(h->b_r[i] * s * std::pow(R, 2.0 - al));
     s *= R2;
   }
   // the radial-derivative polynomials have degree nder - 1: their entry nder
@@ -56,14 +65,31 @@ PairCoef<T> make_pair_coef(const npme_handle *h) {
   // the packed bodies relies on it)
   if (k.nder >= 0 && k.nder <= kMaxDeriv) {
     k.br[k.nder] = k.bi[k.nder] = (T)0;
-    k.br2[k.nder].x = k.br2[k.nder].y = (T)0;
     k.nbc2[k.nder].x = k.nbc2[k.nder].y = (T)0;
   }
   {
     const double al = h->p.funcType == NPME_FUNC_RALPHA ? h->p.alpha : -1.0;
+    // Taylor coefficients of s^a, a = alpha/2, about s = 1 (zero above the
+    // order), and ca = c_n / -a from n = 1 (also defined for a = 0)
+    const double a = 0.5 * al;
+    double c = 1.0, ca = 1.0;
+    for (int i = 0; i <= k.nder && i <= kMaxDeriv; i++) {
+      if (i > 1) ca = ca * (i - 1 - a) / i;
+      if (i > 0) c = -a * ca;
+      k.nc2[i].x = k.nc2[i].y = (T)-c;
+      if (i > 0) k.nq2[i - 1].x = k.nq2[i - 1].y = (T)(-i * ca);
+      if (i == k.nder) k.kn2.x = k.kn2.y = (T)((k.nder - a) * ca);
+    }
+    if (k.split == NPME_SPLIT_LAPLACE_ORIG) {  // dm_eval2<2, 0>: coefficients and constants
+      const double b = h->beta * R;
+      for (int i = 0; i < 10; i++) k.nc2[i].x = k.nc2[i].y = (T)kErfcxFit[i];
+      k.nq2[0].x = k.nq2[0].y = (T)b;
+      k.nq2[1].x = k.nq2[1].y = (T)(-b * b / std::log(2.0));
+      k.kn2.x = k.kn2.y = (T)(2.0 * b / std::sqrt(M_PI));
+    }
     k.invR = 1.0 / R;
     k.vscale = std::pow(R, al);
-    k.gscale = std::pow(R, al - 1.0);
+    k.gscale = (k.split == NPME_SPLIT_LAPLACE_ORIG ? 1.0 : -al) * std::pow(R, al - 1.0);
   }
   return k;
 }
@@ -130,22 +156,64 @@ static void merge_or_defer(npme_handle *h, const DirectArgs &a, cudaStream_t s, 
   }
 }
 
+// Warps per group of a pair-once launch with ngroups groups.  The SMs hold
+// 16 warps each (128 registers a thread), 2,368 in all, and a group is one
+// serial walk of its half-shell list, so with few groups the launch lasts as
+// long as one walk with most of the chip idle, and with about one round of
+// them as long as the heaviest: the walk is split over the warps of a CTA.
+// Measured, whole against split walks: 170 groups (4,000 points) 92 / 26 us
+// with 16 warps, 28 with 8; 1,150 groups (30,000 points in a flat box) 110 /
+// 82 us with 4 warps, 96 with 2, 98 with 8.  From about two rounds on the
+// splitting's own work (every warp stages the targets and walks all segments)
+// costs more than it gives: 3,300 groups 137 / 139 us, 31,700 groups +10 %.
+constexpr int kMaxSplit = 16;
+static int split_warps(long ngroups) {
+  if (ngroups <= 148) return 16;
+  if (ngroups <= 4 * 148) return 8;
+  if (ngroups <= 20 * 148) return 4;
+  return 1;
+}
+
 // FP32 real-DM direct sum with every pair evaluated once (direct_group_sym),
 // then the source-side sums folded into V.
 template <int FUNC, int ND>
-__global__ void __launch_bounds__(32 * kGroupWarps, kGroupMinBlocks) direct_sym_kernel(
+__global__ void __launch_bounds__(32 * kGroupWarps, 4) direct_sym_kernel(
     PairCoef<float> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const float *__restrict__ qs, const double *__restrict__ qcaller,
     const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
     const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, long ngroups,
     float refine2, double fself_r, double *__restrict__ V, float4 *__restrict__ vsrc) {
-  __shared__ float4 tsm[kGroupWarps][32];  // group targets (x, y, z, q), heads
+  __shared__ float4 tsm[kGroupWarps][32];  // group targets in pairs, heads and charges
   __shared__ float4 tlo[kGroupWarps][32];  // residuals of the target coordinates
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long g = (long)blockIdx.x * kGroupWarps + wid;
   if (g >= ngroups) return;  // warp-uniform; nothing below synchronises the block
-  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, groups[g], gcen[g], segs, perm,
-                             refine2, fself_r, V, vsrc, tsm[wid], tlo[wid], lane);
+  double acc[4] = {0, 0, 0, 0};
+  const int4 G = groups[g];
+  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, perm, refine2, vsrc,
+                             tsm[wid], tlo[wid], lane, 0, 1, acc);
+  sym_store(k, G, perm, qcaller, fself_r, V, lane, acc);
+}
+
+// The same with a CTA of blockDim.x / 32 warps per group (split_warps).
+template <int FUNC, int ND>
+__global__ void __launch_bounds__(32 * kMaxSplit) direct_sym_split_kernel(
+    PairCoef<float> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
+    const float *__restrict__ qs, const double *__restrict__ qcaller,
+    const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
+    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, float refine2,
+    double fself_r, double *__restrict__ V, float4 *__restrict__ vsrc) {
+  __shared__ float4 tsm[kMaxSplit][32];
+  __shared__ float4 tlo[kMaxSplit][32];
+  __shared__ double red[kMaxSplit][32][4];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nsplit = blockDim.x >> 5;
+  const long g = blockIdx.x;
+  double acc[4] = {0, 0, 0, 0};
+  const int4 G = groups[g];
+  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, perm, refine2, vsrc,
+                             tsm[wid], tlo[wid], lane, wid, nsplit, acc);
+  reduce_parts(acc, red, wid, nsplit, lane);
+  if (wid == 0) sym_store(k, G, perm, qcaller, fself_r, V, lane, acc);
 }
 
 // V[caller(i)] += scale * vsrc[i] for every brick-order slot i, then
@@ -211,31 +279,20 @@ static void sym_helm_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream_t
 
 template <int FUNC, int ND>
 static void sym_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
-  const long blocks = (h->n_hgroups + kGroupWarps - 1) / kGroupWarps;
-  if (blocks == 0) return;
+  if (h->n_hgroups == 0) return;
   const PairCoef<float> k = make_pair_coef<float>(h);
-  direct_sym_kernel<FUNC, ND><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
-      k, h->d_gpos, h->d_spos, (const float *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
-      h->d_hsegs, h->d_cperm, h->n_hgroups, (float)h->refine2, a.fself_r, a.V, h->d_vsrc);
+  const int split = split_warps(h->n_hgroups);
+  if (split > 1) {
+    direct_sym_split_kernel<FUNC, ND><<<(unsigned)h->n_hgroups, 32 * split, 0, s>>>(
+        k, h->d_gpos, h->d_spos, (const float *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
+        h->d_hsegs, h->d_cperm, (float)h->refine2, a.fself_r, a.V, h->d_vsrc);
+  } else {
+    const long blocks = (h->n_hgroups + kGroupWarps - 1) / kGroupWarps;
+    direct_sym_kernel<FUNC, ND><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
+        k, h->d_gpos, h->d_spos, (const float *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
+        h->d_hsegs, h->d_cperm, h->n_hgroups, (float)h->refine2, a.fself_r, a.V, h->d_vsrc);
+  }
   merge_or_defer(h, a, s, k.vscale, k.gscale);
-}
-
-// FP32 form with the scalar pair kernel (original Ewald split).
-template <int FUNC, int SPLIT, int ND>
-__global__ void __launch_bounds__(32 * kGroupWarps) direct_sym_scalar_kernel(
-    PairCoef<float> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
-    const float *__restrict__ qs, const double *__restrict__ qcaller,
-    const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
-    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, long ngroups,
-    float refine2, double fself_r, double *__restrict__ V, float4 *__restrict__ vsrc) {
-  __shared__ float4 th[kGroupWarps][32];  // group targets: heads, q
-  __shared__ float4 tl[kGroupWarps][32];  // residuals
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long g = (long)blockIdx.x * kGroupWarps + wid;
-  if (g >= ngroups) return;  // warp-uniform
-  direct_group_sym_scalar<FUNC, SPLIT, ND>(k, gpos, spos, qs, qcaller, groups[g], gcen[g], segs,
-                                           perm, refine2, fself_r, V, vsrc, th[wid], tl[wid],
-                                           lane);
 }
 
 // FP64 form for the real built-in kernels (DM and original Ewald).
@@ -327,14 +384,7 @@ static bool sym_launch(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
     return true;
   }
   if (h->fp32 && h->p.EwaldSplit == NPME_SPLIT_LAPLACE_ORIG) {
-    const long blocks = (h->n_hgroups + kGroupWarps - 1) / kGroupWarps;
-    if (blocks > 0) {
-      direct_sym_scalar_kernel<0, 1, 0><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
-          make_pair_coef<float>(h), h->d_gpos, h->d_spos, (const float *)a.q, a.qcaller,
-          h->d_hgroups, h->d_hcen, h->d_hsegs, h->d_cperm, h->n_hgroups, (float)h->refine2,
-          a.fself_r, a.V, h->d_vsrc);
-      merge_or_defer(h, a, s, 1.0, 1.0);
-    }
+    sym_launch_nd<2, 0>(h, a, s);
     return true;
   }
   if (!h->fp32) {
@@ -349,7 +399,9 @@ static bool sym_launch(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
     else if (nd == 8) sym_launch_nd<0, 8>(h, a, s);
     else sym_launch_nd<0, 0>(h, a, s);
   } else {
-    if (nd == 3) sym_launch_nd<1, 3>(h, a, s);
+    // the fixed-order instances hold for alpha < 0 (dm_eval2)
+    if (h->p.alpha >= 0) sym_launch_nd<1, 0>(h, a, s);
+    else if (nd == 3) sym_launch_nd<1, 3>(h, a, s);
     else if (nd == 6) sym_launch_nd<1, 6>(h, a, s);
     else if (nd == 8) sym_launch_nd<1, 8>(h, a, s);
     else sym_launch_nd<1, 0>(h, a, s);
@@ -393,7 +445,7 @@ static void groups_launch(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
     }
     return;
   }
-  switch (SPLIT == 1 ? 0 : h->p.nDeriv) {
+  switch (SPLIT == 1 || (FUNC == 1 && h->p.alpha >= 0) ? 0 : h->p.nDeriv) {
     case 3: groups_launch_nd<CPLX, FUNC, SPLIT, 3>(h, a, s); break;
     case 6: groups_launch_nd<CPLX, FUNC, SPLIT, 6>(h, a, s); break;
     case 8: groups_launch_nd<CPLX, FUNC, SPLIT, 8>(h, a, s); break;
