@@ -104,7 +104,8 @@ typedef struct {
   long nGroups;         /* direct sum: warp groups of <= 32 points */
   double candidatesPerPoint; /* direct sum: staged sources per target */
   int pairsOnce;        /* 1: the direct sum evaluates every pair once, for
-                           both of its points (FP32 real DM kernels) */
+                           both of its points (0 for FP64 Helmholtz, whose
+                           walk does so as well) */
   double pairsOnceCandidatesPerPoint; /* half-shell sources per target */
 } npme_info;
 
@@ -174,8 +175,8 @@ int npme_gpu_calcv_device(npme_handle *h, double *d_V, const double *d_charge,
  * (src/PotentialGenFunc.cpp:140) for the set-up geometry.  Layouts and
  * stream semantics as npme_gpu_calcv_device.  Like the reference's cell-pair
  * loops it evaluates every pair once for both points (built-in kernels and
- * real caller kernels; complex caller kernels and FP64 Helmholtz walk each
- * target's sources), adding the source-side sums with atomics, so repeated
+ * real caller kernels; complex caller kernels, and FP64 Helmholtz with
+ * |k0| Rdir >= 1e5, walk each target's sources), adding the source-side sums with atomics, so repeated
  * calls can differ in the last bits (NPME_PAIRS_ONCE=0 at set-up: one-sided,
  * reproducible). */
 int npme_gpu_direct_sum_device(npme_handle *h, double *d_V, const double *d_charge,

@@ -369,12 +369,15 @@ __device__ __forceinline__ void interp_brick_body(int brick, const int *__restri
     const T sc[4] = {T(1), c1, c2, c3};
     const long o = pt.orig, slot = beg + pi;
     if (CPLX) {
-      // source-side slot (FP32 complex): (V re, V im, x re, x im), (y .., z ..)
+      // source-side slot: (V re, V im, x re, x im), (y .., z ..)
       double d[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       if (vsrc) {
-        float4 *vp = reinterpret_cast<float4 *>(vsrc) + 2 * slot;
-        const float4 a = vp[0], b = vp[1];
-        vp[0] = vp[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        using V4 = typename Vec4<T>::type;
+        V4 *vp = reinterpret_cast<V4 *>(vsrc) + 2 * slot;
+        const V4 a = vp[0], b = vp[1];
+        V4 z;
+        z.x = z.y = z.z = z.w = T(0);
+        vp[0] = vp[1] = z;
         d[0] = a.x, d[1] = a.y, d[2] = a.z, d[3] = a.w;
         d[4] = b.x, d[5] = b.y, d[6] = b.z, d[7] = b.w;
       }
@@ -1630,6 +1633,381 @@ __device__ __forceinline__ void direct_group_sym_scalar(
     acc[0] -= fself_r * qcaller[o];  // src/Interface.cpp:2061-2062
     reinterpret_cast<double4 *>(V)[o] = make_double4(acc[0], acc[1], acc[2], acc[3]);
   }
+}
+
+// 1/sqrt(s) for normal finite s > 0: the hardware's approximation (20 bits or
+// more) and one step of Householder's cubically convergent iteration, y + y e
+// (1/2 + 3/8 e) with e = 1 - s y^2, whose error is 5/16 e^3 < 2^-57.  Five
+// FP64 operations and no branch.
+__device__ __forceinline__ double rsqrt_iter(double s) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+  const double e = fma(-(s * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+template <int N>
+__device__ __forceinline__ double pow_n(double u) {
+  if constexpr (N == 1) {
+    return u;
+  } else {
+    const double h = pow_n<N / 2>(u), h2 = h * h;
+    return N % 2 ? h2 * u : h2;
+  }
+}
+
+// The real DM pair kernel of dm_eval2 in FP64 (coordinates in units of Rdir,
+// s = r^2 in (0, 1]; ND > 0 for alpha < 0, ND = 0 any order and alpha).
+template <int FUNC, int ND>
+__device__ __forceinline__ void dm_eval64(const PairCoef<double> &k, double s, double &f0,
+                                          double &t) {
+  constexpr int nd = dm_degree<ND>();
+  const double u = 1.0 - s;
+  double h = k.nc2[nd].x;
+#pragma unroll
+  for (int n = nd - 1; n >= 1; n--) h = fma(h, u, k.nc2[n].x);
+  const double ri = rsqrt_iter(s), ri2 = ri * ri;
+  const double e0 = FUNC == 1 ? rpow_t(s, k.half_alpha) : ri;
+  f0 = fma(h, u, e0 - 1.0);
+  if constexpr (ND > 0) {
+    t = fma(pow_n<ND>(u), k.kn2.x, f0) * ri2;
+  } else {
+    double d = k.nq2[nd - 1].x;
+#pragma unroll
+    for (int n = nd - 2; n >= 0; n--) d = fma(d, u, k.nq2[n].x);
+    t = fma(e0, ri2, d);
+  }
+}
+
+// FP64 real DM kernels with every unordered pair evaluated once: the walk of
+// direct_group_sym64 (below) in coordinates scaled by 1/Rdir, without
+// branches.  A pair is a hit when r^2 is a normal number below 1 (compared on
+// its high word, an integer operation: the FP64 pipe, at half the FP32 rate,
+// is what bounds the kernel); a miss gets s = 1 and charge 0 on both sides.
+// 35 FP64 operations per pair at order 6, 41 and a hit branch before.  The
+// group's work is shared by nsplit warps as in direct_group_sym.
+template <int FUNC, int ND>
+__device__ __forceinline__ void direct_group_sym64_dm(
+    const PairCoef<double> &k, const double4 *__restrict__ gpos,
+    const double4 *__restrict__ spos, const double *__restrict__ qs,
+    const double *__restrict__ qcaller, const int4 G, const double4 c,
+    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm,
+    double *__restrict__ vsrc, double4 *tsm, int lane, int part, int nsplit,
+    double (&acc)[4]) {
+  const unsigned FULL = 0xffffffffu;
+  const int ti = G.x + lane;
+  const bool active = lane < G.y;
+  const double ir = k.invR, vs = k.vscale, gsc = k.gscale;
+  double tx = 1e150, ty = 1e150, tz = 1e150, tq = 0.0;  // idle lanes: far away, no charge
+  if (active) {
+    const double4 p = gpos[ti];
+    tx = (p.x - c.x) * ir, ty = (p.y - c.y) * ir, tz = (p.z - c.z) * ir;
+    tq = qcaller[perm[ti]];
+  }
+  tsm[lane] = make_double4(tx, ty, tz, tq);
+  __syncwarp();
+  // r^2 in [2^-1022, 1): the high word in [0x00100000, 0x3ff00000)
+  auto inside = [](double r2) {
+    return (unsigned)__double2hiint(r2) - 0x00100000u < 0x3fe00000u;
+  };
+  // pairs inside the group, target side only (each is met from both ends)
+  for (int s = part; s < G.y; s += nsplit) {
+    const double4 S = tsm[s];
+    const double x = tx - S.x, y = ty - S.y, z = tz - S.z;
+    const double r2 = fma(x, x, fma(y, y, z * z));
+    const bool hit = inside(r2);
+    double f0, t;
+    dm_eval64<FUNC, ND>(k, hit ? r2 : 1.0, f0, t);
+    const double q = hit ? S.w : 0.0, gq = t * q;
+    acc[0] = fma(f0, q, acc[0]);
+    acc[1] = fma(-gq, x, acc[1]);
+    acc[2] = fma(-gq, y, acc[2]);
+    acc[3] = fma(-gq, z, acc[3]);
+  }
+  // half-shell segments in chunks of 64 sources (register prefetch)
+  const int stride = 64 * nsplit;
+  SrcCursor cur[2];
+  cur[0] = SrcCursor{G.z, lane + 64 * part};
+  cur[0].normalize(segs, G.w);
+  cur[1] = SrcCursor{cur[0].seg, cur[0].off + 32};
+  cur[1].normalize(segs, G.w);
+  bool v[2];
+  double4 p[2];
+  int slot[2] = {-1, -1};  // source-side slots (brick positions)
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    v[i] = cur[i].seg < G.w;
+    p[i] = make_double4(0, 0, 0, 0);
+    if (v[i]) {
+      const long j = (long)segs[cur[i].seg].x + cur[i].off;
+      p[i] = spos[j], slot[i] = (int)p[i].w, p[i].w = qs[j];
+    }
+  }
+  while (__any_sync(FULL, v[0])) {
+    // empty slots far away on the other side from idle targets, no charge
+    double4 src[2];
+    int to[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      src[i] = make_double4(-1e150, -1e150, -1e150, 0.0);
+      to[i] = v[i] ? slot[i] : -1;
+      if (v[i])
+        src[i] = make_double4((p[i].x - c.x) * ir, (p[i].y - c.y) * ir, (p[i].z - c.z) * ir,
+                              p[i].w);
+      cur[i].off += stride;
+      cur[i].normalize(segs, G.w);
+      v[i] = cur[i].seg < G.w;
+      if (v[i]) {
+        const long j = (long)segs[cur[i].seg].x + cur[i].off;
+        p[i] = spos[j], slot[i] = (int)p[i].w, p[i].w = qs[j];
+      }
+    }
+    double aV = 0, aX = 0, aY = 0, aZ = 0;                   // target side, rotating
+    double S[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};           // source side
+    const int next = (lane + 1) & 31;
+#pragma unroll 2
+    for (int kk = 0; kk < 32; kk++) {
+      const double4 T = tsm[(lane + kk) & 31];
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const double x = T.x - src[i].x, y = T.y - src[i].y, z = T.z - src[i].z;
+        const double r2 = fma(x, x, fma(y, y, z * z));
+        const bool hit = inside(r2);
+        double f0, t;
+        dm_eval64<FUNC, ND>(k, hit ? r2 : 1.0, f0, t);
+        const double qm = hit ? src[i].w : 0.0, qt = hit ? T.w : 0.0;
+        const double gm = t * qm, gt = t * qt;
+        aV = fma(f0, qm, aV);
+        aX = fma(-gm, x, aX);
+        aY = fma(-gm, y, aY);
+        aZ = fma(-gm, z, aZ);
+        S[i][0] = fma(f0, qt, S[i][0]);
+        S[i][1] = fma(gt, x, S[i][1]);
+        S[i][2] = fma(gt, y, S[i][2]);
+        S[i][3] = fma(gt, z, S[i][3]);
+      }
+      aV = __shfl_sync(FULL, aV, next);
+      aX = __shfl_sync(FULL, aX, next);
+      aY = __shfl_sync(FULL, aY, next);
+      aZ = __shfl_sync(FULL, aZ, next);
+    }
+    acc[0] += aV;
+    acc[1] += aX;
+    acc[2] += aY;
+    acc[3] += aZ;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      if (to[i] >= 0) {
+        double *d = vsrc + 4L * to[i];
+        atomicAdd(d, vs * S[i][0]);
+#pragma unroll
+        for (int m = 1; m < 4; m++) atomicAdd(d + m, gsc * S[i][m]);
+      }
+  }
+}
+
+// sin and cos of x in FP64, |x| < kMaxHelmArg, without a branch: Cody-Waite
+// reduction to [-pi/4, pi/4] with pi/2 as the sum of two doubles, Taylor
+// polynomials of degree 15 and 16 (truncation below 5e-17), quadrant by
+// selects.  About half the FP64 operations of the general sincos.
+constexpr double kMaxHelmArg = 1e5;
+__device__ __forceinline__ void sincos_taylor(double x, double &sn, double &cs) {
+  constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
+  const double m = fma(x, 0.63661977236758134308, kMagic), n = m - kMagic;
+  double r = fma(-n, 1.57079632679489661923, x);
+  r = fma(-n, 6.12323399573676603587e-17, r);
+  const double z = r * r;
+  double a = -1.0 / 1307674368000.0;  // -1/15!
+  a = fma(a, z, 1.0 / 6227020800.0);
+  a = fma(a, z, -1.0 / 39916800.0);
+  a = fma(a, z, 1.0 / 362880.0);
+  a = fma(a, z, -1.0 / 5040.0);
+  a = fma(a, z, 1.0 / 120.0);
+  a = fma(a, z, -1.0 / 6.0);
+  const double s = fma(a * z, r, r);
+  double b = 1.0 / 20922789888000.0;  // 1/16!
+  b = fma(b, z, -1.0 / 87178291200.0);
+  b = fma(b, z, 1.0 / 479001600.0);
+  b = fma(b, z, -1.0 / 3628800.0);
+  b = fma(b, z, 1.0 / 40320.0);
+  b = fma(b, z, -1.0 / 720.0);
+  b = fma(b, z, 1.0 / 24.0);
+  b = fma(b, z, -0.5);
+  const double c = fma(b, z, 1.0);
+  const int q = __double2loint(m);  // n mod 2^32
+  sn = q & 1 ? c : s;
+  cs = q & 1 ? s : c;
+  if (q & 2) sn = -sn;
+  if ((q + 1) & 2) cs = -cs;
+}
+
+// Helmholtz DM pair kernel in FP64 (coordinates in units of Rdir, s = r^2 in
+// (0, 1]): F0 = exp(i kap r)/r - P and F1 = (1/r) dF0/dr, P the Taylor
+// polynomial in u = 1 - s (PairCoef; src/KernelFunctionHelmholtz.cpp:506-563).
+template <int ND>
+__device__ __forceinline__ void helm_eval64(const PairCoef<double> &k, double s, double2 &F0,
+                                            double2 &F1) {
+  constexpr int nd = dm_degree<ND>();  // ND = 0: zero-padded to kMaxDeriv
+  const double ri = rsqrt_iter(s), r = s * ri, u = 1.0 - s;
+  double sn, cs;
+  sincos_taylor(k.kapr * r, sn, cs);
+  const double damp = k.kapi != 0.0 ? exp(-k.kapi * r) * ri : ri;
+  const double er = cs * damp, ei = sn * damp;  // exp(i kap r) / r
+  // its radial derivative over r: E (i kap / r - 1 / r^2)
+  const double A = fma(-k.kapi, ri, -ri * ri), B = k.kapr * ri;
+  double pr = k.hc[nd].x, pi = k.hc[nd].y;
+#pragma unroll
+  for (int n = nd - 1; n >= 0; n--) pr = fma(pr, u, k.hc[n].x), pi = fma(pi, u, k.hc[n].y);
+  double dr = k.hd[nd - 1].x, di = k.hd[nd - 1].y;
+#pragma unroll
+  for (int n = nd - 2; n >= 0; n--) dr = fma(dr, u, k.hd[n].x), di = fma(di, u, k.hd[n].y);
+  F0 = make_double2(er + pr, ei + pi);
+  F1 = make_double2(fma(A, er, fma(-B, ei, dr)), fma(A, ei, fma(B, er, di)));
+}
+
+// complex a * b + c on (re, im) doubles
+__device__ __forceinline__ void cfma64(double2 a, double2 b, double &cr, double &ci) {
+  cr = fma(a.x, b.x, fma(-a.y, b.y, cr));
+  ci = fma(a.x, b.y, fma(a.y, b.x, ci));
+}
+
+// FP64 Helmholtz with every unordered pair evaluated once, the complex
+// counterpart of direct_group_sym64_dm: scaled coordinates, misses at s = 1
+// with charge 0, no branch.  One source per lane and chunks of 32 (two would
+// take 170-200 registers and halve the resident warps); the eight target sums
+// rotate one lane down per step, the source sums go to vsrc ([n][8] doubles:
+// V, x, y, z as re, im).  About 105 FP64 operations per pair at order 8; the
+// one-sided walk spends about 130 on each of the pair's two directions.
+// tsm: the targets' x, y, z, Re q, Im q.
+template <int ND>
+__device__ __forceinline__ void direct_group_sym64_helm(
+    const PairCoef<double> &k, const double4 *__restrict__ gpos,
+    const double4 *__restrict__ spos, const double *__restrict__ qs,
+    const double *__restrict__ qcaller, const int4 G, const double4 c,
+    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm,
+    double *__restrict__ vsrc, double (*tsm)[32], int lane, int part, int nsplit,
+    double (&acc)[4], double (&acci)[4]) {
+  const unsigned FULL = 0xffffffffu;
+  const int ti = G.x + lane;
+  const double ir = k.invR, gsc = ir * ir;  // F0 / Rdir, F1 x / Rdir^2
+  double tx = 1e150, ty = 1e150, tz = 1e150;  // idle lanes: far away, no charge
+  double2 tq = make_double2(0.0, 0.0);
+  if (lane < G.y) {
+    const double4 p = gpos[ti];
+    tx = (p.x - c.x) * ir, ty = (p.y - c.y) * ir, tz = (p.z - c.z) * ir;
+    const long o = perm[ti];
+    tq = make_double2(qcaller[2 * o], qcaller[2 * o + 1]);
+  }
+  tsm[0][lane] = tx, tsm[1][lane] = ty, tsm[2][lane] = tz;
+  tsm[3][lane] = tq.x, tsm[4][lane] = tq.y;
+  __syncwarp();
+  auto inside = [](double r2) {  // r^2 in [2^-1022, 1)
+    return (unsigned)__double2hiint(r2) - 0x00100000u < 0x3fe00000u;
+  };
+  // pairs inside the group, target side only (each is met from both ends)
+  for (int s = part; s < G.y; s += nsplit) {
+    const double x = tx - tsm[0][s], y = ty - tsm[1][s], z = tz - tsm[2][s];
+    const double r2 = fma(x, x, fma(y, y, z * z));
+    const bool hit = inside(r2);
+    double2 F0, F1;
+    helm_eval64<ND>(k, hit ? r2 : 1.0, F0, F1);
+    const double2 q = make_double2(hit ? tsm[3][s] : 0.0, hit ? tsm[4][s] : 0.0);
+    double gr = 0, gi = 0;
+    cfma64(F0, q, acc[0], acci[0]);
+    cfma64(F1, q, gr, gi);
+    acc[1] = fma(gr, x, acc[1]), acci[1] = fma(gi, x, acci[1]);
+    acc[2] = fma(gr, y, acc[2]), acci[2] = fma(gi, y, acci[2]);
+    acc[3] = fma(gr, z, acc[3]), acci[3] = fma(gi, z, acci[3]);
+  }
+  const int stride = 32 * nsplit;
+  SrcCursor cur{G.z, lane + 32 * part};
+  cur.normalize(segs, G.w);
+  bool v = cur.seg < G.w;
+  double4 p = make_double4(0, 0, 0, 0);
+  double2 q = make_double2(0, 0);
+  if (v) {
+    const long j = (long)segs[cur.seg].x + cur.off;
+    p = spos[j], q = reinterpret_cast<const double2 *>(qs)[j];
+  }
+  while (__any_sync(FULL, v)) {
+    // empty slots far away on the other side from idle targets, no charge
+    double sx = -1e150, sy = -1e150, sz = -1e150;
+    double2 sq = make_double2(0.0, 0.0);
+    int slot = -1;
+    if (v) {
+      sx = (p.x - c.x) * ir, sy = (p.y - c.y) * ir, sz = (p.z - c.z) * ir;
+      sq = q;
+      slot = (int)p.w;
+    }
+    cur.off += stride;
+    cur.normalize(segs, G.w);
+    v = cur.seg < G.w;
+    if (v) {
+      const long j = (long)segs[cur.seg].x + cur.off;
+      p = spos[j], q = reinterpret_cast<const double2 *>(qs)[j];
+    }
+    double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // target side, rotating
+    double S[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // source side
+    const int next = (lane + 1) & 31;
+#pragma unroll 1
+    for (int kk = 0; kk < 32; kk++) {
+      const int t = (lane + kk) & 31;
+      const double x = tsm[0][t] - sx, y = tsm[1][t] - sy, z = tsm[2][t] - sz;
+      const double r2 = fma(x, x, fma(y, y, z * z));
+      const bool hit = inside(r2);
+      double2 F0, F1;
+      helm_eval64<ND>(k, hit ? r2 : 1.0, F0, F1);
+      const double2 qm = make_double2(hit ? sq.x : 0.0, hit ? sq.y : 0.0);
+      const double2 qt = make_double2(hit ? tsm[3][t] : 0.0, hit ? tsm[4][t] : 0.0);
+      const double gr = fma(F1.x, qm.x, -F1.y * qm.y), gi = fma(F1.x, qm.y, F1.y * qm.x);
+      cfma64(F0, qm, a[0], a[1]);
+      a[2] = fma(gr, x, a[2]), a[3] = fma(gi, x, a[3]);
+      a[4] = fma(gr, y, a[4]), a[5] = fma(gi, y, a[5]);
+      a[6] = fma(gr, z, a[6]), a[7] = fma(gi, z, a[7]);
+      const double hr = fma(F1.x, qt.x, -F1.y * qt.y), hi = fma(F1.x, qt.y, F1.y * qt.x);
+      cfma64(F0, qt, S[0], S[1]);
+      S[2] = fma(-hr, x, S[2]), S[3] = fma(-hi, x, S[3]);
+      S[4] = fma(-hr, y, S[4]), S[5] = fma(-hi, y, S[5]);
+      S[6] = fma(-hr, z, S[6]), S[7] = fma(-hi, z, S[7]);
+#pragma unroll
+      for (int m = 0; m < 8; m++) a[m] = __shfl_sync(FULL, a[m], next);
+    }
+#pragma unroll
+    for (int m = 0; m < 4; m++) acc[m] += a[2 * m], acci[m] += a[2 * m + 1];
+    if (slot >= 0) {
+      double *d = vsrc + 8L * slot;
+#pragma unroll
+      for (int m = 0; m < 8; m++) atomicAdd(d + m, (m < 2 ? ir : gsc) * S[m]);
+    }
+  }
+}
+
+// Its target sums to V, less the self term (src/Interface.cpp:2909-2910).
+__device__ __forceinline__ void store_targets64_cplx(
+    const int4 G, const uint32_t *__restrict__ perm, const double *__restrict__ qcaller,
+    double fself_r, double fself_i, double ir, double *__restrict__ V, int lane,
+    const double (&acc)[4], const double (&acci)[4]) {
+  if (lane >= G.y) return;
+  const long o = perm[G.x + lane];
+  const double qr = qcaller[2 * o], qi = qcaller[2 * o + 1], g = ir * ir;
+  double2 *Vo = reinterpret_cast<double2 *>(V) + 4 * o;
+  Vo[0] = make_double2(ir * acc[0] - (fself_r * qr - fself_i * qi),
+                       ir * acci[0] - (fself_r * qi + fself_i * qr));
+#pragma unroll
+  for (int m = 1; m < 4; m++) Vo[m] = make_double2(g * acc[m], g * acci[m]);
+}
+
+// Target sums of the FP64 pair-once walk to V (sums scaled by vs, gs), less
+// the self term f_LR(0) q (src/Interface.cpp:2061-2062).
+__device__ __forceinline__ void store_targets64(const int4 G, const uint32_t *__restrict__ perm,
+                                                const double *__restrict__ qcaller,
+                                                double fself_r, double vs, double gs,
+                                                double *__restrict__ V, int lane,
+                                                const double (&acc)[4]) {
+  if (lane >= G.y) return;
+  const long o = perm[G.x + lane];
+  reinterpret_cast<double4 *>(V)[o] =
+      make_double4(vs * acc[0] - fself_r * qcaller[o], gs * acc[1], gs * acc[2], gs * acc[3]);
 }
 
 // FP64 direct sum of one warp group with every unordered pair evaluated once

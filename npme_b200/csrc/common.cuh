@@ -47,6 +47,12 @@ struct PairCoef {
   // 0 and gscale = 0.)
   typename Vec2<T>::type nc2[kMaxDeriv + 1], nq2[kMaxDeriv + 1], kn2;
   double invR, vscale, gscale;
+  // Helmholtz in FP64, scaled frame (kap = k0 Rdir): with c_n the Taylor
+  // coefficients of exp(i kap sqrt(s))/sqrt(s) in u = 1 - s, (re, im) pairs
+  // hc[n] = -c_n and hd[n] = 2 (n + 1) c_{n+1}, the negated coefficients of
+  // 2 dP/ds
+  typename Vec2<T>::type hc[kMaxDeriv + 1], hd[kMaxDeriv + 1];
+  T kapr, kapi;
   // Helmholtz packed evaluation: (re, im) pairs of -ar/-ai and -br/-bi
   typename Vec2<T>::type nac2[kMaxDeriv + 1], nbc2[kMaxDeriv + 1];
 };

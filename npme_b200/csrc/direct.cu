@@ -88,6 +88,26 @@ PairCoef<T> make_pair_coef(const npme_handle *h) {
       k.kn2.x = k.kn2.y = (T)(2.0 * b / std::sqrt(M_PI));
     }
     k.invR = 1.0 / R;
+    // Helmholtz: G_n = ((1/x) d/dx)^n exp(i kap x)/x at x = 1 (the recursion of
+    // dm_coefficients with Rdir = 1), c_n = G_n (-1)^n / (2^n n!)
+    if (h->p.funcType == NPME_FUNC_HELMHOLTZ) {
+      typedef std::complex<double> cd;
+      const cd I(0, 1), kap(h->p.k0_r * R, h->p.k0_i * R);
+      k.kapr = (T)kap.real(), k.kapi = (T)kap.imag();
+      cd g0 = std::exp(I * kap), g1 = g0 * (I * kap - 1.0);  // G_n, G_{n+1}
+      double f = 1.0;  // (-1)^n / (2^n n!)
+      for (int i = 0; i <= k.nder && i <= kMaxDeriv; i++) {
+        const cd c = g0 * f;
+        k.hc[i].x = (T)-c.real(), k.hc[i].y = (T)-c.imag();
+        const double fn = -f / (2.0 * (i + 1));
+        if (i < k.nder) {
+          const cd d = 2.0 * (i + 1) * fn * g1;
+          k.hd[i].x = (T)d.real(), k.hd[i].y = (T)d.imag();
+        }
+        const cd g2 = -(2.0 * (i + 2) - 1.0) * g1 - kap * kap * g0;
+        g0 = g1, g1 = g2, f = fn;
+      }
+    }
     k.vscale = std::pow(R, al);
     k.gscale = (k.split == NPME_SPLIT_LAPLACE_ORIG ? 1.0 : -al) * std::pow(R, al - 1.0);
   }
@@ -163,7 +183,8 @@ static void merge_or_defer(npme_handle *h, const DirectArgs &a, cudaStream_t s, 
 // them as long as the heaviest: the walk is split over the warps of a CTA.
 // Measured, whole against split walks: 170 groups (4,000 points) 92 / 26 us
 // with 16 warps, 28 with 8; 1,150 groups (30,000 points in a flat box) 110 /
-// 82 us with 4 warps, 96 with 2, 98 with 8.  From about two rounds on the
+// 82 us with 4 warps, 96 with 2, 98 with 8; 2,000 groups (FP64 Helmholtz,
+// 62,500 points) 1,530 / 1,098 us with 4.  From about two rounds on the
 // splitting's own work (every warp stages the targets and walks all segments)
 // costs more than it gives: 3,300 groups 137 / 139 us, 31,700 groups +10 %.
 constexpr int kMaxSplit = 16;
@@ -307,8 +328,35 @@ __global__ void __launch_bounds__(32 * kGroupWarps) direct_sym64_kernel(
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long g = (long)blockIdx.x * kGroupWarps + wid;
   if (g >= ngroups) return;  // warp-uniform
-  direct_group_sym64<FUNC, SPLIT, ND>(k, gpos, spos, qs, qcaller, groups[g], gcen[g], segs, perm,
-                                      fself_r, V, vsrc, tsm[wid], lane);
+  if constexpr (SPLIT == 0) {
+    double acc[4] = {0, 0, 0, 0};
+    const int4 G = groups[g];
+    direct_group_sym64_dm<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, perm, vsrc,
+                                    tsm[wid], lane, 0, 1, acc);
+    store_targets64(G, perm, qcaller, fself_r, k.vscale, k.gscale, V, lane, acc);
+  } else
+    direct_group_sym64<FUNC, SPLIT, ND>(k, gpos, spos, qs, qcaller, groups[g], gcen[g], segs,
+                                        perm, fself_r, V, vsrc, tsm[wid], lane);
+}
+
+// The DM form with a CTA of blockDim.x / 32 warps per group (split_warps).
+template <int FUNC, int ND>
+__global__ void __launch_bounds__(32 * kMaxSplit) direct_sym64_split_kernel(
+    PairCoef<double> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
+    const double *__restrict__ qs, const double *__restrict__ qcaller,
+    const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
+    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, double fself_r,
+    double *__restrict__ V, double *__restrict__ vsrc) {
+  __shared__ double4 tsm[kMaxSplit][32];
+  __shared__ double red[kMaxSplit][32][4];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nsplit = blockDim.x >> 5;
+  const long g = blockIdx.x;
+  double acc[4] = {0, 0, 0, 0};
+  const int4 G = groups[g];
+  direct_group_sym64_dm<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, perm, vsrc,
+                                  tsm[wid], lane, wid, nsplit, acc);
+  reduce_parts(acc, red, wid, nsplit, lane);
+  if (wid == 0) store_targets64(G, perm, qcaller, fself_r, k.vscale, k.gscale, V, lane, acc);
 }
 
 // V[caller(i)][m] += vsrc[i][m], then vsrc[i] = 0 for the next call.
@@ -329,6 +377,16 @@ template <int FUNC, int SPLIT, int ND>
 static void sym64_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
   const long blocks = (h->n_hgroups + kGroupWarps - 1) / kGroupWarps;
   if (blocks == 0) return;
+  if constexpr (SPLIT == 0) {
+    const int split = split_warps(h->n_hgroups);
+    if (split > 1) {
+      direct_sym64_split_kernel<FUNC, ND><<<(unsigned)h->n_hgroups, 32 * split, 0, s>>>(
+          make_pair_coef<double>(h), h->d_gpos, h->d_spos, (const double *)a.q, a.qcaller,
+          h->d_hgroups, h->d_hcen, h->d_hsegs, h->d_cperm, a.fself_r, a.V, h->d_vsrc64);
+      merge_or_defer(h, a, s, 1.0, 1.0);
+      return;
+    }
+  }
   direct_sym64_kernel<FUNC, SPLIT, ND><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
       make_pair_coef<double>(h), h->d_gpos, h->d_spos, (const double *)a.q, a.qcaller,
       h->d_hgroups, h->d_hcen, h->d_hsegs, h->d_cperm, h->n_hgroups, a.fself_r, a.V,
@@ -336,9 +394,70 @@ static void sym64_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream_t s)
   merge_or_defer(h, a, s, 1.0, 1.0);
 }
 
+// FP64 Helmholtz form: CTAs of kGroupWarps groups (split = 1) or of one group.
+template <int ND, bool SPLIT>
+__global__ void __launch_bounds__(32 * (SPLIT ? kMaxSplit : kGroupWarps), SPLIT ? 1 : 4)
+    direct_sym64_helm_kernel(
+    PairCoef<double> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
+    const double *__restrict__ qs, const double *__restrict__ qcaller,
+    const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
+    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, long ngroups,
+    double fself_r, double fself_i, double *__restrict__ V, double *__restrict__ vsrc) {
+  constexpr int W = SPLIT ? kMaxSplit : kGroupWarps;
+  __shared__ double tsm[W][5][32];  // group targets: x, y, z, q
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nsplit = SPLIT ? blockDim.x >> 5 : 1, part = SPLIT ? wid : 0;
+  const long g = SPLIT ? (long)blockIdx.x : (long)blockIdx.x * kGroupWarps + wid;
+  if (g >= ngroups) return;  // warp-uniform (SPLIT: no CTA is past the end)
+  double acc[4] = {0, 0, 0, 0}, acci[4] = {0, 0, 0, 0};
+  const int4 G = groups[g];
+  direct_group_sym64_helm<ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, perm, vsrc, tsm[wid],
+                              lane, part, nsplit, acc, acci);
+  if constexpr (SPLIT) {
+    __shared__ double red[kMaxSplit][32][4];
+    reduce_parts(acc, red, wid, nsplit, lane);
+    __syncthreads();
+    reduce_parts(acci, red, wid, nsplit, lane);
+    if (wid > 0) return;
+  }
+  store_targets64_cplx(G, perm, qcaller, fself_r, fself_i, k.invR, V, lane, acc, acci);
+}
+
+// Complex V[caller(i)][0..3] += vsrc[i] (re, im pairs), then zero.
+__global__ void merge_source64_cplx_kernel(double4 *__restrict__ vsrc,
+                                           const uint32_t *__restrict__ bperm, long n,
+                                           double *__restrict__ V) {
+  const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n) return;
+  const double4 a = vsrc[2 * s], b = vsrc[2 * s + 1];
+  vsrc[2 * s] = vsrc[2 * s + 1] = make_double4(0, 0, 0, 0);
+  double4 *o = reinterpret_cast<double4 *>(V) + 2 * (long)bperm[s];
+  double4 u = o[0], w = o[1];
+  u.x += a.x, u.y += a.y, u.z += a.z, u.w += a.w;
+  w.x += b.x, w.y += b.y, w.z += b.z, w.w += b.w;
+  o[0] = u, o[1] = w;
+}
+
+template <int ND>
+static void sym64_helm_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
+  const long blocks = (h->n_hgroups + kGroupWarps - 1) / kGroupWarps;
+  if (blocks == 0) return;
+  const PairCoef<double> k = make_pair_coef<double>(h);
+  const int split = split_warps(h->n_hgroups);
+  if (split > 1)
+    direct_sym64_helm_kernel<ND, true><<<(unsigned)h->n_hgroups, 32 * split, 0, s>>>(
+        k, h->d_gpos, h->d_spos, (const double *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
+        h->d_hsegs, h->d_cperm, h->n_hgroups, a.fself_r, a.fself_i, a.V, h->d_vsrc64);
+  else
+    direct_sym64_helm_kernel<ND, false><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
+        k, h->d_gpos, h->d_spos, (const double *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
+        h->d_hsegs, h->d_cperm, h->n_hgroups, a.fself_r, a.fself_i, a.V, h->d_vsrc64);
+  merge_or_defer(h, a, s, 1.0, 1.0);
+}
+
 template <int FUNC, int SPLIT>
 static void sym64_launch(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
-  switch (SPLIT == 1 ? 0 : h->p.nDeriv) {
+  switch (SPLIT == 1 || (FUNC == 1 && h->p.alpha >= 0) ? 0 : h->p.nDeriv) {
     case 3: sym64_launch_nd<FUNC, SPLIT, 3>(h, a, s); break;
     case 6: sym64_launch_nd<FUNC, SPLIT, 6>(h, a, s); break;
     case 8: sym64_launch_nd<FUNC, SPLIT, 8>(h, a, s); break;
@@ -349,7 +468,10 @@ static void sym64_launch(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
 void launch_merge_source(npme_handle *h, double *V, cudaStream_t s, double vs, double gs) {
   const long n = (long)h->n;
   const unsigned blocks = (unsigned)((n + 255) / 256);
-  if (!h->fp32)
+  if (!h->fp32 && h->complex_kernel)
+    merge_source64_cplx_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<double4 *>(h->d_vsrc64),
+                                                      h->d_bperm, n, V);
+  else if (!h->fp32)
     merge_source64_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<double4 *>(h->d_vsrc64),
                                                  h->d_bperm, n, V);
   else if (h->complex_kernel)
@@ -369,13 +491,22 @@ bool pairs_once(const npme_handle *h) {
   if (!h->use_sym || h->n_hgroups == 0) return false;
   if (h->user_kernel) return !h->complex_kernel;  // the functor's scalar pair kernel
   const int f = h->p.funcType;
-  if (f == NPME_FUNC_HELMHOLTZ) return h->fp32;
+  // FP64 Helmholtz: its argument reduction holds for moderate arguments
+  if (f == NPME_FUNC_HELMHOLTZ)
+    return h->fp32 || std::fabs(h->p.k0_r) * h->p.Rdir < kMaxHelmArg;
   return f == NPME_FUNC_LAPLACE || f == NPME_FUNC_RALPHA;
 }
 
 static bool sym_launch(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
   if (!pairs_once(h)) return false;
   const int f = h->p.funcType, nd = h->p.nDeriv;
+  if (f == NPME_FUNC_HELMHOLTZ && !h->fp32) {
+    if (nd == 3) sym64_helm_launch_nd<3>(h, a, s);
+    else if (nd == 6) sym64_helm_launch_nd<6>(h, a, s);
+    else if (nd == 8) sym64_helm_launch_nd<8>(h, a, s);
+    else sym64_helm_launch_nd<0>(h, a, s);
+    return true;
+  }
   if (f == NPME_FUNC_HELMHOLTZ) {
     if (nd == 3) sym_helm_launch_nd<3>(h, a, s);
     else if (nd == 6) sym_helm_launch_nd<6>(h, a, s);

@@ -184,7 +184,7 @@ struct npme_handle {
   // brick order (spos[k].w holds it), so that the interpolation, which visits
   // the points in that order, can fold them into V
   float4 *d_vsrc = nullptr;      // FP32: source-side sums (two float4 if complex), kept zero
-  double *d_vsrc64 = nullptr;    // FP64: source-side sums [n][4], kept zero
+  double *d_vsrc64 = nullptr;    // FP64: source-side sums [n][4] ([8] if complex), kept zero
   // CalcV leaves the source-side sums of its pair-once walk to the
   // interpolation (scale vs for the potential, gs for the gradient)
   bool merge_pending = false;

@@ -781,8 +781,8 @@ int describe(npme_handle *h, SysDesc &D) {
     if ((rc = handle_buffer(h, (void **)&h->d_vsrc, sizeof(float4) * C * n))) return rc;
     cudaMemsetAsync(h->d_vsrc, 0, sizeof(float4) * C * n, h->stream);
   } else {
-    if ((rc = handle_buffer(h, (void **)&h->d_vsrc64, sizeof(double) * 4 * n))) return rc;
-    cudaMemsetAsync(h->d_vsrc64, 0, sizeof(double) * 4 * n, h->stream);
+    if ((rc = handle_buffer(h, (void **)&h->d_vsrc64, sizeof(double) * 4 * C * n))) return rc;
+    cudaMemsetAsync(h->d_vsrc64, 0, sizeof(double) * 4 * C * n, h->stream);
   }
   // grids
   const long *N = gr.N;
