@@ -652,79 +652,116 @@ void launch_count_pairs(npme_handle *h, unsigned long long *d_count, cudaStream_
 // ---------------------------------------------------------------------------
 // Exact sum (src/PotentialLaplace.cpp:40-132, src/PotentialHelmholtz.cpp:41,
 // src/PotentialGenFunc.cpp:321): all pairs j != i with the full kernel, FP64,
-// no self term.  Sources are tiled through shared memory.
+// no self term.  A CTA of 128 targets walks its share of the sources (blockIdx.y
+// of gridDim.y) in shared-memory tiles; with more than one share the partial
+// sums go to scratch and exact_reduce_kernel adds them in order.  Bound by the
+// FP64 pipe: 18 operations per ordered pair for 1/r.
 
 constexpr int kExactBS = 128;
 
+struct ExactArgs {
+  const double *coord, *q;
+  long n;
+  double alpha, k0r, k0i;
+  const uint32_t *tidx;
+  long nt, share;  // targets, sources per share
+  double *out;     // V, or the partial sums [share][target][4 or 8]
+};
+
+// 1/sqrt(r2) of any r2 >= 0: the iteration where it holds, the hardware's 0
+// or infinity elsewhere (coincident points give infinity, as rsqrt does).
+__device__ __forceinline__ double rsqrt_any(double r2) {
+  const double y = rsqrt_iter(r2);
+  const bool normal = (unsigned)__double2hiint(r2) - 0x00100000u < 0x7fe00000u;
+  return normal ? y : rsqrt(r2);
+}
+
+// One ordered pair added to the target's sums.  FUNC as in npme_params; 3:
+// Helmholtz with arguments beyond kMaxHelmArg.
 template <int FUNC>
-__global__ void __launch_bounds__(kExactBS) exact_kernel(const double *__restrict__ coord,
-                                                          const double *__restrict__ q, long n,
-                                                          double alpha, double k0r, double k0i,
-                                                          const uint32_t *__restrict__ tidx,
-                                                          long nt, double *__restrict__ V) {
-  constexpr bool CPLX = FUNC == 2;
-  __shared__ double4 sp[kExactBS];
-  __shared__ double2 sq[kExactBS];
+__device__ __forceinline__ void exact_pair(const ExactArgs &A, double x, double y, double z,
+                                           double r2, double qr, double qi, double (&a)[4],
+                                           double (&ai)[4]) {
+  const double ri = rsqrt_any(r2), ri2 = ri * ri;
+  if constexpr (FUNC < 2) {
+    const double f = FUNC == 0 ? qr * ri : qr * pow(r2, 0.5 * A.alpha);
+    const double g = (FUNC == 0 ? -f : A.alpha * f) * ri2;
+    a[0] += f;
+    a[1] = fma(g, x, a[1]);
+    a[2] = fma(g, y, a[2]);
+    a[3] = fma(g, z, a[3]);
+  } else {
+    const double r = r2 * ri;
+    double sn, cs;
+    if (FUNC == 2) sincos_taylor(A.k0r * r, sn, cs);
+    else sincos(A.k0r * r, &sn, &cs);
+    const double d = A.k0i != 0.0 ? exp(-A.k0i * r) * ri : ri;
+    const double er = cs * d, ei = sn * d;
+    // f1 = f0 (i k0 / r - 1 / r^2)
+    const double u = fma(-A.k0i, ri, -ri2), v = A.k0r * ri;
+    const double f1r = fma(u, er, -v * ei), f1i = fma(u, ei, v * er);
+    a[0] = fma(er, qr, fma(-ei, qi, a[0]));
+    ai[0] = fma(er, qi, fma(ei, qr, ai[0]));
+    const double gr = fma(f1r, qr, -f1i * qi), gi = fma(f1r, qi, f1i * qr);
+    a[1] = fma(gr, x, a[1]), a[2] = fma(gr, y, a[2]), a[3] = fma(gr, z, a[3]);
+    ai[1] = fma(gi, x, ai[1]), ai[2] = fma(gi, y, ai[2]), ai[3] = fma(gi, z, ai[3]);
+  }
+}
+
+template <int FUNC>
+__global__ void __launch_bounds__(kExactBS) exact_kernel(const __grid_constant__ ExactArgs A) {
+  constexpr bool CPLX = FUNC >= 2;
+  __shared__ double4 sp[kExactBS];  // x, y, z, Re q
+  __shared__ double sqi[CPLX ? kExactBS : 1];
   // output row t holds target tidx[t] (every point when tidx is null)
   const long t = blockIdx.x * (long)kExactBS + threadIdx.x;
-  const bool active = t < nt;
-  const long i = active ? (tidx ? (long)tidx[t] : t) : -1;
+  const bool active = t < A.nt;
+  const long i = active ? (A.tidx ? (long)A.tidx[t] : t) : -1;
   double xi = 0, yi = 0, zi = 0;
-  if (active) xi = coord[3 * i], yi = coord[3 * i + 1], zi = coord[3 * i + 2];
+  if (active) xi = A.coord[3 * i], yi = A.coord[3 * i + 1], zi = A.coord[3 * i + 2];
   double a[4] = {0, 0, 0, 0}, ai[4] = {0, 0, 0, 0};
-  for (long j0 = 0; j0 < n; j0 += kExactBS) {
+  const long first = blockIdx.y * A.share, last = min(A.n, first + A.share);
+  for (long j0 = first; j0 < last; j0 += kExactBS) {
     __syncthreads();
     const long j = j0 + threadIdx.x;
-    if (j < n) {
-      sp[threadIdx.x] = make_double4(coord[3 * j], coord[3 * j + 1], coord[3 * j + 2], 0.0);
-      sq[threadIdx.x] = CPLX ? make_double2(q[2 * j], q[2 * j + 1]) : make_double2(q[j], 0.0);
+    if (j < last) {
+      sp[threadIdx.x] = make_double4(A.coord[3 * j], A.coord[3 * j + 1], A.coord[3 * j + 2],
+                                     CPLX ? A.q[2 * j] : A.q[j]);
+      if (CPLX) sqi[threadIdx.x] = A.q[2 * j + 1];
     }
     __syncthreads();
-    const int cnt = (int)min((long)kExactBS, n - j0);
-    for (int s = 0; s < cnt; s++) {
-      if (j0 + s == i) continue;
-      const double x = xi - sp[s].x, y = yi - sp[s].y, z = zi - sp[s].z;
-      const double r2 = x * x + y * y + z * z;
-      if (FUNC == 0) {
-        const double rinv = rsqrt(r2);
-        const double f0 = rinv, f1 = -rinv * rinv * rinv;
-        const double qj = sq[s].x;
-        a[0] += f0 * qj;
-        a[1] += f1 * qj * x;
-        a[2] += f1 * qj * y;
-        a[3] += f1 * qj * z;
-      } else if (FUNC == 1) {
-        const double f0 = pow(r2, 0.5 * alpha), f1 = alpha * f0 / r2;
-        const double qj = sq[s].x;
-        a[0] += f0 * qj;
-        a[1] += f1 * qj * x;
-        a[2] += f1 * qj * y;
-        a[3] += f1 * qj * z;
-      } else {
-        const double r = sqrt(r2);
-        double sn, cs;
-        sincos(k0r * r, &sn, &cs);
-        const double d = exp(-k0i * r) / r;
-        const double er = cs * d, ei = sn * d;
-        const double ikr = -k0i * er - k0r * ei, iki = k0r * er - k0i * ei;
-        const double f1r = (ikr - er / r) / r, f1i = (iki - ei / r) / r;
-        const double qr = sq[s].x, qi = sq[s].y;
-        a[0] += er * qr - ei * qi;
-        ai[0] += er * qi + ei * qr;
-        const double gr = f1r * qr - f1i * qi, gi = f1r * qi + f1i * qr;
-        a[1] += gr * x, a[2] += gr * y, a[3] += gr * z;
-        ai[1] += gi * x, ai[2] += gi * y, ai[3] += gi * z;
+    const int cnt = (int)min((long)kExactBS, last - j0);
+    auto sweep = [&](bool own) {  // own: the target itself may be in the tile
+#pragma unroll 4
+      for (int s = 0; s < cnt; s++) {
+        if (own && j0 + s == i) continue;
+        const double4 S = sp[s];
+        const double x = xi - S.x, y = yi - S.y, z = zi - S.z;
+        exact_pair<FUNC>(A, x, y, z, fma(x, x, fma(y, y, z * z)), S.w, CPLX ? sqi[s] : 0.0, a, ai);
       }
-    }
+    };
+    if (__any_sync(0xffffffffu, i >= j0 && i < j0 + cnt)) sweep(true);
+    else sweep(false);
   }
   if (active) {
+    const long row = (long)blockIdx.y * A.nt + t;
     if (CPLX) {
-      double2 *Vo = reinterpret_cast<double2 *>(V) + 4 * t;
+      double2 *Vo = reinterpret_cast<double2 *>(A.out) + 4 * row;
       for (int m = 0; m < 4; m++) Vo[m] = make_double2(a[m], ai[m]);
     } else {
-      reinterpret_cast<double4 *>(V)[t] = make_double4(a[0], a[1], a[2], a[3]);
+      reinterpret_cast<double4 *>(A.out)[row] = make_double4(a[0], a[1], a[2], a[3]);
     }
   }
+}
+
+// V[i] = sum of the shares' partial sums, in order.
+__global__ void exact_reduce_kernel(const double *__restrict__ part, long m, int shares,
+                                    double *__restrict__ V) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  double v = part[i];
+  for (int s = 1; s < shares; s++) v += part[(long)s * m + i];
+  V[i] = v;
 }
 
 int launch_exact(npme_handle *h, const double *d_q, double *d_V, cudaStream_t s,
@@ -737,17 +774,35 @@ int launch_exact(npme_handle *h, const double *d_q, double *d_V, cudaStream_t s,
     h->launches++;
     return h->uops.exact(h, d_q, d_V, s, d_tidx, nt);
   }
+  // Shares of the sources: about 16 CTAs per SM (two rounds of the 8 that are
+  // resident), so that a few thousand targets fill the chip and the last round
+  // of a larger set is short; at least 1,024 sources each.  Without memory
+  // for the partial sums: one share.
+  const int C = h->complex_kernel ? 2 : 1;
+  long shares = std::min<long>((148L * 16 + blocks - 1) / blocks, (n + 1023) / 1024);
+  shares = std::max<long>(1, shares);
+  if (shares > 1 && handle_buffer(h, (void **)&h->d_part, sizeof(double) * 4 * C * nt * shares))
+    shares = 1;
+  ExactArgs A{h->d_coord, d_q, n, h->p.alpha, h->p.k0_r, h->p.k0_i, d_tidx, nt, 0, d_V};
+  A.share = ((n + shares - 1) / shares + kExactBS - 1) / kExactBS * kExactBS;
+  shares = (n + A.share - 1) / A.share;
+  if (shares > 1) A.out = h->d_part;
   const int f = h->p.funcType;
-  if (f == 0)
-    exact_kernel<0><<<blocks, kExactBS, 0, s>>>(h->d_coord, d_q, n, h->p.alpha, h->p.k0_r,
-                                                 h->p.k0_i, d_tidx, nt, d_V);
-  else if (f == 1)
-    exact_kernel<1><<<blocks, kExactBS, 0, s>>>(h->d_coord, d_q, n, h->p.alpha, h->p.k0_r,
-                                                 h->p.k0_i, d_tidx, nt, d_V);
-  else
-    exact_kernel<2><<<blocks, kExactBS, 0, s>>>(h->d_coord, d_q, n, h->p.alpha, h->p.k0_r,
-                                                 h->p.k0_i, d_tidx, nt, d_V);
+  double diag2 = 0;
+  for (int d = 0; d < 3; d++) diag2 += std::pow(h->bmax[d] - h->bmin[d], 2);
+  const bool near = std::fabs(h->p.k0_r) * std::sqrt(diag2) < kMaxHelmArg;
+  const dim3 grid((unsigned)blocks, (unsigned)shares);
+  if (f == 0) exact_kernel<0><<<grid, kExactBS, 0, s>>>(A);
+  else if (f == 1) exact_kernel<1><<<grid, kExactBS, 0, s>>>(A);
+  else if (near) exact_kernel<2><<<grid, kExactBS, 0, s>>>(A);
+  else exact_kernel<3><<<grid, kExactBS, 0, s>>>(A);
   h->launches++;
+  if (shares > 1) {
+    const long m = nt * 4 * C;
+    exact_reduce_kernel<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(h->d_part, m, (int)shares,
+                                                                    d_V);
+    h->launches++;
+  }
   return NPME_OK;
 }
 

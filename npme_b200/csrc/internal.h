@@ -137,6 +137,7 @@ struct npme_handle {
   double *d_V_exact = nullptr;
   int *d_err = nullptr;          // device error flag
   uint32_t *d_tidx = nullptr;    // target list of the exact subset sum
+  double *d_part = nullptr;      // partial sums of the exact sum's source shares
   size_t dev_bytes = 0;
   std::map<void *, size_t> caps;  // pointer field -> capacity of its buffer
   // kernel-transform construction scratch (kept to reuse across set-ups)
