@@ -36,7 +36,7 @@ struct BatchSys {
   const BrickPoint<float> *bpts;
   const uint32_t *cperm;  // targets: group order -> caller index
   const uint32_t *dperm;  // direct-sum sources: source order -> caller index
-  float *qb, *qc;
+  float *qc;
   const int *brick_list, *brick_start;
   int nb2, nb3;
   float *grid;    // real N1 N2 N3 (real kernels) or complex (Helmholtz)
@@ -82,7 +82,7 @@ __global__ void batch_gather_kernel(const BatchSys *__restrict__ sys,
        u += (long long)gridDim.x * blockDim.x) {
     const int s = find_sys(off, count, u);
     const BatchSys &S = sys[s];
-    gather_body<float, CPLX>(S.q, S.bpts, S.dperm, S.qb, S.qc, (long)(u - off[s]));
+    gather_body<float, CPLX>(S.q, S.dperm, S.qc, (long)(u - off[s]));
   }
 }
 
@@ -90,12 +90,12 @@ template <int P, bool CPLX>
 __global__ void __launch_bounds__(256) batch_spread_kernel(const BatchSys *__restrict__ sys,
                                                            const long long *__restrict__ off,
                                                            int count) {
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const long long u = blockIdx.x;
   const int s = find_sys(off, count, u);
   const BatchSys &S = sys[s];
-  spread_brick_fixed<P, CPLX>(S.brick_list[u - off[s]], S.brick_start, S.bpts, S.qb, S.grid,
-                              S.nb2, S.nb3, S.g1, S.g2, S.g3, reinterpret_cast<int *>(smem_raw));
+  spread_brick<float, P, CPLX>(S.brick_list[u - off[s]], S.brick_start, S.bpts, S.q, S.grid,
+                               S.nb2, S.nb3, S.g1, S.g2, S.g3, smem_raw);
 }
 
 // one warp per spectrum row of one system (units: rows)
@@ -124,7 +124,7 @@ template <int P, bool CPLX>
 __global__ void __launch_bounds__(256) batch_interp_kernel(const BatchSys *__restrict__ sys,
                                                            const long long *__restrict__ off,
                                                            int count) {
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const long long u = blockIdx.x;
   const int s = find_sys(off, count, u);
   const BatchSys &S = sys[s];
@@ -324,7 +324,6 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     S.bpts = (const BrickPoint<float> *)h->d_bpts;
     S.cperm = h->d_cperm;
     S.dperm = h->d_dperm;
-    S.qb = (float *)h->d_qb;
     S.qc = (float *)h->d_qc;
     S.brick_list = h->d_brick_list;
     S.brick_start = h->d_brick_start;
@@ -468,17 +467,17 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     return (unsigned)std::max<long long>(1, std::min<long long>((units + threads - 1) / threads, cap));
   };
 
-  // 1. gather
+  // 1. gather, then 2. direct sums, on the second stream, beside the
+  // reciprocal sums
+  cudaEventRecord(b->ev_fork, s);
+  cudaStreamWaitEvent(b->stream2, b->ev_fork, 0);
   for (auto &kv : gath) {
     Class &c = kv.second;
     const unsigned g = grid_of(c.off.back(), 256, 148 * 16);
-    if (kv.first) batch_gather_kernel<true><<<g, 256, 0, s>>>(D(c), O(c), (int)c.members.size());
-    else batch_gather_kernel<false><<<g, 256, 0, s>>>(D(c), O(c), (int)c.members.size());
+    if (kv.first) batch_gather_kernel<true><<<g, 256, 0, b->stream2>>>(D(c), O(c), (int)c.members.size());
+    else batch_gather_kernel<false><<<g, 256, 0, b->stream2>>>(D(c), O(c), (int)c.members.size());
     b->launches++;
   }
-  // 2. direct sums on the second stream, overlapped with the reciprocal sums
-  cudaEventRecord(b->ev_fork, s);
-  cudaStreamWaitEvent(b->stream2, b->ev_fork, 0);
   for (auto &kv : dir) {
     Class &c = kv.second;
     const npme_handle *h0 = hs[f32[c.members[0]]];
@@ -541,8 +540,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     const int cnt = (int)c.members.size();
 #define NPME_BS(PP, CX)                                                                    \
   {                                                                                        \
-    constexpr int TL = kBrick + PP - 1;                                                    \
-    const size_t smem = 2 * sizeof(int) * TL * TL * TL * (CX ? 2 : 1);                     \
+    const size_t smem = spread_smem<float, PP, CX>();                                      \
     auto kern = batch_spread_kernel<PP, CX>;                                               \
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
     kern<<<(unsigned)nb, 256, smem, s>>>(D(c), O(c), cnt);                                 \

@@ -18,22 +18,18 @@ constexpr int kGroupMinBlocks = NPME_GROUP_MIN_BLOCKS;  // resident CTAs asked o
 #endif
 constexpr int kDirectUnroll = NPME_DIRECT_UNROLL;  // pair-loop unroll factor
 
-// Charges into brick order (spread/interp) and the direct sum's source
-// order (dperm: source slot -> caller index).
+// Charges into the direct sum's source order (dperm: source slot -> caller
+// index) and the bulk precision; the spread reads the caller's charges itself.
 template <typename T, bool CPLX>
 __device__ __forceinline__ void gather_body(const double *__restrict__ q,
-                                            const BrickPoint<T> *__restrict__ bp,
                                             const uint32_t *__restrict__ dperm,
-                                            T *__restrict__ qb, T *__restrict__ qc, long i) {
-  const uint32_t ob = bp[i].orig, oc = dperm[i];
+                                            T *__restrict__ qc, long i) {
+  const long o = dperm[i];
   if (CPLX) {
-    qb[2 * i] = (T)q[2 * (long)ob];
-    qb[2 * i + 1] = (T)q[2 * (long)ob + 1];
-    qc[2 * i] = (T)q[2 * (long)oc];
-    qc[2 * i + 1] = (T)q[2 * (long)oc + 1];
+    qc[2 * i] = (T)q[2 * o];
+    qc[2 * i + 1] = (T)q[2 * o + 1];
   } else {
-    qb[i] = (T)q[ob];
-    qc[i] = (T)q[oc];
+    qc[i] = (T)q[o];
   }
 }
 
@@ -66,9 +62,9 @@ __device__ __forceinline__ int brick_point(int nb, int vw, int lane) {
 template <typename T, int P, bool CPLX>
 __device__ __forceinline__ void spread_brick_body(int brick, const int *__restrict__ brick_start,
                                                   const BrickPoint<T> *__restrict__ bp,
-                                                  const T *__restrict__ q, T *__restrict__ grid,
-                                                  int nb2, int nb3, long N1, long N2, long N3,
-                                                  T *tile) {
+                                                  const double *__restrict__ q,
+                                                  T *__restrict__ grid, int nb2, int nb3, long N1,
+                                                  long N2, long N3, T *tile) {
   constexpr int TL = kBrick + P - 1;
   constexpr int TV = TL * TL * TL;
   constexpr int C = CPLX ? 2 : 1;
@@ -80,8 +76,7 @@ __device__ __forceinline__ void spread_brick_body(int brick, const int *__restri
   for (int vw = threadIdx.x >> 5; vw < nvw; vw += blockDim.x >> 5) {
     const int pi = brick_point(nbp, vw, lane);
     if (pi < 0) continue;
-    const int i = beg + pi;
-    const BrickPoint<T> pt = bp[i];
+    const BrickPoint<T> pt = bp[beg + pi];
     T w1[P], w2[P], w3[P], dummy[P];
     bspline_weights<T, P, false>(pt.u[0], w1, dummy);
     bspline_weights<T, P, false>(pt.u[1], w2, dummy);
@@ -89,7 +84,7 @@ __device__ __forceinline__ void spread_brick_body(int brick, const int *__restri
     const int l1 = (int)(pt.g0 >> 20) - b1 * kBrick;
     const int l2 = (int)((pt.g0 >> 10) & 1023u) - b2 * kBrick;
     const int l3 = (int)(pt.g0 & 1023u) - b3 * kBrick;
-    const T qr = q[C * (long)i], qi = CPLX ? q[2 * (long)i + 1] : T(0);
+    const T qr = (T)q[C * (long)pt.orig], qi = CPLX ? (T)q[2 * (long)pt.orig + 1] : T(0);
 #pragma unroll(kStencilUnroll<P>)
     for (int t1 = 0; t1 < P; t1++) {
 #pragma unroll
@@ -134,7 +129,7 @@ __device__ __forceinline__ void spread_brick_body(int brick, const int *__restri
 template <int P, bool CPLX>
 __device__ __forceinline__ void spread_brick_fixed(int brick, const int *__restrict__ brick_start,
                                                    const BrickPoint<float> *__restrict__ bp,
-                                                   const float *__restrict__ q,
+                                                   const double *__restrict__ q,
                                                    float *__restrict__ grid, int nb2, int nb3,
                                                    long N1, long N2, long N3, int *tile) {
   constexpr int TL = kBrick + P - 1;
@@ -146,7 +141,11 @@ __device__ __forceinline__ void spread_brick_fixed(int brick, const int *__restr
   for (int t = threadIdx.x; t < 2 * TV * C; t += blockDim.x) tile[t] = 0;
   const int beg = brick_start[brick], nbp = brick_start[brick + 1] - beg;
   float m = 0.f;
-  for (int i = threadIdx.x; i < nbp * C; i += blockDim.x) m = fmaxf(m, fabsf(q[C * (long)beg + i]));
+  for (int i = threadIdx.x; i < nbp; i += blockDim.x) {
+    const long o = bp[beg + i].orig;
+    m = fmaxf(m, fabsf((float)q[C * o]));
+    if (CPLX) m = fmaxf(m, fabsf((float)q[2 * o + 1]));
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -166,8 +165,7 @@ __device__ __forceinline__ void spread_brick_fixed(int brick, const int *__restr
   for (int vw = threadIdx.x >> 5; vw < nvw; vw += nw) {
     const int pi = brick_point(nbp, vw, lane);
     if (pi < 0) continue;
-    const int i = beg + pi;
-    const BrickPoint<float> pt = bp[i];
+    const BrickPoint<float> pt = bp[beg + pi];
     float w1[P], w2[P], w3[P], dummy[P];
     bspline_weights<float, P, false>(pt.u[0], w1, dummy);
     bspline_weights<float, P, false>(pt.u[1], w2, dummy);
@@ -175,7 +173,8 @@ __device__ __forceinline__ void spread_brick_fixed(int brick, const int *__restr
     const int l1 = (int)(pt.g0 >> 20) - b1 * kBrick;
     const int l2 = (int)((pt.g0 >> 10) & 1023u) - b2 * kBrick;
     const int l3 = (int)(pt.g0 & 1023u) - b3 * kBrick;
-    const float qr = q[C * (long)i] * S, qi = CPLX ? q[2 * (long)i + 1] * S : 0.f;
+    const float qr = (float)q[C * (long)pt.orig] * S;
+    const float qi = CPLX ? (float)q[2 * (long)pt.orig + 1] * S : 0.f;
 #pragma unroll(kStencilUnroll<P>)
     for (int t1 = 0; t1 < P; t1++) {
 #pragma unroll
@@ -218,6 +217,213 @@ __device__ __forceinline__ void spread_brick_fixed(int brick, const int *__restr
       }
     }
   }
+}
+
+// Spreading without atomics, orders up to 8: the CTA's warp w takes the
+// brick's points whose stencil starts at x = w of the tile, so that all of them
+// touch the tile's planes w .. w + P - 1, and keeps those planes in registers:
+// lane (z, y half) holds P x H sums, H = half of the tile's y range.  A point
+// is one sweep of multiply-adds of its zero-padded weights over these registers
+// (weights of a batch of points computed one point per lane, passed through
+// shared memory).  Most of them multiply zeros (36 of 224 cells per plane are
+// in the stencil at order 6), but they run on the FMA pipes of four schedulers,
+// where the shared-memory atomics queue in one pipe, two per contribution with
+// two wavefronts each (spread_brick_fixed).  At the end the warps add their
+// planes to the shared tile in P steps, each on a plane of its own, and the
+// tile goes to the global grid with atomics.  Sums are in T: two
+// roundings per contribution (q w3, then times w2; the product with w1 is
+// fused), one fewer than with the products of the fixed-point form.
+template <typename T, int P, bool CPLX>
+struct SpreadOwner {
+  static constexpr bool kUse = P <= 8;
+  static constexpr int TL = kBrick + P - 1, H = (TL + 1) / 2;
+  static constexpr int C = CPLX ? 2 : 1;
+  // complex FP64 sums do not fit the registers together: one pass per part
+  static constexpr int CC = (CPLX && sizeof(T) == 4) ? 2 : 1;
+  static constexpr int kBatch = sizeof(T) == 4 ? 32 : 16;  // points per batch
+  static constexpr int kRow = 20, kX = 12;  // padded rows: z and y weights; x weights and q
+  static constexpr size_t kWarpBytes = sizeof(T) * kBatch * (2 * kRow + kX) + sizeof(int) * 64;
+  static constexpr size_t kBytes = kBrick * kWarpBytes + sizeof(T) * C * TL * TL * TL;
+};
+
+template <typename T, int P, bool CPLX>
+__device__ __forceinline__ void spread_brick_owner(int brick, const int *__restrict__ brick_start,
+                                                   const BrickPoint<T> *__restrict__ bp,
+                                                   const double *__restrict__ q,
+                                                   T *__restrict__ grid, int nb2, int nb3, long N1,
+                                                   long N2, long N3, unsigned char *smem) {
+  using S = SpreadOwner<T, P, CPLX>;
+  constexpr int TL = S::TL, TV = TL * TL * TL, H = S::H, C = S::C, CC = S::CC, KB = S::kBatch;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, zl = lane & 15, half = lane >> 4;
+  T *tile = reinterpret_cast<T *>(smem + kBrick * S::kWarpBytes);
+  T *wz = reinterpret_cast<T *>(smem + w * S::kWarpBytes);
+  T *wy = wz + KB * S::kRow, *wx = wy + KB * S::kRow;
+  int *list = reinterpret_cast<int *>(wx + KB * S::kX);
+  const int b3 = brick % nb3, b2 = (brick / nb3) % nb2, b1 = brick / (nb3 * nb2);
+  const int beg = brick_start[brick], nbp = brick_start[brick + 1] - beg;
+  for (int t = threadIdx.x; t < TV * C; t += blockDim.x) tile[t] = T(0);
+  for (int pass = 0; pass < C / CC; pass++) {
+    T acc[CC][P][H];
+#pragma unroll
+    for (int c = 0; c < CC; c++)
+#pragma unroll
+      for (int x = 0; x < P; x++)
+#pragma unroll
+        for (int h = 0; h < H; h++) acc[c][x][h] = T(0);
+    auto batch = [&](int n) {  // points list[0 .. n) into the sums
+      if (lane < n) {
+        const BrickPoint<T> pt = bp[beg + list[lane]];
+        T a[P], dummy[P];
+        T *rz = wz + lane * S::kRow, *ry = wy + lane * S::kRow, *rx = wx + lane * S::kX;
+        using V4 = typename Vec4<T>::type;
+        V4 zero;
+        zero.x = zero.y = zero.z = zero.w = T(0);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          reinterpret_cast<V4 *>(rz)[i] = zero, reinterpret_cast<V4 *>(ry)[i] = zero;
+        const long o = pt.orig;
+        T qz = T(1);
+        if (CC == 2) {
+          rx[8] = (T)q[2 * o], rx[9] = (T)q[2 * o + 1];
+        } else {
+          qz = (T)q[C * o + pass];
+        }
+        bspline_weights<T, P, false>(pt.u[2], a, dummy);
+        const int l3 = (int)(pt.g0 & 1023u) - b3 * kBrick;
+#pragma unroll
+        for (int t = 0; t < P; t++) rz[l3 + t] = CC == 2 ? a[t] : qz * a[t];
+        bspline_weights<T, P, false>(pt.u[1], a, dummy);
+        const int l2 = (int)((pt.g0 >> 10) & 1023u) - b2 * kBrick;
+#pragma unroll
+        for (int t = 0; t < P; t++) {
+          const int y = l2 + t;
+          ry[y < H ? y : 8 + y - H] = a[t];
+        }
+        bspline_weights<T, P, false>(pt.u[0], a, dummy);
+#pragma unroll
+        for (int t = 0; t < P; t++) rx[t] = a[t];
+      }
+      __syncwarp();
+#pragma unroll 1
+      for (int p = 0; p < n; p++) {
+        using V4 = typename Vec4<T>::type;
+        const T z = wz[p * S::kRow + zl];
+        T y[8], x[8];
+        const V4 *vy = reinterpret_cast<const V4 *>(wy + p * S::kRow + 8 * half);
+        const V4 *vx = reinterpret_cast<const V4 *>(wx + p * S::kX);
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const V4 ay = vy[i], ax = vx[i];
+          y[4 * i] = ay.x, y[4 * i + 1] = ay.y, y[4 * i + 2] = ay.z, y[4 * i + 3] = ay.w;
+          x[4 * i] = ax.x, x[4 * i + 1] = ax.y, x[4 * i + 2] = ax.z, x[4 * i + 3] = ax.w;
+        }
+#pragma unroll
+        for (int c = 0; c < CC; c++) {
+          const T s = CC == 2 ? z * wx[p * S::kX + 8 + c] : z;
+#pragma unroll
+          for (int h = 0; h < H; h++) {
+            const T v = s * y[h];
+#pragma unroll
+            for (int i = 0; i < P; i++) acc[c][i][h] = fma(x[i], v, acc[c][i][h]);
+          }
+        }
+      }
+      __syncwarp();
+    };
+    // the warp's points, in batches
+    int cnt = 0;
+    for (int c0 = 0; c0 < nbp; c0 += 32) {
+      const int i = c0 + lane;
+      const bool mine = i < nbp && (int)(bp[beg + i].g0 >> 20) - b1 * kBrick == w;
+      const unsigned m = __ballot_sync(FULL, mine);
+      if (mine) list[cnt + __popc(m & ((1u << lane) - 1u))] = i;
+      cnt += __popc(m);
+      __syncwarp();
+      while (cnt >= KB) {
+        batch(KB);
+        const int rest = cnt - KB, next = lane < rest ? list[KB + lane] : 0;
+        __syncwarp();
+        if (lane < rest) list[lane] = next;
+        __syncwarp();
+        cnt = rest;
+      }
+    }
+    if (cnt > 0) batch(cnt);
+    // planes w + s of all warps are different ones in every step s
+#pragma unroll
+    for (int s = 0; s < P; s++) {
+      __syncthreads();
+#pragma unroll
+      for (int h = 0; h < H; h++) {
+        const int y = half * H + h;
+        if (y < TL && zl < TL) {
+          T *d = tile + C * (((w + s) * TL + y) * TL + zl) + pass;
+#pragma unroll
+          for (int c = 0; c < CC; c++) d[c] += acc[c][s][h];
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // the tile's rows to the grid, FP32 in pieces of 16 bytes: one vector atomic
+  // each (the atomic units count requests, and with 4 to 7 tile values per grid
+  // point they, not the sums, would be the bound).  A row starts at a multiple
+  // of 8 values; rows of the grid that are not 16-byte aligned, and pieces past
+  // the end of a row, go value by value.
+  constexpr int kPiece = sizeof(T) == 4 ? 4 / C : 1;  // grid points per piece
+  constexpr int kPieces = (TL + kPiece - 1) / kPiece;
+  const long g1 = (long)b1 * kBrick, g2 = (long)b2 * kBrick, g3 = (long)b3 * kBrick;
+  const bool aligned = (N3 * C) % 4 == 0;
+  for (int t = threadIdx.x; t < TL * TL * kPieces; t += blockDim.x) {
+    const int row = t / kPieces, i3 = (t - row * kPieces) * kPiece;
+    const int i1 = row / TL, i2 = row - i1 * TL;
+    if (g1 + i1 >= N1 || g2 + i2 >= N2) continue;  // always zero there
+    T *d = grid + C * (((g1 + i1) * N2 + (g2 + i2)) * N3 + (g3 + i3));
+    T v[kPiece * C];
+    bool any = false;
+#pragma unroll
+    for (int m = 0; m < kPiece * C; m++) {
+      v[m] = i3 + m / C < TL ? tile[C * (row * TL + i3) + m] : T(0);
+      any |= v[m] != T(0);
+    }
+    if (!any) continue;
+    if constexpr (sizeof(T) == 4) {
+      if (aligned && g3 + i3 + kPiece <= N3) {
+        atomicAdd(reinterpret_cast<float4 *>(d), make_float4(v[0], v[1], v[2], v[3]));
+        continue;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < kPiece * C; m++)
+      if (v[m] != T(0) && g3 + i3 + m / C < N3) atomicAdd(d + m, v[m]);
+  }
+}
+
+// The spread body of an order and precision, and its shared memory.
+template <typename T, int P, bool CPLX>
+__device__ __forceinline__ void spread_brick(int brick, const int *__restrict__ brick_start,
+                                             const BrickPoint<T> *__restrict__ bp,
+                                             const double *__restrict__ q, T *__restrict__ grid,
+                                             int nb2, int nb3, long N1, long N2, long N3,
+                                             unsigned char *smem) {
+  if constexpr (SpreadOwner<T, P, CPLX>::kUse)
+    spread_brick_owner<T, P, CPLX>(brick, brick_start, bp, q, grid, nb2, nb3, N1, N2, N3, smem);
+  else if constexpr (std::is_same<T, float>::value)
+    spread_brick_fixed<P, CPLX>(brick, brick_start, bp, q, grid, nb2, nb3, N1, N2, N3,
+                                reinterpret_cast<int *>(smem));
+  else
+    spread_brick_body<T, P, CPLX>(brick, brick_start, bp, q, grid, nb2, nb3, N1, N2, N3,
+                                  reinterpret_cast<T *>(smem));
+}
+
+template <typename T, int P, bool CPLX>
+constexpr size_t spread_smem() {
+  constexpr int TL = kBrick + P - 1;
+  // fixed point: two int words per tile value; FP64: one double
+  return SpreadOwner<T, P, CPLX>::kUse
+             ? SpreadOwner<T, P, CPLX>::kBytes
+             : (sizeof(T) == 4 ? 8 : sizeof(T)) * TL * TL * TL * (CPLX ? 2 : 1);
 }
 
 // X(k) *= G(|k1|, |k2|, k3) on the R2C half spectrum (src/RecSumV.cpp:639-707),

@@ -126,7 +126,6 @@ struct npme_handle {
   int *d_brick_start = nullptr;  // [n_bricks + 1]
   int *d_brick_list = nullptr;   // non-empty brick ids
   uint32_t *d_cperm = nullptr;   // group order (direct-sum targets) -> caller index
-  void *d_qb = nullptr;          // charges in brick order (T or T2)
   void *d_qc = nullptr;          // charges in the direct sum's source order (T or T2)
   void *d_grid = nullptr;        // spread grid, real N1 N2 N3 (or complex)
   void *d_kgrid = nullptr;       // transformed grid N1 N2 (N3/2+1) complex (real kernels)
@@ -268,8 +267,7 @@ int build_kernel_transform(npme_handle *h);  // F-hat, lambda^2 -> d_G
 // a built-in kernel (real, complex), the rest one by one on their own
 // streams.  status[k] gets each handle's result.
 void build_kernel_transforms(npme_handle **hs, int R, npme_handle *owner, int *status);
-void launch_gather_charges(npme_handle *h, const double *d_q, cudaStream_t s);
-void launch_spread(npme_handle *h, cudaStream_t s);
+void launch_spread(npme_handle *h, const double *d_q, cudaStream_t s);
 void launch_multiply(npme_handle *h, cudaStream_t s);
 void launch_interp(npme_handle *h, double *d_V, cudaStream_t s);
 

@@ -624,17 +624,21 @@ static void tmark(npme_handle *h, int i, cudaStream_t s) {
 static int enqueue_calcv(npme_handle *h, double *d_V, const double *d_charge, cudaStream_t s) {
   h->launches = 0;
   tmark(h, 0, s);
-  npme::launch_gather_charges(h, d_charge, s);
-  CK(cudaGetLastError());  // launch errors are checked before cuFFT runs
-  tmark(h, 1, s);
-  // the direct sum runs on stream2 beside the reciprocal sum; in the serial
-  // timing mode it starts after the reciprocal chain, so that each stage's
-  // events time that stage alone
+  // the direct sum, with the gather of its charges, runs on stream2 beside the
+  // reciprocal sum, which reads the caller's charges itself; in the serial
+  // timing mode the gather comes first and the direct sum after the reciprocal
+  // chain, so that each stage's events time that stage alone
   const bool serial = h->timing.enabled && h->timing.serial;
+  if (h->timing.enabled) {
+    npme::launch_gather_direct(h, d_charge, h->d_qc, s);
+    CK(cudaGetLastError());
+  }
+  tmark(h, 1, s);
   h->merge_pending = false;
   auto fork_direct = [&]() -> int {
     CK(cudaEventRecord(h->ev_fork, s));
     CK(cudaStreamWaitEvent(h->stream2, h->ev_fork, 0));
+    if (!h->timing.enabled) npme::launch_gather_direct(h, d_charge, h->d_qc, h->stream2);
     tmark(h, 8, h->stream2);
     if (npme::launch_direct(h, d_charge, d_V, h->stream2))
       return fail(h, NPME_ECUDA, "direct-sum launch of the caller-defined kernel failed");
@@ -646,7 +650,7 @@ static int enqueue_calcv(npme_handle *h, double *d_V, const double *d_charge, cu
   int frc;
   if (!serial && (frc = fork_direct())) return frc;
   if (npme::grid_clear(h, s)) return fail(h, NPME_ECUDA, "clearing the spread grid failed");
-  npme::launch_spread(h, s);
+  npme::launch_spread(h, d_charge, s);
   CK(cudaGetLastError());
   tmark(h, 2, s);
   if (h->own_fft) {

@@ -817,58 +817,15 @@ void build_kernel_transforms(npme_handle **hs, int R, npme_handle *owner, int *s
 }
 
 // ---------------------------------------------------------------------------
-// Per-call charge gather into brick order (spread/interp) and the direct
-// sum's source order, converted to the bulk precision.
+// Per-call charge gather into the direct sum's source order, converted to the
+// bulk precision.
 
 template <typename T, bool CPLX>
-__global__ void gather_kernel(const double *__restrict__ q, const BrickPoint<T> *__restrict__ bp,
-                              const uint32_t *__restrict__ dperm, T *__restrict__ qb,
+__global__ void gather_kernel(const double *__restrict__ q, const uint32_t *__restrict__ dperm,
                               T *__restrict__ qc, long n) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
        i += (long)gridDim.x * blockDim.x)
-    gather_body<T, CPLX>(q, bp, dperm, qb, qc, i);
-}
-
-void launch_gather_charges(npme_handle *h, const double *d_q, cudaStream_t s) {
-  const int threads = 256;
-  const int blocks = (int)std::min<long>((h->n + threads - 1) / threads, 148 * 16);
-  if (h->fp32) {
-    if (h->complex_kernel)
-      gather_kernel<float, true><<<blocks, threads, 0, s>>>(
-          d_q, (const BrickPoint<float> *)h->d_bpts, h->d_dperm, (float *)h->d_qb,
-          (float *)h->d_qc, (long)h->n);
-    else
-      gather_kernel<float, false><<<blocks, threads, 0, s>>>(
-          d_q, (const BrickPoint<float> *)h->d_bpts, h->d_dperm, (float *)h->d_qb,
-          (float *)h->d_qc, (long)h->n);
-  } else {
-    if (h->complex_kernel)
-      gather_kernel<double, true><<<blocks, threads, 0, s>>>(
-          d_q, (const BrickPoint<double> *)h->d_bpts, h->d_dperm, (double *)h->d_qb,
-          (double *)h->d_qc, (long)h->n);
-    else
-      gather_kernel<double, false><<<blocks, threads, 0, s>>>(
-          d_q, (const BrickPoint<double> *)h->d_bpts, h->d_dperm, (double *)h->d_qb,
-          (double *)h->d_qc, (long)h->n);
-  }
-  h->launches++;
-}
-
-// Charges into the direct-sum order only (the bare short-range sum).
-template <typename T, bool CPLX>
-__global__ void gather_one_kernel(const double *__restrict__ q,
-                                  const uint32_t *__restrict__ perm, T *__restrict__ dst,
-                                  long n) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
-       i += (long)gridDim.x * blockDim.x) {
-    const long o = perm[i];
-    if (CPLX) {
-      dst[2 * i] = (T)q[2 * o];
-      dst[2 * i + 1] = (T)q[2 * o + 1];
-    } else {
-      dst[i] = (T)q[o];
-    }
-  }
+    gather_body<T, CPLX>(q, dperm, qc, i);
 }
 
 void launch_gather_direct(npme_handle *h, const double *d_q, void *d_qdst, cudaStream_t s) {
@@ -877,14 +834,14 @@ void launch_gather_direct(npme_handle *h, const double *d_q, void *d_qdst, cudaS
   const long n = (long)h->n;
   if (h->fp32) {
     if (h->complex_kernel)
-      gather_one_kernel<float, true><<<blocks, threads, 0, s>>>(d_q, h->d_dperm, (float *)d_qdst, n);
+      gather_kernel<float, true><<<blocks, threads, 0, s>>>(d_q, h->d_dperm, (float *)d_qdst, n);
     else
-      gather_one_kernel<float, false><<<blocks, threads, 0, s>>>(d_q, h->d_dperm, (float *)d_qdst, n);
+      gather_kernel<float, false><<<blocks, threads, 0, s>>>(d_q, h->d_dperm, (float *)d_qdst, n);
   } else {
     if (h->complex_kernel)
-      gather_one_kernel<double, true><<<blocks, threads, 0, s>>>(d_q, h->d_dperm, (double *)d_qdst, n);
+      gather_kernel<double, true><<<blocks, threads, 0, s>>>(d_q, h->d_dperm, (double *)d_qdst, n);
     else
-      gather_one_kernel<double, false><<<blocks, threads, 0, s>>>(d_q, h->d_dperm, (double *)d_qdst, n);
+      gather_kernel<double, false><<<blocks, threads, 0, s>>>(d_q, h->d_dperm, (double *)d_qdst, n);
   }
   h->launches++;
 }
@@ -904,51 +861,45 @@ void launch_gather_direct(npme_handle *h, const double *d_q, void *d_qdst, cudaS
 template <typename T, int P, bool CPLX>
 __global__ void __launch_bounds__(256) spread_kernel(
     const int *__restrict__ brick_list, const int *__restrict__ brick_start,
-    const BrickPoint<T> *__restrict__ bp, const T *__restrict__ q, T *__restrict__ grid,
+    const BrickPoint<T> *__restrict__ bp, const double *__restrict__ q, T *__restrict__ grid,
     int nb2, int nb3, long N1, long N2, long N3) {
-  extern __shared__ unsigned char smem_raw[];
-  if constexpr (std::is_same<T, float>::value)
-    spread_brick_fixed<P, CPLX>(brick_list[blockIdx.x], brick_start, bp, q, grid, nb2, nb3, N1,
-                                N2, N3, reinterpret_cast<int *>(smem_raw));
-  else
-    spread_brick_body<T, P, CPLX>(brick_list[blockIdx.x], brick_start, bp, q, grid, nb2, nb3, N1,
-                                  N2, N3, reinterpret_cast<T *>(smem_raw));
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  spread_brick<T, P, CPLX>(brick_list[blockIdx.x], brick_start, bp, q, grid, nb2, nb3, N1, N2, N3,
+                           smem_raw);
 }
 
 template <typename T, bool CPLX, int P>
-static void spread_dispatch(npme_handle *h, cudaStream_t s) {
-  constexpr int TL = kBrick + P - 1;
-  // FP32: two int words per tile value; FP64: one double
-  const size_t smem = (sizeof(T) == 4 ? 8 : sizeof(T)) * TL * TL * TL * (CPLX ? 2 : 1);
+static void spread_dispatch(npme_handle *h, const double *d_q, cudaStream_t s) {
+  const size_t smem = spread_smem<T, P, CPLX>();
   auto kern = spread_kernel<T, P, CPLX>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   kern<<<(unsigned)h->n_nonempty, 256, smem, s>>>(
       h->d_brick_list, h->d_brick_start, (const BrickPoint<T> *)h->d_bpts,
-      (const T *)h->d_qb, (T *)h->d_grid, (int)h->grid.nb[1], (int)h->grid.nb[2], h->gd[0],
+      d_q, (T *)h->d_grid, (int)h->grid.nb[1], (int)h->grid.nb[2], h->gd[0],
       h->gd[1], h->gd[2]);
 }
 
 template <typename T, bool CPLX>
-static void spread_order(npme_handle *h, cudaStream_t s) {
+static void spread_order(npme_handle *h, const double *d_q, cudaStream_t s) {
   switch (h->grid.order) {
-    case 4: spread_dispatch<T, CPLX, 4>(h, s); break;
-    case 6: spread_dispatch<T, CPLX, 6>(h, s); break;
-    case 8: spread_dispatch<T, CPLX, 8>(h, s); break;
-    case 10: spread_dispatch<T, CPLX, 10>(h, s); break;
-    case 12: spread_dispatch<T, CPLX, 12>(h, s); break;
-    case 14: spread_dispatch<T, CPLX, 14>(h, s); break;
-    case 16: spread_dispatch<T, CPLX, 16>(h, s); break;
+    case 4: spread_dispatch<T, CPLX, 4>(h, d_q, s); break;
+    case 6: spread_dispatch<T, CPLX, 6>(h, d_q, s); break;
+    case 8: spread_dispatch<T, CPLX, 8>(h, d_q, s); break;
+    case 10: spread_dispatch<T, CPLX, 10>(h, d_q, s); break;
+    case 12: spread_dispatch<T, CPLX, 12>(h, d_q, s); break;
+    case 14: spread_dispatch<T, CPLX, 14>(h, d_q, s); break;
+    case 16: spread_dispatch<T, CPLX, 16>(h, d_q, s); break;
   }
 }
 
-void launch_spread(npme_handle *h, cudaStream_t s) {
+void launch_spread(npme_handle *h, const double *d_q, cudaStream_t s) {
   if (h->n_nonempty == 0) return;
   if (h->fp32) {
-    if (h->complex_kernel) spread_order<float, true>(h, s);
-    else spread_order<float, false>(h, s);
+    if (h->complex_kernel) spread_order<float, true>(h, d_q, s);
+    else spread_order<float, false>(h, d_q, s);
   } else {
-    if (h->complex_kernel) spread_order<double, true>(h, s);
-    else spread_order<double, false>(h, s);
+    if (h->complex_kernel) spread_order<double, true>(h, d_q, s);
+    else spread_order<double, false>(h, d_q, s);
   }
   h->launches++;
 }
@@ -1020,7 +971,7 @@ __global__ void __launch_bounds__(256) interp_kernel(
     const BrickPoint<T> *__restrict__ bp, const T *__restrict__ theta, double *__restrict__ V,
     int nb2, int nb3, long N1, long N2, long N3, T c1, T c2, T c3, void *vsrc, double vs,
     double gs) {
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   interp_brick_body<T, P, CPLX>(brick_list[blockIdx.x], brick_start, bp, theta, V, nb2, nb3, N1,
                                 N2, N3, c1, c2, c3, reinterpret_cast<T *>(smem_raw), vsrc, vs,
                                 gs);

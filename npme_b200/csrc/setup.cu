@@ -771,7 +771,6 @@ int describe(npme_handle *h, SysDesc &D) {
       (rc = handle_buffer(h, (void **)&h->d_gcen, sizeof(double4) * D.ngb)) ||
       (rc = handle_buffer(h, (void **)&h->d_hgroups, sizeof(int4) * D.ngb)) ||
       (rc = handle_buffer(h, (void **)&h->d_hcen, sizeof(double4) * D.ngb)) ||
-      (rc = handle_buffer(h, &h->d_qb, sizeof(T) * C * n)) ||
       (rc = handle_buffer(h, &h->d_qc, sizeof(T) * C * n)) ||
       (rc = handle_buffer(h, (void **)&h->d_q_in, sizeof(double) * C * n)) ||
       (rc = handle_buffer(h, (void **)&h->d_V, sizeof(double) * 4 * C * n)))
