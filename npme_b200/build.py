@@ -17,12 +17,13 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libnpme_gpu.so")
-SOURCES = ["npme_gpu.cu", "setup.cu", "recsum.cu", "direct.cu", "noalloc.cu", "batch.cu", "fft.cu", "fftk.cu",
+SOURCES = ["npme_gpu.cu", "setup.cu", "recsum.cu", "direct.cu", "noalloc.cu", "batch.cu", "batch_direct.cu",
+           "fft.cu", "fftk.cu",
            "server.cu", "choose.cu"]
 APPS = os.path.join(HERE, "apps")
 BIN = os.path.join(HERE, "bin")
 APPS_SRC = ["npme", "compareV", "makeRandomBox"]
-HEADERS = ["common.cuh", "bodies.cuh", "internal.h", "fft_own.cuh",
+HEADERS = ["common.cuh", "bodies.cuh", "internal.h", "fft_own.cuh", "batch.cuh",
            os.path.join("..", "..", "include", "npme_gpu.h")]
 
 

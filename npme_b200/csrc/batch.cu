@@ -25,54 +25,11 @@
 #include <tuple>
 #include <vector>
 
+#include "batch.cuh"
 #include "bodies.cuh"
 #include "internal.h"
 
 namespace npme {
-
-struct BatchSys {
-  const double *q;  // caller charges (device)
-  double *V;        // caller output (device)
-  const BrickPoint<float> *bpts;
-  const uint32_t *cperm;  // targets: group order -> caller index
-  const uint32_t *dperm;  // direct-sum sources: source order -> caller index
-  float *qc;
-  const int *brick_list, *brick_start;
-  int nb2, nb3;
-  float *grid;    // real N1 N2 N3 (real kernels) or complex (Helmholtz)
-  float2 *kgrid;  // R2C half spectrum (real kernels)
-  const float *G;
-  long N1, N2, N3;  // FFT box
-  long g1, g2, g3;  // dimensions the grid is stored with
-  float c1, c2, c3;
-  const double4 *gpos, *spos;
-  const int4 *groups;
-  const double4 *gcen;
-  const int2 *segs;
-  // pair-once walk: half-shell groups and segments, source-side sums
-  const int4 *hgroups;
-  const double4 *hcen;
-  const int2 *hsegs;
-  float4 *vsrc;            // source-side sums, slot = brick-order position
-  const uint32_t *bperm;   // brick-order position -> caller index
-  float refine2;
-  double fself_r, fself_i;
-  // pair-once systems: the interpolation adds the source-side sums into V
-  // (potential times vs, gradient times gs) and clears them
-  int fold;
-  double vs, gs;
-};
-
-__device__ __forceinline__ int find_sys(const long long *__restrict__ off, int count,
-                                        long long u) {
-  int lo = 0, hi = count - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (off[mid] <= u) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
 
 template <bool CPLX>
 __global__ void batch_gather_kernel(const BatchSys *__restrict__ sys,
@@ -84,6 +41,21 @@ __global__ void batch_gather_kernel(const BatchSys *__restrict__ sys,
     const BatchSys &S = sys[s];
     gather_body<float, CPLX>(S.q, S.dperm, S.qc, (long)(u - off[s]));
   }
+}
+
+// Zeroes the spread grids of a spread class; CTAs of kClearFloats floats each,
+// off: prefix sums of the systems' CTAs.
+constexpr long kClearFloats = 16384;
+template <bool CPLX>
+__global__ void __launch_bounds__(256) batch_clear_kernel(const BatchSys *__restrict__ sys,
+                                                          const long long *__restrict__ off,
+                                                          int count) {
+  const int s = find_sys(off, count, blockIdx.x);
+  const BatchSys &S = sys[s];
+  const long n = (CPLX ? 2 : 1) * S.g1 * S.g2 * S.g3;  // even: so are the dimensions
+  const long a = (blockIdx.x - off[s]) * kClearFloats, b = min(n, a + kClearFloats);
+  for (long i = a + 2 * threadIdx.x; i < b; i += 512)
+    *reinterpret_cast<float2 *>(S.grid + i) = make_float2(0.f, 0.f);
 }
 
 template <int P, bool CPLX>
@@ -134,50 +106,6 @@ __global__ void __launch_bounds__(256) batch_interp_kernel(const BatchSys *__res
                                     S.fold ? (void *)S.vsrc : nullptr, S.vs, S.gs);
 }
 
-template <bool CPLX, int FUNC, int SPLIT, int ND>
-__global__ void __launch_bounds__(32 * kGroupWarps, kGroupMinBlocks) batch_direct_kernel(
-    PairCoef<float> k, const BatchSys *__restrict__ sys, const long long *__restrict__ off,
-    int count) {
-  __shared__ float4 sp[kGroupWarps][32];
-  __shared__ float4 slo[kGroupWarps][32];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long u = (long long)blockIdx.x * kGroupWarps + wid;
-  if (u >= off[count]) return;  // warp-uniform
-  const int s = find_sys(off, count, u);
-  const BatchSys &S = sys[s];
-  const long g = (long)(u - off[s]);
-  direct_group_body<CPLX, FUNC, SPLIT, ND>(k, S.gpos, S.spos, S.qc, S.q, S.groups[g], S.gcen[g],
-                                           S.segs, S.cperm, S.refine2, S.fself_r, S.fself_i, S.V,
-                                           sp[wid], slo[wid], lane);
-}
-
-// Pair-once direct sums of a batch: KIND 0 the packed real body
-// (direct_group_sym), 1 Helmholtz DM.
-template <int KIND, int FUNC, int ND>
-__global__ void __launch_bounds__(32 * kGroupWarps) batch_sym_kernel(
-    PairCoef<float> k, const BatchSys *__restrict__ sys, const long long *__restrict__ off,
-    int count) {
-  __shared__ float4 ta[kGroupWarps][32];
-  __shared__ float4 tb[kGroupWarps][32];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long u = (long long)blockIdx.x * kGroupWarps + wid;
-  if (u >= off[count]) return;  // warp-uniform
-  const int s = find_sys(off, count, u);
-  const BatchSys &S = sys[s];
-  const long g = (long)(u - off[s]);
-  if constexpr (KIND == 0) {
-    double acc[4] = {0, 0, 0, 0};
-    const int4 G = S.hgroups[g];
-    direct_group_sym<FUNC, ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.cperm,
-                               S.refine2, S.vsrc, ta[wid], tb[wid], lane, 0, 1, acc);
-    sym_store(k, G, S.cperm, S.q, S.fself_r, S.V, lane, acc);
-  } else {
-    direct_group_sym_helm<ND>(k, S.gpos, S.spos, S.qc, S.q, S.hgroups[g], S.hcen[g], S.hsegs,
-                              S.cperm, S.refine2, S.fself_r, S.fself_i, S.V, S.vsrc, ta[wid],
-                              tb[wid], lane);
-  }
-}
-
 }  // namespace npme
 
 using npme::BatchSys;
@@ -185,6 +113,10 @@ using npme::BatchSys;
 struct npme_batch {
   int device = 0;
   cudaStream_t stream2 = nullptr;
+  // the direct-sum classes beyond the first run beside it
+  static constexpr int kSide = 3;
+  cudaStream_t side[kSide] = {};
+  cudaEvent_t ev_side[kSide] = {}, ev_gather = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_done = nullptr;
   bool pending = false;  // ev_done recorded: buffers and members may be in use
   unsigned char *h_pinned = nullptr;  // host image of the descriptor block
@@ -232,11 +164,16 @@ int npme_gpu_batch_create(int device, npme_batch **out) {
   b->device = device;
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking);
+  for (int i = 0; i < npme_batch::kSide && e == cudaSuccess; i++) {
+    e = cudaStreamCreateWithFlags(&b->side[i], cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_side[i], cudaEventDisableTiming);
+  }
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_gather, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming);
   if (e != cudaSuccess) {
-    delete b;
+    npme_gpu_batch_destroy(b);
     return NPME_ECUDA;
   }
   *out = b;
@@ -249,6 +186,11 @@ int npme_gpu_batch_destroy(npme_batch *b) {
   if (b->pending) cudaEventSynchronize(b->ev_done);
   if (b->stream2) cudaStreamSynchronize(b->stream2);
   if (b->stream2) cudaStreamDestroy(b->stream2);
+  for (int i = 0; i < npme_batch::kSide; i++) {
+    if (b->side[i]) cudaStreamDestroy(b->side[i]);
+    if (b->ev_side[i]) cudaEventDestroy(b->ev_side[i]);
+  }
+  if (b->ev_gather) cudaEventDestroy(b->ev_gather);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
   if (b->ev_join) cudaEventDestroy(b->ev_join);
   if (b->ev_done) cudaEventDestroy(b->ev_done);
@@ -359,6 +301,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   }
 
   // launch classes
+  std::map<int, Class> clr;  // key: complex (members with the library's transforms)
   std::map<int, Class> gath, mult;                           // key: complex (mult: cuFFT members)
   std::map<int, FftClass> own;                               // key: complex
   std::map<std::pair<int, int>, Class> spr;                  // (order, complex)
@@ -368,7 +311,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     const npme_handle *h = hs[f32[k]];
     const int cx = h->complex_kernel ? 1 : 0;
     gath[cx].members.push_back(k);
-    if (h->own_fft) own[cx].members.push_back(k);
+    if (h->own_fft) own[cx].members.push_back(k), clr[cx].members.push_back(k);
     else mult[cx].members.push_back(k);
     spr[{h->grid.order, cx}].members.push_back(k);
     const DKey key(pairs_once(h) ? 1 : 0, h->p.funcType, h->p.EwaldSplit, h->p.nDeriv,
@@ -380,6 +323,11 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   auto units_mult = [&](int k) {  // spectrum rows
     const long *N = hs[f32[k]]->grid.N;
     return (long long)N[0] * N[1];
+  };
+  auto units_clear = [&](int k) {
+    const npme_handle *h = hs[f32[k]];
+    const long n = (h->complex_kernel ? 2 : 1) * h->gd[0] * h->gd[1] * h->gd[2];
+    return (long long)((n + kClearFloats - 1) / kClearFloats);
   };
   auto units_dir = [&](int k) {
     const npme_handle *h = hs[f32[k]];
@@ -399,6 +347,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     all.push_back(&c);
   };
   for (auto &kv : gath) lay(kv.second, units_gather);
+  for (auto &kv : clr) lay(kv.second, units_clear);
   for (auto &kv : mult) lay(kv.second, units_mult);
   for (auto &kv : spr) lay(kv.second, units_spread);  // spread and interpolation: bricks
   for (auto &kv : dir) lay(kv.second, units_dir);
@@ -478,59 +427,42 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     else batch_gather_kernel<false><<<g, 256, 0, b->stream2>>>(D(c), O(c), (int)c.members.size());
     b->launches++;
   }
+  cudaEventRecord(b->ev_gather, b->stream2);
+  int nclass = 0;  // direct-sum launches so far
   for (auto &kv : dir) {
     Class &c = kv.second;
     const npme_handle *h0 = hs[f32[c.members[0]]];
     const PairCoef<float> k = make_pair_coef<float>(h0);
     const long long ng = c.off.back();
     if (ng == 0) continue;
-    const unsigned g = (unsigned)((ng + kGroupWarps - 1) / kGroupWarps);
-    const int cnt = (int)c.members.size();
-    const int f = h0->p.funcType, sp = h0->p.EwaldSplit;
-    // fixed-order instances: see dm_eval2 for alpha
-    const int nd = sp == 1 || (f == NPME_FUNC_RALPHA && h0->p.alpha >= 0) ? 0 : h0->p.nDeriv;
-    if (std::get<0>(kv.first)) {  // pair-once walk, then the source-side sums
-#define NPME_BSYM(KD, FN, ND) \
-  batch_sym_kernel<KD, FN, ND><<<g, 32 * kGroupWarps, 0, b->stream2>>>(k, D(c), O(c), cnt)
-#define NPME_BSYM_ND(KD, FN)                \
-  switch (nd) {                             \
-    case 3: NPME_BSYM(KD, FN, 3); break;    \
-    case 6: NPME_BSYM(KD, FN, 6); break;    \
-    case 8: NPME_BSYM(KD, FN, 8); break;    \
-    default: NPME_BSYM(KD, FN, 0); break;   \
-  }
-      if (f == NPME_FUNC_HELMHOLTZ) { NPME_BSYM_ND(1, 2); }
-      else if (sp == NPME_SPLIT_LAPLACE_ORIG) { NPME_BSYM(0, 2, 0); }
-      else if (f == NPME_FUNC_RALPHA) { NPME_BSYM_ND(0, 1); }
-      else { NPME_BSYM_ND(0, 0); }
-#undef NPME_BSYM_ND
-#undef NPME_BSYM
-      // the source-side sums are folded into V by the interpolation below
-      b->launches++;
-      continue;
+    // classes beyond the first on streams of their own: a class has its own
+    // tail of late CTAs, which the others fill
+    cudaStream_t ds = b->stream2;
+    if (nclass > 0) {
+      const int i = (nclass - 1) % npme_batch::kSide;
+      ds = b->side[i];
+      if (nclass <= npme_batch::kSide) cudaStreamWaitEvent(ds, b->ev_gather, 0);
     }
-#define NPME_BD(CX, FN, SL, ND) \
-  batch_direct_kernel<CX, FN, SL, ND><<<g, 32 * kGroupWarps, 0, b->stream2>>>(k, D(c), O(c), cnt)
-#define NPME_BD_ND(CX, FN, SL)               \
-  switch (nd) {                              \
-    case 3: NPME_BD(CX, FN, SL, 3); break;   \
-    case 6: NPME_BD(CX, FN, SL, 6); break;   \
-    case 8: NPME_BD(CX, FN, SL, 8); break;   \
-    default: NPME_BD(CX, FN, SL, 0); break;  \
-  }
-    if (f == NPME_FUNC_HELMHOLTZ) { NPME_BD_ND(true, 2, 0); }
-    else if (sp == NPME_SPLIT_LAPLACE_ORIG) { NPME_BD(false, 0, 1, 0); }
-    else if (f == NPME_FUNC_RALPHA) { NPME_BD_ND(false, 1, 0); }
-    else { NPME_BD_ND(false, 0, 0); }
-#undef NPME_BD_ND
-#undef NPME_BD
+    launch_batch_direct(k, std::get<0>(kv.first) != 0, h0->p.alpha >= 0, D(c), O(c),
+                        (int)c.members.size(), ng, ds);
+    nclass++;
     b->launches++;
+  }
+  for (int i = 0; i < std::min(nclass - 1, (int)npme_batch::kSide); i++) {
+    cudaEventRecord(b->ev_side[i], b->side[i]);
+    cudaStreamWaitEvent(b->stream2, b->ev_side[i], 0);
   }
   cudaEventRecord(b->ev_join, b->stream2);
   // 3. spread (grids zeroed first)
-  for (int k = 0; k < m; k++) {
-    grid_clear(hs[f32[k]], s);
+  for (auto &kv : clr) {
+    Class &c = kv.second;
+    const unsigned g = (unsigned)c.off.back();
+    if (kv.first) batch_clear_kernel<true><<<g, 256, 0, s>>>(D(c), O(c), (int)c.members.size());
+    else batch_clear_kernel<false><<<g, 256, 0, s>>>(D(c), O(c), (int)c.members.size());
+    b->launches++;
   }
+  for (int k = 0; k < m; k++)
+    if (!hs[f32[k]]->own_fft) grid_clear(hs[f32[k]], s);
   for (auto &kv : spr) {
     Class &c = kv.second;
     const long long nb = c.off.back();
