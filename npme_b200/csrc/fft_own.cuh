@@ -32,6 +32,7 @@
 namespace npme {
 
 constexpr int kFftThreads = 256;
+constexpr int kFftMaxLines = 4;  // log2 of the lines per CTA at most
 
 template <typename T>
 using Cx = typename Vec2<T>::type;
@@ -206,46 +207,64 @@ __device__ __forceinline__ void dft(Cx<T> (&v)[R]) {
   }
 }
 
-// One Stockham pass over the CTA's lines: butterfly j of a line reads
-// elements j + r N/R and writes (j / Ns) Ns R + j mod Ns + r Ns.  load(n)
-// and store(n, v) address element n of the thread's line.
-template <typename T, int DIR, int R, class Load, class Store>
+// Largest radix first; even radices only where half of the line is zero or
+// unwanted (HIN, HOUT below).
+#define NPME_FFT_EVEN(CASE) CASE(16) CASE(12) CASE(10) CASE(8) CASE(6) CASE(4) CASE(2)
+#define NPME_FFT_ALL(CASE) NPME_FFT_EVEN(CASE) CASE(9) CASE(5) CASE(3)
+
+// One Stockham pass over a line: butterfly j reads elements j + r N/R and
+// writes (j / Ns) Ns R + j mod Ns + r Ns; element n is at src[n ss], dst[n ds].
+// HIN (first pass): the elements from N/2 on are zeros that are not read.  HOUT
+// (last pass): those from N/2 on are not written.  Both are half of the
+// butterfly's values for an even radix, known at compile time.
+template <typename T, int DIR, int R, bool HIN, bool HOUT, class SS, class DS>
 __device__ __forceinline__ void fft_pass_r(const FftPass &p, int N, int j0, int dj, const Cx<T> *tw,
-                                           const Load &load, const Store &store) {
+                                           const Cx<T> *src, SS ss, Cx<T> *dst, DS ds) {
+  static_assert(R % 2 == 0 || (!HIN && !HOUT), "even radix");
   const int nb = N / R;
   for (int j = j0; j < nb; j += dj) {
     const int q = p.Ns == 1 ? j : (int)__umulhi((unsigned)j, p.magic), k = j - q * p.Ns;
     Cx<T> v[R];
+    const Cx<T> *in = src + j * ss;
+    const SS sstep = nb * ss;
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = load(j + r * nb);
-    if (p.Ns > 1) {
+    for (int r = 0; r < R; r++) {
+      if (HIN && r >= R / 2) {
+        v[r] = Cx<T>{};
+      } else {
+        v[r] = *in;
+        in += sstep;
+      }
+    }
+    if (!HIN && p.Ns > 1) {
+      const Cx<T> *t = tw;
       const int step = k * p.step;
 #pragma unroll
-      for (int r = 1; r < R; r++) v[r] = ctw<DIR>(v[r], tw[r * step]);
+      for (int r = 1; r < R; r++) {
+        t += step;
+        v[r] = ctw<DIR>(v[r], *t);
+      }
     }
     dft<T, DIR, R>(v);
-    const int base = q * p.Ns * R + k;
+    Cx<T> *out = dst + (q * p.Ns * R + k) * ds;
+    const DS dstep = p.Ns * ds;
 #pragma unroll
-    for (int r = 0; r < R; r++) store(base + r * p.Ns, v[r]);
+    for (int r = 0; r < (HOUT ? R / 2 : R); r++) {
+      *out = v[r];
+      out += dstep;
+    }
   }
 }
 
-template <typename T, int DIR, class Load, class Store>
+template <typename T, int DIR, bool HIN, bool HOUT, class SS, class DS>
 __device__ __forceinline__ void fft_pass(const FftPass &p, int N, int j0, int dj, const Cx<T> *tw,
-                                         const Load &load, const Store &store) {
+                                         const Cx<T> *src, SS ss, Cx<T> *dst, DS ds) {
 #define NPME_FFT_CASE(RR) \
-  case RR: fft_pass_r<T, DIR, RR>(p, N, j0, dj, tw, load, store); break
-  switch (p.R) {
-    NPME_FFT_CASE(16);
-    NPME_FFT_CASE(12);
-    NPME_FFT_CASE(10);
-    NPME_FFT_CASE(9);
-    NPME_FFT_CASE(8);
-    NPME_FFT_CASE(6);
-    NPME_FFT_CASE(5);
-    NPME_FFT_CASE(4);
-    NPME_FFT_CASE(3);
-    NPME_FFT_CASE(2);
+  case RR: fft_pass_r<T, DIR, RR, HIN, HOUT>(p, N, j0, dj, tw, src, ss, dst, ds); break;
+  if constexpr (HIN || HOUT) {
+    switch (p.R) { NPME_FFT_EVEN(NPME_FFT_CASE) }
+  } else {
+    switch (p.R) { NPME_FFT_ALL(NPME_FFT_CASE) }
   }
 #undef NPME_FFT_CASE
 }
@@ -256,62 +275,59 @@ __device__ __forceinline__ void fft_pass(const FftPass &p, int N, int j0, int dj
 // reads for its butterfly j.  mul(n, v): the product at element n.
 template <typename T, int R, class Mul>
 __device__ __forceinline__ void fft_turn_r(const FftPass &p, int N, int j0, int dj,
-                                           const Cx<T> *tw, const Cx<T> *in, Cx<T> *out,
+                                           const Cx<T> *tw, const Cx<T> *src, Cx<T> *dst,
                                            int pitch, const Mul &mul) {
   const int nb = N / R;
   for (int j = j0; j < nb; j += dj) {
     Cx<T> v[R];
+    const Cx<T> *in = src + j * pitch, *t = tw;
+    const int sstep = nb * pitch, step = j * p.step;
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = in[(j + r * nb) * pitch];
-    const int step = j * p.step;
+    for (int r = 0; r < R; r++) {
+      v[r] = *in;
+      in += sstep;
+    }
 #pragma unroll
-    for (int r = 1; r < R; r++) v[r] = ctw<-1>(v[r], tw[r * step]);
+    for (int r = 1; r < R; r++) {
+      t += step;
+      v[r] = ctw<-1>(v[r], *t);
+    }
     dft<T, -1, R>(v);
 #pragma unroll
     for (int r = 0; r < R; r++) v[r] = mul(j + r * nb, v[r]);
     dft<T, 1, R>(v);
+    Cx<T> *out = dst + j * R * pitch;
 #pragma unroll
-    for (int r = 0; r < R; r++) out[(j * R + r) * pitch] = v[r];
+    for (int r = 0; r < R; r++) {
+      *out = v[r];
+      out += pitch;
+    }
   }
 }
 
 template <typename T, class Mul>
 __device__ __forceinline__ void fft_turn(const FftPass &p, int N, int j0, int dj,
-                                         const Cx<T> *tw, const Cx<T> *in, Cx<T> *out, int pitch,
+                                         const Cx<T> *tw, const Cx<T> *src, Cx<T> *dst, int pitch,
                                          const Mul &mul) {
 #define NPME_FFT_CASE(RR) \
-  case RR: fft_turn_r<T, RR>(p, N, j0, dj, tw, in, out, pitch, mul); break
-  switch (p.R) {
-    NPME_FFT_CASE(16);
-    NPME_FFT_CASE(12);
-    NPME_FFT_CASE(10);
-    NPME_FFT_CASE(9);
-    NPME_FFT_CASE(8);
-    NPME_FFT_CASE(6);
-    NPME_FFT_CASE(5);
-    NPME_FFT_CASE(4);
-    NPME_FFT_CASE(3);
-    NPME_FFT_CASE(2);
-  }
+  case RR: fft_turn_r<T, RR>(p, N, j0, dj, tw, src, dst, pitch, mul); break;
+  switch (p.R) { NPME_FFT_ALL(NPME_FFT_CASE) }
 #undef NPME_FFT_CASE
 }
 
-// A transform of the CTA's lines in shared memory buffers s0 and s1 ([n *
-// pitch] of this thread's line): passes [from, to), the first of them
-// reading `cur`.  Returns the buffer that holds the result.  Barriers after
-// every pass.
+// Passes [from, to) of a transform in shared memory (the thread's line at cur,
+// the other buffer at other), a barrier after each; returns the buffer that
+// holds the result.  Dead lines only meet the barriers.
 template <typename T, int DIR>
 __device__ __forceinline__ Cx<T> *fft_middle(const FftAxis &a, int from, int to, int j0, int dj,
-                                             const Cx<T> *tw, Cx<T> *cur, Cx<T> *other,
-                                             int pitch) {
+                                             const Cx<T> *tw, Cx<T> *cur, Cx<T> *other, int pitch,
+                                             bool live = true) {
   for (int i = from; i < to; i++) {
-    const Cx<T> *in = cur;
-    Cx<T> *out = other;
-    fft_pass<T, DIR>(a.p[i], a.N, j0, dj, tw, [=](int n) { return in[n * pitch]; },
-                     [=](int n, Cx<T> v) { out[n * pitch] = v; });
+    if (live) fft_pass<T, DIR, false, false>(a.p[i], a.N, j0, dj, tw, cur, pitch, other, pitch);
     __syncthreads();
-    other = cur;
-    cur = out;
+    Cx<T> *t = cur;
+    cur = other;
+    other = t;
   }
   return cur;
 }
@@ -327,7 +343,7 @@ __device__ __forceinline__ void load_twiddles(const FftAxis &a, Cx<T> *tw) {
 template <typename T, int DIR>
 __device__ __forceinline__ void fft_y_body(const FftJob &J, long u, unsigned char *smem) {
   using C = Cx<T>;
-  const FftAxis &a = J.y;
+  const FftAxis &a = DIR < 0 ? J.y : J.yi;
   const int B = 1 << a.lb;
   C *tw = reinterpret_cast<C *>(smem), *s0 = tw + a.twlen, *s1 = s0 + (long)a.N * B;
   const int b = threadIdx.x & (B - 1), j0 = threadIdx.x >> a.lb, dj = kFftThreads >> a.lb;
@@ -336,18 +352,11 @@ __device__ __forceinline__ void fft_y_body(const FftJob &J, long u, unsigned cha
   const bool live = x < J.H[0] && k < J.K;
   C *g = static_cast<C *>(J.spec) + (long)x * J.N[1] * J.KP + k;
   const long st = J.KP;
-  const int nin = DIR < 0 ? J.H[1] : J.N[1], nout = DIR < 0 ? J.N[1] : J.H[1];
   load_twiddles<T>(a, tw);
-  C *o0 = s0 + b;
-  fft_pass<T, DIR>(a.p[0], a.N, j0, dj, tw,
-                   [=](int n) { return live && n < nin ? g[n * st] : C{}; },
-                   [=](int n, C v) { o0[n * B] = v; });
+  if (live) fft_pass<T, DIR, DIR<0, false>(a.p[0], a.N, j0, dj, tw, g, st, s0 + b, B);
   __syncthreads();
-  const C *in = fft_middle<T, DIR>(a, 1, a.np - 1, j0, dj, tw, s0 + b, s1 + b, B);
-  fft_pass<T, DIR>(a.p[a.np - 1], a.N, j0, dj, tw, [=](int n) { return in[n * B]; },
-                   [=](int n, C v) {
-                     if (live && n < nout) g[n * st] = v;
-                   });
+  const C *in = fft_middle<T, DIR>(a, 1, a.np - 1, j0, dj, tw, s0 + b, s1 + b, B, live);
+  if (live) fft_pass<T, DIR, false, (DIR > 0)>(a.p[a.np - 1], a.N, j0, dj, tw, in, B, g, st);
 }
 
 // Lines along x: forward, times G, inverse, in place on the spectrum; unit
@@ -356,41 +365,35 @@ __device__ __forceinline__ void fft_y_body(const FftJob &J, long u, unsigned cha
 template <typename T, bool CPLX>
 __device__ __forceinline__ void fft_x_body(const FftJob &J, long u, unsigned char *smem) {
   using C = Cx<T>;
-  const FftAxis &a = J.x;
+  const FftAxis &a = J.x, &ai = J.xi;
   const int B = 1 << a.lb;
   C *tw = reinterpret_cast<C *>(smem), *s0 = tw + a.twlen, *s1 = s0 + (long)a.N * B;
   const int b = threadIdx.x & (B - 1), j0 = threadIdx.x >> a.lb, dj = kFftThreads >> a.lb;
   const int line = (int)(u << a.lb) + b;
-  const int N1 = J.N[0], H1 = J.H[0], N2 = J.N[1], N3 = J.N[2];
+  const int N1 = J.N[0], N2 = J.N[1], N3 = J.N[2];
   const int k2 = line / J.KP, k3 = line - k2 * J.KP;
   const bool live = k2 < N2 && k3 < J.K;
   C *g = static_cast<C *>(J.spec) + line;
   const long st = (long)N2 * J.KP;
   const int M2 = N2 / 2 + 1, M3 = N3 / 2 + 1;
-  const int f2 = k2 <= N2 / 2 ? k2 : N2 - k2, f3 = k3 <= N3 / 2 ? k3 : N3 - k3;
+  const int f2 = min(k2, N2 - k2), f3 = min(k3, N3 - k3);
   const long gst = (long)M2 * M3;
   using GT = typename std::conditional<CPLX, C, T>::type;
-  const GT *G = static_cast<const GT *>(J.G) + (live ? (long)f2 * M3 + f3 : 0);
+  const GT *G = static_cast<const GT *>(J.G) + ((long)f2 * M3 + f3);  // read for live lines
   load_twiddles<T>(a, tw);
-  C *o0 = s0 + b;
-  fft_pass<T, -1>(a.p[0], N1, j0, dj, tw,
-                  [=](int n) { return live && n < H1 ? g[n * st] : C{}; },
-                  [=](int n, C v) { o0[n * B] = v; });
+  if (live) fft_pass<T, -1, true, false>(a.p[0], N1, j0, dj, tw, g, st, s0 + b, B);
   __syncthreads();
-  C *cur = fft_middle<T, -1>(a, 1, a.np - 1, j0, dj, tw, s0 + b, s1 + b, B);
+  C *cur = fft_middle<T, -1>(a, 1, a.np - 1, j0, dj, tw, s0 + b, s1 + b, B, live);
   C *out = cur == s0 + b ? s1 + b : s0 + b;
-  fft_turn<T>(a.p[a.np - 1], N1, j0, dj, tw, cur, out, B, [=](int n, C v) {
-    const GT w = G[(n <= N1 / 2 ? n : N1 - n) * gst];
-    if constexpr (CPLX) return cx<T>(v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x);
-    else return cx<T>(v.x * w, v.y * w);
-  });
+  if (live)
+    fft_turn<T>(a.p[a.np - 1], N1, j0, dj, tw, cur, out, B, [=](int n, C v) {
+      const GT w = G[min(n, N1 - n) * gst];
+      if constexpr (CPLX) return cx<T>(v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x);
+      else return cx<T>(v.x * w, v.y * w);
+    });
   __syncthreads();
-  const FftAxis &ai = J.xi;
-  const C *in = fft_middle<T, 1>(ai, 1, ai.np - 1, j0, dj, tw, out, cur, B);
-  fft_pass<T, 1>(ai.p[ai.np - 1], N1, j0, dj, tw, [=](int n) { return in[n * B]; },
-                 [=](int n, C v) {
-                   if (live && n < H1) g[n * st] = v;
-                 });
+  const C *in = fft_middle<T, 1>(ai, 1, ai.np - 1, j0, dj, tw, out, cur, B, live);
+  if (live) fft_pass<T, 1, false, true>(ai.p[ai.np - 1], N1, j0, dj, tw, in, B, g, st);
 }
 
 // Rows along z; unit u: rows u B ... of the H1 H2 rows.  Forward: the grid's
@@ -401,58 +404,57 @@ __device__ __forceinline__ void fft_x_body(const FftJob &J, long u, unsigned cha
 template <typename T, bool CPLX, int DIR>
 __device__ __forceinline__ void fft_z_body(const FftJob &J, long u, unsigned char *smem) {
   using C = Cx<T>;
-  const FftAxis &a = J.z;  // length N3 (complex kernels) or H3
+  __shared__ long srow[1 << kFftMaxLines];   // the rows' places in the spectrum
+  const FftAxis &a = DIR < 0 ? J.z : J.zi;  // length N3 (complex kernels) or H3
   const int B = 1 << a.lb, P = B + 1, L = a.N, H3 = J.H[2];
   C *tw = reinterpret_cast<C *>(smem), *s0 = tw + a.twlen, *s1 = s0 + (long)(L + 1) * P;
   const int b = threadIdx.x & (B - 1), j0 = threadIdx.x >> a.lb, dj = kFftThreads >> a.lb;
-  const int row0 = (int)(u << a.lb), rows = J.H[0] * J.H[1];
+  const int row0 = (int)(u << a.lb), rows = min(B, J.H[0] * J.H[1] - row0);
+  const bool live = b < rows;
   // grid rows as complex values: H3 (complex kernels) or H3 / 2 pairs
   const int gl = CPLX ? H3 : H3 / 2;
-  C *grid = static_cast<C *>(J.grid), *spec = static_cast<C *>(J.spec);
-  // rows of the octant (x, y) in the spectrum: x N2 + y
-  auto srow = [&](int row) {
-    const int x = row / J.H[1];
-    return spec + ((long)x * J.N[1] + (row - x * J.H[1])) * J.KP;
-  };
+  C *grid = static_cast<C *>(J.grid) + (long)row0 * gl, *spec = static_cast<C *>(J.spec);
+  if (threadIdx.x < rows) {
+    const int row = row0 + threadIdx.x, x = row / J.H[1];
+    srow[threadIdx.x] = ((long)x * J.N[1] + (row - x * J.H[1])) * J.KP;
+  }
   load_twiddles<T>(a, tw);
   // element i of row r of the batch -> (r, i), i fastest
   auto sweep = [&](int len, auto f) {
     const unsigned m = 0xffffffffu / (unsigned)len + 1;  // ceil(2^32 / len), len > 1
-    for (int t = threadIdx.x; t < (len << a.lb); t += kFftThreads) {
-      const int r = (int)__umulhi((unsigned)t, m), i = t - r * len;
-      if (row0 + r < rows) f(r, i);
+    for (int t = threadIdx.x; t < len * rows; t += kFftThreads) {
+      const int r = (int)__umulhi((unsigned)t, m);
+      f(r, t - r * len, t);
     }
   };
   if (DIR < 0) {
-    sweep(gl, [&](int r, int i) { s0[i * P + r] = grid[(long)(row0 + r) * gl + i]; });
+    // the rows are contiguous in the grid
+    sweep(gl, [&](int r, int i, int t) { s0[i * P + r] = grid[t]; });
     __syncthreads();
-    const C *in = s0 + b;
-    C *out = s1 + b;
-    fft_pass<T, -1>(a.p[0], L, j0, dj, tw, [=](int n) { return n < gl ? in[n * P] : C{}; },
-                    [=](int n, C v) { out[n * P] = v; });
+    if (live) fft_pass<T, -1, true, false>(a.p[0], L, j0, dj, tw, s0 + b, P, s1 + b, P);
     __syncthreads();
-    const C *Z = fft_middle<T, -1>(a, 1, a.np, j0, dj, tw, s1 + b, s0 + b, P) - b;
+    const C *Z = fft_middle<T, -1>(a, 1, a.np, j0, dj, tw, s1 + b, s0 + b, P, live) - b;
     if (CPLX) {
-      sweep(L, [&](int r, int k) { srow(row0 + r)[k] = Z[k * P + r]; });
+      sweep(L, [&](int r, int k, int) { spec[srow[r] + k] = Z[k * P + r]; });
     } else {
-      sweep(L + 1, [&](int r, int k) {
+      sweep(L + 1, [&](int r, int k, int) {
         const C z = Z[(k == L ? 0 : k) * P + r], m = Z[(k == 0 ? 0 : L - k) * P + r];
         const C e = cx<T>(T(0.5) * (z.x + m.x), T(0.5) * (z.y - m.y));
         const C d = cx<T>(T(0.5) * (z.x - m.x), T(0.5) * (z.y + m.y));
         const C w = tw[k];  // table of the length-N3 transform
         // -i w d
         const C wd = cx<T>(w.x * d.x - w.y * d.y, w.x * d.y + w.y * d.x);
-        srow(row0 + r)[k] = cx<T>(e.x + wd.y, e.y - wd.x);
+        spec[srow[r] + k] = cx<T>(e.x + wd.y, e.y - wd.x);
       });
     }
   } else {
-    C *cur = s0;
+    __syncthreads();
     if (CPLX) {
-      sweep(L, [&](int r, int k) { s0[k * P + r] = srow(row0 + r)[k]; });
+      sweep(L, [&](int r, int k, int) { s0[k * P + r] = spec[srow[r] + k]; });
     } else {
-      sweep(L + 1, [&](int r, int k) { s1[k * P + r] = srow(row0 + r)[k]; });
+      sweep(L + 1, [&](int r, int k, int) { s1[k * P + r] = spec[srow[r] + k]; });
       __syncthreads();
-      sweep(L, [&](int r, int k) {
+      sweep(L, [&](int r, int k, int) {
         const C z = s1[k * P + r], m = s1[(L - k) * P + r];
         const C e = cx<T>(z.x + m.x, z.y - m.y), d = cx<T>(z.x - m.x, z.y + m.y);
         const C w = tw[k];
@@ -462,8 +464,12 @@ __device__ __forceinline__ void fft_z_body(const FftJob &J, long u, unsigned cha
       });
     }
     __syncthreads();
-    const C *Z = fft_middle<T, 1>(a, 0, a.np, j0, dj, tw, cur + b, s1 + b, P) - b;
-    sweep(gl, [&](int r, int i) { grid[(long)(row0 + r) * gl + i] = Z[i * P + r]; });
+    C *in = fft_middle<T, 1>(a, 0, a.np - 1, j0, dj, tw, s0 + b, s1 + b, P, live);
+    C *out = in == s0 + b ? s1 + b : s0 + b;
+    if (live) fft_pass<T, 1, false, true>(a.p[a.np - 1], L, j0, dj, tw, in, P, out, P);
+    __syncthreads();
+    const C *Z = out - b;
+    sweep(gl, [&](int r, int i, int t) { grid[t] = Z[i * P + r]; });
   }
 }
 

@@ -69,10 +69,11 @@ __global__ void __launch_bounds__(kFftThreads)
 
 namespace {
 
-// Radices of N, largest first: as few as possible, then the smallest largest
-// one; empty when N has a factor other than 2, 3 and 5 or fewer than two
+// Radices of N, as few as possible, then the smallest largest one; an even one
+// first (half of the line is zero at the start and unwanted at the end of the
+// reverse order); none above `largest`; empty when N has a factor other than 2, 3 and 5 or fewer than two
 // passes.
-std::vector<int> radices(long N) {
+std::vector<int> radices(long N, int largest = 16) {
   static const int kR[] = {16, 12, 10, 9, 8, 6, 5, 4, 3, 2};
   // products of at most `left` radices, none above cap
   struct Search {
@@ -90,10 +91,15 @@ std::vector<int> radices(long N) {
   };
   std::vector<int> r;
   for (int passes = 2; passes <= 8; passes++)
-    for (int i = 9; i >= 0; i--) {
+    for (int i = 9; i >= 0 && kR[i] <= largest; i--) {
       r.clear();
       if (Search::run(N, passes, kR[i], r)) {
-        if (r.size() < 2) r.clear();
+        if (r.size() < 2 || N % 2) r.clear();
+        for (size_t k = 0; k < r.size(); k++)
+          if (r[k] % 2 == 0) {
+            std::swap(r[0], r[k]);
+            break;
+          }
         return r;
       }
     }
@@ -137,11 +143,13 @@ int twiddles(npme_handle *h, long N, const void **out) {
 
 // Passes of a length-N transform whose twiddles are every `stride`-th entry
 // of a table.
-void make_axis(FftAxis &a, long N, int stride, bool reverse = false) {
+void make_axis(FftAxis &a, long N, int stride, bool fp32, bool reverse) {
   a.N = (int)N;
   a.np = 0;
   int Ns = 1;
-  std::vector<int> radix = radices(N);
+  // radix 9 and more take two doubles too many per value for two resident CTAs
+  // in FP64 (128 registers): 256^3 in FP64 235 us with them, 209 without
+  std::vector<int> radix = radices(N, fp32 ? 16 : 8);
   if (reverse) std::reverse(radix.begin(), radix.end());
   for (int R : radix) {
     FftPass &p = a.p[a.np++];
@@ -165,7 +173,7 @@ size_t own_fft_smem(const FftJob &j, int axis, size_t cbytes) {
 // Shared memory of a CTA: at most about half of an SM's while 8 lines or more
 // fit that, so that two or more are resident.  Two lines of the greatest
 // length (2,048) fit a CTA in FP64 (229,472 bytes along z, complex).
-static constexpr size_t kFftSmem = 100 * 1024, kFftSmemMax = 227 * 1024;
+static constexpr size_t kFftSmem = 100 * 1024, kFftSmemMax = 226 * 1024;
 
 bool own_fft_lengths(const long N[3]) {
   for (int a = 0; a < 3; a++)
@@ -182,10 +190,11 @@ int own_fft_prepare(npme_handle *h) {
   j.K = cx ? j.N[2] : j.H[2] + 1;
   j.KP = (j.K + 3) & ~3;
   j.grid = h->d_grid, j.spec = h->d_kgrid, j.G = h->d_G;
-  make_axis(j.x, N[0], 1);
-  make_axis(j.xi, N[0], 1, true);
-  make_axis(j.y, N[1], 1);
-  make_axis(j.z, cx ? N[2] : N[2] / 2, cx ? 1 : 2);
+  for (int r = 0; r < 2; r++) {
+    make_axis(r ? j.xi : j.x, N[0], 1, h->fp32, r != 0);
+    make_axis(r ? j.yi : j.y, N[1], 1, h->fp32, r != 0);
+    make_axis(r ? j.zi : j.z, cx ? N[2] : N[2] / 2, cx ? 1 : 2, h->fp32, r != 0);
+  }
   int rc;
   if ((rc = twiddles(h, N[0], &j.x.tw)) || (rc = twiddles(h, N[1], &j.y.tw)) ||
       (rc = twiddles(h, N[2], &j.z.tw)))
@@ -197,7 +206,7 @@ int own_fft_prepare(npme_handle *h) {
   for (int a = 0; a < 3; a++) {
     // 16 lines (128 bytes of a row in FP32), fewer when they do not fit or
     // when the pass would leave SMs without a CTA
-    int lb = 4;
+    int lb = kFftMaxLines;
     for (ax[a]->lb = lb; lb > 1; lb--) {
       ax[a]->lb = lb;
       if (own_fft_smem(j, a, cb) <= kFftSmem && (lb <= 3 || (lines[a] >> lb) >= 148)) break;
@@ -205,6 +214,8 @@ int own_fft_prepare(npme_handle *h) {
     ax[a]->lb = std::max(lb, 1);
     *units[a] = (lines[a] + (1L << ax[a]->lb) - 1) >> ax[a]->lb;
   }
+  j.xi.lb = j.x.lb, j.yi.lb = j.y.lb, j.zi.lb = j.z.lb;
+  j.xi.tw = j.x.tw, j.yi.tw = j.y.tw, j.zi.tw = j.z.tw;
   return NPME_OK;
 }
 

@@ -81,7 +81,7 @@ struct FftJob {
   const void *G;
   int H[3], N[3];
   int K, KP;       // values per spectrum row, and its pitch
-  FftAxis x, xi, y, z;  // xi: x with the passes in reverse order
+  FftAxis x, y, z, xi, yi, zi;  // forward; inverse, the passes in reverse order
   long ux, uy, uz; // CTAs of each pass
 };
 
