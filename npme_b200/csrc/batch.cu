@@ -287,6 +287,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     S.hgroups = h->d_hgroups;
     S.hcen = h->d_hcen;
     S.hsegs = h->d_hsegs;
+    S.hzones = h->d_hzones;
     S.vsrc = h->d_vsrc;
     S.bperm = h->d_bperm;
     S.refine2 = (float)h->refine2;

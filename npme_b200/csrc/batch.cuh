@@ -27,6 +27,7 @@ struct BatchSys {
   const int2 *segs;
   // pair-once walk: half-shell groups and segments, source-side sums
   const int4 *hgroups;
+  const int2 *hzones;
   const double4 *hcen;
   const int2 *hsegs;
   float4 *vsrc;            // source-side sums, slot = brick-order position

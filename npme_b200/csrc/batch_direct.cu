@@ -42,19 +42,21 @@ __global__ void __launch_bounds__(32 * kGroupWarps, 4) batch_sym_kernel(
   if constexpr (KIND == 0) {
     double acc[4] = {0, 0, 0, 0};
     const int4 G = S.hgroups[g];
-    direct_group_sym<FUNC, ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.cperm,
-                               S.refine2, S.vsrc, ta[wid], tb[wid], lane, 0, 1, acc);
+    direct_group_sym<FUNC, ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.hzones[g],
+                               S.cperm, S.refine2, S.vsrc, ta[wid], tb[wid], lane, 0, 1, acc);
     sym_store(k, G, S.cperm, S.q, S.fself_r, S.V, lane, acc);
   } else {
-    direct_group_sym_helm<ND>(k, S.gpos, S.spos, S.qc, S.q, S.hgroups[g], S.hcen[g], S.hsegs,
-                              S.cperm, S.refine2, S.fself_r, S.fself_i, S.V, S.vsrc, ta[wid],
-                              tb[wid], lane);
+    double acc[4] = {0, 0, 0, 0}, acci[4] = {0, 0, 0, 0};
+    const int4 G = S.hgroups[g];
+    direct_group_sym_helm<ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.hzones[g],
+                              S.cperm, S.refine2, S.vsrc, ta[wid], tb[wid], lane, 0, 1, acc, acci);
+    store_targets_cplx(G, S.cperm, S.q, S.fself_r, S.fself_i, 1.0, 1.0, S.V, lane, acc, acci);
   }
 }
 
 // The pair-once walk with a CTA of kGroupWarps warps per group, for classes
 // with few groups (split_warps in direct.cu): four warps per group.
-template <int FUNC, int ND>
+template <int KIND, int FUNC, int ND>
 __global__ void __launch_bounds__(32 * kGroupWarps, 4) batch_sym_split_kernel(
     PairCoef<float> k, const BatchSys *__restrict__ sys, const long long *__restrict__ off,
     int count) {
@@ -66,12 +68,24 @@ __global__ void __launch_bounds__(32 * kGroupWarps, 4) batch_sym_split_kernel(
   const int s = find_sys(off, count, u);
   const BatchSys &S = sys[s];
   const long g = (long)(u - off[s]);
-  double acc[4] = {0, 0, 0, 0};
+  double acc[4] = {0, 0, 0, 0}, acci[4] = {0, 0, 0, 0};
   const int4 G = S.hgroups[g];
-  direct_group_sym<FUNC, ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.cperm,
-                             S.refine2, S.vsrc, ta[wid], tb[wid], lane, wid, kGroupWarps, acc);
-  reduce_parts(acc, red, wid, kGroupWarps, lane);
-  if (wid == 0) sym_store(k, G, S.cperm, S.q, S.fself_r, S.V, lane, acc);
+  if constexpr (KIND == 0) {
+    direct_group_sym<FUNC, ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.hzones[g],
+                               S.cperm, S.refine2, S.vsrc, ta[wid], tb[wid], lane, wid,
+                               kGroupWarps, acc);
+    reduce_parts(acc, red, wid, kGroupWarps, lane);
+    if (wid == 0) sym_store(k, G, S.cperm, S.q, S.fself_r, S.V, lane, acc);
+  } else {
+    direct_group_sym_helm<ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.hzones[g],
+                              S.cperm, S.refine2, S.vsrc, ta[wid], tb[wid], lane, wid,
+                              kGroupWarps, acc, acci);
+    reduce_parts(acc, red, wid, kGroupWarps, lane);
+    __syncthreads();
+    reduce_parts(acci, red, wid, kGroupWarps, lane);
+    if (wid == 0)
+      store_targets_cplx(G, S.cperm, S.q, S.fself_r, S.fself_i, 1.0, 1.0, S.V, lane, acc, acci);
+  }
 }
 
 void launch_batch_direct(const PairCoef<float> &k, bool once, bool alpha_positive,
@@ -85,8 +99,9 @@ void launch_batch_direct(const PairCoef<float> &k, bool once, bool alpha_positiv
   // batch runs beside other launches, so fewer groups take no more warps
   const bool split = ng <= 20 * 148;
 #define NPME_BSYM(KD, FN, ND)                                                              \
-  if (KD == 0 && split)                                                                    \
-    batch_sym_split_kernel<FN, ND><<<(unsigned)ng, 32 * kGroupWarps, 0, s>>>(k, sys, off, count); \
+  if (split)                                                                               \
+    batch_sym_split_kernel<KD, FN, ND>                                                     \
+        <<<(unsigned)ng, 32 * kGroupWarps, 0, s>>>(k, sys, off, count);                     \
   else                                                                                     \
     batch_sym_kernel<KD, FN, ND><<<g, 32 * kGroupWarps, 0, s>>>(k, sys, off, count)
 #define NPME_BSYM_ND(KD, FN)                \
@@ -98,12 +113,7 @@ void launch_batch_direct(const PairCoef<float> &k, bool once, bool alpha_positiv
   }
   if (once) {  // the source-side sums are folded into V by the interpolation
     if (f == NPME_FUNC_HELMHOLTZ) {
-      switch (nd) {
-        case 3: batch_sym_kernel<1, 2, 3><<<g, 32 * kGroupWarps, 0, s>>>(k, sys, off, count); break;
-        case 6: batch_sym_kernel<1, 2, 6><<<g, 32 * kGroupWarps, 0, s>>>(k, sys, off, count); break;
-        case 8: batch_sym_kernel<1, 2, 8><<<g, 32 * kGroupWarps, 0, s>>>(k, sys, off, count); break;
-        default: batch_sym_kernel<1, 2, 0><<<g, 32 * kGroupWarps, 0, s>>>(k, sys, off, count); break;
-      }
+      NPME_BSYM_ND(1, 2);
     } else if (sp == NPME_SPLIT_LAPLACE_ORIG) {
       NPME_BSYM(0, 2, 0);
     } else if (f == NPME_FUNC_RALPHA) {

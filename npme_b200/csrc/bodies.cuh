@@ -819,6 +819,64 @@ struct SrcCursor {
   }
 };
 
+// A lane's K positions (lane, lane + 32, ...) in the chunks of 32 K sources of a
+// group's half-shell segments, zone by zone (both halves of the targets, lower,
+// upper half: setup.cu); a chunk belongs to one zone.  Of nsplit warps that
+// share the group, warp `part` takes every nsplit-th chunk of a zone.  ZONED =
+// false: the zones are one (the set-up makes them so for these kernels).
+template <int K, bool ZONED = true>
+struct ZoneWalk {
+  const int2 *__restrict__ segs;
+  int ends[3];  // of the zones' segments
+  int zone, lane, first, stride;
+  SrcCursor cur[K];
+  bool v[K];
+
+  __device__ __forceinline__ ZoneWalk(const int2 *__restrict__ segs_, const int4 G,
+                                      const int2 zones, int lane_, int part, int nsplit)
+      : segs(segs_), ends{zones.x, zones.y, G.w}, zone(0), lane(lane_),
+        first(lane_ + 32 * K * part), stride(32 * K * nsplit) {
+    start(G.z);
+    skip();
+  }
+  __device__ __forceinline__ int end() const {
+    return !ZONED ? ends[2] : zone == 0 ? ends[0] : zone == 1 ? ends[1] : ends[2];
+  }
+  __device__ __forceinline__ void start(int seg) {
+    cur[0] = SrcCursor{seg, first};
+    cur[0].normalize(segs, end());
+    v[0] = cur[0].seg < end();
+#pragma unroll
+    for (int i = 1; i < K; i++) {
+      cur[i] = SrcCursor{cur[i - 1].seg, cur[i - 1].off + 32};
+      cur[i].normalize(segs, end());
+      v[i] = cur[i].seg < end();
+    }
+  }
+  // on to the zone that has a chunk left (the valid lanes are a prefix)
+  __device__ __forceinline__ void skip() {
+    if (!ZONED) return;
+    while (zone < 2 && !__any_sync(0xffffffffu, v[0])) {
+      const int seg = end();
+      zone++;
+      start(seg);
+    }
+  }
+  __device__ __forceinline__ bool any() const { return __any_sync(0xffffffffu, v[0]); }
+  __device__ __forceinline__ void next() {
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+      cur[i].off += stride;
+      cur[i].normalize(segs, end());
+      v[i] = cur[i].seg < end();
+    }
+    skip();
+  }
+  __device__ __forceinline__ long index(int i) const {
+    return (long)segs[cur[i].seg].x + cur[i].off;
+  }
+};
+
 // Real derivative-match kernels (1/r, r^alpha) of the FP32 direct sum with
 // packed arithmetic: every lane evaluates its target against two sources per
 // step with sm_100's two-wide FP32 instructions (__fadd2_rn / __fmul2_rn /
@@ -1007,21 +1065,27 @@ __device__ __forceinline__ float2 rotate2(float2 v, int src) {
   return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
-// The 16 steps of one chunk; target sums rotate after each.
+// The steps of one chunk, 16 over all target pairs or 8 over one half of them
+// (zone 1: pairs 0-7, zone 2: pairs 8-15); target sums rotate after each.
 template <int FUNC, int ND, bool CHECKED>
 __device__ __forceinline__ void sym_sweep(const PairCoef<float> &k, const float4 *tsm,
                                           const float4 *tlo, const SymSource (&src)[2],
-                                          float refine2, int lane, float2 &aV, float2 &aX,
-                                          float2 &aY, float2 &aZ, float2 (&S)[2][4]) {
+                                          float refine2, int lane, int zone, float2 &aV,
+                                          float2 &aX, float2 &aY, float2 &aZ,
+                                          float2 (&S)[2][4]) {
   constexpr int kUnroll = CHECKED ? 1 : 8;
   const int next = (lane + 1) & 31;
+  const int mask = zone == 0 ? 15 : 7, from = zone == 2 ? 8 : 0;
+#pragma unroll 1
+  for (int k0 = 0; k0 <= mask; k0 += 8) {
 #pragma unroll kUnroll
-  for (int kk = 0; kk < 16; kk++) {
-    const int j = (lane + kk) & 15;
-    sym_step<FUNC, ND, CHECKED>(k, tsm[j], tsm[16 + j], tlo + j, tlo + 16 + j, src, refine2, aV,
-                                aX, aY, aZ, S);
-    aV = rotate2(aV, next), aX = rotate2(aX, next);
-    aY = rotate2(aY, next), aZ = rotate2(aZ, next);
+    for (int kk = 0; kk < 8; kk++) {
+      const int j = from + ((lane + k0 + kk) & mask);
+      sym_step<FUNC, ND, CHECKED>(k, tsm[j], tsm[16 + j], tlo + j, tlo + 16 + j, src, refine2,
+                                  aV, aX, aY, aZ, S);
+      aV = rotate2(aV, next), aX = rotate2(aX, next);
+      aY = rotate2(aY, next), aZ = rotate2(aZ, next);
+    }
   }
 }
 
@@ -1046,6 +1110,8 @@ __device__ __forceinline__ void sym_sweep(const PairCoef<float> &k, const float4
 // vsrc (FP32, scaled frame; slot = the source's brick-order position, from
 // spos[j].w) with one vector atomic per source, and folded into V by the
 // interpolation (CalcV) or by merge_source_kernel.
+// r^alpha: sources that only one half of the targets (16 in z order) can reach
+// are met by that half alone, in half the steps.
 // The group's work is shared by nsplit warps of the CTA, warp `part` taking
 // chunks part, part + nsplit, ... (and every nsplit-th source of the pairs
 // inside the group); the caller adds their acc.
@@ -1053,9 +1119,9 @@ template <int FUNC, int ND>
 __device__ __forceinline__ void direct_group_sym(
     const PairCoef<float> &k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const float *__restrict__ qs, const double *__restrict__ qcaller, const int4 G,
-    const double4 c, const int2 *__restrict__ segs, const uint32_t *__restrict__ perm,
-    float refine2, float4 *__restrict__ vsrc, float4 *tsm, float4 *tlo, int lane, int part,
-    int nsplit, double (&acc)[4]) {
+    const double4 c, const int2 *__restrict__ segs, const int2 zones,
+    const uint32_t *__restrict__ perm, float refine2, float4 *__restrict__ vsrc, float4 *tsm,
+    float4 *tlo, int lane, int part, int nsplit, double (&acc)[4]) {
   const unsigned FULL = 0xffffffffu;
   const int tid = 2 * (lane & 15) + (lane >> 4);  // the lane's target in the group
   // absent targets sit far outside the cutoff with charge 0
@@ -1112,36 +1178,31 @@ __device__ __forceinline__ void direct_group_sym(
   // and l + 32 of the chunk (register prefetch of the next chunk)
   const double rfs = sqrt((double)refine2) + c.w * ir;
   const double near2 = rfs * rfs;
-  const int stride = 64 * nsplit;
-  SrcCursor cur[2];
-  cur[0] = SrcCursor{G.z, lane + 64 * part};
-  cur[0].normalize(segs, G.w);
-  cur[1] = SrcCursor{cur[0].seg, cur[0].off + 32};
-  cur[1].normalize(segs, G.w);
-  bool v[2];
+  constexpr bool kZoned = FUNC == 1;  // measured: set-up (describe)
+  ZoneWalk<2, kZoned> walk(segs, G, zones, lane, part, nsplit);
   double4 p[2];
   float q[2];
 #pragma unroll
   for (int i = 0; i < 2; i++) {
-    v[i] = cur[i].seg < G.w;
     p[i] = make_double4(0, 0, 0, 0);
     q[i] = 0.f;
-    if (v[i]) {
-      const long j = (long)segs[cur[i].seg].x + cur[i].off;
+    if (walk.v[i]) {
+      const long j = walk.index(i);
       p[i] = spos[j], q[i] = qs[j];
     }
   }
-  while (__any_sync(FULL, v[0])) {
+  while (walk.any()) {
     // this chunk's sources, relative to the group centre; empty slots far
     // away (on the other side from absent targets) with charge 0
     SymSource src[2];
     int slot[2];  // source-side slots: the sources' brick-order positions
     bool checked = odd_group;
+    const int zone = kZoned ? walk.zone : 0;
 #pragma unroll
     for (int i = 0; i < 2; i++) {
       float hx = -1e18f, hy = -1e18f, hz = -1e18f, lx = 0.f, ly = 0.f, lz = 0.f, qv = 0.f;
       slot[i] = -1;
-      if (v[i]) {
+      if (walk.v[i]) {
         const double dx = (p[i].x - c.x) * ir, dy = (p[i].y - c.y) * ir,
                      dz = (p[i].z - c.z) * ir;
         hx = (float)dx, hy = (float)dy, hz = (float)dz;
@@ -1156,28 +1217,35 @@ __device__ __forceinline__ void direct_group_sym(
       src[i].z = make_float2(-hz, -hz), src[i].q = make_float2(qv, qv);
       src[i].lx = make_float2(-lx, -lx), src[i].ly = make_float2(-ly, -ly);
       src[i].lz = make_float2(-lz, -lz);
-      // prefetch the next chunk
-      cur[i].off += stride;
-      cur[i].normalize(segs, G.w);
-      v[i] = cur[i].seg < G.w;
-      if (v[i]) {
-        const long j = (long)segs[cur[i].seg].x + cur[i].off;
+    }
+    // prefetch the next chunk
+    walk.next();
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      if (walk.v[i]) {
+        const long j = walk.index(i);
         p[i] = spos[j], q[i] = qs[j];
       }
-    }
     float2 aV = make_float2(0.f, 0.f), aX = aV, aY = aV, aZ = aV;
     float2 S[2][4];
 #pragma unroll
     for (int i = 0; i < 2; i++) S[i][0] = S[i][1] = S[i][2] = S[i][3] = make_float2(0.f, 0.f);
     if (__any_sync(FULL, checked))
-      sym_sweep<FUNC, ND, true>(k, tsm, tlo, src, refine2, lane, aV, aX, aY, aZ, S);
+      sym_sweep<FUNC, ND, true>(k, tsm, tlo, src, refine2, lane, zone, aV, aX, aY, aZ, S);
     else
-      sym_sweep<FUNC, ND, false>(k, tsm, tlo, src, refine2, lane, aV, aX, aY, aZ, S);
-    // lanes l and l + 16 hold half of the sums of target pair l mod 16 each
-    const bool hi = lane >= 16;
+      sym_sweep<FUNC, ND, false>(k, tsm, tlo, src, refine2, lane, zone, aV, aX, aY, aZ, S);
+    // lanes l and l + 16 hold half of the sums of target pair l mod 16 each;
+    // after a sweep over one half of the pairs lanes l, l + 8, l + 16 and l + 24
+    // hold a quarter each of pair l mod 8 of that half
+    const bool hi = lane >= 16, other_half = zone != 0 && (lane >> 3 & 1) != zone - 1;
     auto total = [&](float2 a) {
+      if (zone != 0) {
+        a.x += __shfl_xor_sync(FULL, a.x, 8);
+        a.y += __shfl_xor_sync(FULL, a.y, 8);
+      }
       const float give = hi ? a.x : a.y, keep = hi ? a.y : a.x;
-      return keep + __shfl_xor_sync(FULL, give, 16);
+      const float sum = keep + __shfl_xor_sync(FULL, give, 16);
+      return other_half ? 0.f : sum;
     };
     acc[0] += (double)total(aV);
     acc[1] -= (double)total(aX);
@@ -1329,18 +1397,17 @@ template <int ND>
 __device__ __forceinline__ void direct_group_sym_helm(
     const PairCoef<float> &k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const float *__restrict__ qs, const double *__restrict__ qcaller, const int4 G,
-    const double4 c, const int2 *__restrict__ segs, const uint32_t *__restrict__ perm,
-    float refine2, double fself_r, double fself_i, double *__restrict__ V,
-    float4 *__restrict__ vsrc, float4 *th, float4 *tl, int lane) {
+    const double4 c, const int2 *__restrict__ segs, const int2 zones,
+    const uint32_t *__restrict__ perm, float refine2, float4 *__restrict__ vsrc, float4 *th,
+    float4 *tl, int lane, int part, int nsplit, double (&acc)[4], double (&acci)[4]) {
   const unsigned FULL = 0xffffffffu;
   const int ti = G.x + lane;
   const bool active = lane < G.y;
   float tx = 1e18f, ty = 1e18f, tz = 1e18f, tlx = 0.f, tly = 0.f, tlz = 0.f;
   float2 tq = make_float2(0.f, 0.f);
-  long o = 0;
   if (active) {
     const double4 p = gpos[ti];
-    o = perm[ti];
+    const long o = perm[ti];
     const double dx = p.x - c.x, dy = p.y - c.y, dz = p.z - c.z;
     tx = (float)dx, ty = (float)dy, tz = (float)dz;
     tlx = (float)(dx - (double)tx), tly = (float)(dy - (double)ty), tlz = (float)(dz - (double)tz);
@@ -1351,12 +1418,11 @@ __device__ __forceinline__ void direct_group_sym_helm(
   __syncwarp();
   const float R2 = k.R2;
   const unsigned rb = __float_as_uint(R2);
-  double acc[4] = {0, 0, 0, 0}, acci[4] = {0, 0, 0, 0};
 
   // pairs inside the group, target side only, differences always refined
   {
     float2 Pv = make_float2(0.f, 0.f), Gx = Pv, Gy = Pv, Gz = Pv;
-    for (int s = 0; s < G.y; s++) {
+    for (int s = part; s < G.y; s += nsplit) {
       const float4 S = th[s], L = tl[s];
       const float x = (tx - S.x) + (tlx - L.x), y = (ty - S.y) + (tly - L.y),
                   z = (tz - S.z) + (tlz - L.z);
@@ -1375,52 +1441,54 @@ __device__ __forceinline__ void direct_group_sym_helm(
     acc[2] += Gy.x, acci[2] += Gy.y, acc[3] += Gz.x, acci[3] += Gz.y;
   }
 
-  SrcCursor ca{G.z, lane};
-  ca.normalize(segs, G.w);
-  SrcCursor cb{ca.seg, ca.off + 32};
-  cb.normalize(segs, G.w);
-  bool va = ca.seg < G.w, vb = cb.seg < G.w;
-  long ja = -1, jb = -1;
-  double4 pa = make_double4(0, 0, 0, 0), pb = pa;
-  float2 qa = make_float2(0.f, 0.f), qb = qa;
-  if (va) ja = (long)segs[ca.seg].x + ca.off, pa = spos[ja], qa = make_float2(qs[2 * ja], qs[2 * ja + 1]);
-  if (vb) jb = (long)segs[cb.seg].x + cb.off, pb = spos[jb], qb = make_float2(qs[2 * jb], qs[2 * jb + 1]);
-  while (__any_sync(FULL, va)) {
+  ZoneWalk<2> walk(segs, G, zones, lane, part, nsplit);
+  double4 p[2];
+  float2 q[2];
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    p[i] = make_double4(0, 0, 0, 0);
+    q[i] = make_float2(0.f, 0.f);
+    if (walk.v[i]) {
+      const long j = walk.index(i);
+      p[i] = spos[j], q[i] = make_float2(qs[2 * j], qs[2 * j + 1]);
+    }
+  }
+  while (walk.any()) {
+    const int zone = walk.zone;
     // this chunk's two sources of the lane; empty slots far away on the
     // other side from idle targets, with charge 0
     float sx[2] = {-1e18f, -1e18f}, sy[2] = {-1e18f, -1e18f}, sz[2] = {-1e18f, -1e18f};
     float lx[2] = {0.f, 0.f}, ly[2] = {0.f, 0.f}, lz[2] = {0.f, 0.f};
     float2 sq[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-    const long kidx[2] = {va ? (long)pa.w : -1, vb ? (long)pb.w : -1};  // brick positions
-    if (va) {
-      const double dx = pa.x - c.x, dy = pa.y - c.y, dz = pa.z - c.z;
-      sx[0] = (float)dx, sy[0] = (float)dy, sz[0] = (float)dz;
-      lx[0] = (float)(dx - (double)sx[0]), ly[0] = (float)(dy - (double)sy[0]);
-      lz[0] = (float)(dz - (double)sz[0]);
-      sq[0] = qa;
+    int kidx[2];  // brick positions
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      kidx[i] = -1;
+      if (walk.v[i]) {
+        const double dx = p[i].x - c.x, dy = p[i].y - c.y, dz = p[i].z - c.z;
+        sx[i] = (float)dx, sy[i] = (float)dy, sz[i] = (float)dz;
+        lx[i] = (float)(dx - (double)sx[i]), ly[i] = (float)(dy - (double)sy[i]);
+        lz[i] = (float)(dz - (double)sz[i]);
+        sq[i] = q[i];
+        kidx[i] = (int)p[i].w;
+      }
     }
-    if (vb) {
-      const double dx = pb.x - c.x, dy = pb.y - c.y, dz = pb.z - c.z;
-      sx[1] = (float)dx, sy[1] = (float)dy, sz[1] = (float)dz;
-      lx[1] = (float)(dx - (double)sx[1]), ly[1] = (float)(dy - (double)sy[1]);
-      lz[1] = (float)(dz - (double)sz[1]);
-      sq[1] = qb;
-    }
-    ca.off += 64;
-    ca.normalize(segs, G.w);
-    cb.off += 64;
-    cb.normalize(segs, G.w);
-    va = ca.seg < G.w, vb = cb.seg < G.w;
-    if (va) ja = (long)segs[ca.seg].x + ca.off, pa = spos[ja], qa = make_float2(qs[2 * ja], qs[2 * ja + 1]);
-    if (vb) jb = (long)segs[cb.seg].x + cb.off, pb = spos[jb], qb = make_float2(qs[2 * jb], qs[2 * jb + 1]);
+    walk.next();
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      if (walk.v[i]) {
+        const long j = walk.index(i);
+        p[i] = spos[j], q[i] = make_float2(qs[2 * j], qs[2 * j + 1]);
+      }
 
     float2 Pv = make_float2(0.f, 0.f), Gx = Pv, Gy = Pv, Gz = Pv;  // target side, rotating
     float2 SV[2], SX[2], SY[2], SZ[2];                              // source side
 #pragma unroll
     for (int u = 0; u < 2; u++) SV[u] = SX[u] = SY[u] = SZ[u] = make_float2(0.f, 0.f);
     const int src = (lane + 1) & 31;
-    for (int kk = 0; kk < 32; kk++) {
-      const int tt = (lane + kk) & 31;
+    const int mask = zone == 0 ? 31 : 15, from = zone == 2 ? 16 : 0;
+    for (int kk = 0; kk <= mask; kk++) {
+      const int tt = from + ((lane + kk) & mask);
       const float4 T = th[tt], L = tl[tt];
       float x[2], y[2], z[2], rr[2];
       bool hit[2];
@@ -1461,24 +1529,44 @@ __device__ __forceinline__ void direct_group_sym_helm(
       Gy.x = __shfl_sync(FULL, Gy.x, src), Gy.y = __shfl_sync(FULL, Gy.y, src);
       Gz.x = __shfl_sync(FULL, Gz.x, src), Gz.y = __shfl_sync(FULL, Gz.y, src);
     }
-    acc[0] += Pv.x, acci[0] += Pv.y, acc[1] += Gx.x, acci[1] += Gx.y;
-    acc[2] += Gy.x, acci[2] += Gy.y, acc[3] += Gz.x, acci[3] += Gz.y;
+    if (zone != 0) {  // lanes l and l + 16 hold half of the sums of one target
+      float2 *const sums[4] = {&Pv, &Gx, &Gy, &Gz};
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        sums[m]->x += __shfl_xor_sync(FULL, sums[m]->x, 16);
+        sums[m]->y += __shfl_xor_sync(FULL, sums[m]->y, 16);
+      }
+    }
+    if (zone == 0 || lane >> 4 == zone - 1) {
+      acc[0] += Pv.x, acci[0] += Pv.y, acc[1] += Gx.x, acci[1] += Gx.y;
+      acc[2] += Gy.x, acci[2] += Gy.y, acc[3] += Gz.x, acci[3] += Gz.y;
+    }
 #pragma unroll
     for (int u = 0; u < 2; u++) {
       if (kidx[u] >= 0) {
-        atomicAdd(vsrc + 2 * kidx[u], make_float4(SV[u].x, SV[u].y, SX[u].x, SX[u].y));
-        atomicAdd(vsrc + 2 * kidx[u] + 1, make_float4(SY[u].x, SY[u].y, SZ[u].x, SZ[u].y));
+        atomicAdd(vsrc + 2L * kidx[u], make_float4(SV[u].x, SV[u].y, SX[u].x, SX[u].y));
+        atomicAdd(vsrc + 2L * kidx[u] + 1, make_float4(SY[u].x, SY[u].y, SZ[u].x, SZ[u].y));
       }
     }
   }
-  if (active) {
-    const double qr = qcaller[2 * o], qi = qcaller[2 * o + 1];
-    acc[0] -= fself_r * qr - fself_i * qi;  // src/Interface.cpp:2909-2910
-    acci[0] -= fself_r * qi + fself_i * qr;
-    double2 *Vo = reinterpret_cast<double2 *>(V) + 4 * o;
+}
+
+// Target sums of a complex walk to V (potential times vs, gradient times gs),
+// less the self term (src/Interface.cpp:2909-2910).
+__device__ __forceinline__ void store_targets_cplx(const int4 G, const uint32_t *__restrict__ perm,
+                                                   const double *__restrict__ qcaller,
+                                                   double fself_r, double fself_i, double vs,
+                                                   double gs, double *__restrict__ V, int lane,
+                                                   const double (&acc)[4],
+                                                   const double (&acci)[4]) {
+  if (lane >= G.y) return;
+  const long o = perm[G.x + lane];
+  const double qr = qcaller[2 * o], qi = qcaller[2 * o + 1];
+  double2 *Vo = reinterpret_cast<double2 *>(V) + 4 * o;
+  Vo[0] = make_double2(vs * acc[0] - (fself_r * qr - fself_i * qi),
+                       vs * acci[0] - (fself_r * qi + fself_i * qr));
 #pragma unroll
-    for (int m = 0; m < 4; m++) Vo[m] = make_double2(acc[m], acci[m]);
-  }
+  for (int m = 1; m < 4; m++) Vo[m] = make_double2(gs * acc[m], gs * acci[m]);
 }
 
 // FP32 direct sum of one warp group (see direct.cu for the scheme): targets
@@ -1897,7 +1985,7 @@ __device__ __forceinline__ void direct_group_sym64_dm(
     const PairCoef<double> &k, const double4 *__restrict__ gpos,
     const double4 *__restrict__ spos, const double *__restrict__ qs,
     const double *__restrict__ qcaller, const int4 G, const double4 c,
-    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm,
+    const int2 *__restrict__ segs, const int2 zones, const uint32_t *__restrict__ perm,
     double *__restrict__ vsrc, double4 *tsm, int lane, int part, int nsplit,
     double (&acc)[4]) {
   const unsigned FULL = 0xffffffffu;
@@ -1931,49 +2019,45 @@ __device__ __forceinline__ void direct_group_sym64_dm(
     acc[3] = fma(-gq, z, acc[3]);
   }
   // half-shell segments in chunks of 64 sources (register prefetch)
-  const int stride = 64 * nsplit;
-  SrcCursor cur[2];
-  cur[0] = SrcCursor{G.z, lane + 64 * part};
-  cur[0].normalize(segs, G.w);
-  cur[1] = SrcCursor{cur[0].seg, cur[0].off + 32};
-  cur[1].normalize(segs, G.w);
-  bool v[2];
+  ZoneWalk<2> walk(segs, G, zones, lane, part, nsplit);
   double4 p[2];
   int slot[2] = {-1, -1};  // source-side slots (brick positions)
 #pragma unroll
   for (int i = 0; i < 2; i++) {
-    v[i] = cur[i].seg < G.w;
     p[i] = make_double4(0, 0, 0, 0);
-    if (v[i]) {
-      const long j = (long)segs[cur[i].seg].x + cur[i].off;
+    if (walk.v[i]) {
+      const long j = walk.index(i);
       p[i] = spos[j], slot[i] = (int)p[i].w, p[i].w = qs[j];
     }
   }
-  while (__any_sync(FULL, v[0])) {
+  while (walk.any()) {
+    const int zone = walk.zone;
     // empty slots far away on the other side from idle targets, no charge
     double4 src[2];
     int to[2];
 #pragma unroll
     for (int i = 0; i < 2; i++) {
       src[i] = make_double4(-1e150, -1e150, -1e150, 0.0);
-      to[i] = v[i] ? slot[i] : -1;
-      if (v[i])
+      to[i] = walk.v[i] ? slot[i] : -1;
+      if (walk.v[i])
         src[i] = make_double4((p[i].x - c.x) * ir, (p[i].y - c.y) * ir, (p[i].z - c.z) * ir,
                               p[i].w);
-      cur[i].off += stride;
-      cur[i].normalize(segs, G.w);
-      v[i] = cur[i].seg < G.w;
-      if (v[i]) {
-        const long j = (long)segs[cur[i].seg].x + cur[i].off;
+    }
+    walk.next();
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      if (walk.v[i]) {
+        const long j = walk.index(i);
         p[i] = spos[j], slot[i] = (int)p[i].w, p[i].w = qs[j];
       }
-    }
     double aV = 0, aX = 0, aY = 0, aZ = 0;                   // target side, rotating
     double S[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};           // source side
     const int next = (lane + 1) & 31;
+    // all targets, or the half that the zone reaches
+    const int mask = zone == 0 ? 31 : 15, from = zone == 2 ? 16 : 0;
 #pragma unroll 2
-    for (int kk = 0; kk < 32; kk++) {
-      const double4 T = tsm[(lane + kk) & 31];
+    for (int kk = 0; kk <= mask; kk++) {
+      const double4 T = tsm[from + ((lane + kk) & mask)];
 #pragma unroll
       for (int i = 0; i < 2; i++) {
         const double x = T.x - src[i].x, y = T.y - src[i].y, z = T.z - src[i].z;
@@ -1997,10 +2081,16 @@ __device__ __forceinline__ void direct_group_sym64_dm(
       aY = __shfl_sync(FULL, aY, next);
       aZ = __shfl_sync(FULL, aZ, next);
     }
-    acc[0] += aV;
-    acc[1] += aX;
-    acc[2] += aY;
-    acc[3] += aZ;
+    if (zone != 0) {  // lanes l and l + 16 hold half of the sums of one target
+      aV += __shfl_xor_sync(FULL, aV, 16), aX += __shfl_xor_sync(FULL, aX, 16);
+      aY += __shfl_xor_sync(FULL, aY, 16), aZ += __shfl_xor_sync(FULL, aZ, 16);
+    }
+    if (zone == 0 || lane >> 4 == zone - 1) {
+      acc[0] += aV;
+      acc[1] += aX;
+      acc[2] += aY;
+      acc[3] += aZ;
+    }
 #pragma unroll
     for (int i = 0; i < 2; i++)
       if (to[i] >= 0) {
@@ -2090,7 +2180,7 @@ __device__ __forceinline__ void direct_group_sym64_helm(
     const PairCoef<double> &k, const double4 *__restrict__ gpos,
     const double4 *__restrict__ spos, const double *__restrict__ qs,
     const double *__restrict__ qcaller, const int4 G, const double4 c,
-    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm,
+    const int2 *__restrict__ segs, const int2 zones, const uint32_t *__restrict__ perm,
     double *__restrict__ vsrc, double (*tsm)[32], int lane, int part, int nsplit,
     double (&acc)[4], double (&acci)[4]) {
   const unsigned FULL = 0xffffffffu;
@@ -2125,39 +2215,36 @@ __device__ __forceinline__ void direct_group_sym64_helm(
     acc[2] = fma(gr, y, acc[2]), acci[2] = fma(gi, y, acci[2]);
     acc[3] = fma(gr, z, acc[3]), acci[3] = fma(gi, z, acci[3]);
   }
-  const int stride = 32 * nsplit;
-  SrcCursor cur{G.z, lane + 32 * part};
-  cur.normalize(segs, G.w);
-  bool v = cur.seg < G.w;
+  ZoneWalk<1> walk(segs, G, zones, lane, part, nsplit);
   double4 p = make_double4(0, 0, 0, 0);
   double2 q = make_double2(0, 0);
-  if (v) {
-    const long j = (long)segs[cur.seg].x + cur.off;
+  if (walk.v[0]) {
+    const long j = walk.index(0);
     p = spos[j], q = reinterpret_cast<const double2 *>(qs)[j];
   }
-  while (__any_sync(FULL, v)) {
+  while (walk.any()) {
+    const int zone = walk.zone;
     // empty slots far away on the other side from idle targets, no charge
     double sx = -1e150, sy = -1e150, sz = -1e150;
     double2 sq = make_double2(0.0, 0.0);
     int slot = -1;
-    if (v) {
+    if (walk.v[0]) {
       sx = (p.x - c.x) * ir, sy = (p.y - c.y) * ir, sz = (p.z - c.z) * ir;
       sq = q;
       slot = (int)p.w;
     }
-    cur.off += stride;
-    cur.normalize(segs, G.w);
-    v = cur.seg < G.w;
-    if (v) {
-      const long j = (long)segs[cur.seg].x + cur.off;
+    walk.next();
+    if (walk.v[0]) {
+      const long j = walk.index(0);
       p = spos[j], q = reinterpret_cast<const double2 *>(qs)[j];
     }
     double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // target side, rotating
     double S[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // source side
     const int next = (lane + 1) & 31;
+    const int mask = zone == 0 ? 31 : 15, from = zone == 2 ? 16 : 0;
 #pragma unroll 1
-    for (int kk = 0; kk < 32; kk++) {
-      const int t = (lane + kk) & 31;
+    for (int kk = 0; kk <= mask; kk++) {
+      const int t = from + ((lane + kk) & mask);
       const double x = tsm[0][t] - sx, y = tsm[1][t] - sy, z = tsm[2][t] - sz;
       const double r2 = fma(x, x, fma(y, y, z * z));
       const bool hit = inside(r2);
@@ -2178,29 +2265,18 @@ __device__ __forceinline__ void direct_group_sym64_helm(
 #pragma unroll
       for (int m = 0; m < 8; m++) a[m] = __shfl_sync(FULL, a[m], next);
     }
+    if (zone != 0)  // lanes l and l + 16 hold half of the sums of one target
 #pragma unroll
-    for (int m = 0; m < 4; m++) acc[m] += a[2 * m], acci[m] += a[2 * m + 1];
+      for (int m = 0; m < 8; m++) a[m] += __shfl_xor_sync(FULL, a[m], 16);
+    if (zone == 0 || lane >> 4 == zone - 1)
+#pragma unroll
+      for (int m = 0; m < 4; m++) acc[m] += a[2 * m], acci[m] += a[2 * m + 1];
     if (slot >= 0) {
       double *d = vsrc + 8L * slot;
 #pragma unroll
       for (int m = 0; m < 8; m++) atomicAdd(d + m, (m < 2 ? ir : gsc) * S[m]);
     }
   }
-}
-
-// Its target sums to V, less the self term (src/Interface.cpp:2909-2910).
-__device__ __forceinline__ void store_targets64_cplx(
-    const int4 G, const uint32_t *__restrict__ perm, const double *__restrict__ qcaller,
-    double fself_r, double fself_i, double ir, double *__restrict__ V, int lane,
-    const double (&acc)[4], const double (&acci)[4]) {
-  if (lane >= G.y) return;
-  const long o = perm[G.x + lane];
-  const double qr = qcaller[2 * o], qi = qcaller[2 * o + 1], g = ir * ir;
-  double2 *Vo = reinterpret_cast<double2 *>(V) + 4 * o;
-  Vo[0] = make_double2(ir * acc[0] - (fself_r * qr - fself_i * qi),
-                       ir * acci[0] - (fself_r * qi + fself_i * qr));
-#pragma unroll
-  for (int m = 1; m < 4; m++) Vo[m] = make_double2(g * acc[m], g * acci[m]);
 }
 
 // Target sums of the FP64 pair-once walk to V (sums scaled by vs, gs), less

@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(32 * kGroupWarps, 4) direct_sym_kernel(
     PairCoef<float> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const float *__restrict__ qs, const double *__restrict__ qcaller,
     const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
-    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, long ngroups,
+    const int2 *__restrict__ segs, const int2 *__restrict__ zones,
+    const uint32_t *__restrict__ perm, long ngroups,
     float refine2, double fself_r, double *__restrict__ V, float4 *__restrict__ vsrc) {
   __shared__ float4 tsm[kGroupWarps][32];  // group targets in pairs, heads and charges
   __shared__ float4 tlo[kGroupWarps][32];  // residuals of the target coordinates
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(32 * kGroupWarps, 4) direct_sym_kernel(
   if (g >= ngroups) return;  // warp-uniform; nothing below synchronises the block
   double acc[4] = {0, 0, 0, 0};
   const int4 G = groups[g];
-  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, perm, refine2, vsrc,
+  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, refine2, vsrc,
                              tsm[wid], tlo[wid], lane, 0, 1, acc);
   sym_store(k, G, perm, qcaller, fself_r, V, lane, acc);
 }
@@ -222,8 +223,9 @@ __global__ void __launch_bounds__(32 * kMaxSplit) direct_sym_split_kernel(
     PairCoef<float> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const float *__restrict__ qs, const double *__restrict__ qcaller,
     const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
-    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, float refine2,
-    double fself_r, double *__restrict__ V, float4 *__restrict__ vsrc) {
+    const int2 *__restrict__ segs, const int2 *__restrict__ zones,
+    const uint32_t *__restrict__ perm, float refine2, double fself_r, double *__restrict__ V,
+    float4 *__restrict__ vsrc) {
   __shared__ float4 tsm[kMaxSplit][32];
   __shared__ float4 tlo[kMaxSplit][32];
   __shared__ double red[kMaxSplit][32][4];
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(32 * kMaxSplit) direct_sym_split_kernel(
   const long g = blockIdx.x;
   double acc[4] = {0, 0, 0, 0};
   const int4 G = groups[g];
-  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, perm, refine2, vsrc,
+  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, refine2, vsrc,
                              tsm[wid], tlo[wid], lane, wid, nsplit, acc);
   reduce_parts(acc, red, wid, nsplit, lane);
   if (wid == 0) sym_store(k, G, perm, qcaller, fself_r, V, lane, acc);
@@ -254,22 +256,36 @@ __global__ void merge_source_kernel(float4 *__restrict__ vsrc, const uint32_t *_
   *o = v;
 }
 
-// FP32 Helmholtz DM form (direct_group_sym_helm).
-template <int ND>
-__global__ void __launch_bounds__(32 * kGroupWarps) direct_sym_helm_kernel(
+// FP32 Helmholtz DM form (direct_group_sym_helm): CTAs of kGroupWarps groups, or
+// (SPLIT) of one group.
+template <int ND, bool SPLIT>
+__global__ void __launch_bounds__(32 * (SPLIT ? kMaxSplit : kGroupWarps), SPLIT ? 1 : 4)
+    direct_sym_helm_kernel(
     PairCoef<float> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const float *__restrict__ qs, const double *__restrict__ qcaller,
     const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
-    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, long ngroups,
-    float refine2, double fself_r, double fself_i, double *__restrict__ V,
-    float4 *__restrict__ vsrc) {
-  __shared__ float4 th[kGroupWarps][32];  // group targets: heads, Re q
-  __shared__ float4 tl[kGroupWarps][32];  // residuals, Im q
+    const int2 *__restrict__ segs, const int2 *__restrict__ zones,
+    const uint32_t *__restrict__ perm, long ngroups, float refine2, double fself_r,
+    double fself_i, double *__restrict__ V, float4 *__restrict__ vsrc) {
+  constexpr int W = SPLIT ? kMaxSplit : kGroupWarps;
+  __shared__ float4 th[W][32];  // group targets: heads, Re q
+  __shared__ float4 tl[W][32];  // residuals, Im q
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long g = (long)blockIdx.x * kGroupWarps + wid;
-  if (g >= ngroups) return;  // warp-uniform
-  direct_group_sym_helm<ND>(k, gpos, spos, qs, qcaller, groups[g], gcen[g], segs, perm, refine2,
-                            fself_r, fself_i, V, vsrc, th[wid], tl[wid], lane);
+  const int nsplit = SPLIT ? blockDim.x >> 5 : 1, part = SPLIT ? wid : 0;
+  const long g = SPLIT ? (long)blockIdx.x : (long)blockIdx.x * kGroupWarps + wid;
+  if (g >= ngroups) return;  // warp-uniform (SPLIT: no CTA is past the end)
+  double acc[4] = {0, 0, 0, 0}, acci[4] = {0, 0, 0, 0};
+  const int4 G = groups[g];
+  direct_group_sym_helm<ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, refine2,
+                            vsrc, th[wid], tl[wid], lane, part, nsplit, acc, acci);
+  if constexpr (SPLIT) {
+    __shared__ double red[kMaxSplit][32][4];
+    reduce_parts(acc, red, wid, nsplit, lane);
+    __syncthreads();
+    reduce_parts(acci, red, wid, nsplit, lane);
+    if (wid > 0) return;
+  }
+  store_targets_cplx(G, perm, qcaller, fself_r, fself_i, 1.0, 1.0, V, lane, acc, acci);
 }
 
 // Complex V[caller(i)][0..3] += vsrc[2i], vsrc[2i + 1] (re, im pairs), then zero.
@@ -291,10 +307,18 @@ template <int ND>
 static void sym_helm_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
   const long blocks = (h->n_hgroups + kGroupWarps - 1) / kGroupWarps;
   if (blocks == 0) return;
-  direct_sym_helm_kernel<ND><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
-      make_pair_coef<float>(h), h->d_gpos, h->d_spos, (const float *)a.q, a.qcaller,
-      h->d_hgroups, h->d_hcen, h->d_hsegs, h->d_cperm, h->n_hgroups, (float)h->refine2,
-      a.fself_r, a.fself_i, a.V, h->d_vsrc);
+  const PairCoef<float> k = make_pair_coef<float>(h);
+  const int split = split_warps(h->n_hgroups);
+  if (split > 1)
+    direct_sym_helm_kernel<ND, true><<<(unsigned)h->n_hgroups, 32 * split, 0, s>>>(
+        k, h->d_gpos, h->d_spos, (const float *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
+        h->d_hsegs, h->d_hzones, h->d_cperm, h->n_hgroups, (float)h->refine2, a.fself_r,
+        a.fself_i, a.V, h->d_vsrc);
+  else
+    direct_sym_helm_kernel<ND, false><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
+        k, h->d_gpos, h->d_spos, (const float *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
+        h->d_hsegs, h->d_hzones, h->d_cperm, h->n_hgroups, (float)h->refine2, a.fself_r,
+        a.fself_i, a.V, h->d_vsrc);
   merge_or_defer(h, a, s, 1.0, 1.0);
 }
 
@@ -306,12 +330,12 @@ static void sym_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
   if (split > 1) {
     direct_sym_split_kernel<FUNC, ND><<<(unsigned)h->n_hgroups, 32 * split, 0, s>>>(
         k, h->d_gpos, h->d_spos, (const float *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
-        h->d_hsegs, h->d_cperm, (float)h->refine2, a.fself_r, a.V, h->d_vsrc);
+        h->d_hsegs, h->d_hzones, h->d_cperm, (float)h->refine2, a.fself_r, a.V, h->d_vsrc);
   } else {
     const long blocks = (h->n_hgroups + kGroupWarps - 1) / kGroupWarps;
     direct_sym_kernel<FUNC, ND><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
         k, h->d_gpos, h->d_spos, (const float *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
-        h->d_hsegs, h->d_cperm, h->n_hgroups, (float)h->refine2, a.fself_r, a.V, h->d_vsrc);
+        h->d_hsegs, h->d_hzones, h->d_cperm, h->n_hgroups, (float)h->refine2, a.fself_r, a.V, h->d_vsrc);
   }
   merge_or_defer(h, a, s, k.vscale, k.gscale);
 }
@@ -322,7 +346,8 @@ __global__ void __launch_bounds__(32 * kGroupWarps) direct_sym64_kernel(
     PairCoef<double> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const double *__restrict__ qs, const double *__restrict__ qcaller,
     const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
-    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, long ngroups,
+    const int2 *__restrict__ segs, const int2 *__restrict__ zones,
+    const uint32_t *__restrict__ perm, long ngroups,
     double fself_r, double *__restrict__ V, double *__restrict__ vsrc) {
   __shared__ double4 tsm[kGroupWarps][32];  // group targets (x, y, z, q)
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -331,7 +356,7 @@ __global__ void __launch_bounds__(32 * kGroupWarps) direct_sym64_kernel(
   if constexpr (SPLIT == 0) {
     double acc[4] = {0, 0, 0, 0};
     const int4 G = groups[g];
-    direct_group_sym64_dm<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, perm, vsrc,
+    direct_group_sym64_dm<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, vsrc,
                                     tsm[wid], lane, 0, 1, acc);
     store_targets64(G, perm, qcaller, fself_r, k.vscale, k.gscale, V, lane, acc);
   } else
@@ -345,7 +370,8 @@ __global__ void __launch_bounds__(32 * kMaxSplit) direct_sym64_split_kernel(
     PairCoef<double> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const double *__restrict__ qs, const double *__restrict__ qcaller,
     const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
-    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, double fself_r,
+    const int2 *__restrict__ segs, const int2 *__restrict__ zones,
+    const uint32_t *__restrict__ perm, double fself_r,
     double *__restrict__ V, double *__restrict__ vsrc) {
   __shared__ double4 tsm[kMaxSplit][32];
   __shared__ double red[kMaxSplit][32][4];
@@ -353,7 +379,7 @@ __global__ void __launch_bounds__(32 * kMaxSplit) direct_sym64_split_kernel(
   const long g = blockIdx.x;
   double acc[4] = {0, 0, 0, 0};
   const int4 G = groups[g];
-  direct_group_sym64_dm<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, perm, vsrc,
+  direct_group_sym64_dm<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, vsrc,
                                   tsm[wid], lane, wid, nsplit, acc);
   reduce_parts(acc, red, wid, nsplit, lane);
   if (wid == 0) store_targets64(G, perm, qcaller, fself_r, k.vscale, k.gscale, V, lane, acc);
@@ -382,14 +408,14 @@ static void sym64_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream_t s)
     if (split > 1) {
       direct_sym64_split_kernel<FUNC, ND><<<(unsigned)h->n_hgroups, 32 * split, 0, s>>>(
           make_pair_coef<double>(h), h->d_gpos, h->d_spos, (const double *)a.q, a.qcaller,
-          h->d_hgroups, h->d_hcen, h->d_hsegs, h->d_cperm, a.fself_r, a.V, h->d_vsrc64);
+          h->d_hgroups, h->d_hcen, h->d_hsegs, h->d_hzones, h->d_cperm, a.fself_r, a.V, h->d_vsrc64);
       merge_or_defer(h, a, s, 1.0, 1.0);
       return;
     }
   }
   direct_sym64_kernel<FUNC, SPLIT, ND><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
       make_pair_coef<double>(h), h->d_gpos, h->d_spos, (const double *)a.q, a.qcaller,
-      h->d_hgroups, h->d_hcen, h->d_hsegs, h->d_cperm, h->n_hgroups, a.fself_r, a.V,
+      h->d_hgroups, h->d_hcen, h->d_hsegs, h->d_hzones, h->d_cperm, h->n_hgroups, a.fself_r, a.V,
       h->d_vsrc64);
   merge_or_defer(h, a, s, 1.0, 1.0);
 }
@@ -401,7 +427,8 @@ __global__ void __launch_bounds__(32 * (SPLIT ? kMaxSplit : kGroupWarps), SPLIT 
     PairCoef<double> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const double *__restrict__ qs, const double *__restrict__ qcaller,
     const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
-    const int2 *__restrict__ segs, const uint32_t *__restrict__ perm, long ngroups,
+    const int2 *__restrict__ segs, const int2 *__restrict__ zones,
+    const uint32_t *__restrict__ perm, long ngroups,
     double fself_r, double fself_i, double *__restrict__ V, double *__restrict__ vsrc) {
   constexpr int W = SPLIT ? kMaxSplit : kGroupWarps;
   __shared__ double tsm[W][5][32];  // group targets: x, y, z, q
@@ -411,7 +438,7 @@ __global__ void __launch_bounds__(32 * (SPLIT ? kMaxSplit : kGroupWarps), SPLIT 
   if (g >= ngroups) return;  // warp-uniform (SPLIT: no CTA is past the end)
   double acc[4] = {0, 0, 0, 0}, acci[4] = {0, 0, 0, 0};
   const int4 G = groups[g];
-  direct_group_sym64_helm<ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, perm, vsrc, tsm[wid],
+  direct_group_sym64_helm<ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, vsrc, tsm[wid],
                               lane, part, nsplit, acc, acci);
   if constexpr (SPLIT) {
     __shared__ double red[kMaxSplit][32][4];
@@ -420,7 +447,8 @@ __global__ void __launch_bounds__(32 * (SPLIT ? kMaxSplit : kGroupWarps), SPLIT 
     reduce_parts(acci, red, wid, nsplit, lane);
     if (wid > 0) return;
   }
-  store_targets64_cplx(G, perm, qcaller, fself_r, fself_i, k.invR, V, lane, acc, acci);
+  store_targets_cplx(G, perm, qcaller, fself_r, fself_i, k.invR, k.invR * k.invR, V, lane, acc,
+                     acci);
 }
 
 // Complex V[caller(i)][0..3] += vsrc[i] (re, im pairs), then zero.
@@ -447,11 +475,11 @@ static void sym64_helm_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream
   if (split > 1)
     direct_sym64_helm_kernel<ND, true><<<(unsigned)h->n_hgroups, 32 * split, 0, s>>>(
         k, h->d_gpos, h->d_spos, (const double *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
-        h->d_hsegs, h->d_cperm, h->n_hgroups, a.fself_r, a.fself_i, a.V, h->d_vsrc64);
+        h->d_hsegs, h->d_hzones, h->d_cperm, h->n_hgroups, a.fself_r, a.fself_i, a.V, h->d_vsrc64);
   else
     direct_sym64_helm_kernel<ND, false><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
         k, h->d_gpos, h->d_spos, (const double *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
-        h->d_hsegs, h->d_cperm, h->n_hgroups, a.fself_r, a.fself_i, a.V, h->d_vsrc64);
+        h->d_hsegs, h->d_hzones, h->d_cperm, h->n_hgroups, a.fself_r, a.fself_i, a.V, h->d_vsrc64);
   merge_or_defer(h, a, s, 1.0, 1.0);
 }
 
@@ -487,15 +515,15 @@ void launch_merge_source(npme_handle *h, double *V, cudaStream_t s, double vs, d
 // Ewald split, in FP64 the real kernels (any order, original Ewald
 // included); FP64 Helmholtz and caller-defined complex kernels walk the full
 // segments.
-bool pairs_once(const npme_handle *h) {
-  if (!h->use_sym || h->n_hgroups == 0) return false;
-  if (h->user_kernel) return !h->complex_kernel;  // the functor's scalar pair kernel
-  const int f = h->p.funcType;
+bool needs_full_lists(const npme_handle *h) {
+  if (!h->use_sym) return true;
+  if (h->user_kernel) return h->complex_kernel;  // real: the functor's scalar pair kernel
   // FP64 Helmholtz: its argument reduction holds for moderate arguments
-  if (f == NPME_FUNC_HELMHOLTZ)
-    return h->fp32 || std::fabs(h->p.k0_r) * h->p.Rdir < kMaxHelmArg;
-  return f == NPME_FUNC_LAPLACE || f == NPME_FUNC_RALPHA;
+  return h->p.funcType == NPME_FUNC_HELMHOLTZ && !h->fp32 &&
+         !(std::fabs(h->p.k0_r) * h->p.Rdir < kMaxHelmArg);
 }
+
+bool pairs_once(const npme_handle *h) { return h->n_hgroups > 0 && !needs_full_lists(h); }
 
 static bool sym_launch(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
   if (!pairs_once(h)) return false;
@@ -605,9 +633,10 @@ int launch_direct(npme_handle *h, const double *d_q, double *d_V, cudaStream_t s
   return launch_direct_args(h, a, s);
 }
 
-// Ordered pairs with 0 < r <= Rdir (FP64 distances) over the one-sided group
-// walk, every target of a group against every source of its segments: the
-// work count of the roofline report (set-up only, not on the CalcV path).
+// Unordered pairs with 0 < r <= Rdir (FP64 distances) over the pair-once
+// lists: every target of a group against the later ones of its group and every
+// source of its half-shell segments: the work count of the roofline report
+// (not on the CalcV path).
 __global__ void __launch_bounds__(32 * kGroupWarps) count_pairs_kernel(
     const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const int4 *__restrict__ groups, const int2 *__restrict__ segs, long ngroups, double R2,
@@ -620,6 +649,17 @@ __global__ void __launch_bounds__(32 * kGroupWarps) count_pairs_kernel(
   const int4 G = groups[g];
   const double4 t = lane < G.y ? gpos[G.x + lane] : make_double4(1e150, 1e150, 1e150, 0.0);
   unsigned long long mine = 0;
+  auto count_chunk = [&](int from, int cnt) {
+    for (int s = from; s < cnt; s++) {
+      const double4 q = sp[wid][s];
+      const double x = t.x - q.x, y = t.y - q.y, z = t.z - q.z;
+      const double r2 = x * x + y * y + z * z;
+      mine += (r2 <= R2 && r2 > 0.0) ? 1ull : 0ull;
+    }
+  };
+  sp[wid][lane] = t;
+  __syncwarp();
+  if (lane < G.y) count_chunk(lane + 1, G.y);
   SrcCursor cur{G.z, lane};
   cur.normalize(segs, G.w);
   while (__any_sync(FULL, cur.seg < G.w)) {
@@ -628,12 +668,7 @@ __global__ void __launch_bounds__(32 * kGroupWarps) count_pairs_kernel(
     __syncwarp();
     if (v) sp[wid][lane] = spos[(long)segs[cur.seg].x + cur.off];
     __syncwarp();
-    for (int s = 0; s < cnt; s++) {
-      const double4 q = sp[wid][s];
-      const double x = t.x - q.x, y = t.y - q.y, z = t.z - q.z;
-      const double r2 = x * x + y * y + z * z;
-      mine += (r2 <= R2 && r2 > 0.0) ? 1ull : 0ull;
-    }
+    count_chunk(0, cnt);
     cur.off += 32;
     cur.normalize(segs, G.w);
   }
@@ -643,10 +678,11 @@ __global__ void __launch_bounds__(32 * kGroupWarps) count_pairs_kernel(
 }
 
 void launch_count_pairs(npme_handle *h, unsigned long long *d_count, cudaStream_t s) {
-  const long blocks = (h->n_groups + kGroupWarps - 1) / kGroupWarps;
+  const long blocks = (h->n_hgroups + kGroupWarps - 1) / kGroupWarps;
   if (blocks == 0) return;
   count_pairs_kernel<<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
-      h->d_gpos, h->d_spos, h->d_groups, h->d_segs, h->n_groups, h->p.Rdir * h->p.Rdir, d_count);
+      h->d_gpos, h->d_spos, h->d_hgroups, h->d_hsegs, h->n_hgroups, h->p.Rdir * h->p.Rdir,
+      d_count);
 }
 
 // ---------------------------------------------------------------------------

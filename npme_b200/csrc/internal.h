@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <chrono>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <string>
@@ -159,8 +160,9 @@ struct npme_handle {
   // direct sum (both precisions): warp groups of <= 32 z-sorted points of
   // one xy column and, per group, the source segments (neighbour-column z
   // ranges) that can hold a point within Rdir of the group.  Built once per
-  // geometry.
-  long n_groups = 0, n_segs = 0;
+  // geometry; these lists only for handles that take the one-sided walk
+  // (needs_full_lists).
+  long n_groups = 0;
   double cand_per_point = 0;     // staged source candidates per target point
   double refine2 = 0;            // r^2 below which pair differences are refined
   double4 *d_gpos = nullptr;     // targets in group order, FP64 positions
@@ -175,9 +177,12 @@ struct npme_handle {
   // with their half-shell segments (sources in later coarse columns, or later
   // in the group's own column), ordered by their own work
   bool use_sym = true;
-  long n_hgroups = 0, n_hsegs = 0;
+  long n_hgroups = 0;
   double hcand_per_point = 0;    // half-shell candidates per target point
   int4 *d_hgroups = nullptr;
+  // per group the ends of the segments within reach of both halves of its
+  // targets and of the lower half only; the upper half's follow up to the end
+  int2 *d_hzones = nullptr;
   double4 *d_hcen = nullptr;
   int2 *d_hsegs = nullptr;
   // the source-side sums are indexed by the source point's position in the
@@ -230,8 +235,9 @@ int device_bbox(npme_handle *h, const double *coord, double mn[3], double mx[3])
 // handles of one precision in one pass on stream s (each with its box, grid
 // geometry and bmin / bmax set, its coordinates on its own stream); hs[0]
 // owns the scratch.  Enqueued without waiting: the counts reach
-// hs[0]->h_counts with the caller's synchronisation.
-int setup_geometry(npme_handle **hs, int R, cudaStream_t s);
+// hs[0]->h_counts with the caller's synchronisation.  hook runs once the
+// buffers of all systems are allocated, before anything else is enqueued.
+int setup_geometry(npme_handle **hs, int R, cudaStream_t s, const std::function<int()> &hook);
 // after that synchronisation: system r's counts (from owner) into handle h,
 // and its stencil check
 int finish_setup(npme_handle *h, const npme_handle *owner, int r);
@@ -263,9 +269,9 @@ size_t own_fft_smem(const FftJob &j, int axis, size_t cbytes);
 // recsum.cu
 int build_kernel_transform(npme_handle *h);  // F-hat, lambda^2 -> d_G
 // The kernel transforms of several handles (one precision), on the owner's
-// stream: one launch per stage for every class of two or more handles with
+// second stream, beside the geometry on its first: one launch per stage for every class of two or more handles with
 // a built-in kernel (real, complex), the rest one by one on their own
-// streams.  status[k] gets each handle's result.
+// second streams.  status[k] gets each handle's result.
 void build_kernel_transforms(npme_handle **hs, int R, npme_handle *owner, int *status);
 void launch_spread(npme_handle *h, const double *d_q, cudaStream_t s);
 void launch_multiply(npme_handle *h, cudaStream_t s);
@@ -294,6 +300,8 @@ int noalloc_preload(std::string &err);
 // true when the direct sum takes the pair-once form (FP32 real DM kernels
 // with the half-shell lists built)
 bool pairs_once(const npme_handle *h);
+// true when it walks each target's sources instead (known before the set-up)
+bool needs_full_lists(const npme_handle *h);
 // V[caller(s)] += the source-side sums of the pair-once walk (times vs for
 // the potential, gs for the gradient; FP32 real, FP32 complex or FP64 by the
 // handle), and zeroes them for the next call

@@ -176,8 +176,7 @@ void release(npme_handle *h) {
   }
   if (!h->caps.empty()) cudaStreamSynchronize(h->stream);
   h->caps.clear();
-  h->n_groups = h->n_segs = 0;
-  h->n_hgroups = h->n_hsegs = 0;
+  h->n_groups = h->n_hgroups = 0;
   h->dev_bytes = 0;
   h->ready = false;
 }
@@ -464,36 +463,43 @@ int npme::setup_many(npme_handle **hs, int R, const size_t *n, const double *con
     if (group.empty()) continue;
     npme_handle *owner = group[0];
     int rc;
+    // FFT plans and kernel transforms depend on the boxes only: they are
+    // enqueued on second streams as soon as the buffers exist and run beside
+    // the geometry
+    auto transforms = [&]() -> int {
+      std::vector<npme_handle *> kt;
+      std::vector<int> kidx;
+      for (size_t k = 0; k < group.size(); k++) {
+        st[idx[k]] = npme::prepare_plans(group[k]);
+        if (!st[idx[k]]) kt.push_back(group[k]), kidx.push_back(idx[k]);
+      }
+      if (kt.empty()) return NPME_OK;
+      npme::StepTimer t("set-up: kernel transforms enqueue", kt.size());
+      std::vector<int> kst(kt.size(), NPME_OK);
+      npme::build_kernel_transforms(kt.data(), (int)kt.size(), owner, kst.data());
+      for (size_t k = 0; k < kt.size(); k++) st[kidx[k]] = kst[k];
+      return NPME_OK;
+    };
     {
       npme::StepTimer t("set-up: geometry enqueue", group.size());
-      rc = npme::setup_geometry(group.data(), (int)group.size(), owner->stream);
+      rc = npme::setup_geometry(group.data(), (int)group.size(), owner->stream, transforms);
     }
     if (rc) {
       for (size_t k = 0; k < group.size(); k++) {
+        cudaStreamSynchronize(group[k]->stream2);  // transforms already enqueued
         if (group[k] != owner) group[k]->err = owner->err;
         st[idx[k]] = rc;
       }
       continue;
     }
-    std::vector<npme_handle *> kt;
-    std::vector<int> kidx;
-    for (size_t k = 0; k < group.size(); k++) {
-      st[idx[k]] = npme::prepare_plans(group[k]);
-      if (!st[idx[k]]) kt.push_back(group[k]), kidx.push_back(idx[k]);
-    }
-    if (!kt.empty()) {
-      npme::StepTimer t("set-up: kernel transforms enqueue", kt.size());
-      std::vector<int> kst(kt.size(), NPME_OK);
-      npme::build_kernel_transforms(kt.data(), (int)kt.size(), owner, kst.data());
-      for (size_t k = 0; k < kt.size(); k++) st[kidx[k]] = kst[k];
-    }
     npme::StepTimer t_wait("set-up: wait for the device and read the counts", group.size());
-    // the owner's stream carries the shared passes; every handle's stream
-    // its own transform: CalcV may be enqueued on any stream, so the set-up
-    // completes here (and the counts arrive)
+    // the owner's streams carry the shared passes; every handle's streams its
+    // own copies and transform: CalcV may be enqueued on any stream, so the
+    // set-up completes here (and the counts arrive)
     for (size_t k = 0; k < group.size(); k++) {
       npme_handle *h = group[k];
-      const cudaError_t e = cudaStreamSynchronize(h->stream);
+      cudaError_t e = cudaStreamSynchronize(h->stream);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream2);
       if (e != cudaSuccess && !st[idx[k]])
         st[idx[k]] = fail(h, NPME_ECUDA, std::string("set-up: ") + cudaGetErrorString(e));
     }
@@ -882,13 +888,13 @@ int npme_gpu_count_pairs(npme_handle *h, unsigned long long *unordered_pairs) {
   CK(cudaMalloc(&d_count, sizeof(unsigned long long)));
   cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), h->stream);
   npme::launch_count_pairs(h, d_count, h->stream);
-  unsigned long long ordered = 0;
-  cudaError_t e = cudaMemcpyAsync(&ordered, d_count, sizeof(ordered), cudaMemcpyDeviceToHost,
+  unsigned long long pairs = 0;
+  cudaError_t e = cudaMemcpyAsync(&pairs, d_count, sizeof(pairs), cudaMemcpyDeviceToHost,
                                   h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   cudaFree(d_count);
   if (e != cudaSuccess) return fail(h, NPME_ECUDA, cudaGetErrorString(e));
-  *unordered_pairs = ordered / 2;
+  *unordered_pairs = pairs;
   return NPME_OK;
 }
 

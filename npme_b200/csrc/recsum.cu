@@ -692,8 +692,8 @@ static int kt_launch_one(npme_handle *h, const KtSys &d, cudaStream_t s) {
 
 int build_kernel_transform(npme_handle *h) {
   KtSys d;
-  const int rc = kt_prepare(h, h->stream, &d);
-  return rc ? rc : kt_launch_one(h, d, h->stream);
+  const int rc = kt_prepare(h, h->stream2, &d);
+  return rc ? rc : kt_launch_one(h, d, h->stream2);
 }
 
 // Layout of one class of handles (the same precision and kernel type,
@@ -738,15 +738,15 @@ static void kt_launch_class(const KtSys *dd, int R, bool cplx, bool fp32, long t
   }
 }
 
-// The kernel transforms of a set-up pass (one precision), on the owner's
+// The kernel transforms of a set-up pass (one precision), on the owner's second
 // stream: a class of two or more handles (built-in real kernels, built-in
 // complex kernels) in one launch per stage, caller-defined kernels and
-// classes of one handle by handle on their own streams.  One launch per
+// classes of one handle by handle on their own second streams.  One launch per
 // stage instead of five per handle: about 4 % more served capacity at the
 // best passes of a serving stream.
 void build_kernel_transforms(npme_handle **hs, int R, npme_handle *owner, int *status) {
   npme_handle *h = owner;  // errors of the shared steps are recorded on the owner
-  const cudaStream_t s = owner->stream;
+  const cudaStream_t s = owner->stream2;
   std::vector<int> cls(R, -1);
   int count[2] = {0, 0};
   for (int r = 0; r < R; r++)
@@ -802,7 +802,10 @@ void build_kernel_transforms(npme_handle **hs, int R, npme_handle *owner, int *s
   KtSys *hd = static_cast<KtSys *>(h->h_ktdesc);
   if (n0) std::copy(ds[0].begin(), ds[0].end(), hd);
   if (n1) std::copy(ds[1].begin(), ds[1].end(), hd + n0);
-  cudaError_t e = cudaMemcpyAsync(h->d_ktdesc, hd, bytes, cudaMemcpyHostToDevice, s);
+  // the descriptor buffer comes from the owner's stream
+  cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(s, h->ev_fork, 0);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h->d_ktdesc, hd, bytes, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) {
     const KtSys *dd = static_cast<const KtSys *>(h->d_ktdesc);
     const bool fp32 = owner->fp32;

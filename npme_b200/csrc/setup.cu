@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -154,6 +155,9 @@ struct SysDesc {
   BinGeom g;
   GroupGeom gg;
   long n, nbt, ncol, nscol, ngb;
+  long wmax;         // segments of a group at most: the stride of its list
+  bool full;         // the one-sided walk's lists are wanted too
+  bool zones;        // the half shell's segments are cut into zones
   long p_off, b_off, c_off, s_off, g_off;
   const double *coord;
   void *bpts;        // BrickPoint<T>[n]
@@ -163,23 +167,27 @@ struct SysDesc {
   double4 *gpos, *spos;
   int2 *segs, *hsegs;
   int4 *groups, *hgroups;
+  int2 *hzones;
   double4 *gcen, *hcen;
 };
 
 // Per system, accumulated on the device.
+constexpr int kWorkBins = 1024;
 struct SysStats {
   long long bad;                   // lowest index whose stencil leaves the octant
   unsigned long long cand, hcand;  // staged (target, source) candidates, both walks
+  // groups per work bin and the places handed out in each, full and half lists
+  int bins[2][kWorkBins], taken[2][kWorkBins];
 };
 
 // The counts the host reads once the set-up has completed.
 struct SetupCounts {
   long long bad;
   unsigned long long cand, hcand;
-  int ngroups, nnonempty, nsegs, nhsegs;
+  int ngroups, nnonempty;
 };
 
-constexpr int kZField = 20;  // bits of the quantised-z field of the column keys
+constexpr int kMaxZBits = 20;  // bits of the quantised z at most
 
 // The system owning element x of an index space with starts off[0..R).
 __device__ __forceinline__ int owner(const long *__restrict__ off, int R, long x) {
@@ -192,27 +200,30 @@ __device__ __forceinline__ int owner(const long *__restrict__ off, int R, long x
   return lo;
 }
 
-__global__ void init_sys_stats_kernel(const SysDesc *__restrict__ d, int R, SysStats *st) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  st[r].bad = d[r].n;
-  st[r].cand = st[r].hcand = 0;
+// one CTA per system
+__global__ void init_sys_stats_kernel(const SysDesc *__restrict__ d, SysStats *st) {
+  SysStats &S = st[blockIdx.x];
+  if (threadIdx.x == 0) {
+    S.bad = d[blockIdx.x].n;
+    S.cand = S.hcand = 0;
+  }
+  for (int i = threadIdx.x; i < 2 * kWorkBins; i += blockDim.x)
+    S.bins[i / kWorkBins][i % kWorkBins] = S.taken[i / kWorkBins][i % kWorkBins] = 0;
 }
 
 // Per point: the spread/interpolation record, its brick-and-bank sort key,
-// its (coarse column, quantised z) and (fine column, quantised z) sort keys;
-// per brick and column the point counts.  Arithmetic as the host restatement
+// its (coarse column, quantised z) and (fine column, quantised z) sort keys (z
+// in the low zf bits).  Arithmetic as the host restatement
 // of the reference (explicit round-to-nearest operations, no contraction),
 // so that every point lands in the same brick, bank and column on any
 // machine.
 template <typename T>
 __global__ void bin_kernel(const SysDesc *__restrict__ d, const long *__restrict__ poff, int R,
-                           long P, int bbits, int cbits, int sbits,
+                           long P, int bbits, int cbits, int sbits, int zf,
                            BrickPoint<T> *__restrict__ pts, unsigned long long *__restrict__ bkey,
                            unsigned long long *__restrict__ ckey,
                            unsigned long long *__restrict__ skey, unsigned *__restrict__ iota,
-                           int *__restrict__ bcount, int *__restrict__ ccount,
-                           int *__restrict__ scount, SysStats *st) {
+                           SysStats *st) {
   const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= P) return;
   const int r = owner(poff, R, p);
@@ -245,9 +256,6 @@ __global__ void bin_kernel(const SysDesc *__restrict__ d, const long *__restrict
   bp.orig = (uint32_t)i;
   pts[p] = bp;
   bkey[p] = ((unsigned long long)r << (bbits + 5)) | ((unsigned long long)bid << 5) | key;
-  // every point is counted in the brick its key names (a point outside the
-  // octant in brick 0), so that the brick starts index the sorted keys
-  atomicAdd(&bcount[D.b_off + bid], 1);
   int cs[2], ss[2];
 #pragma unroll
   for (int a = 0; a < 2; a++) {
@@ -259,11 +267,106 @@ __global__ void bin_kernel(const SysDesc *__restrict__ d, const long *__restrict
   const unsigned long long cc = (unsigned long long)(cs[0] * g.nc[1] + cs[1]);
   const unsigned long long sc = (unsigned long long)(ss[0] * g.ns[1] + ss[1]);
   const unsigned long long zq = zquant(x[2], g.zmin, g.zscale, g.zbits);
-  ckey[p] = ((unsigned long long)r << (cbits + kZField)) | (cc << kZField) | zq;
-  skey[p] = ((unsigned long long)r << (sbits + kZField)) | (sc << kZField) | zq;
-  atomicAdd(&ccount[D.c_off + (long)cc], 1);
-  atomicAdd(&scount[D.s_off + (long)sc], 1);
+  ckey[p] = ((unsigned long long)r << (cbits + zf)) | (cc << zf) | zq;
+  skey[p] = ((unsigned long long)r << (sbits + zf)) | (sc << zf) | zq;
   iota[p] = (unsigned)p;
+}
+
+// Where every brick, coarse column and fine column of the batch begins in its
+// sorted keys (one thread per slot, binary search), and P past the last: the
+// counts are differences of neighbours.  The slot after a system's last brick
+// or column is where the next system begins.  (Counting with atomics in the
+// binning took three quarters of it: a few hundred columns share all points.)
+__global__ void starts_kernel(const SysDesc *__restrict__ d, int R,
+                              const long *__restrict__ boff, const long *__restrict__ coff,
+                              const long *__restrict__ soff, long P, long B, long C, long S,
+                              int bbits, int cbits, int sbits, int zf,
+                              const unsigned long long *__restrict__ bkey,
+                              const unsigned long long *__restrict__ ckey,
+                              const unsigned long long *__restrict__ skey,
+                              int *__restrict__ bstart, int *__restrict__ cstart,
+                              int *__restrict__ sstart) {
+  long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned long long *key = bkey;
+  int *out = bstart;
+  long last = B;
+  const long *off = boff;
+  int idbits = bbits, low = 5;
+  if (t > B) {
+    t -= B + 1, key = ckey, out = cstart, last = C, off = coff, idbits = cbits, low = zf;
+    if (t > C) t -= C + 1, key = skey, out = sstart, last = S, off = soff, idbits = sbits;
+  }
+  if (t > last) return;
+  if (t == last) {
+    out[t] = (int)P;
+    return;
+  }
+  const int r = owner(off, R, t);
+  const unsigned long long want = (((unsigned long long)r << idbits) + (t - off[r])) << low;
+  long lo = 0, hi = P;
+  while (lo < hi) {
+    const long m = (lo + hi) >> 1;
+    if (key[m] < want) lo = m + 1;
+    else hi = m;
+  }
+  out[t] = (int)lo;
+}
+
+// What the two scans of a set-up add up: non-empty bricks (CTA 0) and groups
+// per coarse column (CTA 1).
+struct NonEmpty {
+  const int *start;
+  __host__ __device__ int operator()(int i) const { return start[i + 1] > start[i]; }
+};
+struct GroupsOf {
+  const int *start;
+  __host__ __device__ int operator()(int i) const { return (start[i + 1] - start[i] + 31) / 32; }
+};
+
+// Both exclusive sums in one launch, a CTA each, for up to kOneScan elements.
+constexpr long kOneScan = 1L << 16;
+__global__ void __launch_bounds__(1024) scans_kernel(const int *__restrict__ bstart, int B,
+                                                     int *__restrict__ pos,
+                                                     const int *__restrict__ cstart, int C,
+                                                     int *__restrict__ goff) {
+  __shared__ int warp_sum[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool first = blockIdx.x == 0;
+  const int n = first ? B : C;
+  int *out = first ? pos : goff;
+  // consecutive elements per thread: one pass of loads, one CTA-wide scan
+  const int per = (n + 1023) / 1024, i0 = threadIdx.x * per, i1 = min(n, i0 + per);
+  int sum = 0;
+  for (int i = i0; i < i1; i++) sum += first ? NonEmpty{bstart}(i) : GroupsOf{cstart}(i);
+  int inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  if (lane == 31) warp_sum[w] = inc;
+  __syncthreads();
+  if (w == 0) {
+    int v = warp_sum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    warp_sum[lane] = v;
+  }
+  __syncthreads();
+  int run = inc - sum + (w > 0 ? warp_sum[w - 1] : 0);
+  for (int i = i0; i < i1; i++) {
+    out[i] = run;
+    run += first ? NonEmpty{bstart}(i) : GroupsOf{cstart}(i);
+  }
+}
+
+template <class F>
+__global__ void values_kernel(F f, long n, int *__restrict__ out) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = f((int)i);
 }
 
 // Brick order inside each brick in rounds over the banks: round r holds the
@@ -271,34 +374,32 @@ __global__ void bin_kernel(const SysDesc *__restrict__ d, const long *__restrict
 // ascending, i.e. the order of a stable sort by (system, brick, rank inside
 // the bank, bank).  Input: the point indices sorted by (system, brick, bank)
 // and those keys; one warp per brick slot, lane b owns bank b (keys carry the
-// bank in their low 5 bits).
-__global__ void round_place_kernel(const unsigned long long *__restrict__ key,
-                                   const unsigned *__restrict__ in, const int *__restrict__ bstart,
-                                   const int *__restrict__ bcount, long B,
-                                   unsigned *__restrict__ out) {
-  const long b = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+// bank in their low 5 bits), whose run is found where the bank changes.
+constexpr int kPlaceWarps = 8;
+__global__ void __launch_bounds__(32 * kPlaceWarps)
+    round_place_kernel(const unsigned long long *__restrict__ key,
+                       const unsigned *__restrict__ in, const int *__restrict__ bstart, long B,
+                       unsigned *__restrict__ out) {
+  __shared__ int run[kPlaceWarps][33];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long b = (long)blockIdx.x * kPlaceWarps + w;
   if (b >= B) return;  // warp-uniform
-  const int c = bcount[b];
+  const int s = bstart[b], c = bstart[b + 1] - s;
   if (c == 0) return;
-  const long s = bstart[b], e = s + c;
-  // first position in [s, e) whose bank is >= v (banks ascend in the brick)
-  auto first = [&](unsigned v) {
-    long lo = s, hi = e;
-    while (lo < hi) {
-      const long m = (lo + hi) >> 1;
-      if ((unsigned)(key[m] & 31ull) < v) lo = m + 1;
-      else hi = m;
-    }
-    return lo;
-  };
-  const long lo = first((unsigned)lane), hi = first((unsigned)lane + 1u);
-  const int cnt = (int)(hi - lo);
+  // run[v]: first position whose bank is >= v
+  for (int i = lane; i <= c; i += 32) {
+    const int prev = i > 0 ? (int)(key[s + i - 1] & 31ull) : -1;
+    const int cur = i < c ? (int)(key[s + i] & 31ull) : 32;
+    for (int v = prev + 1; v <= cur; v++) run[w][v] = s + i;
+  }
+  __syncwarp();
+  const int lo = run[w][lane], cnt = run[w][lane + 1] - lo;
   int rounds = cnt;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) rounds = max(rounds, __shfl_xor_sync(0xffffffffu, rounds, o));
   const unsigned below = (1u << lane) - 1u;
-  long base = s;
+  int base = s;
+#pragma unroll 4
   for (int r = 0; r < rounds; r++) {
     const unsigned m = __ballot_sync(0xffffffffu, cnt > r);
     if (cnt > r) out[base + __popc(m & below)] = in[lo + r];
@@ -308,50 +409,40 @@ __global__ void round_place_kernel(const unsigned long long *__restrict__ key,
 
 // Final brick order of every system: its records, the brick-order
 // permutation, and each point's brick-order position (the slot of its
-// source-side direct-sum sums).
+// source-side direct-sum sums); and every system's brick starts (local
+// positions) and non-empty brick list.
 template <typename T>
 __global__ void place_bricks_kernel(const SysDesc *__restrict__ d, const long *__restrict__ poff,
-                                    int R, long P, const unsigned *__restrict__ order,
+                                    const long *__restrict__ boff, int R, long P, long B,
+                                    const unsigned *__restrict__ order,
                                     const BrickPoint<T> *__restrict__ pts,
+                                    const int *__restrict__ start, const int *__restrict__ pos,
                                     unsigned *__restrict__ bpos) {
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= P) return;
-  const int r = owner(poff, R, k);
-  const SysDesc &D = d[r];
-  const long p = order[k], kl = k - D.p_off;
-  reinterpret_cast<BrickPoint<T> *>(D.bpts)[kl] = pts[p];
-  D.bperm[kl] = (uint32_t)(p - D.p_off);
-  bpos[p] = (unsigned)kl;
-}
-
-// flag[b] = 1 for non-empty brick slots (end slots are empty)
-__global__ void nonempty_flags_kernel(const int *__restrict__ count, long nb,
-                                      int *__restrict__ flag) {
-  const long b = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < nb) flag[b] = count[b] > 0;
-}
-
-// Every system's brick starts (local positions) and non-empty brick list.
-__global__ void bricks_kernel(const SysDesc *__restrict__ d, const long *__restrict__ boff, int R,
-                              long B, const int *__restrict__ count, const int *__restrict__ start,
-                              const int *__restrict__ pos) {
-  const long slot = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot >= B) return;
-  const int r = owner(boff, R, slot);
-  const SysDesc &D = d[r];
-  const long b = slot - D.b_off;  // 0 .. nbt (end slot)
-  D.brick_start[b] = start[slot] - start[D.b_off];
-  if (b < D.nbt && count[slot] > 0) D.brick_list[pos[slot] - pos[D.b_off]] = (int)b;
+  if (k < P) {
+    const int r = owner(poff, R, k);
+    const SysDesc &D = d[r];
+    const long p = order[k], kl = k - D.p_off;
+    reinterpret_cast<BrickPoint<T> *>(D.bpts)[kl] = pts[p];
+    D.bperm[kl] = (uint32_t)(p - D.p_off);
+    bpos[p] = (unsigned)kl;
+  }
+  if (k < B) {
+    const int r = owner(boff, R, k);
+    const SysDesc &D = d[r];
+    const long b = k - D.b_off;  // 0 .. nbt (end slot)
+    D.brick_start[b] = start[k] - start[D.b_off];
+    if (b < D.nbt && start[k + 1] > start[k]) D.brick_list[pos[k] - pos[D.b_off]] = (int)b;
+  }
 }
 
 // The direct sum's two orders of every system: local permutations, FP64
-// positions (a source's w holds its brick-order position), the sources'
-// quantised z, and each point's position in the target (group) order.
+// positions (a source's w holds its brick-order position) and each point's
+// position in the target (group) order.
 __global__ void place_orders_kernel(const SysDesc *__restrict__ d, const long *__restrict__ poff,
                                     int R, long P, const unsigned *__restrict__ corder,
                                     const unsigned *__restrict__ sorder,
-                                    const unsigned long long *__restrict__ skey,
-                                    const unsigned *__restrict__ bpos, unsigned *__restrict__ zq,
+                                    const unsigned *__restrict__ bpos,
                                     unsigned *__restrict__ cpos) {
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= P) return;
@@ -365,40 +456,8 @@ __global__ void place_orders_kernel(const SysDesc *__restrict__ d, const long *_
   D.gpos[kl] = make_double4(x[0], x[1], x[2], 0.0);
   const long ps = sorder[k], is = ps - D.p_off;
   D.sperm[kl] = (uint32_t)is;
-  zq[k] = (unsigned)(skey[k] & ((1ull << kZField) - 1ull));
   const double *y = D.coord + 3 * is;
   D.spos[kl] = make_double4(y[0], y[1], y[2], (double)bpos[ps]);
-}
-
-__global__ void gather_u32_kernel(const unsigned *__restrict__ src,
-                                  const unsigned *__restrict__ perm, long n,
-                                  unsigned *__restrict__ out) {
-  const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) out[k] = src[perm[k]];
-}
-
-// groups per coarse column slot: ceil(count / 32) (end slots: 0)
-__global__ void groups_per_column_kernel(const int *__restrict__ ccount, long ncol,
-                                         int *__restrict__ gcount) {
-  const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < ncol) gcount[c] = (ccount[c] + 31) / 32;
-}
-
-// The groups of every column: points [p0, p1) of the batch's target order
-// (runs of 32 in the column), the column and the system.
-__global__ void group_records_kernel(const SysDesc *__restrict__ d, const long *__restrict__ coff,
-                                     int R, long C, const int *__restrict__ cstart,
-                                     const int *__restrict__ goff, int4 *__restrict__ grec) {
-  const long slot = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot >= C) return;
-  const int r = owner(coff, R, slot);
-  const SysDesc &D = d[r];
-  const long c = slot - D.c_off;
-  if (c >= D.ncol) return;  // end slot
-  const int p_end = cstart[slot + 1];
-  long gs = D.g_off + (goff[slot] - goff[D.c_off]);
-  for (int p0 = cstart[slot]; p0 < p_end; p0 += 32, gs++)
-    grec[gs] = make_int4(p0, min(p0 + 32, p_end), (int)c, r);
 }
 
 // the number of groups of system D (on the device)
@@ -406,25 +465,79 @@ __device__ __forceinline__ long sys_groups(const SysDesc &D, const int *__restri
   return goff[D.c_off + D.ncol] - goff[D.c_off];
 }
 
-// Bounding box of every group (warp per group slot): lo/hi corners, and the
-// frame origin (centre) with the half diagonal in w.
-__global__ void group_box_kernel(const SysDesc *__restrict__ d, const long *__restrict__ goffs,
-                                 int R, long G, const int *__restrict__ goff,
-                                 const int4 *__restrict__ grec, double4 *__restrict__ blo,
-                                 double4 *__restrict__ bhi, double4 *__restrict__ cen) {
+// first index in [a, b) with f(index) >= x
+template <class F>
+__device__ __forceinline__ int lower_idx(const F &f, int a, int b, unsigned x) {
+  while (a < b) {
+    const int m = (a + b) >> 1;
+    if (f(m) < x) a = m + 1;
+    else b = m;
+  }
+  return a;
+}
+
+// Bin of a group's work (staged sources): 32 bins per power of two, the
+// heaviest first.
+__device__ __forceinline__ int work_bin(unsigned long long work) {
+  const unsigned u = __float_as_uint((float)min(work, 0x7fffffffull)) >> 18;  // 5 mantissa bits
+  const unsigned one = 0x3f800000u >> 18;                                     // bin of 1
+  return kWorkBins - 1 - (int)min(u > one ? u - one : 0u, (unsigned)kWorkBins - 1);
+}
+
+// One warp per group slot: the group's points (a run of 32 of one coarse
+// column of the batch's target order), its bounding box and frame origin, and
+// its source segments (lanes over the fine columns of the group's window in
+// (s0, s1) order, so that a group's segments come in the same order as a
+// sequential sweep).  A fine column contributes the z range of its sources
+// within Rdir of the group's box: |dz| <= sqrt(Rdir^2 - d_xy^2), d_xy the xy
+// distance from the box to the column; the half shell keeps the fine columns of
+// later coarse columns and, in the group's own coarse column, the sources after
+// the group in the group order.  The half shell's ranges are cut into three
+// zones: within reach of both halves of the group (its targets are in z order),
+// of the lower or of the upper half only; the walks spend half the steps on the
+// last two.  Positions are the batch's (cstart, sstart); the written segments
+// and group records are the system's own (local).  A group's segments start at
+// its number times a bound of their count, so that no pass over all groups has
+// to count them first.
+__global__ void __launch_bounds__(256)
+    groups_kernel(const SysDesc *__restrict__ d, const long *__restrict__ goffs, int R, long G,
+                  const int *__restrict__ goff, const int *__restrict__ cstart,
+                  const int *__restrict__ sstart, const unsigned long long *__restrict__ skey,
+                  int zf, const unsigned *__restrict__ sorder,
+                  const unsigned *__restrict__ cpos, int4 *__restrict__ ug,
+                  int4 *__restrict__ uh, int2 *__restrict__ uz, double4 *__restrict__ cen, int *__restrict__ bin,
+                  int *__restrict__ hbin, SysStats *st) {
   const long slot = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (slot >= G) return;  // warp-uniform
   const int r = owner(goffs, R, slot);
   const SysDesc &D = d[r];
-  if (slot - D.g_off >= sys_groups(D, goff)) return;  // a spare slot of the bound
-  const int4 Gr = grec[slot];
+  const int gi = (int)(slot - D.g_off);
+  if (gi >= sys_groups(D, goff)) return;  // a spare slot of the bound
+  const GroupGeom &gg = D.gg;
+  const unsigned FULL = 0xffffffffu;
+  const unsigned zmask = (unsigned)((1ull << zf) - 1ull);
+  // the coarse column: the last with at most gi groups before it
+  int c, p0, p1;
+  {
+    const int *go = goff + D.c_off;
+    const int want = go[0] + gi;
+    int a = 0, b = (int)D.ncol;  // first column in (a, b] with more than gi groups before it
+    while (a < b) {
+      const int m = (a + b + 1) >> 1;
+      if (go[m] <= want) a = m;
+      else b = m - 1;
+    }
+    c = a;
+    p0 = cstart[D.c_off + c] + 32 * (want - go[c]);
+    p1 = min(p0 + 32, cstart[D.c_off + c + 1]);
+  }
+  const int pl = (int)D.p_off;  // batch position -> system position
   double l[3] = {1e300, 1e300, 1e300}, h[3] = {-1e300, -1e300, -1e300};
-  if (Gr.x + lane < Gr.y) {
-    const double4 p = D.gpos[Gr.x + lane - D.p_off];
+  if (p0 + lane < p1) {
+    const double4 p = D.gpos[p0 + lane - pl];
     l[0] = h[0] = p.x, l[1] = h[1] = p.y, l[2] = h[2] = p.z;
   }
-  const unsigned FULL = 0xffffffffu;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -433,8 +546,6 @@ __global__ void group_box_kernel(const SysDesc *__restrict__ d, const long *__re
       h[a] = fmax(h[a], __shfl_xor_sync(FULL, h[a], o));
     }
   if (lane == 0) {
-    blo[slot] = make_double4(l[0], l[1], l[2], 0.0);
-    bhi[slot] = make_double4(h[0], h[1], h[2], 0.0);
     const double dx = __dsub_rn(h[0], l[0]), dy = __dsub_rn(h[1], l[1]),
                  dz = __dsub_rn(h[2], l[2]);
     cen[slot] = make_double4(
@@ -443,179 +554,180 @@ __global__ void group_box_kernel(const SysDesc *__restrict__ d, const long *__re
         __dmul_rn(0.5, __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
                                             __dmul_rn(dz, dz)))));
   }
-}
-
-// first index in [a, b) with v[index] >= x (lower) or > x (upper)
-__device__ __forceinline__ int lower_idx(const unsigned *__restrict__ v, int a, int b, unsigned x) {
-  while (a < b) {
-    const int m = (a + b) >> 1;
-    if (v[m] < x) a = m + 1;
-    else b = m;
-  }
-  return a;
-}
-__device__ __forceinline__ int upper_idx(const unsigned *__restrict__ v, int a, int b, unsigned x) {
-  while (a < b) {
-    const int m = (a + b) >> 1;
-    if (v[m] <= x) a = m + 1;
-    else b = m;
-  }
-  return a;
-}
-
-// Source segments of every group (warp per group slot; lanes over the fine
-// columns of the group's window in (s0, s1) order, so that a group's
-// segments come in the same order as a sequential sweep).  A fine column
-// contributes the z range of its sources within Rdir of the group's box:
-// |dz| <= sqrt(Rdir^2 - d_xy^2), d_xy the xy distance from the box to the
-// column; the half shell keeps the fine columns of later coarse columns and,
-// in the group's own coarse column, the sources after the group in the
-// group order.  Positions are the batch's (cstart, sstart, fcpos); the
-// written segments and group records are the system's own (local).  FILL =
-// false counts (segments, work, candidates); FILL = true writes the
-// segments at the offsets of the count pass.
-template <bool FILL>
-__global__ void group_segments_kernel(const SysDesc *__restrict__ d, const long *__restrict__ goffs,
-                                      int R, long G, const int *__restrict__ goff,
-                                      const int4 *__restrict__ grec,
-                                      const double4 *__restrict__ blo,
-                                      const double4 *__restrict__ bhi,
-                                      const int *__restrict__ sstart,
-                                      const unsigned *__restrict__ zq,
-                                      const unsigned *__restrict__ fcpos, int *__restrict__ nseg,
-                                      int *__restrict__ nhseg, unsigned *__restrict__ work,
-                                      unsigned *__restrict__ hwork,
-                                      const int *__restrict__ segoff,
-                                      const int *__restrict__ hsegoff, int4 *__restrict__ ug,
-                                      int4 *__restrict__ uh, SysStats *st) {
-  const long slot = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (slot >= G) return;  // warp-uniform
-  const int r = owner(goffs, R, slot);
-  const SysDesc &D = d[r];
-  if (slot - D.g_off >= sys_groups(D, goff)) return;  // a spare slot of the bound
-  const GroupGeom &gg = D.gg;
-  const unsigned FULL = 0xffffffffu;
-  const int4 Gr = grec[slot];
-  const int p0 = Gr.x, p1 = Gr.y, c = Gr.z;
-  const double4 L = blo[slot], Hh = bhi[slot];
-  const double bl[2] = {L.x, L.y}, bh[2] = {Hh.x, Hh.y};
   int lo[2], hi[2];
 #pragma unroll
   for (int a = 0; a < 2; a++) {
     // one column of margin on each side: the distance test below decides
-    lo[a] = max(0, (int)floor((bl[a] - gg.R - gg.mn[a]) / gg.sedge[a]) - 1);
-    hi[a] = min(gg.ns[a] - 1, (int)floor((bh[a] + gg.R - gg.mn[a]) / gg.sedge[a]) + 1);
+    lo[a] = max(0, (int)floor((l[a] - gg.R - gg.mn[a]) / gg.sedge[a]) - 1);
+    hi[a] = min(gg.ns[a] - 1, (int)floor((h[a] + gg.R - gg.mn[a]) / gg.sedge[a]) + 1);
   }
   const int w1 = hi[1] - lo[1] + 1;
   const int nwin = (hi[0] - lo[0] + 1) * w1;
-  int ns_ = 0, nh_ = 0;
-  unsigned long long wk = 0, hwk = 0;
-  const int base = FILL ? segoff[slot] - segoff[D.g_off] : 0;
-  const int hbase = FILL ? hsegoff[slot] - hsegoff[D.g_off] : 0;
-  const int pl = (int)D.p_off;  // batch position -> system position
+  // z extents of the group's halves (targets 0-15 and 16-31)
+  double zl = l[2], zh = h[2], hl[2], hh[2];
+  {
+    double a = 1e300, b = -1e300;
+    if (p0 + lane < p1) a = b = D.gpos[p0 + lane - pl].z;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      a = fmin(a, __shfl_xor_sync(FULL, a, o));
+      b = fmax(b, __shfl_xor_sync(FULL, b, o));
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      hl[i] = __shfl_sync(FULL, a, 16 * i), hh[i] = __shfl_sync(FULL, b, 16 * i);
+  }
+  const int cl = min(16, p1 - p0), cu = p1 - p0 - cl;  // targets of the halves
+  const long stride = D.zones ? 3 * D.wmax : D.wmax;
+  const int base = (int)(gi * stride);
+  auto zq = [&](int i) { return (unsigned)skey[i] & zmask; };
+  auto zquantum = [&](double z) { return zquant(z, gg.zmin, gg.zscale, gg.zbits); };
+  // Window column t: [a, b) the sources within reach of the group (one-sided
+  // walk); of those in the half shell, [u[0], v[0]) within reach of both
+  // halves, [u[1], v[1]) of the lower and [u[2], v[2]) of the upper one only
+  // (whole quanta: every source within reach is inside).
+  auto column = [&](int t, int &a, int &b, int (&u)[3], int (&v)[3]) {
+    a = b = 0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) u[i] = v[i] = 0;
+    if (t >= nwin) return;
+    const int s0 = lo[0] + t / w1, s1 = lo[1] + t % w1;
+    const long sc = D.s_off + (long)s0 * gg.ns[1] + s1;
+    const int zb = sstart[sc], ze = sstart[sc + 1];
+    if (ze <= zb) return;
+    const double l0 = __dadd_rn(gg.mn[0], __dmul_rn((double)s0, gg.sedge[0]));
+    const double h0 = __dadd_rn(l0, gg.sedge[0]);
+    const double l1 = __dadd_rn(gg.mn[1], __dmul_rn((double)s1, gg.sedge[1]));
+    const double h1 = __dadd_rn(l1, gg.sedge[1]);
+    const double dx = fmax(0.0, fmax(__dsub_rn(l0, h[0]), __dsub_rn(l[0], h0)));
+    const double dy = fmax(0.0, fmax(__dsub_rn(l1, h[1]), __dsub_rn(l[1], h1)));
+    const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+    if (d2 > gg.R2) return;
+    const double hz = __dsqrt_rn(__dsub_rn(gg.R2, d2));
+    a = lower_idx(zq, zb, ze, zquantum(__dsub_rn(zl, hz)));
+    b = lower_idx(zq, a, ze, zquantum(__dadd_rn(zh, hz)) + 1u);
+    const long cc = (long)(s0 / kSourceSplit) * gg.nc1 + s1 / kSourceSplit;
+    if (b <= a || cc < c) return;
+    const int a2 =
+        cc == c ? lower_idx([&](int i) { return cpos[sorder[i]]; }, a, b, (unsigned)p1) : a;
+    if (a2 >= b) return;
+    if (!D.zones) {
+      u[0] = a2, v[0] = b;
+      return;
+    }
+    if (cu == 0) {
+      u[1] = a2, v[1] = b;
+      return;
+    }
+    // the halves are in z order: the lower reaches [a2, e), the upper [f, b)
+    const int e = lower_idx(zq, a2, b, zquantum(__dadd_rn(hh[0], hz)) + 1u);
+    const int f = lower_idx(zq, a2, b, zquantum(__dsub_rn(hl[1], hz)));
+    u[0] = f, v[0] = max(e, f);
+    u[1] = a2, v[1] = min(e, f);
+    u[2] = max(e, f), v[2] = b;
+  };
+  // segments of every zone, then their places: both halves, lower, upper
+  int n[3] = {0, 0, 0}, nf = 0;
+  unsigned long long src[4] = {0, 0, 0, 0};  // sources per zone; one-sided walk
   for (int t0 = 0; t0 < nwin; t0 += 32) {
-    const int t = t0 + lane;
-    bool has = false, hhas = false;
-    int a = 0, b = 0, a2 = 0;
-    if (t < nwin) {
-      const int s0 = lo[0] + t / w1, s1 = lo[1] + t % w1;
-      const long sc = D.s_off + (long)s0 * gg.ns[1] + s1;
-      const int zb = sstart[sc], ze = sstart[sc + 1];
-      if (ze > zb) {
-        const double l0 = __dadd_rn(gg.mn[0], __dmul_rn((double)s0, gg.sedge[0]));
-        const double h0 = __dadd_rn(l0, gg.sedge[0]);
-        const double l1 = __dadd_rn(gg.mn[1], __dmul_rn((double)s1, gg.sedge[1]));
-        const double h1 = __dadd_rn(l1, gg.sedge[1]);
-        const double dx = fmax(0.0, fmax(__dsub_rn(l0, bh[0]), __dsub_rn(bl[0], h0)));
-        const double dy = fmax(0.0, fmax(__dsub_rn(l1, bh[1]), __dsub_rn(bl[1], h1)));
-        const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-        if (d2 <= gg.R2) {
-          const double hz = __dsqrt_rn(__dsub_rn(gg.R2, d2));
-          const double zlo = __dsub_rn(L.z, hz), zhi = __dadd_rn(Hh.z, hz);
-          // whole quanta: every source with zlo <= z <= zhi is inside [a, b)
-          a = lower_idx(zq, zb, ze, zquant(zlo, gg.zmin, gg.zscale, gg.zbits));
-          b = upper_idx(zq, a, ze, zquant(zhi, gg.zmin, gg.zscale, gg.zbits));
-          has = b > a;
-          const long cc = (long)(s0 / kSourceSplit) * gg.nc1 + s1 / kSourceSplit;
-          if (has && cc >= c) {
-            a2 = cc == c ? lower_idx(fcpos, a, b, (unsigned)p1) : a;
-            hhas = b > a2;
-          }
-        }
-      }
+    int a, b, u[3], v[3];
+    column(t0 + lane, a, b, u, v);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      n[i] += __popc(__ballot_sync(FULL, v[i] > u[i]));
+      src[i] += (unsigned)max(0, v[i] - u[i]);
     }
-    const unsigned m = __ballot_sync(FULL, has), hm = __ballot_sync(FULL, hhas);
+    src[3] += (unsigned)(b - a);
+  }
+  int at[3] = {base, base + n[0], base + n[0] + n[1]};
+  for (int t0 = 0; t0 < nwin; t0 += 32) {
+    int a, b, u[3], v[3];
+    column(t0 + lane, a, b, u, v);
     const unsigned below = (1u << lane) - 1u;
-    if (FILL) {
-      if (has) D.segs[base + ns_ + __popc(m & below)] = make_int2(a - pl, b - a);
-      if (hhas) D.hsegs[hbase + nh_ + __popc(hm & below)] = make_int2(a2 - pl, b - a2);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const unsigned m = __ballot_sync(FULL, v[i] > u[i]);
+      if (v[i] > u[i]) D.hsegs[at[i] + __popc(m & below)] = make_int2(u[i] - pl, v[i] - u[i]);
+      at[i] += __popc(m);
     }
-    ns_ += __popc(m);
-    nh_ += __popc(hm);
-    if (has) wk += (unsigned long long)(b - a);
-    if (hhas) hwk += (unsigned long long)(b - a2);
+    if (D.full) {
+      const unsigned m = __ballot_sync(FULL, b > a);
+      if (b > a) D.segs[gi * D.wmax + nf + __popc(m & below)] = make_int2(a - pl, b - a);
+      nf += __popc(m);
+    }
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    wk += __shfl_xor_sync(FULL, wk, o);
-    hwk += __shfl_xor_sync(FULL, hwk, o);
-  }
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < 4; i++) src[i] += __shfl_xor_sync(FULL, src[i], o);
   if (lane == 0) {
-    if (FILL) {
-      ug[slot] = make_int4(p0 - pl, p1 - p0, base, base + ns_);
-      uh[slot] = make_int4(p0 - pl, p1 - p0, hbase, hbase + nh_);
-    } else {
-      nseg[slot] = ns_;
-      nhseg[slot] = nh_;
-      // sources staged by the group (at most n: its segments are disjoint)
-      work[slot] = (unsigned)min(wk, 0xffffffffull);
-      hwork[slot] = (unsigned)min(hwk, 0xffffffffull);
-      atomicAdd(&st[r].cand, wk * (unsigned long long)(p1 - p0));
-      atomicAdd(&st[r].hcand, hwk * (unsigned long long)(p1 - p0));
+    uh[slot] = make_int4(p0 - pl, p1 - p0, base, base + n[0] + n[1] + n[2]);
+    uz[slot] = make_int2(base + n[0], base + n[0] + n[1]);
+    const int hb = work_bin(2 * src[0] + src[1] + src[2]);
+    hbin[slot] = hb;
+    atomicAdd(&st[r].bins[1][hb], 1);
+    if (D.full) {
+      ug[slot] = make_int4(p0 - pl, p1 - p0, (int)(gi * D.wmax), (int)(gi * D.wmax) + nf);
+      const int fb = work_bin(src[3]);
+      bin[slot] = fb;
+      atomicAdd(&st[r].bins[0][fb], 1);
     }
+    atomicAdd(&st[r].cand, src[3] * (unsigned long long)(p1 - p0));
+    atomicAdd(&st[r].hcand, src[0] * (unsigned long long)(p1 - p0) +
+                                src[1] * (unsigned long long)cl + src[2] * (unsigned long long)cu);
   }
 }
 
-// Sort key of a group slot: the system, then the work, heaviest first; spare
-// slots of a system's bound last.
-__global__ void work_key_kernel(const SysDesc *__restrict__ d, const long *__restrict__ goffs,
-                                int R, long G, const int *__restrict__ goff,
-                                const unsigned *__restrict__ work, int wbits,
-                                unsigned long long *__restrict__ key, unsigned *__restrict__ iota) {
-  const long slot = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot >= G) return;
-  const int r = owner(goffs, R, slot);
-  const SysDesc &D = d[r];
-  const unsigned long long mask = (1ull << wbits) - 1ull;
-  const bool real = slot - D.g_off < sys_groups(D, goff);
-  const unsigned long long w = real ? mask - min((unsigned long long)work[slot], mask) : mask;
-  key[slot] = ((unsigned long long)r << wbits) | w;
-  iota[slot] = (unsigned)slot;
-}
-
-// A system's final group records and frame origins, in work order.
-__global__ void order_groups_kernel(const SysDesc *__restrict__ d, const long *__restrict__ goffs,
-                                    int R, long G, const int *__restrict__ goff,
-                                    const unsigned *__restrict__ ord,
-                                    const int4 *__restrict__ gin, const double4 *__restrict__ cin,
-                                    bool half) {
-  const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= G) return;
-  const int r = owner(goffs, R, k);
-  const SysDesc &D = d[r];
-  const long dest = k - D.g_off;
-  if (dest >= sys_groups(D, goff)) return;
-  const long s = ord[k];
-  (half ? D.hgroups : D.groups)[dest] = gin[s];
-  (half ? D.hcen : D.gcen)[dest] = cin[s];
+// A system's final group records and frame origins, heaviest bin first (the
+// order inside a bin is that of the atomics: it decides only which warp walks
+// a group, no result), so that the last wave of a direct-sum launch holds the
+// light ones.  Grid: (CTAs of 256 slots of the longest system, systems, lists).
+__global__ void __launch_bounds__(256)
+    order_groups_kernel(const SysDesc *__restrict__ d, const int *__restrict__ goff,
+                        const int4 *__restrict__ ug, const int4 *__restrict__ uh,
+                        const int2 *__restrict__ uz, const double4 *__restrict__ cen, const int *__restrict__ bin,
+                        const int *__restrict__ hbin, SysStats *st) {
+  __shared__ int first[kWorkBins];
+  __shared__ int warp_sum[8];
+  const SysDesc &D = d[blockIdx.y];
+  SysStats &S = st[blockIdx.y];
+  const bool half = blockIdx.z == 0;
+  if (!half && !D.full) return;
+  const long n = sys_groups(D, goff), g0 = (long)blockIdx.x * 256;
+  if (g0 >= n) return;
+  // exclusive sum of the bins, four per thread
+  constexpr int K = kWorkBins / 256;
+  const int *bins = S.bins[half ? 1 : 0];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int v[K], sum = 0;
+#pragma unroll
+  for (int i = 0; i < K; i++) v[i] = bins[K * threadIdx.x + i], sum += v[i];
+  int inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) warp_sum[w] = inc;
+  __syncthreads();
+  int run = inc - sum;
+  for (int i = 0; i < w; i++) run += warp_sum[i];
+#pragma unroll
+  for (int i = 0; i < K; i++) first[K * threadIdx.x + i] = run, run += v[i];
+  __syncthreads();
+  const long k = g0 + threadIdx.x;
+  if (k >= n) return;
+  const long s = D.g_off + k;
+  const int b = (half ? hbin : bin)[s];
+  const int dest = first[b] + atomicAdd(&S.taken[half ? 1 : 0][b], 1);
+  (half ? D.hgroups : D.groups)[dest] = (half ? uh : ug)[s];
+  if (half) D.hzones[dest] = uz[s];
+  (half ? D.hcen : D.gcen)[dest] = cen[s];
 }
 
 __global__ void collect_counts_kernel(const SysDesc *__restrict__ d, int R,
                                       const SysStats *__restrict__ st,
                                       const int *__restrict__ goff, const int *__restrict__ pos,
-                                      const int *__restrict__ segoff,
-                                      const int *__restrict__ hsegoff,
                                       SetupCounts *__restrict__ out) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= R) return;
@@ -625,8 +737,6 @@ __global__ void collect_counts_kernel(const SysDesc *__restrict__ d, int R,
   out[r].hcand = st[r].hcand;
   out[r].ngroups = (int)sys_groups(D, goff);
   out[r].nnonempty = pos[D.b_off + D.nbt] - pos[D.b_off];
-  out[r].nsegs = segoff[D.g_off + D.ngb] - segoff[D.g_off];
-  out[r].nhsegs = hsegoff[D.g_off + D.ngb] - hsegoff[D.g_off];
 }
 
 int bits_for(unsigned long long v) {  // bits to hold values < v
@@ -641,10 +751,9 @@ inline unsigned blocks_for(long n, int t = 256) { return (unsigned)((n + t - 1) 
 // first) and reused by its next set-up.
 enum Scratch {
   kPts, kBKey, kBKeyOut, kIota, kBPerm, kCKey, kSKey, kKeyOut, kCOrder, kSOrder, kBOrder,
-  kCounts3, kBStart, kFlag, kPos, kCStart, kSStart, kZs, kCPos, kFCPos, kGCount, kGOff,
-  kGRec, kBLo, kBHi, kCen, kGroupCounters, kSegOff, kHSegOff, kUGroups, kUHGroups,
-  kWKey, kWKeyOut, kOrd, kGIota, kStats, kSysStats, kDesc, kOffs, kCub, kBPos, kCountsDev,
-  kScratchCount
+  kBStart, kValues, kPos, kCStart, kSStart, kCPos, kGOff, kCen, kBins, kUGroups, kUHGroups,
+  kUZones,
+  kStats, kSysStats, kDesc, kOffs, kCub, kBPos, kCountsDev, kScratchCount
 };
 static_assert(kScratchCount <= kSetupScratch, "raise kSetupScratch");
 
@@ -723,7 +832,7 @@ int describe(npme_handle *h, SysDesc &D) {
   }
   {
     const double H = h->bmax[2] - h->bmin[2];
-    g.zbits = std::max(8, std::min(kZField,
+    g.zbits = std::max(8, std::min(kMaxZBits,
                                    (int)std::ceil(std::log2(std::max(1.0, 1024.0 * H / e)))));
     g.zmin = h->bmin[2];
     g.zscale = (double)((1u << g.zbits) - 1u) / std::max(H, 1e-300);
@@ -746,15 +855,29 @@ int describe(npme_handle *h, SysDesc &D) {
   //   groups   <= n / 32 + non-empty columns <= n / 32 + min(n, ncol)
   //   segments <= groups x the fine columns of a group's window (a group lies
   //               in one coarse column, so its window spans at most
-  //               (edge + 2 Rdir) / sedge + 4 fine columns per axis)
+  //               (edge + 2 Rdir) / sedge + 4 fine columns per axis, one more
+  //               for rounding)
   //   non-empty bricks <= min(n, nbt)
   D.ngb = n / 32 + std::min(n, D.ncol) + 1;
   long wmax = 1;
   for (int a = 0; a < 2; a++)
-    wmax *= std::min<long>(g.ns[a], (long)std::floor((g.edge[a] + 2.0 * Rd) / g.sedge[a]) + 4);
+    wmax *= std::min<long>(g.ns[a], (long)std::floor((g.edge[a] + 2.0 * Rd) / g.sedge[a]) + 5);
+  D.wmax = wmax;
+  D.full = needs_full_lists(h);
   const long nsb = D.ngb * wmax;
   if (nsb >= (1L << 31))  // int offsets in the group records
     return record_error(h, NPME_EINVAL, "too many direct-sum source segments (2^31)");
+  // Zones leave an eighth of the pairs out (at density 1 and Rdir 8 a quarter of
+  // the candidates reach one half of a group only) but cost shorter lists.  They
+  // gain where a pair is expensive and the lists are long: FP64 1M 6,411 ->
+  // 6,131 us, FP64 Helmholtz 62,500 1,088 -> 1,037, FP32 r^-0.5 500k 1,778 ->
+  // 1,731, FP32 Helmholtz 250k 1,257 -> 1,239; FP32 1/r 1M 3,121 -> 3,168, and
+  // with few groups, whose walks are split, 4,000 points 26 -> 41, 30,000 82 ->
+  // 98.  Not where three segments per column would exceed the offsets.
+  const long min_points = sizeof(T) == 8 ? 32L * 4 * 148 : 32L * 20 * 148;
+  D.zones = n >= min_points && 3 * nsb < (1L << 31) &&
+            (sizeof(T) == 8 || h->p.funcType == NPME_FUNC_RALPHA ||
+             h->p.funcType == NPME_FUNC_HELMHOLTZ);
   const int C = h->complex_kernel ? 2 : 1;
   if ((rc = handle_buffer(h, &h->d_bpts, sizeof(BrickPoint<T>) * n)) ||
       (rc = handle_buffer(h, (void **)&h->d_brick_start, sizeof(int) * (D.nbt + 1))) ||
@@ -765,15 +888,17 @@ int describe(npme_handle *h, SysDesc &D) {
       (rc = handle_buffer(h, (void **)&h->d_bperm, sizeof(uint32_t) * n)) ||
       (rc = handle_buffer(h, (void **)&h->d_gpos, sizeof(double4) * n)) ||
       (rc = handle_buffer(h, (void **)&h->d_spos, sizeof(double4) * n)) ||
-      (rc = handle_buffer(h, (void **)&h->d_segs, sizeof(int2) * nsb)) ||
-      (rc = handle_buffer(h, (void **)&h->d_hsegs, sizeof(int2) * nsb)) ||
-      (rc = handle_buffer(h, (void **)&h->d_groups, sizeof(int4) * D.ngb)) ||
-      (rc = handle_buffer(h, (void **)&h->d_gcen, sizeof(double4) * D.ngb)) ||
+      (rc = handle_buffer(h, (void **)&h->d_hsegs, sizeof(int2) * nsb * (D.zones ? 3 : 1))) ||
+      (rc = handle_buffer(h, (void **)&h->d_hzones, sizeof(int2) * D.ngb)) ||
       (rc = handle_buffer(h, (void **)&h->d_hgroups, sizeof(int4) * D.ngb)) ||
       (rc = handle_buffer(h, (void **)&h->d_hcen, sizeof(double4) * D.ngb)) ||
       (rc = handle_buffer(h, &h->d_qc, sizeof(T) * C * n)) ||
       (rc = handle_buffer(h, (void **)&h->d_q_in, sizeof(double) * C * n)) ||
       (rc = handle_buffer(h, (void **)&h->d_V, sizeof(double) * 4 * C * n)))
+    return rc;
+  if (D.full && ((rc = handle_buffer(h, (void **)&h->d_segs, sizeof(int2) * nsb)) ||
+                 (rc = handle_buffer(h, (void **)&h->d_groups, sizeof(int4) * D.ngb)) ||
+                 (rc = handle_buffer(h, (void **)&h->d_gcen, sizeof(double4) * D.ngb))))
     return rc;
   // source-side sums of the pair-once walk start (and are kept) at zero
   if (h->fp32) {
@@ -811,7 +936,7 @@ int describe(npme_handle *h, SysDesc &D) {
   D.cperm = h->d_cperm, D.sperm = h->d_sperm, D.bperm = h->d_bperm;
   D.gpos = h->d_gpos, D.spos = h->d_spos;
   D.segs = h->d_segs, D.hsegs = h->d_hsegs;
-  D.groups = h->d_groups, D.hgroups = h->d_hgroups;
+  D.groups = h->d_groups, D.hgroups = h->d_hgroups, D.hzones = h->d_hzones;
   D.gcen = h->d_gcen, D.hcen = h->d_hcen;
   h->d_dperm = h->d_sperm;  // direct-sum charges are gathered into the source order
   return NPME_OK;
@@ -820,13 +945,16 @@ int describe(npme_handle *h, SysDesc &D) {
 // Brick order, direct-sum orders, warp groups and segment lists of R systems
 // of one precision in one pass on stream s (h0 = hs[0] owns the scratch).
 // Enqueued without waiting; the counts arrive in h0->h_counts with the
-// caller's synchronisation.
+// caller's synchronisation.  `hook` runs when the systems' buffers are
+// allocated and nothing of the geometry is enqueued yet.
 template <typename T>
-int geometry_batch(npme_handle **hs, int R, cudaStream_t s) {
+int geometry_batch(npme_handle **hs, int R, cudaStream_t s, const std::function<int()> &hook) {
   npme_handle *h = hs[0];
   int rc;
   std::vector<SysDesc> ds(R);
-  long P = 0, B = 0, C = 0, S = 0, G = 0, nmax = 1, nbtmax = 1, ncolmax = 1, nscolmax = 1;
+  long P = 0, B = 0, C = 0, S = 0, G = 0, gmax = 1, nbtmax = 1, ncolmax = 1, nscolmax = 1;
+  int zf = 1;
+  bool full = false;
   for (int r = 0; r < R; r++) {
     if ((rc = describe<T>(hs[r], ds[r]))) {
       if (hs[r] != h) h->err = hs[r]->err;
@@ -835,7 +963,8 @@ int geometry_batch(npme_handle **hs, int R, cudaStream_t s) {
     SysDesc &D = ds[r];
     D.p_off = P, D.b_off = B, D.c_off = C, D.s_off = S, D.g_off = G;
     P += D.n, B += D.nbt + 1, C += D.ncol + 1, S += D.nscol + 1, G += D.ngb;
-    nmax = std::max(nmax, D.n), nbtmax = std::max(nbtmax, D.nbt);
+    gmax = std::max(gmax, D.ngb), nbtmax = std::max(nbtmax, D.nbt);
+    zf = std::max(zf, D.g.zbits), full = full || D.full;
     ncolmax = std::max(ncolmax, D.ncol), nscolmax = std::max(nscolmax, D.nscol);
     // the system's coordinates and buffers (on its own stream) come first
     if (hs[r]->stream != s) {
@@ -843,12 +972,12 @@ int geometry_batch(npme_handle **hs, int R, cudaStream_t s) {
       SCK(cudaStreamWaitEvent(s, hs[r]->ev_fork, 0));
     }
   }
+  if (hook && (rc = hook())) return rc;
   if (P >= (1L << 31) || B >= (1L << 31) || G >= (1L << 31))
     return record_error(h, NPME_EINVAL, "set-up batch too large for 32-bit indices");
   const int rbits = bits_for((unsigned long long)R);
   const int bbits = bits_for(nbtmax), cbits = bits_for(ncolmax), sbits = bits_for(nscolmax);
-  const int wbits = bits_for((unsigned long long)nmax + 1) + 1;
-  if (rbits + bbits + 5 > 64 || rbits + sbits + kZField > 64)
+  if (rbits + bbits + 5 > 64 || rbits + sbits + zf > 64)
     return record_error(h, NPME_EINVAL, "set-up batch keys exceed 64 bits");
 
   // descriptors and the index-space starts (points, bricks, columns, fine
@@ -872,12 +1001,16 @@ int geometry_batch(npme_handle **hs, int R, cudaStream_t s) {
   }
   SCK(cudaMemcpyAsync(dd, hd, sizeof(SysDesc) * R, cudaMemcpyHostToDevice, s));
   SCK(cudaMemcpyAsync(offs, ho, sizeof(long) * 5 * R, cudaMemcpyHostToDevice, s));
-  const long *poff = offs, *boff = offs + R, *coff = offs + 2 * R, *goffs = offs + 4 * R;
+  const long *poff = offs, *boff = offs + R, *coff = offs + 2 * R, *soff = offs + 3 * R,
+             *goffs = offs + 4 * R;
 
   BrickPoint<T> *pts;
   unsigned long long *bkey, *bkey_out, *ckey, *skey, *key_out;
-  unsigned *iota, *border, *corder, *sorder, *border2, *bpos, *zs, *cpos, *fcpos;
-  int *counts, *bstart, *flag, *pos, *cstart, *sstart, *gcount, *goff;
+  unsigned *iota, *border, *corder, *sorder, *border2, *bpos, *cpos;
+  int *bstart, *pos, *cstart, *sstart, *goff, *bins;
+  int4 *ug, *uh;
+  int2 *uz;
+  double4 *cen;
   SysStats *st;
   if ((rc = scratch(h, kPts, sizeof(BrickPoint<T>) * P, &pts)) ||
       (rc = scratch(h, kBKey, sizeof(unsigned long long) * P, &bkey)) ||
@@ -891,105 +1024,64 @@ int geometry_batch(npme_handle **hs, int R, cudaStream_t s) {
       (rc = scratch(h, kCOrder, sizeof(unsigned) * P, &corder)) ||
       (rc = scratch(h, kSOrder, sizeof(unsigned) * P, &sorder)) ||
       (rc = scratch(h, kBPos, sizeof(unsigned) * P, &bpos)) ||
-      (rc = scratch(h, kZs, sizeof(unsigned) * P, &zs)) ||
       (rc = scratch(h, kCPos, sizeof(unsigned) * P, &cpos)) ||
-      (rc = scratch(h, kFCPos, sizeof(unsigned) * P, &fcpos)) ||
-      (rc = scratch(h, kCounts3, sizeof(int) * (B + C + S), &counts)) ||
-      (rc = scratch(h, kBStart, sizeof(int) * B, &bstart)) ||
-      (rc = scratch(h, kFlag, sizeof(int) * B, &flag)) ||
+      (rc = scratch(h, kBStart, sizeof(int) * (B + 1), &bstart)) ||
       (rc = scratch(h, kPos, sizeof(int) * B, &pos)) ||
-      (rc = scratch(h, kCStart, sizeof(int) * C, &cstart)) ||
-      (rc = scratch(h, kSStart, sizeof(int) * S, &sstart)) ||
-      (rc = scratch(h, kGCount, sizeof(int) * C, &gcount)) ||
+      (rc = scratch(h, kCStart, sizeof(int) * (C + 1), &cstart)) ||
+      (rc = scratch(h, kSStart, sizeof(int) * (S + 1), &sstart)) ||
       (rc = scratch(h, kGOff, sizeof(int) * C, &goff)) ||
-      (rc = scratch(h, kSysStats, sizeof(SysStats) * R, &st)))
-    return rc;
-  int *bcount = counts, *ccount = counts + B, *scount = counts + B + C;
-
-  // --- binning: records, keys and counts of every point ---
-  SCK(cudaMemsetAsync(counts, 0, sizeof(int) * (B + C + S), s));
-  init_sys_stats_kernel<<<blocks_for(R, 64), 64, 0, s>>>(dd, R, st);
-  bin_kernel<T><<<blocks_for(P), 256, 0, s>>>(dd, poff, R, P, bbits, cbits, sbits, pts, bkey,
-                                              ckey, skey, iota, bcount, ccount, scount, st);
-  SCK(cudaGetLastError());
-
-  // --- brick order: by (system, brick), inside a brick in rounds over the
-  // banks: a sort by (system, brick, bank, index), then each brick's banks
-  // interleaved in rounds ---
-  if ((rc = sort_pairs(h, bkey, bkey_out, iota, border, P, rbits + bbits + 5, s))) return rc;
-  if ((rc = exclusive_sum(h, bcount, bstart, B, s))) return rc;
-  round_place_kernel<<<blocks_for(32 * B), 256, 0, s>>>(bkey_out, border, bstart, bcount, B,
-                                                       border2);
-  place_bricks_kernel<T><<<blocks_for(P), 256, 0, s>>>(dd, poff, R, P, border2, pts, bpos);
-  nonempty_flags_kernel<<<blocks_for(B), 256, 0, s>>>(bcount, B, flag);
-  if ((rc = exclusive_sum(h, flag, pos, B, s))) return rc;
-  bricks_kernel<<<blocks_for(B), 256, 0, s>>>(dd, boff, R, B, bcount, bstart, pos);
-
-  // --- direct-sum orders: (system, column, quantised z, index) for targets
-  // and sources, one radix sort each ---
-  if ((rc = sort_pairs(h, ckey, key_out, iota, corder, P, rbits + cbits + kZField, s)) ||
-      (rc = sort_pairs(h, skey, key_out, iota, sorder, P, rbits + sbits + kZField, s)))
-    return rc;
-  place_orders_kernel<<<blocks_for(P), 256, 0, s>>>(dd, poff, R, P, corder, sorder, key_out, bpos,
-                                                    zs, cpos);
-  gather_u32_kernel<<<blocks_for(P), 256, 0, s>>>(cpos, sorder, P, fcpos);
-  if ((rc = exclusive_sum(h, ccount, cstart, C, s))) return rc;
-  if ((rc = exclusive_sum(h, scount, sstart, S, s))) return rc;
-  groups_per_column_kernel<<<blocks_for(C), 256, 0, s>>>(ccount, C, gcount);
-  if ((rc = exclusive_sum(h, gcount, goff, C, s))) return rc;
-  SCK(cudaGetLastError());
-
-  // --- warp groups and their source segments ---
-  int4 *grec, *ug, *uh;
-  double4 *blo, *bhi, *cen;
-  int *nseg, *segoff, *hsegoff;
-  unsigned long long *wkey, *wkey_out;
-  unsigned *ord, *giota;
-  if ((rc = scratch(h, kGRec, sizeof(int4) * G, &grec)) ||
-      (rc = scratch(h, kBLo, sizeof(double4) * G, &blo)) ||
-      (rc = scratch(h, kBHi, sizeof(double4) * G, &bhi)) ||
       (rc = scratch(h, kCen, sizeof(double4) * G, &cen)) ||
-      (rc = scratch(h, kGroupCounters, sizeof(int) * 4 * (G + 1), &nseg)) ||
-      (rc = scratch(h, kSegOff, sizeof(int) * (G + 1), &segoff)) ||
-      (rc = scratch(h, kHSegOff, sizeof(int) * (G + 1), &hsegoff)) ||
+      (rc = scratch(h, kBins, sizeof(int) * 2 * G, &bins)) ||
       (rc = scratch(h, kUGroups, sizeof(int4) * G, &ug)) ||
       (rc = scratch(h, kUHGroups, sizeof(int4) * G, &uh)) ||
-      (rc = scratch(h, kWKey, sizeof(unsigned long long) * G, &wkey)) ||
-      (rc = scratch(h, kWKeyOut, sizeof(unsigned long long) * G, &wkey_out)) ||
-      (rc = scratch(h, kOrd, sizeof(unsigned) * G, &ord)) ||
-      (rc = scratch(h, kGIota, sizeof(unsigned) * G, &giota)))
+      (rc = scratch(h, kUZones, sizeof(int2) * G, &uz)) ||
+      (rc = scratch(h, kSysStats, sizeof(SysStats) * R, &st)))
     return rc;
-  // segment counts and work of both lists in one block, one clear (spare
-  // slots of the bounds: no segments, no work)
-  int *nhseg = nseg + (G + 1);
-  unsigned *work = (unsigned *)(nhseg + (G + 1)), *hwork = work + (G + 1);
-  SCK(cudaMemsetAsync(nseg, 0, sizeof(int) * 4 * (G + 1), s));
-  group_records_kernel<<<blocks_for(C), 256, 0, s>>>(dd, coff, R, C, cstart, goff, grec);
-  group_box_kernel<<<blocks_for(32 * G), 256, 0, s>>>(dd, goffs, R, G, goff, grec, blo, bhi, cen);
-  group_segments_kernel<false><<<blocks_for(32 * G), 256, 0, s>>>(
-      dd, goffs, R, G, goff, grec, blo, bhi, sstart, zs, fcpos, nseg, nhseg, work, hwork, nullptr,
-      nullptr, nullptr, nullptr, st);
-  if ((rc = exclusive_sum(h, nseg, segoff, G + 1, s))) return rc;
-  if ((rc = exclusive_sum(h, nhseg, hsegoff, G + 1, s))) return rc;
-  group_segments_kernel<true><<<blocks_for(32 * G), 256, 0, s>>>(
-      dd, goffs, R, G, goff, grec, blo, bhi, sstart, zs, fcpos, nullptr, nullptr, nullptr,
-      nullptr, segoff, hsegoff, ug, uh, st);
-  // heaviest groups first, so that the last wave of a direct-sum launch
-  // holds the light ones (each list by its own work; ties keep the column
-  // order)
-  for (int half = 0; half < 2; half++) {
-    work_key_kernel<<<blocks_for(G), 256, 0, s>>>(dd, goffs, R, G, goff, half ? hwork : work,
-                                                  wbits, wkey, giota);
-    if ((rc = sort_pairs(h, wkey, wkey_out, giota, ord, G, rbits + wbits, s))) return rc;
-    order_groups_kernel<<<blocks_for(G), 256, 0, s>>>(dd, goffs, R, G, goff, ord,
-                                                      half ? uh : ug, cen, half != 0);
+
+  // --- binning: records and keys of every point ---
+  init_sys_stats_kernel<<<R, 256, 0, s>>>(dd, st);
+  bin_kernel<T><<<blocks_for(P), 256, 0, s>>>(dd, poff, R, P, bbits, cbits, sbits, zf, pts, bkey,
+                                              ckey, skey, iota, st);
+  SCK(cudaGetLastError());
+
+  // --- the three orders: (system, brick, bank, index) for the bricks,
+  // (system, column, quantised z, index) for the direct sum's targets and
+  // sources, one radix sort each (the sorted source keys take the place of the
+  // unsorted target keys) ---
+  if ((rc = sort_pairs(h, bkey, bkey_out, iota, border, P, rbits + bbits + 5, s)) ||
+      (rc = sort_pairs(h, ckey, key_out, iota, corder, P, rbits + cbits + zf, s)) ||
+      (rc = sort_pairs(h, skey, ckey, iota, sorder, P, rbits + sbits + zf, s)))
+    return rc;
+  starts_kernel<<<blocks_for(B + C + S + 3), 256, 0, s>>>(dd, R, boff, coff, soff, P, B, C, S,
+                                                         bbits, cbits, sbits, zf, bkey_out,
+                                                         key_out, ckey, bstart, cstart, sstart);
+  if (std::max(B, C) <= kOneScan) {
+    scans_kernel<<<2, 1024, 0, s>>>(bstart, (int)B, pos, cstart, (int)C, goff);
+  } else {
+    int *values;
+    if ((rc = scratch(h, kValues, sizeof(int) * std::max(B, C), &values))) return rc;
+    values_kernel<<<blocks_for(B), 256, 0, s>>>(NonEmpty{bstart}, B, values);
+    if ((rc = exclusive_sum(h, values, pos, B, s))) return rc;
+    values_kernel<<<blocks_for(C), 256, 0, s>>>(GroupsOf{cstart}, C, values);
+    if ((rc = exclusive_sum(h, values, goff, C, s))) return rc;
   }
+  round_place_kernel<<<blocks_for(B, kPlaceWarps), 32 * kPlaceWarps, 0, s>>>(bkey_out, border,
+                                                                            bstart, B, border2);
+  place_bricks_kernel<T><<<blocks_for(std::max(P, B)), 256, 0, s>>>(
+      dd, poff, boff, R, P, B, border2, pts, bstart, pos, bpos);
+  place_orders_kernel<<<blocks_for(P), 256, 0, s>>>(dd, poff, R, P, corder, sorder, bpos, cpos);
+  SCK(cudaGetLastError());
+
+  // --- warp groups and their source segments, heaviest groups first ---
+  groups_kernel<<<blocks_for(32 * G), 256, 0, s>>>(dd, goffs, R, G, goff, cstart, sstart, ckey, zf,
+                                                  sorder, cpos, ug, uh, uz, cen, bins, bins + G, st);
+  const dim3 og((unsigned)blocks_for(gmax), (unsigned)R, full ? 2 : 1);
+  order_groups_kernel<<<og, 256, 0, s>>>(dd, goff, ug, uh, uz, cen, bins, bins + G, st);
   // the counts, for the host to read when the set-up has completed
   SetupCounts *dc;
   if ((rc = scratch(h, kCountsDev, sizeof(SetupCounts) * R, &dc))) return rc;
   if ((rc = pinned_block(h, &h->h_counts, &h->counts_cap, sizeof(SetupCounts) * R))) return rc;
-  collect_counts_kernel<<<blocks_for(R, 64), 64, 0, s>>>(dd, R, st, goff, pos, segoff, hsegoff,
-                                                         dc);
+  collect_counts_kernel<<<blocks_for(R, 64), 64, 0, s>>>(dd, R, st, goff, pos, dc);
   SCK(cudaMemcpyAsync(h->h_counts, dc, sizeof(SetupCounts) * R, cudaMemcpyDeviceToHost, s));
   SCK(cudaGetLastError());
   return NPME_OK;
@@ -1031,8 +1123,9 @@ int device_bbox(npme_handle *h, const double *coord, double mn[3], double mx[3])
   return NPME_OK;
 }
 
-int setup_geometry(npme_handle **hs, int R, cudaStream_t s) {
-  return hs[0]->fp32 ? geometry_batch<float>(hs, R, s) : geometry_batch<double>(hs, R, s);
+int setup_geometry(npme_handle **hs, int R, cudaStream_t s, const std::function<int()> &hook) {
+  return hs[0]->fp32 ? geometry_batch<float>(hs, R, s, hook)
+                     : geometry_batch<double>(hs, R, s, hook);
 }
 
 int finish_setup(npme_handle *h, const npme_handle *owner, int r) {
@@ -1060,8 +1153,6 @@ int finish_setup(npme_handle *h, const npme_handle *owner, int r) {
   }
   h->n_nonempty = c.nnonempty;
   h->n_groups = h->n_hgroups = c.ngroups;
-  h->n_segs = c.nsegs;
-  h->n_hsegs = c.nhsegs;
   h->cand_per_point = (double)c.cand / (double)n;
   h->hcand_per_point = (double)c.hcand / (double)n;
   return NPME_OK;
