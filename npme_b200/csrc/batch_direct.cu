@@ -27,64 +27,42 @@ __global__ void __launch_bounds__(32 * kGroupWarps, kGroupMinBlocks) batch_direc
 
 // Pair-once direct sums of a batch: KIND 0 the packed real body
 // (direct_group_sym), 1 Helmholtz DM.
-template <int KIND, int FUNC, int ND>
-__global__ void __launch_bounds__(32 * kGroupWarps, 4) batch_sym_kernel(
+// SPLIT: a CTA of kGroupWarps warps per group, for classes with few groups
+// (split_warps in direct.cu).
+template <int KIND, int FUNC, int ND, bool SPLIT>
+__global__ void __launch_bounds__(32 * kGroupWarps, KIND == 0 ? NPME_MB : 4) batch_sym_kernel(
     PairCoef<float> k, const BatchSys *__restrict__ sys, const long long *__restrict__ off,
     int count) {
-  __shared__ float4 ta[kGroupWarps][32];
-  __shared__ float4 tb[kGroupWarps][32];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long u = (long long)blockIdx.x * kGroupWarps + wid;
-  if (u >= off[count]) return;  // warp-uniform
+  const int part = SPLIT ? wid : 0, nsplit = SPLIT ? kGroupWarps : 1;
+  const long long u = SPLIT ? (long long)blockIdx.x : (long long)blockIdx.x * kGroupWarps + wid;
+  if (u >= off[count]) return;  // warp-uniform (SPLIT: no CTA is past the end)
   const int s = find_sys(off, count, u);
   const BatchSys &S = sys[s];
   const long g = (long)(u - off[s]);
   if constexpr (KIND == 0) {
-    double acc[4] = {0, 0, 0, 0};
-    const int4 G = S.hgroups[g];
-    direct_group_sym<FUNC, ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.hzones[g],
-                               S.cperm, S.refine2, S.vsrc, ta[wid], tb[wid], lane, 0, 1, acc);
-    sym_store(k, G, S.cperm, S.q, S.fself_r, S.V, lane, acc);
+    __shared__ SymWarp W[kGroupWarps];
+    direct_group_sym<FUNC, ND>(k, S.gpos, S.spos, S.qc, S.q, S.hgroups[g], S.hcen[g], S.hsegs,
+                               S.hzones[g], S.cperm, S.refine2, S.vsrc, W[wid], lane, part,
+                               nsplit);
+    if (SPLIT) __syncthreads();
+    if (!SPLIT || wid == 0)
+      sym_store(k, S.hgroups[g], S.cperm, S.q, S.fself_r, S.V, lane, &W[wid], nsplit);
   } else {
+    __shared__ float4 ta[kGroupWarps][32], tb[kGroupWarps][32];
     double acc[4] = {0, 0, 0, 0}, acci[4] = {0, 0, 0, 0};
     const int4 G = S.hgroups[g];
     direct_group_sym_helm<ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.hzones[g],
-                              S.cperm, S.refine2, S.vsrc, ta[wid], tb[wid], lane, 0, 1, acc, acci);
+                              S.cperm, S.refine2, S.vsrc, ta[wid], tb[wid], lane, part, nsplit,
+                              acc, acci);
+    if constexpr (SPLIT) {
+      __shared__ double red[kGroupWarps][32][4];
+      reduce_parts(acc, red, wid, kGroupWarps, lane);
+      __syncthreads();
+      reduce_parts(acci, red, wid, kGroupWarps, lane);
+      if (wid > 0) return;
+    }
     store_targets_cplx(G, S.cperm, S.q, S.fself_r, S.fself_i, 1.0, 1.0, S.V, lane, acc, acci);
-  }
-}
-
-// The pair-once walk with a CTA of kGroupWarps warps per group, for classes
-// with few groups (split_warps in direct.cu): four warps per group.
-template <int KIND, int FUNC, int ND>
-__global__ void __launch_bounds__(32 * kGroupWarps, 4) batch_sym_split_kernel(
-    PairCoef<float> k, const BatchSys *__restrict__ sys, const long long *__restrict__ off,
-    int count) {
-  __shared__ float4 ta[kGroupWarps][32];
-  __shared__ float4 tb[kGroupWarps][32];
-  __shared__ double red[kGroupWarps][32][4];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long u = blockIdx.x;
-  const int s = find_sys(off, count, u);
-  const BatchSys &S = sys[s];
-  const long g = (long)(u - off[s]);
-  double acc[4] = {0, 0, 0, 0}, acci[4] = {0, 0, 0, 0};
-  const int4 G = S.hgroups[g];
-  if constexpr (KIND == 0) {
-    direct_group_sym<FUNC, ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.hzones[g],
-                               S.cperm, S.refine2, S.vsrc, ta[wid], tb[wid], lane, wid,
-                               kGroupWarps, acc);
-    reduce_parts(acc, red, wid, kGroupWarps, lane);
-    if (wid == 0) sym_store(k, G, S.cperm, S.q, S.fself_r, S.V, lane, acc);
-  } else {
-    direct_group_sym_helm<ND>(k, S.gpos, S.spos, S.qc, S.q, G, S.hcen[g], S.hsegs, S.hzones[g],
-                              S.cperm, S.refine2, S.vsrc, ta[wid], tb[wid], lane, wid,
-                              kGroupWarps, acc, acci);
-    reduce_parts(acc, red, wid, kGroupWarps, lane);
-    __syncthreads();
-    reduce_parts(acci, red, wid, kGroupWarps, lane);
-    if (wid == 0)
-      store_targets_cplx(G, S.cperm, S.q, S.fself_r, S.fself_i, 1.0, 1.0, S.V, lane, acc, acci);
   }
 }
 
@@ -100,10 +78,10 @@ void launch_batch_direct(const PairCoef<float> &k, bool once, bool alpha_positiv
   const bool split = ng <= 20 * 148;
 #define NPME_BSYM(KD, FN, ND)                                                              \
   if (split)                                                                               \
-    batch_sym_split_kernel<KD, FN, ND>                                                     \
+    batch_sym_kernel<KD, FN, ND, true>                                                     \
         <<<(unsigned)ng, 32 * kGroupWarps, 0, s>>>(k, sys, off, count);                     \
   else                                                                                     \
-    batch_sym_kernel<KD, FN, ND><<<g, 32 * kGroupWarps, 0, s>>>(k, sys, off, count)
+    batch_sym_kernel<KD, FN, ND, false><<<g, 32 * kGroupWarps, 0, s>>>(k, sys, off, count)
 #define NPME_BSYM_ND(KD, FN)                \
   switch (nd) {                             \
     case 3: NPME_BSYM(KD, FN, 3); break;    \

@@ -12,6 +12,12 @@ namespace npme {
 #ifndef NPME_GROUP_MIN_BLOCKS
 #define NPME_GROUP_MIN_BLOCKS 1
 #endif
+#ifndef NPME_U
+#define NPME_U 8
+#endif
+#ifndef NPME_MB
+#define NPME_MB 4
+#endif
 constexpr int kGroupMinBlocks = NPME_GROUP_MIN_BLOCKS;  // resident CTAs asked of ptxas
 #ifndef NPME_DIRECT_UNROLL
 #define NPME_DIRECT_UNROLL 8
@@ -990,11 +996,23 @@ __device__ __forceinline__ void direct_group_packed(
 }
 
 // The two sources of a lane in the pair-once sweep: coordinates relative to
-// the group centre, negated (so that t + (-s) gives t - s exactly), and the
-// residuals of their rounding, each as the pair (v, v) that meets two
-// targets at once.
+// the group centre, negated (so that t + (-s) gives t - s exactly), each as the
+// pair (v, v) that meets two targets at once.
 struct SymSource {
-  float2 x, y, z, q, lx, ly, lz;
+  float2 x, y, z, q;
+};
+
+// What a warp of the pair-once sweep keeps in shared memory: the group's targets
+// in pairs (t[j] = x0 x1 y0 y1, t[16 + j] = z0 z1 q0 q1), the residuals of
+// their coordinates and, for the chunks that need them, of the sources' (negated,
+// as the coordinates), the target sums across chunks, and the group's centre
+// with near2 (below).  The last three would take 20 registers that are used once
+// per chunk.
+struct SymWarp {
+  float4 t[32], lo[32];
+  float res[2][3][32];
+  double acc[4][32];
+  double4 c;
 };
 
 // One step of the Newton's-third-law sweep (below): the lane's two sources
@@ -1007,10 +1025,11 @@ struct SymSource {
 // recomputed from heads and residuals, coincident points are no pair, and
 // misses also get charge 0 (a non-finite charge stays out of their sums).
 template <int FUNC, int ND, bool CHECKED>
-__device__ __forceinline__ void sym_step(const PairCoef<float> &k, const float4 A, const float4 B,
-                                         const float4 *la, const float4 *lb,
-                                         const SymSource (&src)[2], float refine2, float2 &aV,
+__device__ __forceinline__ void sym_step(const PairCoef<float> &k, const SymWarp &W, int j,
+                                         int lane, const SymSource (&src)[2], float refine2,
+                                         float2 &aV,
                                          float2 &aX, float2 &aY, float2 &aZ, float2 (&S)[2][4]) {
+  const float4 A = W.t[j], B = W.t[16 + j];
   float2 x[2], y[2], z[2], s[2], qs[2], qt[2];
 #pragma unroll
   for (int i = 0; i < 2; i++) {
@@ -1022,10 +1041,11 @@ __device__ __forceinline__ void sym_step(const PairCoef<float> &k, const float4 
     qt[i] = make_float2(B.z, B.w);
     if (CHECKED) {
       if (fminf(r2.x, r2.y) < refine2) {  // exact differences from head + residual
-        const float4 LA = *la, LB = *lb;
-        x[i] = __fadd2_rn(x[i], __fadd2_rn(make_float2(LA.x, LA.y), src[i].lx));
-        y[i] = __fadd2_rn(y[i], __fadd2_rn(make_float2(LA.z, LA.w), src[i].ly));
-        z[i] = __fadd2_rn(z[i], __fadd2_rn(make_float2(LB.x, LB.y), src[i].lz));
+        const float4 LA = W.lo[j], LB = W.lo[16 + j];
+        const float lx = W.res[i][0][lane], ly = W.res[i][1][lane], lz = W.res[i][2][lane];
+        x[i] = __fadd2_rn(x[i], __fadd2_rn(make_float2(LA.x, LA.y), make_float2(lx, lx)));
+        y[i] = __fadd2_rn(y[i], __fadd2_rn(make_float2(LA.z, LA.w), make_float2(ly, ly)));
+        z[i] = __fadd2_rn(z[i], __fadd2_rn(make_float2(LB.x, LB.y), make_float2(lz, lz)));
         r2 = __ffma2_rn(x[i], x[i], __ffma2_rn(y[i], y[i], __fmul2_rn(z[i], z[i])));
       }
       // a pair is inside iff 0 < r^2 <= 1, i.e. bits(r^2) - 1 < bits(1) as
@@ -1068,12 +1088,12 @@ __device__ __forceinline__ float2 rotate2(float2 v, int src) {
 // The steps of one chunk, 16 over all target pairs or 8 over one half of them
 // (zone 1: pairs 0-7, zone 2: pairs 8-15); target sums rotate after each.
 template <int FUNC, int ND, bool CHECKED>
-__device__ __forceinline__ void sym_sweep(const PairCoef<float> &k, const float4 *tsm,
-                                          const float4 *tlo, const SymSource (&src)[2],
-                                          float refine2, int lane, int zone, float2 &aV,
+__device__ __forceinline__ void sym_sweep(const PairCoef<float> &k, const SymWarp &W,
+                                          const SymSource (&src)[2], float refine2, int lane,
+                                          int zone, float2 &aV,
                                           float2 &aX, float2 &aY, float2 &aZ,
                                           float2 (&S)[2][4]) {
-  constexpr int kUnroll = CHECKED ? 1 : 8;
+  constexpr int kUnroll = CHECKED ? 1 : NPME_U;
   const int next = (lane + 1) & 31;
   const int mask = zone == 0 ? 15 : 7, from = zone == 2 ? 8 : 0;
 #pragma unroll 1
@@ -1081,8 +1101,7 @@ __device__ __forceinline__ void sym_sweep(const PairCoef<float> &k, const float4
 #pragma unroll kUnroll
     for (int kk = 0; kk < 8; kk++) {
       const int j = from + ((lane + k0 + kk) & mask);
-      sym_step<FUNC, ND, CHECKED>(k, tsm[j], tsm[16 + j], tlo + j, tlo + 16 + j, src, refine2,
-                                  aV, aX, aY, aZ, S);
+      sym_step<FUNC, ND, CHECKED>(k, W, j, lane, src, refine2, aV, aX, aY, aZ, S);
       aV = rotate2(aV, next), aX = rotate2(aX, next);
       aY = rotate2(aY, next), aZ = rotate2(aZ, next);
     }
@@ -1114,14 +1133,14 @@ __device__ __forceinline__ void sym_sweep(const PairCoef<float> &k, const float4
 // are met by that half alone, in half the steps.
 // The group's work is shared by nsplit warps of the CTA, warp `part` taking
 // chunks part, part + nsplit, ... (and every nsplit-th source of the pairs
-// inside the group); the caller adds their acc.
+// inside the group); the caller adds their sums (sym_store).
 template <int FUNC, int ND>
 __device__ __forceinline__ void direct_group_sym(
     const PairCoef<float> &k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const float *__restrict__ qs, const double *__restrict__ qcaller, const int4 G,
     const double4 c, const int2 *__restrict__ segs, const int2 zones,
-    const uint32_t *__restrict__ perm, float refine2, float4 *__restrict__ vsrc, float4 *tsm,
-    float4 *tlo, int lane, int part, int nsplit, double (&acc)[4]) {
+    const uint32_t *__restrict__ perm, float refine2, float4 *__restrict__ vsrc, SymWarp &W,
+    int lane, int part, int nsplit) {
   const unsigned FULL = 0xffffffffu;
   const int tid = 2 * (lane & 15) + (lane >> 4);  // the lane's target in the group
   // absent targets sit far outside the cutoff with charge 0
@@ -1134,24 +1153,27 @@ __device__ __forceinline__ void direct_group_sym(
     tlx = (float)(dx - (double)tx), tly = (float)(dy - (double)ty), tlz = (float)(dz - (double)tz);
     tq = (float)qcaller[perm[G.x + tid]];
   }
-  // tsm[j] = (x0 x1 y0 y1), tsm[16 + j] = (z0 z1 q0 q1) of target pair j; tlo
-  // the residuals
+  refine2 = (float)((double)refine2 * ir * ir);
   {
-    float *ts = reinterpret_cast<float *>(tsm), *tl = reinterpret_cast<float *>(tlo);
+    float *ts = reinterpret_cast<float *>(W.t), *tl = reinterpret_cast<float *>(W.lo);
     const int at = 4 * (lane & 15) + (lane >> 4);
     ts[at] = tx, ts[at + 2] = ty, ts[at + 64] = tz, ts[at + 66] = tq;
     tl[at] = tlx, tl[at + 2] = tly, tl[at + 64] = tlz, tl[at + 66] = 0.f;
   }
+  if (lane == 0) {
+    // a chunk with a source nearer to the centre than this takes the checked steps
+    const double rfs = sqrt((double)refine2) + c.w * ir;
+    W.c = make_double4(c.x, c.y, c.z, rfs * rfs);
+  }
   __syncwarp();
-  refine2 = (float)((double)refine2 * ir * ir);
   // a non-finite charge in the group: every chunk takes the checked steps
   const bool odd_group = __any_sync(FULL, !(fabsf(tq) <= 3.402823466e38f));
 
   // pairs inside the group, from both sides; the differences are always
   // refined (head difference + residual difference)
   {
-    const float *ts = reinterpret_cast<const float *>(tsm),
-                *tl = reinterpret_cast<const float *>(tlo);
+    const float *ts = reinterpret_cast<const float *>(W.t),
+                *tl = reinterpret_cast<const float *>(W.lo);
     const unsigned rb = __float_as_uint(1.f);
     float aV = 0.f, aX = 0.f, aY = 0.f, aZ = 0.f;
     for (int s = part; s < G.y; s += nsplit) {
@@ -1168,16 +1190,14 @@ __device__ __forceinline__ void direct_group_sym(
       aY = fmaf(g, y, aY);
       aZ = fmaf(g, z, aZ);
     }
-    acc[0] += (double)aV;
-    acc[1] -= (double)aX;
-    acc[2] -= (double)aY;
-    acc[3] -= (double)aZ;
+    W.acc[0][lane] = (double)aV;
+    W.acc[1][lane] = -(double)aX;
+    W.acc[2][lane] = -(double)aY;
+    W.acc[3][lane] = -(double)aZ;
   }
 
   // half-shell segments in chunks of 64 sources: lane l holds positions l
   // and l + 32 of the chunk (register prefetch of the next chunk)
-  const double rfs = sqrt((double)refine2) + c.w * ir;
-  const double near2 = rfs * rfs;
   constexpr bool kZoned = FUNC == 1;  // measured: set-up (describe)
   ZoneWalk<2, kZoned> walk(segs, G, zones, lane, part, nsplit);
   double4 p[2];
@@ -1198,25 +1218,36 @@ __device__ __forceinline__ void direct_group_sym(
     int slot[2];  // source-side slots: the sources' brick-order positions
     bool checked = odd_group;
     const int zone = kZoned ? walk.zone : 0;
+    {
+      const double4 o = W.c;
+      double d[2][3];
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-      float hx = -1e18f, hy = -1e18f, hz = -1e18f, lx = 0.f, ly = 0.f, lz = 0.f, qv = 0.f;
-      slot[i] = -1;
-      if (walk.v[i]) {
-        const double dx = (p[i].x - c.x) * ir, dy = (p[i].y - c.y) * ir,
-                     dz = (p[i].z - c.z) * ir;
-        hx = (float)dx, hy = (float)dy, hz = (float)dz;
-        lx = (float)(dx - (double)hx), ly = (float)(dy - (double)hy),
-        lz = (float)(dz - (double)hz);
-        qv = q[i];
-        slot[i] = (int)p[i].w;
-        checked = checked || dx * dx + dy * dy + dz * dz < near2 ||
-                  !(fabsf(qv) <= 3.402823466e38f);
+      for (int i = 0; i < 2; i++) {
+        float hx = -1e18f, hy = -1e18f, hz = -1e18f, qv = 0.f;
+        slot[i] = -1;
+        d[i][0] = d[i][1] = d[i][2] = -1e18;
+        if (walk.v[i]) {
+          d[i][0] = (p[i].x - o.x) * ir, d[i][1] = (p[i].y - o.y) * ir;
+          d[i][2] = (p[i].z - o.z) * ir;
+          hx = (float)d[i][0], hy = (float)d[i][1], hz = (float)d[i][2];
+          qv = q[i];
+          slot[i] = (int)p[i].w;
+          checked = checked ||
+                    d[i][0] * d[i][0] + d[i][1] * d[i][1] + d[i][2] * d[i][2] < o.w ||
+                    !(fabsf(qv) <= 3.402823466e38f);
+        }
+        src[i].x = make_float2(-hx, -hx), src[i].y = make_float2(-hy, -hy);
+        src[i].z = make_float2(-hz, -hz), src[i].q = make_float2(qv, qv);
       }
-      src[i].x = make_float2(-hx, -hx), src[i].y = make_float2(-hy, -hy);
-      src[i].z = make_float2(-hz, -hz), src[i].q = make_float2(qv, qv);
-      src[i].lx = make_float2(-lx, -lx), src[i].ly = make_float2(-ly, -ly);
-      src[i].lz = make_float2(-lz, -lz);
+      checked = __any_sync(FULL, checked);
+      if (checked) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          W.res[i][0][lane] = -(float)(d[i][0] + (double)src[i].x.x);
+          W.res[i][1][lane] = -(float)(d[i][1] + (double)src[i].y.x);
+          W.res[i][2][lane] = -(float)(d[i][2] + (double)src[i].z.x);
+        }
+      }
     }
     // prefetch the next chunk
     walk.next();
@@ -1230,10 +1261,10 @@ __device__ __forceinline__ void direct_group_sym(
     float2 S[2][4];
 #pragma unroll
     for (int i = 0; i < 2; i++) S[i][0] = S[i][1] = S[i][2] = S[i][3] = make_float2(0.f, 0.f);
-    if (__any_sync(FULL, checked))
-      sym_sweep<FUNC, ND, true>(k, tsm, tlo, src, refine2, lane, zone, aV, aX, aY, aZ, S);
+    if (checked)
+      sym_sweep<FUNC, ND, true>(k, W, src, refine2, lane, zone, aV, aX, aY, aZ, S);
     else
-      sym_sweep<FUNC, ND, false>(k, tsm, tlo, src, refine2, lane, zone, aV, aX, aY, aZ, S);
+      sym_sweep<FUNC, ND, false>(k, W, src, refine2, lane, zone, aV, aX, aY, aZ, S);
     // lanes l and l + 16 hold half of the sums of target pair l mod 16 each;
     // after a sweep over one half of the pairs lanes l, l + 8, l + 16 and l + 24
     // hold a quarter each of pair l mod 8 of that half
@@ -1247,10 +1278,10 @@ __device__ __forceinline__ void direct_group_sym(
       const float sum = keep + __shfl_xor_sync(FULL, give, 16);
       return other_half ? 0.f : sum;
     };
-    acc[0] += (double)total(aV);
-    acc[1] -= (double)total(aX);
-    acc[2] -= (double)total(aY);
-    acc[3] -= (double)total(aZ);
+    W.acc[0][lane] += (double)total(aV);
+    W.acc[1][lane] -= (double)total(aX);
+    W.acc[2][lane] -= (double)total(aY);
+    W.acc[3][lane] -= (double)total(aZ);
 #pragma unroll
     for (int i = 0; i < 2; i++)
       if (slot[i] >= 0)
@@ -1273,15 +1304,21 @@ __device__ __forceinline__ void reduce_parts(double (&acc)[4], double (*red)[32]
       for (int m = 0; m < 4; m++) acc[m] += red[w][lane][m];
 }
 
-// The target sums of direct_group_sym to V, less the self term f_LR(0) q
-// (src/Interface.cpp:2061-2062).
+// The target sums of direct_group_sym (of nsplit warps) to V, less the self term
+// f_LR(0) q (src/Interface.cpp:2061-2062).
 __device__ __forceinline__ void sym_store(const PairCoef<float> &k, const int4 G,
                                           const uint32_t *__restrict__ perm,
                                           const double *__restrict__ qcaller, double fself_r,
-                                          double *__restrict__ V, int lane,
-                                          const double (&acc)[4]) {
+                                          double *__restrict__ V, int lane, const SymWarp *W,
+                                          int nsplit) {
   const int tid = 2 * (lane & 15) + (lane >> 4);
   if (tid >= G.y) return;
+  double acc[4];
+#pragma unroll
+  for (int m = 0; m < 4; m++) acc[m] = W[0].acc[m][lane];
+  for (int w = 1; w < nsplit; w++)
+#pragma unroll
+    for (int m = 0; m < 4; m++) acc[m] += W[w].acc[m][lane];
   const long o = perm[G.x + tid];
   const double vs = k.vscale, gs = k.gscale;
   reinterpret_cast<double4 *>(V)[o] =

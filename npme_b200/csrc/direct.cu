@@ -198,23 +198,20 @@ static int split_warps(long ngroups) {
 // FP32 real-DM direct sum with every pair evaluated once (direct_group_sym),
 // then the source-side sums folded into V.
 template <int FUNC, int ND>
-__global__ void __launch_bounds__(32 * kGroupWarps, 4) direct_sym_kernel(
+__global__ void __launch_bounds__(32 * kGroupWarps, NPME_MB) direct_sym_kernel(
     PairCoef<float> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const float *__restrict__ qs, const double *__restrict__ qcaller,
     const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
     const int2 *__restrict__ segs, const int2 *__restrict__ zones,
-    const uint32_t *__restrict__ perm, long ngroups,
-    float refine2, double fself_r, double *__restrict__ V, float4 *__restrict__ vsrc) {
-  __shared__ float4 tsm[kGroupWarps][32];  // group targets in pairs, heads and charges
-  __shared__ float4 tlo[kGroupWarps][32];  // residuals of the target coordinates
+    const uint32_t *__restrict__ perm, long ngroups, float refine2, double fself_r,
+    double *__restrict__ V, float4 *__restrict__ vsrc) {
+  __shared__ SymWarp W[kGroupWarps];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long g = (long)blockIdx.x * kGroupWarps + wid;
   if (g >= ngroups) return;  // warp-uniform; nothing below synchronises the block
-  double acc[4] = {0, 0, 0, 0};
-  const int4 G = groups[g];
-  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, refine2, vsrc,
-                             tsm[wid], tlo[wid], lane, 0, 1, acc);
-  sym_store(k, G, perm, qcaller, fself_r, V, lane, acc);
+  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, groups[g], gcen[g], segs, zones[g], perm,
+                             refine2, vsrc, W[wid], lane, 0, 1);
+  sym_store(k, groups[g], perm, qcaller, fself_r, V, lane, &W[wid], 1);
 }
 
 // The same with a CTA of blockDim.x / 32 warps per group (split_warps).
@@ -226,17 +223,14 @@ __global__ void __launch_bounds__(32 * kMaxSplit) direct_sym_split_kernel(
     const int2 *__restrict__ segs, const int2 *__restrict__ zones,
     const uint32_t *__restrict__ perm, float refine2, double fself_r, double *__restrict__ V,
     float4 *__restrict__ vsrc) {
-  __shared__ float4 tsm[kMaxSplit][32];
-  __shared__ float4 tlo[kMaxSplit][32];
-  __shared__ double red[kMaxSplit][32][4];
+  __shared__ SymWarp W[kMaxSplit];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nsplit = blockDim.x >> 5;
   const long g = blockIdx.x;
-  double acc[4] = {0, 0, 0, 0};
   const int4 G = groups[g];
-  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, refine2, vsrc,
-                             tsm[wid], tlo[wid], lane, wid, nsplit, acc);
-  reduce_parts(acc, red, wid, nsplit, lane);
-  if (wid == 0) sym_store(k, G, perm, qcaller, fself_r, V, lane, acc);
+  direct_group_sym<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, refine2,
+                             vsrc, W[wid], lane, wid, nsplit);
+  __syncthreads();
+  if (wid == 0) sym_store(k, G, perm, qcaller, fself_r, V, lane, W, nsplit);
 }
 
 // V[caller(i)] += scale * vsrc[i] for every brick-order slot i, then
