@@ -113,6 +113,7 @@ using npme::BatchSys;
 struct npme_batch {
   int device = 0;
   cudaStream_t stream2 = nullptr;
+  cudaStream_t hi = nullptr;  // reciprocal chain: its CTAs go before the direct sums'
   // the direct-sum classes beyond the first run beside it
   static constexpr int kSide = 3;
   cudaStream_t side[kSide] = {};
@@ -164,6 +165,9 @@ int npme_gpu_batch_create(int device, npme_batch **out) {
   b->device = device;
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking);
+  int prio_lo = 0, prio_hi = 0;
+  if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
+  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->hi, cudaStreamNonBlocking, prio_hi);
   for (int i = 0; i < npme_batch::kSide && e == cudaSuccess; i++) {
     e = cudaStreamCreateWithFlags(&b->side[i], cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_side[i], cudaEventDisableTiming);
@@ -186,6 +190,7 @@ int npme_gpu_batch_destroy(npme_batch *b) {
   if (b->pending) cudaEventSynchronize(b->ev_done);
   if (b->stream2) cudaStreamSynchronize(b->stream2);
   if (b->stream2) cudaStreamDestroy(b->stream2);
+  if (b->hi) cudaStreamDestroy(b->hi);
   for (int i = 0; i < npme_batch::kSide; i++) {
     if (b->side[i]) cudaStreamDestroy(b->side[i]);
     if (b->ev_side[i]) cudaEventDestroy(b->ev_side[i]);
@@ -231,7 +236,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     if (!d_V[i] || !d_q[i]) return bfail(b, NPME_EINVAL, "null buffer in batch");
   }
   if (cudaSetDevice(b->device) != cudaSuccess) return bfail(b, NPME_ECUDA, "cudaSetDevice");
-  cudaStream_t s = (cudaStream_t)stream;
+  const cudaStream_t user = (cudaStream_t)stream;
   b->launches = 0;
 
   // FP64 (plain) and caller-defined-kernel members take their ordinary path
@@ -249,7 +254,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   const int m = (int)f32.size();
   if (m == 0) {
     // the members' own CalcVs are on `stream`: npme_gpu_batch_sync waits for them
-    if (cudaEventRecord(b->ev_done, s) != cudaSuccess)
+    if (cudaEventRecord(b->ev_done, user) != cudaSuccess)
       return bfail(b, NPME_ECUDA, "batch: event record failed");
     b->pending = true;
     return NPME_OK;
@@ -410,7 +415,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     for (size_t t = 0; t < c.members.size(); t++) dj[t] = hs[f32[c.members[t]]]->fft;
     memcpy(b->h_pinned + c.off_at, c.off.data(), sizeof(long long) * c.off.size());
   }
-  cudaMemcpyAsync(b->d_block, b->h_pinned, bytes, cudaMemcpyHostToDevice, s);
+  cudaMemcpyAsync(b->d_block, b->h_pinned, bytes, cudaMemcpyHostToDevice, user);
   auto D = [&](const Class &c) { return (const BatchSys *)(b->d_block + c.desc_at); };
   auto O = [&](const Class &c) { return (const long long *)(b->d_block + c.off_at); };
   auto grid_of = [](long long units, int threads, int cap) {
@@ -419,7 +424,9 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
 
   // 1. gather, then 2. direct sums, on the second stream, beside the
   // reciprocal sums
-  cudaEventRecord(b->ev_fork, s);
+  const cudaStream_t s = b->hi;  // the reciprocal chain
+  cudaEventRecord(b->ev_fork, user);
+  cudaStreamWaitEvent(s, b->ev_fork, 0);
   cudaStreamWaitEvent(b->stream2, b->ev_fork, 0);
   for (auto &kv : gath) {
     Class &c = kv.second;
@@ -561,6 +568,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     b->launches++;
   }
   cudaEventRecord(b->ev_done, s);
+  cudaStreamWaitEvent(user, b->ev_done, 0);
   b->pending = true;
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return bfail(b, NPME_ECUDA, std::string("batch: ") + cudaGetErrorString(e));

@@ -111,7 +111,8 @@ struct npme_handle {
 
   cudaStream_t stream = nullptr;
   cudaStream_t stream2 = nullptr;  // direct sum runs here, overlapped with the FFTs
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t stream_hi = nullptr;  // reciprocal chain: its CTAs go before the direct sum's
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_chain = nullptr;
   // shared plans (not owned): (y, z) slab transforms forward and inverse,
   // and the transforms along x (fft.cu)
   npme::FFTPlan *pf = nullptr, *pi = nullptr, *px = nullptr;
