@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(32 * kGroupWarps, kGroupMinBlocks) batch_direc
 // SPLIT: a CTA of kGroupWarps warps per group, for classes with few groups
 // (split_warps in direct.cu).
 template <int KIND, int FUNC, int ND, bool SPLIT>
-__global__ void __launch_bounds__(32 * kGroupWarps, KIND == 0 ? NPME_MB : 4) batch_sym_kernel(
+__global__ void __launch_bounds__(32 * kGroupWarps, 4) batch_sym_kernel(
     PairCoef<float> k, const BatchSys *__restrict__ sys, const long long *__restrict__ off,
     int count) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;

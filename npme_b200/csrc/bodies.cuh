@@ -12,12 +12,6 @@ namespace npme {
 #ifndef NPME_GROUP_MIN_BLOCKS
 #define NPME_GROUP_MIN_BLOCKS 1
 #endif
-#ifndef NPME_U
-#define NPME_U 8
-#endif
-#ifndef NPME_MB
-#define NPME_MB 4
-#endif
 constexpr int kGroupMinBlocks = NPME_GROUP_MIN_BLOCKS;  // resident CTAs asked of ptxas
 #ifndef NPME_DIRECT_UNROLL
 #define NPME_DIRECT_UNROLL 8
@@ -339,9 +333,18 @@ __device__ __forceinline__ void spread_brick_owner(int brick, const int *__restr
     };
     // the warp's points, in batches
     int cnt = 0;
+    uint32_t g0[4];  // four chunks of origins in flight (137 -> 131 us at 1M, FP32 order 6)
     for (int c0 = 0; c0 < nbp; c0 += 32) {
-      const int i = c0 + lane;
-      const bool mine = i < nbp && (int)(bp[beg + i].g0 >> 20) - b1 * kBrick == w;
+      if ((c0 & 127) == 0) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int i = c0 + 32 * u + lane;
+          g0[u] = i < nbp ? bp[beg + i].g0 : 0xffffffffu;
+        }
+      }
+      const int i = c0 + lane, u = c0 >> 5 & 3;
+      const uint32_t g = u < 2 ? (u == 0 ? g0[0] : g0[1]) : (u == 2 ? g0[2] : g0[3]);
+      const bool mine = i < nbp && (int)(g >> 20) - b1 * kBrick == w;
       const unsigned m = __ballot_sync(FULL, mine);
       if (mine) list[cnt + __popc(m & ((1u << lane) - 1u))] = i;
       cnt += __popc(m);
@@ -1001,6 +1004,10 @@ __device__ __forceinline__ void direct_group_packed(
 struct SymSource {
   float2 x, y, z, q;
 };
+// Sources per lane.  One (80 registers, 24 resident warps per SM instead of 16)
+// was slower, 3,293-3,377 us against 3,094 for 1/r at 1M: twice the shuffles and
+// shared loads per pair, and latency is not what bounds the sweep.
+constexpr int kSymSources = 2;
 
 // What a warp of the pair-once sweep keeps in shared memory: the group's targets
 // in pairs (t[j] = x0 x1 y0 y1, t[16 + j] = z0 z1 q0 q1), the residuals of
@@ -1010,7 +1017,7 @@ struct SymSource {
 // per chunk.
 struct SymWarp {
   float4 t[32], lo[32];
-  float res[2][3][32];
+  float res[kSymSources][3][32];
   double acc[4][32];
   double4 c;
 };
@@ -1026,13 +1033,14 @@ struct SymWarp {
 // misses also get charge 0 (a non-finite charge stays out of their sums).
 template <int FUNC, int ND, bool CHECKED>
 __device__ __forceinline__ void sym_step(const PairCoef<float> &k, const SymWarp &W, int j,
-                                         int lane, const SymSource (&src)[2], float refine2,
+                                         int lane, const SymSource (&src)[kSymSources], float refine2,
                                          float2 &aV,
-                                         float2 &aX, float2 &aY, float2 &aZ, float2 (&S)[2][4]) {
+                                         float2 &aX, float2 &aY, float2 &aZ, float2 (&S)[kSymSources][4]) {
   const float4 A = W.t[j], B = W.t[16 + j];
-  float2 x[2], y[2], z[2], s[2], qs[2], qt[2];
+  float2 x[kSymSources], y[kSymSources], z[kSymSources], s[kSymSources], qs[kSymSources],
+      qt[kSymSources];
 #pragma unroll
-  for (int i = 0; i < 2; i++) {
+  for (int i = 0; i < kSymSources; i++) {
     x[i] = __fadd2_rn(make_float2(A.x, A.y), src[i].x);
     y[i] = __fadd2_rn(make_float2(A.z, A.w), src[i].y);
     z[i] = __fadd2_rn(make_float2(B.x, B.y), src[i].z);
@@ -1065,7 +1073,7 @@ __device__ __forceinline__ void sym_step(const PairCoef<float> &k, const SymWarp
     }
   }
 #pragma unroll
-  for (int i = 0; i < 2; i++) {
+  for (int i = 0; i < kSymSources; i++) {
     float2 f0, t;  // t = -f1
     dm_eval2<FUNC, ND, !CHECKED>(k, s[i], f0, t);
     const float2 gs = __fmul2_rn(t, qs[i]), gt = __fmul2_rn(t, qt[i]);
@@ -1089,11 +1097,11 @@ __device__ __forceinline__ float2 rotate2(float2 v, int src) {
 // (zone 1: pairs 0-7, zone 2: pairs 8-15); target sums rotate after each.
 template <int FUNC, int ND, bool CHECKED>
 __device__ __forceinline__ void sym_sweep(const PairCoef<float> &k, const SymWarp &W,
-                                          const SymSource (&src)[2], float refine2, int lane,
+                                          const SymSource (&src)[kSymSources], float refine2, int lane,
                                           int zone, float2 &aV,
                                           float2 &aX, float2 &aY, float2 &aZ,
-                                          float2 (&S)[2][4]) {
-  constexpr int kUnroll = CHECKED ? 1 : NPME_U;
+                                          float2 (&S)[kSymSources][4]) {
+  constexpr int kUnroll = CHECKED ? 1 : 8;
   const int next = (lane + 1) & 31;
   const int mask = zone == 0 ? 15 : 7, from = zone == 2 ? 8 : 0;
 #pragma unroll 1
@@ -1199,11 +1207,11 @@ __device__ __forceinline__ void direct_group_sym(
   // half-shell segments in chunks of 64 sources: lane l holds positions l
   // and l + 32 of the chunk (register prefetch of the next chunk)
   constexpr bool kZoned = FUNC == 1;  // measured: set-up (describe)
-  ZoneWalk<2, kZoned> walk(segs, G, zones, lane, part, nsplit);
-  double4 p[2];
-  float q[2];
+  ZoneWalk<kSymSources, kZoned> walk(segs, G, zones, lane, part, nsplit);
+  double4 p[kSymSources];
+  float q[kSymSources];
 #pragma unroll
-  for (int i = 0; i < 2; i++) {
+  for (int i = 0; i < kSymSources; i++) {
     p[i] = make_double4(0, 0, 0, 0);
     q[i] = 0.f;
     if (walk.v[i]) {
@@ -1214,15 +1222,15 @@ __device__ __forceinline__ void direct_group_sym(
   while (walk.any()) {
     // this chunk's sources, relative to the group centre; empty slots far
     // away (on the other side from absent targets) with charge 0
-    SymSource src[2];
-    int slot[2];  // source-side slots: the sources' brick-order positions
+    SymSource src[kSymSources];
+    int slot[kSymSources];  // source-side slots: the sources' brick-order positions
     bool checked = odd_group;
     const int zone = kZoned ? walk.zone : 0;
     {
       const double4 o = W.c;
-      double d[2][3];
+      double d[kSymSources][3];
 #pragma unroll
-      for (int i = 0; i < 2; i++) {
+      for (int i = 0; i < kSymSources; i++) {
         float hx = -1e18f, hy = -1e18f, hz = -1e18f, qv = 0.f;
         slot[i] = -1;
         d[i][0] = d[i][1] = d[i][2] = -1e18;
@@ -1242,7 +1250,7 @@ __device__ __forceinline__ void direct_group_sym(
       checked = __any_sync(FULL, checked);
       if (checked) {
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < kSymSources; i++) {
           W.res[i][0][lane] = -(float)(d[i][0] + (double)src[i].x.x);
           W.res[i][1][lane] = -(float)(d[i][1] + (double)src[i].y.x);
           W.res[i][2][lane] = -(float)(d[i][2] + (double)src[i].z.x);
@@ -1252,15 +1260,15 @@ __device__ __forceinline__ void direct_group_sym(
     // prefetch the next chunk
     walk.next();
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < kSymSources; i++)
       if (walk.v[i]) {
         const long j = walk.index(i);
         p[i] = spos[j], q[i] = qs[j];
       }
     float2 aV = make_float2(0.f, 0.f), aX = aV, aY = aV, aZ = aV;
-    float2 S[2][4];
+    float2 S[kSymSources][4];
 #pragma unroll
-    for (int i = 0; i < 2; i++) S[i][0] = S[i][1] = S[i][2] = S[i][3] = make_float2(0.f, 0.f);
+    for (int i = 0; i < kSymSources; i++) S[i][0] = S[i][1] = S[i][2] = S[i][3] = make_float2(0.f, 0.f);
     if (checked)
       sym_sweep<FUNC, ND, true>(k, W, src, refine2, lane, zone, aV, aX, aY, aZ, S);
     else
@@ -1283,7 +1291,7 @@ __device__ __forceinline__ void direct_group_sym(
     W.acc[2][lane] -= (double)total(aY);
     W.acc[3][lane] -= (double)total(aZ);
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < kSymSources; i++)
       if (slot[i] >= 0)
         atomicAdd(vsrc + slot[i], make_float4(S[i][0].x + S[i][0].y, S[i][1].x + S[i][1].y,
                                               S[i][2].x + S[i][2].y, S[i][3].x + S[i][3].y));

@@ -198,7 +198,7 @@ static int split_warps(long ngroups) {
 // FP32 real-DM direct sum with every pair evaluated once (direct_group_sym),
 // then the source-side sums folded into V.
 template <int FUNC, int ND>
-__global__ void __launch_bounds__(32 * kGroupWarps, NPME_MB) direct_sym_kernel(
+__global__ void __launch_bounds__(32 * kGroupWarps, 4) direct_sym_kernel(
     PairCoef<float> k, const double4 *__restrict__ gpos, const double4 *__restrict__ spos,
     const float *__restrict__ qs, const double *__restrict__ qcaller,
     const int4 *__restrict__ groups, const double4 *__restrict__ gcen,
