@@ -709,19 +709,18 @@ __device__ __forceinline__ void dm_eval2(const PairCoef<float> &k, float2 s, flo
   constexpr int nd = dm_degree<ND>();
   const float2 one = make_float2(1.f, 1.f), mone = make_float2(-1.f, -1.f);
   if constexpr (FUNC == 2) {  // original Ewald split: not zero at s = 1
-    // erfc(x) = exp(-x^2) erfcx(x), x = beta r; erfcx a polynomial in tau = (x
-    // - 3)/(x + 3) over x + 3, so that the exponential serves f0 and t
+    // erfc(x) = exp(-x^2) erfcx(x), x = beta r; erfcx a polynomial in v = x / (x
+    // + 2) (kErfcxFit), so that the exponential serves f0 and t
     const float2 ri = rsqrt2<FTZ>(s);
     const float2 x = __fmul2_rn(__fmul2_rn(s, k.nq2[0]), ri);
-    const float2 d = __fadd2_rn(x, make_float2(3.f, 3.f));
-    const float2 w = make_float2(rcp_approx(d.x), rcp_approx(d.y));
-    const float2 tau = __ffma2_rn(w, make_float2(-6.f, -6.f), one);
+    const float2 d = __fadd2_rn(x, make_float2(2.f, 2.f));
+    const float2 v = __fmul2_rn(x, make_float2(rcp_approx(d.x), rcp_approx(d.y)));
     float2 h = k.nc2[9];
 #pragma unroll
-    for (int n = 8; n >= 0; n--) h = __ffma2_rn(h, tau, k.nc2[n]);
+    for (int n = 8; n >= 0; n--) h = __ffma2_rn(h, v, k.nc2[n]);
     const float2 a = __fmul2_rn(s, k.nq2[1]);
     const float2 e = make_float2(ex2_approx(a.x), ex2_approx(a.y));
-    f0 = __fmul2_rn(__fmul2_rn(__fmul2_rn(h, w), e), ri);
+    f0 = __fmul2_rn(__fmul2_rn(__ffma2_rn(h, v, one), e), ri);
     t = __fmul2_rn(__ffma2_rn(e, k.kn2, f0), __fmul2_rn(ri, ri));
     return;
   }

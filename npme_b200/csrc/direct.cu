@@ -24,14 +24,16 @@
 
 namespace npme {
 
-// Original Ewald split in FP32: erfcx(x) (x + 3) = sum_n e_n tau^n with tau =
-// (x - 3)/(x + 3), a relative-error fit of degree 9 over 0 <= x <= 12 (error
-// 5e-09, below FP32 rounding; beyond x = 10.2 exp(-x^2) is zero in FP32).
+// Original Ewald split in FP32: erfcx(x) = 1 + v sum_n e_n v^n with v = x / (x +
+// 2), a fit of degree 9 over 0 <= x <= 12 (error 2e-09, below FP32 rounding;
+// beyond x = 10.2 exp(-x^2) is zero in FP32).  In v the value at x = 0 is exact
+// and the rounding errors near it, where the pairs that matter most are, grow
+// with v: 2e-08 RMS for x < 0.3.
 constexpr double kErfcxFit[10] = {
-    1.0740069096e+00, -8.8339451071e-01, 5.9022814413e-01, 
-    -3.1046536357e-01, 1.1953133388e-01, -2.6843410022e-02, 
-    -1.2380858249e-03, 3.0828154886e-03, -4.6349936557e-04, 
-    -3.1471575889e-04};
+    -2.2567580482e+00, 1.7432280943e+00, -2.7456315043e-01,
+    -3.1246204138e-01, 1.2640637311e-02, 7.3816158880e-02,
+    3.7015627549e-02, 2.7656030148e-02, -8.1190085803e-02,
+    3.0625252134e-02};
 
 template <typename T>
 PairCoef<T> make_pair_coef(const npme_handle *h) {
