@@ -281,9 +281,11 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     S.G = (const float *)h->d_G;
     S.N1 = h->grid.N[0], S.N2 = h->grid.N[1], S.N3 = h->grid.N[2];
     S.g1 = h->gd[0], S.g2 = h->gd[1], S.g3 = h->gd[2];
-    S.c1 = (float)(h->grid.N[0] / h->box[6]);
-    S.c2 = (float)(h->grid.N[1] / h->box[7]);
-    S.c3 = (float)(h->grid.N[2] / h->box[8]);
+    const int P = h->grid.order;
+    const double dw = npme::spline_scale(P) / npme::spline_scale(P - 1);
+    S.c1 = (float)(h->grid.N[0] / h->box[6] * dw);
+    S.c2 = (float)(h->grid.N[1] / h->box[7] * dw);
+    S.c3 = (float)(h->grid.N[2] / h->box[8] * dw);
     S.gpos = h->d_gpos;
     S.spos = h->d_spos;
     S.groups = h->d_groups;

@@ -508,7 +508,8 @@ __device__ __forceinline__ double2 fhat_sample_body(const LR &lr, long idx, int 
 // the brick's theta tile of (kBrick + P - 1)^3 grid points is read into
 // shared memory once, then every point gathers its p^3 stencil from the
 // tile: V += sum theta B1 B2 B3, grad += (N/L) sum theta dB ..., added into
-// the caller-order output.  With vsrc (CalcV after a pair-once direct sum)
+// the caller-order output; c1, c2, c3 are N/L times the scale of weights to
+// that of their derivatives (bspline_weights).  With vsrc (CalcV after a pair-once direct sum)
 // the point's source-side direct-sum slot (same brick-order position) is
 // added in the same read-modify-write of V (potential scaled by vs,
 // gradient by gs) and cleared for the next call.

@@ -79,11 +79,39 @@ __device__ __forceinline__ double erfc_t(double x) { return erfc(x); }
 __device__ __forceinline__ void sincos_t(float x, float *s, float *c) { sincosf(x, s, c); }
 __device__ __forceinline__ void sincos_t(double x, double *s, double *c) { sincos(x, s, c); }
 
-// Cardinal B-spline weights of order P at the stencil points u + t,
-// t = 0..P-1, with u = w + mStart in [0, 1] (the reference evaluates
-// B_P(w + m) for m = mStart..mStart+P-1, src/RecSumQ.cpp:58-84).  Raised by
-// B_{j+1}(x) = [x B_j(x) + (j + 1 - x) B_j(x - 1)] / j.  The derivative uses
-// dB_P/dw (x) = B_{P-1}(x) - B_{P-1}(x - 1) (src/Bspline.cpp:16766).
+// The recursion's division by j as a multiplication by a power of two (exact, and
+// free within a multiply-add), which leaves the weights of order P scaled by
+// spline_scale(P) in (1/2, 1]: the kernel transform takes the scale out again, in
+// FP64 (lambda2_host).  Rounded reciprocals 1/3, 1/5, 1/6, 1/7 made every FP32
+// weight of order 8 too large by 1e-7, the potential by 5e-7 in all.
+__host__ __device__ constexpr double spline_step(int j) {
+  switch (j) {
+    case 0: case 1: return 1.0;
+    case 2: return 0.5;
+    case 3: case 4: case 5: return 0.25;
+    case 6: case 7: case 8: case 9: case 10: case 12: return 0.125;
+    default: return 0.0625;
+  }
+}
+__host__ __device__ constexpr double spline_scale(int P) {
+  double s = 1.0;
+  for (int j = 2; j < P; j++) s *= j * spline_step(j);
+  return s;
+}
+
+// Cardinal B-spline weights of order P, times spline_scale(P), at the stencil
+// points u + t, t = 0..P-1, with u = w + mStart in [0, 1] (the reference
+// evaluates B_P(w + m) for m = mStart..mStart+P-1, src/RecSumQ.cpp:58-84).
+// Raised by B_{j+1}(x) = [x B_j(x) + (j + 1 - x) B_j(x - 1)] / j.  The derivative
+// uses dB_P/dw (x) = B_{P-1}(x) - B_{P-1}(x - 1) (src/Bspline.cpp:16766); dw is
+// times spline_scale(P - 1).
+// The weights that spread FP32 charges are multiples of 2^-24 (so that their sum
+// is exact) and add up to spline_scale(P) exactly: the net charge of a grid, which
+// a neutral system's long-range potential hangs on, was off by 1e-7 of each
+// charge.  With both, the error of r^-0.5 at 200k points went from 5e-07-1.2e-06
+// (by the charges drawn) to 2.2e-07-2.7e-07, at 0-3 us of 131 for spreading.
+// Interpolation leaves its weights as they are: rounding them too gained less
+// and cost it 30 us of 100 at 1M points.
 template <typename T, int P, bool DERIV>
 __device__ __forceinline__ void bspline_weights(T u, T (&w)[P], T (&dw)[P]) {
   T c[P];
@@ -100,14 +128,28 @@ __device__ __forceinline__ void bspline_weights(T u, T (&w)[P], T (&dw)[P]) {
         dw[t] = cur - prev;
       }
     }
-    const T inv = T(1) / T(j);
+    const T step = T(spline_step(j));
 #pragma unroll
     for (int k = j; k >= 0; k--) {
-      const T x = u + T(k);
       const T left = (k <= j - 1) ? c[k] : T(0);
       const T right = (k >= 1) ? c[k - 1] : T(0);
-      c[k] = (x * left + (T(j + 1) - x) * right) * inv;
+      if constexpr (sizeof(T) == 4) {
+        const T x = fma(u, step, T(k) * step);
+        c[k] = x * left + (T(j + 1) * step - x) * right;
+      } else {
+        const T x = u + T(k);
+        c[k] = (x * left + (T(j + 1) - x) * right) * step;
+      }
     }
+  }
+  if constexpr (sizeof(T) == 4 && !DERIV) {
+    T rest = T(spline_scale(P));
+#pragma unroll
+    for (int t = 0; t < P; t++) {
+      c[t] = (c[t] + T(1)) - T(1);
+      rest -= c[t];
+    }
+    c[P / 2] += rest;
   }
 #pragma unroll
   for (int t = 0; t < P; t++) w[t] = c[t];

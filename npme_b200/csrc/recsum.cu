@@ -304,11 +304,14 @@ static double bspline_host(int n, double w) {
   return c[i0];
 }
 
-// |1/sum_p B_n(p) exp(-2 pi i k p / N)|^2 for k = 0..N/2 (src/RecSumV.cpp:565-581)
+// |1/sum_p B_n(p) exp(-2 pi i k p / N)|^2 for k = 0..N/2 (src/RecSumV.cpp:565-581),
+// over the square of the scale that spreading and interpolation leave in the
+// weights of an axis (spline_step)
 static void lambda2_host(long N, int order, std::vector<double> &out) {
   std::vector<double> b(order + 1);
   for (int p = 0; p <= order; p++) b[p] = bspline_host(order, p);
   out.resize(N / 2 + 1);
+  const double scale = spline_scale(order);
   for (long k = 0; k <= N / 2; k++) {
     const double z = (double)k / (double)N;
     double dr = 0, di = 0;
@@ -316,7 +319,7 @@ static void lambda2_host(long N, int order, std::vector<double> &out) {
       dr += b[p] * std::cos(2.0 * M_PI * z * p);
       di -= b[p] * std::sin(2.0 * M_PI * z * p);
     }
-    out[k] = 1.0 / (dr * dr + di * di);
+    out[k] = 1.0 / ((dr * dr + di * di) * (scale * scale));
   }
 }
 
@@ -985,12 +988,14 @@ static void interp_dispatch(npme_handle *h, double *d_V, cudaStream_t s) {
   constexpr int TL = kBrick + P - 1;
   const size_t smem = sizeof(T) * TL * TL * TL * (CPLX ? 2 : 1);
   const double *L = h->box + 6;
+  constexpr double dw = spline_scale(P) / spline_scale(P - 1);  // of the derivatives' weights
   auto kern = interp_kernel<T, P, CPLX>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   kern<<<(unsigned)h->n_nonempty, 256, smem, s>>>(
       h->d_brick_list, h->d_brick_start, (const BrickPoint<T> *)h->d_bpts, (const T *)h->d_grid,
       d_V, (int)h->grid.nb[1], (int)h->grid.nb[2], h->gd[0], h->gd[1], h->gd[2],
-      (T)(h->grid.N[0] / L[0]), (T)(h->grid.N[1] / L[1]), (T)(h->grid.N[2] / L[2]),
+      (T)(h->grid.N[0] / L[0] * dw), (T)(h->grid.N[1] / L[1] * dw),
+      (T)(h->grid.N[2] / L[2] * dw),
       h->merge_pending ? (h->fp32 ? (void *)h->d_vsrc : (void *)h->d_vsrc64) : nullptr,
       h->merge_vs, h->merge_gs);
 }
