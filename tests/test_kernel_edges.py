@@ -1,0 +1,233 @@
+"""Edges of the kernels' tilings and of the rules that choose between them:
+transform lengths, B-spline orders, warps per target group, source zones,
+runtime exponents, and what a non-finite charge reaches.
+
+Tolerances (relative 2-norm): FP64 against the oracle 1e-12 (the same
+algorithm; sums of up to 1e4 terms in another order), the two FP64 walks of
+the same pairs 1e-13; FP32 against FP64 1e-5 for V and 3e-5 for the gradient
+(the stated bound of the FP32 mode), the two FP32 walks 1e-6.
+"""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from conftest import rel
+import npme_b200
+from npme_b200 import api
+from npme_b200.workloads import Workload
+from oracle import orcbind as ob
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": (1e-12, 1e-12), "fp32": (1e-5, 3e-5)}
+WALKS = {"fp64": 1e-13, "fp32": 1e-6}
+
+
+def check(V, Vo, prec, scale=1.0):
+    assert rel(V[:, 0], Vo[:, 0]) < scale * TOL[prec][0]
+    assert rel(V[:, 1:], Vo[:, 1:]) < scale * TOL[prec][1]
+
+
+def system(n, func="laplace", split="dm", box=(10.0, 10.0, 10.0), grid=(48, 48, 48), order=6,
+           Rdir=4.0, alpha=-0.5, k0=0.5, **kw):
+    cplx = func == "helmholtz"
+    return Workload("edge", n, box, func, split, order, grid, Rdir, alpha=alpha,
+                    k0=k0 if cplx else 0.0, complex_charge=cplx, seed=7000 + n, **kw)
+
+
+def direct(s, q):
+    import torch
+    cplx = np.iscomplexobj(q)
+    dq = torch.from_numpy(np.ascontiguousarray(q)).cuda()
+    dV = torch.zeros((len(q), 8 if cplx else 4), dtype=torch.float64, device="cuda")
+    st = torch.cuda.Stream()
+    st.wait_stream(torch.cuda.current_stream())
+    s.direct_sum_device(dV.data_ptr(), dq.data_ptr(), st.cuda_stream)
+    st.synchronize()
+    V = dV.cpu().numpy()
+    return V.view(np.complex128) if cplx else V
+
+
+def both_walks(w, prec, monkeypatch):
+    """The direct sum with every pair once and from both sides."""
+    c, q = w.generate()
+    out = {}
+    for mode in ("0", "1"):
+        monkeypatch.setenv("NPME_PAIRS_ONCE", mode)
+        with npme_b200.Solver(api.params_from_workload(w, precision=prec)) as s:
+            out[mode] = direct(s.setup(c), q)
+    return c, q, out["0"], out["1"]
+
+
+# Lengths: the shortest, every radix (2, 3, 4, 5, 6, 8, 9, 10, 12, 16) and odd
+# ones, long ones in each place (2,048 is the longest), and one with a prime
+# factor above 5, which the library's own transforms leave to cuFFT.
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("func", ["laplace", "helmholtz"])
+@pytest.mark.parametrize("grid,order", [
+    ((20, 20, 20), 4), ((24, 36, 60), 4), ((100, 72, 40), 6), ((108, 80, 64), 6),
+    ((64, 96, 144), 6), ((180, 48, 200), 6), ((64, 28, 96), 6), ((2048, 32, 36), 6),
+    ((32, 2048, 60), 6), ((32, 40, 2048), 6), ((1920, 32, 32), 6), ((32, 36, 2000), 6),
+    ((36, 32, 1620), 6)])
+def test_transform_lengths(grid, order, func, prec):
+    w = system(300, func, grid=grid, order=order)
+    c, q = w.generate()
+    with npme_b200.Solver(api.params_from_workload(w, precision=prec)) as s:
+        V = s.setup(c).calcv(q)
+    check(V, ob.calcv(ob.params_from_workload(w), c, q), prec)
+
+
+# Orders up to 8 accumulate a brick in registers, larger ones in shared memory;
+# one point, points that fill one brick (several batches a warp) with two far
+# corners, and a uniform system.
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("func", ["laplace", "helmholtz"])
+@pytest.mark.parametrize("order", [4, 6, 8, 10])
+@pytest.mark.parametrize("shape", ["one", "brick", "uniform"])
+def test_spread_orders(shape, order, func, prec):
+    w = system({"one": 1, "brick": 2746, "uniform": 1500}[shape], func, order=order)
+    c, q = w.generate()
+    q = q + 1.5  # one sign: the smooth part is as large as the rest
+    if shape == "brick":
+        g = np.arange(14) * 0.06 + 5.0
+        c[:2744] = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
+        c[2744:] = [[0.0, 0.0, 0.0], [10.0, 10.0, 10.0]]
+    Vo = ob.calcv(ob.params_from_workload(w), c, q)
+    with npme_b200.Solver(api.params_from_workload(w, precision=prec)) as s:
+        V = s.setup(c).calcv(q)
+    if shape == "one":  # a cancellation: against the scale of its terms
+        assert np.abs(V - Vo).max() <= TOL[prec][0] * np.abs(q[0])
+    else:
+        check(V, Vo, prec)
+
+
+# Warps per group of 32 targets: 16 up to 148 groups, 8 up to 592, 4 up to
+# 2,960, else one; sources by target halves from 18,944 points (FP64) and
+# 94,720 (FP32 r^alpha and Helmholtz).
+@pytest.mark.parametrize("func,split,prec,n", [
+    (f, s, p, n)
+    for f, s, p, sizes in [
+        ("laplace", "dm", "fp32", (31, 3000, 15000, 60000, 100001)),
+        ("laplace", "orig", "fp32", (31, 15000, 100001)),
+        ("ralpha", "dm", "fp32", (31, 3000, 94719, 94720)),
+        ("helmholtz", "dm", "fp32", (31, 3000, 15000, 94719, 94720)),
+        ("laplace", "dm", "fp64", (31, 3000, 18943, 18944, 100001)),
+        ("laplace", "orig", "fp64", (3000, 18944)),
+        ("ralpha", "dm", "fp64", (3000, 18943, 18944)),
+        ("helmholtz", "dm", "fp64", (31, 3000, 18943, 18944, 100001))]
+    for n in sizes])
+def test_group_splits_and_zones(func, split, prec, n, monkeypatch):
+    side = max(n, 1000) ** (1 / 3)
+    w = system(n, func, split, box=(side, 1.5 * side, side / 1.5), Rdir=3.5)
+    _, _, two, one = both_walks(w, prec, monkeypatch)
+    assert rel(one[:, 0], two[:, 0]) < WALKS[prec]
+    assert rel(one[:, 1:], two[:, 1:]) < WALKS[prec]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("alpha,nd", [(1.0, 6), (3.0, 3), (0.5, 8), (-3.0, 6), (-2.5, 10),
+                                      (-1.0, 3)])
+def test_exponents(alpha, nd, prec, monkeypatch):
+    w = system(2500, "ralpha", alpha=alpha, nDeriv=nd)
+    c, q, two, one = both_walks(w, prec, monkeypatch)
+    Vo = ob.direct(ob.params_from_workload(w), c, q)
+    for V in (two, one):
+        check(V, Vo, prec)
+
+
+# Damped waves, and |k0| Rdir on both sides of 1e5, above which the FP64 pairs
+# are evaluated from both sides with the library's sine and cosine.  At order 2
+# the matched polynomial's terms reach (k0 Rdir)^2 times the sum, so the walks
+# differ by their rounding (eps 1e10 at most), relative to the polynomial.
+@pytest.mark.parametrize("k0,nd,tol", [(0.5, 6, 1e-13), (1.1 + 0.2j, 8, 1e-12),
+                                       (3.0 - 0.4j, 4, 1e-12), (24999.0, 2, 1e-9),
+                                       (25001.0, 2, 1e-9)])
+def test_fp64_helmholtz_wave_numbers(k0, nd, tol, monkeypatch):
+    w = system(1500, "helmholtz", k0=k0, nDeriv=nd)
+    c, q, two, one = both_walks(w, "fp64", monkeypatch)
+    assert rel(one, two) < tol
+    if abs(k0) < 100:
+        Vo = ob.direct(ob.params_from_workload(w), c, q)
+        assert rel(one, Vo) < 10 * tol
+
+
+# The exact sum: partial groups, coincident points (whose gradients are not
+# finite) and target subsets, which divide the sources among several CTAs.
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("func,alpha", [("laplace", -1.0), ("ralpha", 2.0), ("helmholtz", -1.0)])
+@pytest.mark.parametrize("n", [1, 2, 33, 257, 5001])
+def test_exact_sum_shares(n, func, alpha, prec):
+    w = system(n, func, alpha=alpha)
+    c, q = w.generate()
+    q = q + 0.5
+    same = [0, n // 2, n - 1] if n > 2 else []
+    c[same] = c[:1]
+    targets = np.unique(np.linspace(0, n - 1, 37).astype(np.uint32))
+    with npme_b200.Solver(api.params_from_workload(w, precision=prec)) as s:
+        s.setup(c)
+        V, Vs = s.calcv_exact(q), s.calcv_exact_subset(targets, q)
+        V1 = s.calcv_exact_subset(targets[-1:], q)
+    Vo = ob.exact(ob.params_from_workload(w), c, q)
+    single = np.setdiff1d(np.arange(n), same)
+    scale = np.abs(Vo[single]).max() if n > 1 else 1.0
+    for got, rows in ((V, np.arange(n)), (Vs, targets), (V1, targets[-1:])):
+        ok = np.isin(rows, single)
+        assert (np.abs(got[ok] - Vo[rows[ok]]) <= 1e-12 * scale).all()
+        assert not np.isfinite(got[~ok, 1:]).any()
+
+
+# A non-finite charge reaches the points within the cutoff and no others.
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+@pytest.mark.parametrize("func,split,prec", [
+    ("laplace", "dm", "fp32"), ("laplace", "orig", "fp32"), ("ralpha", "dm", "fp32"),
+    ("helmholtz", "dm", "fp32"), ("laplace", "dm", "fp64"), ("ralpha", "dm", "fp64"),
+    ("helmholtz", "dm", "fp64")])
+@pytest.mark.parametrize("n", [3000, 20000])
+def test_non_finite_charge_stays_local(n, func, split, prec, bad):
+    side = n ** (1 / 3)
+    w = system(n, func, split, box=(side, side, side), Rdir=3.5)
+    c, q = w.generate()
+    k = n // 3
+    with npme_b200.Solver(api.params_from_workload(w, precision=prec)) as s:
+        s.setup(c)
+        q[k] = 0.0
+        V0 = direct(s, q)
+        q[k] = bad
+        V = direct(s, q)
+    r = np.linalg.norm(c - c[k], axis=1)
+    far = r > w.Rdir * (1 + 1e-6)
+    assert rel(V[far], V0[far]) < WALKS[prec]
+    assert not np.isfinite(V[(r > 0) & (r < 0.9 * w.Rdir), 0]).any()
+
+
+# Batches: the members' classes (function, order, exponent) with few and many
+# groups, beside each other, against each member's own CalcV.
+def test_batch_classes():
+    import torch
+    members = [system(40), system(1200, order=8, nDeriv=8), system(9000, box=(20.0, 20.0, 20.0)),
+               system(40000, box=(33.0, 33.0, 33.0), grid=(64, 80, 96)),
+               system(3000, split="orig"), system(2000, "ralpha"),
+               system(2000, "ralpha", alpha=2.0),
+               system(2500, "helmholtz"), system(12000, "helmholtz", box=(20.0, 20.0, 24.0)),
+               system(1000, grid=(56, 48, 44))]
+    solvers, qs, outs, alone = [], [], [], []
+    for w in members:
+        c, q = w.generate()
+        s = npme_b200.Solver(api.params_from_workload(w, precision="fp32")).setup(c)
+        alone.append(s.calcv(q))
+        solvers.append(s)
+        qs.append(torch.from_numpy(np.ascontiguousarray(q)).cuda())
+        outs.append(torch.empty((w.n, 8 if np.iscomplexobj(q) else 4), dtype=torch.float64,
+                                device="cuda"))
+    torch.cuda.synchronize()
+    b = api.Batch()
+    b.calcv(solvers, [o.data_ptr() for o in outs], [q.data_ptr() for q in qs])
+    b.sync()
+    for o, V in zip(outs, alone):
+        got = o.cpu().numpy()
+        got = got.view(np.complex128) if np.iscomplexobj(V) else got
+        assert rel(got[:, 0], V[:, 0]) < 1e-6 and rel(got[:, 1:], V[:, 1:]) < 1e-6
+    b.close()
+    for s in solvers:
+        s.close()
