@@ -176,8 +176,8 @@ int npme_gpu_calcv_device(npme_handle *h, double *d_V, const double *d_charge,
  * stream semantics as npme_gpu_calcv_device.  Like the reference's cell-pair
  * loops it evaluates every pair once for both points (built-in kernels and
  * real caller kernels; complex caller kernels, and FP64 Helmholtz with
- * |k0| Rdir >= 1e5, walk each target's sources), adding the source-side sums with atomics, so repeated
- * calls can differ in the last bits (NPME_PAIRS_ONCE=0 at set-up: one-sided,
+ * |k0| Rdir >= 1e5, walk each target's sources), adding the source-side sums
+ * with atomics, so repeated calls can differ in the last bits (NPME_PAIRS_ONCE=0 at set-up: one-sided,
  * reproducible). */
 int npme_gpu_direct_sum_device(npme_handle *h, double *d_V, const double *d_charge,
                                void *stream);

@@ -433,7 +433,8 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   for (auto &kv : gath) {
     Class &c = kv.second;
     const unsigned g = grid_of(c.off.back(), 256, 148 * 16);
-    if (kv.first) batch_gather_kernel<true><<<g, 256, 0, b->stream2>>>(D(c), O(c), (int)c.members.size());
+    const int m = (int)c.members.size();
+    if (kv.first) batch_gather_kernel<true><<<g, 256, 0, b->stream2>>>(D(c), O(c), m);
     else batch_gather_kernel<false><<<g, 256, 0, b->stream2>>>(D(c), O(c), (int)c.members.size());
     b->launches++;
   }

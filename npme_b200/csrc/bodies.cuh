@@ -1033,9 +1033,9 @@ struct SymWarp {
 // misses also get charge 0 (a non-finite charge stays out of their sums).
 template <int FUNC, int ND, bool CHECKED>
 __device__ __forceinline__ void sym_step(const PairCoef<float> &k, const SymWarp &W, int j,
-                                         int lane, const SymSource (&src)[kSymSources], float refine2,
-                                         float2 &aV,
-                                         float2 &aX, float2 &aY, float2 &aZ, float2 (&S)[kSymSources][4]) {
+                                         int lane, const SymSource (&src)[kSymSources],
+                                         float refine2, float2 &aV, float2 &aX, float2 &aY,
+                                         float2 &aZ, float2 (&S)[kSymSources][4]) {
   const float4 A = W.t[j], B = W.t[16 + j];
   float2 x[kSymSources], y[kSymSources], z[kSymSources], s[kSymSources], qs[kSymSources],
       qt[kSymSources];
@@ -1097,8 +1097,8 @@ __device__ __forceinline__ float2 rotate2(float2 v, int src) {
 // (zone 1: pairs 0-7, zone 2: pairs 8-15); target sums rotate after each.
 template <int FUNC, int ND, bool CHECKED>
 __device__ __forceinline__ void sym_sweep(const PairCoef<float> &k, const SymWarp &W,
-                                          const SymSource (&src)[kSymSources], float refine2, int lane,
-                                          int zone, float2 &aV,
+                                          const SymSource (&src)[kSymSources], float refine2,
+                                          int lane, int zone, float2 &aV,
                                           float2 &aX, float2 &aY, float2 &aZ,
                                           float2 (&S)[kSymSources][4]) {
   constexpr int kUnroll = CHECKED ? 1 : 8;
@@ -1268,7 +1268,8 @@ __device__ __forceinline__ void direct_group_sym(
     float2 aV = make_float2(0.f, 0.f), aX = aV, aY = aV, aZ = aV;
     float2 S[kSymSources][4];
 #pragma unroll
-    for (int i = 0; i < kSymSources; i++) S[i][0] = S[i][1] = S[i][2] = S[i][3] = make_float2(0.f, 0.f);
+    for (int i = 0; i < kSymSources; i++)
+      S[i][0] = S[i][1] = S[i][2] = S[i][3] = make_float2(0.f, 0.f);
     if (checked)
       sym_sweep<FUNC, ND, true>(k, W, src, refine2, lane, zone, aV, aX, aY, aZ, S);
     else
@@ -2343,8 +2344,8 @@ __device__ __forceinline__ void store_targets64(const int4 G, const uint32_t *__
 // sources of a 64-source chunk of the half-shell segments, target (l + k)
 // mod 32 meets lane l at step k and its sums rotate one lane down per step;
 // the source-side sums of a chunk go to vsrc ([n][4] doubles, slot = the
-// source's brick-order position) with one FP64 atomic per component.  Pairs inside the group are a first,
-// one-sided pass.  Same pair arithmetic as direct_group_fp64.
+// source's brick-order position) with one FP64 atomic per component.  Pairs
+// inside the group are a first, one-sided pass.  Same pair arithmetic as direct_group_fp64.
 template <int FUNC, int SPLIT, int ND, class PK = BuiltinPair>
 __device__ __forceinline__ void direct_group_sym64(
     const PairCoef<double> &k, const double4 *__restrict__ gpos,

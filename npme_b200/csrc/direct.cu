@@ -331,7 +331,8 @@ static void sym_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream_t s) {
     const long blocks = (h->n_hgroups + kGroupWarps - 1) / kGroupWarps;
     direct_sym_kernel<FUNC, ND><<<(unsigned)blocks, 32 * kGroupWarps, 0, s>>>(
         k, h->d_gpos, h->d_spos, (const float *)a.q, a.qcaller, h->d_hgroups, h->d_hcen,
-        h->d_hsegs, h->d_hzones, h->d_cperm, h->n_hgroups, (float)h->refine2, a.fself_r, a.V, h->d_vsrc);
+        h->d_hsegs, h->d_hzones, h->d_cperm, h->n_hgroups, (float)h->refine2, a.fself_r, a.V,
+        h->d_vsrc);
   }
   merge_or_defer(h, a, s, k.vscale, k.gscale);
 }
@@ -352,7 +353,8 @@ __global__ void __launch_bounds__(32 * kGroupWarps) direct_sym64_kernel(
   if constexpr (SPLIT == 0) {
     double acc[4] = {0, 0, 0, 0};
     const int4 G = groups[g];
-    direct_group_sym64_dm<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, vsrc,
+    direct_group_sym64_dm<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm,
+                                    vsrc,
                                     tsm[wid], lane, 0, 1, acc);
     store_targets64(G, perm, qcaller, fself_r, k.vscale, k.gscale, V, lane, acc);
   } else
@@ -375,7 +377,8 @@ __global__ void __launch_bounds__(32 * kMaxSplit) direct_sym64_split_kernel(
   const long g = blockIdx.x;
   double acc[4] = {0, 0, 0, 0};
   const int4 G = groups[g];
-  direct_group_sym64_dm<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, vsrc,
+  direct_group_sym64_dm<FUNC, ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm,
+                                  vsrc,
                                   tsm[wid], lane, wid, nsplit, acc);
   reduce_parts(acc, red, wid, nsplit, lane);
   if (wid == 0) store_targets64(G, perm, qcaller, fself_r, k.vscale, k.gscale, V, lane, acc);
@@ -404,7 +407,8 @@ static void sym64_launch_nd(npme_handle *h, const DirectArgs &a, cudaStream_t s)
     if (split > 1) {
       direct_sym64_split_kernel<FUNC, ND><<<(unsigned)h->n_hgroups, 32 * split, 0, s>>>(
           make_pair_coef<double>(h), h->d_gpos, h->d_spos, (const double *)a.q, a.qcaller,
-          h->d_hgroups, h->d_hcen, h->d_hsegs, h->d_hzones, h->d_cperm, a.fself_r, a.V, h->d_vsrc64);
+          h->d_hgroups, h->d_hcen, h->d_hsegs, h->d_hzones, h->d_cperm, a.fself_r, a.V,
+          h->d_vsrc64);
       merge_or_defer(h, a, s, 1.0, 1.0);
       return;
     }
@@ -434,7 +438,8 @@ __global__ void __launch_bounds__(32 * (SPLIT ? kMaxSplit : kGroupWarps), SPLIT 
   if (g >= ngroups) return;  // warp-uniform (SPLIT: no CTA is past the end)
   double acc[4] = {0, 0, 0, 0}, acci[4] = {0, 0, 0, 0};
   const int4 G = groups[g];
-  direct_group_sym64_helm<ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, vsrc, tsm[wid],
+  direct_group_sym64_helm<ND>(k, gpos, spos, qs, qcaller, G, gcen[g], segs, zones[g], perm, vsrc,
+                              tsm[wid],
                               lane, part, nsplit, acc, acci);
   if constexpr (SPLIT) {
     __shared__ double red[kMaxSplit][32][4];

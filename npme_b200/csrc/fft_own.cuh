@@ -20,9 +20,9 @@
 // held in shared memory as [element][line], so that consecutive threads touch
 // consecutive lines: Stockham passes of radix 16, 12, 10, 9, 8, 6, 5, 4, 3 and
 // 2, two buffers, one barrier per pass; nearly every length up to 256 takes two
-// passes, i.e. crosses shared memory once.  Along x and y, consecutive lines are consecutive in
-// memory, and the first pass loads from and the last pass stores to global
-// memory directly; along z the rows are loaded and stored element by element
+// passes, i.e. crosses shared memory once.  Along x and y, consecutive lines are
+// consecutive in memory, and the first pass loads from and the last pass stores
+// to global memory directly; along z the rows are loaded and stored element by element
 // (coalesced) with a padded line pitch in shared memory, and real rows are
 // transformed as complex ones of half the length.
 #pragma once

@@ -69,10 +69,10 @@ __global__ void __launch_bounds__(kFftThreads)
 
 namespace {
 
-// Radices of N, as few as possible, then the smallest largest one; an even one
-// first (half of the line is zero at the start and unwanted at the end of the
-// reverse order); none above `largest`; empty when N has a factor other than 2, 3 and 5 or fewer than two
-// passes.
+// Radices of N, as few as possible, then the smallest largest one, none above
+// `largest`; an even one first (half of the line is zero at the start and
+// unwanted at the end of the reverse order).  Empty when N has a factor other
+// than 2, 3 and 5 or takes fewer than two passes.
 std::vector<int> radices(long N, int largest = 16) {
   static const int kR[] = {16, 12, 10, 9, 8, 6, 5, 4, 3, 2};
   // products of at most `left` radices, none above cap

@@ -270,9 +270,9 @@ size_t own_fft_smem(const FftJob &j, int axis, size_t cbytes);
 // recsum.cu
 int build_kernel_transform(npme_handle *h);  // F-hat, lambda^2 -> d_G
 // The kernel transforms of several handles (one precision), on the owner's
-// second stream, beside the geometry on its first: one launch per stage for every class of two or more handles with
-// a built-in kernel (real, complex), the rest one by one on their own
-// second streams.  status[k] gets each handle's result.
+// second stream, beside the geometry on its first: one launch per stage for
+// every class of two or more handles with a built-in kernel (real, complex), the
+// rest one by one on their own second streams.  status[k] gets each handle's result.
 void build_kernel_transforms(npme_handle **hs, int R, npme_handle *owner, int *status);
 void launch_spread(npme_handle *h, const double *d_q, cudaStream_t s);
 void launch_multiply(npme_handle *h, cudaStream_t s);

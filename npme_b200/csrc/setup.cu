@@ -505,7 +505,8 @@ __global__ void __launch_bounds__(256)
                   const int *__restrict__ sstart, const unsigned long long *__restrict__ skey,
                   int zf, const unsigned *__restrict__ sorder,
                   const unsigned *__restrict__ cpos, int4 *__restrict__ ug,
-                  int4 *__restrict__ uh, int2 *__restrict__ uz, double4 *__restrict__ cen, int *__restrict__ bin,
+                  int4 *__restrict__ uh, int2 *__restrict__ uz,
+                  double4 *__restrict__ cen, int *__restrict__ bin,
                   int *__restrict__ hbin, SysStats *st) {
   const long slot = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -685,7 +686,8 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     order_groups_kernel(const SysDesc *__restrict__ d, const int *__restrict__ goff,
                         const int4 *__restrict__ ug, const int4 *__restrict__ uh,
-                        const int2 *__restrict__ uz, const double4 *__restrict__ cen, const int *__restrict__ bin,
+                        const int2 *__restrict__ uz, const double4 *__restrict__ cen,
+                        const int *__restrict__ bin,
                         const int *__restrict__ hbin, SysStats *st) {
   __shared__ int first[kWorkBins];
   __shared__ int warp_sum[8];
@@ -1074,7 +1076,8 @@ int geometry_batch(npme_handle **hs, int R, cudaStream_t s, const std::function<
 
   // --- warp groups and their source segments, heaviest groups first ---
   groups_kernel<<<blocks_for(32 * G), 256, 0, s>>>(dd, goffs, R, G, goff, cstart, sstart, ckey, zf,
-                                                  sorder, cpos, ug, uh, uz, cen, bins, bins + G, st);
+                                                  sorder, cpos, ug, uh, uz, cen, bins,
+                                                  bins + G, st);
   const dim3 og((unsigned)blocks_for(gmax), (unsigned)R, full ? 2 : 1);
   order_groups_kernel<<<og, 256, 0, s>>>(dd, goff, ug, uh, uz, cen, bins, bins + G, st);
   // the counts, for the host to read when the set-up has completed
