@@ -109,9 +109,10 @@ struct npme_handle {
   npme::CellGeom cells;
   long n_bricks = 0, n_nonempty = 0;
 
+  // set-up, host entry points and the reciprocal chain, at high priority: the
+  // chain's CTAs go before the direct sum's
   cudaStream_t stream = nullptr;
   cudaStream_t stream2 = nullptr;  // direct sum runs here, overlapped with the FFTs
-  cudaStream_t stream_hi = nullptr;  // reciprocal chain: its CTAs go before the direct sum's
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_chain = nullptr;
   // shared plans (not owned): (y, z) slab transforms forward and inverse,
   // and the transforms along x (fft.cu)

@@ -401,7 +401,6 @@ static int setup_prepare(npme_handle *h, size_t n, const double *coord) {
   // src/Interface.cpp:1958-1987).
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->stream2) cudaStreamSynchronize(h->stream2);
-  if (h->stream_hi) cudaStreamSynchronize(h->stream_hi);
   h->ready = false;
   h->setup_gen++;  // a captured CalcV belongs to the previous geometry
   h->n = n;
@@ -554,12 +553,11 @@ int npme_gpu_create(const npme_params *p, npme_handle **out) {
   }
   h->device = p->device;
   cudaError_t e = cudaSetDevice(h->device);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking);
   int prio_lo = 0, prio_hi = 0;
   if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
   if (e == cudaSuccess)
-    e = cudaStreamCreateWithPriority(&h->stream_hi, cudaStreamNonBlocking, prio_hi);
+    e = cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, prio_hi);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_chain, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming);
@@ -595,7 +593,6 @@ int npme_gpu_set_params(npme_handle *h, const npme_params *p) {
   // work already enqueued may still read the handle's buffers and plans
   if (h->stream) CK(cudaStreamSynchronize(h->stream));
   if (h->stream2) CK(cudaStreamSynchronize(h->stream2));
-  if (h->stream_hi) CK(cudaStreamSynchronize(h->stream_hi));
   const npme_params old = h->p;
   h->p = q;
   if ((rc = apply_params(h))) {
@@ -615,7 +612,6 @@ int npme_gpu_set_user_kernel(npme_handle *h, const npme_user_ops *ops) {
   if (!h->user_kernel) return fail(h, NPME_EINVAL, "the handle's funcType is not NPME_FUNC_USER");
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->stream2) cudaStreamSynchronize(h->stream2);
-  if (h->stream_hi) cudaStreamSynchronize(h->stream_hi);
   h->uops = *ops;
   h->fself_r = ops->fself, h->fself_i = ops->fself_i;
   h->complex_kernel = ops->complex_kernel != 0;
@@ -635,8 +631,8 @@ static void tmark(npme_handle *h, int i, cudaStream_t s) {
 }
 
 // Enqueues one CalcV on the caller's stream (the launches; no checks): the
-// reciprocal chain on the high-priority stream and the direct sum, with the
-// gather of its charges, on stream2, both forked from the caller's stream; the
+// reciprocal chain on the handle's high-priority stream and the direct sum, with
+// the gather of its charges, on stream2, both forked from the caller's stream; the
 // interpolation joins them and the caller's stream waits for it.  The chain is a
 // row of short launches, the direct sum one long one that would otherwise hold
 // every SM while the chain waits in between: a flat 30k system took 141 us with
@@ -646,7 +642,7 @@ static void tmark(npme_handle *h, int i, cudaStream_t s) {
 // sum starts after it, so that each stage's events time that stage alone.
 static int enqueue_calcv(npme_handle *h, double *d_V, const double *d_charge, cudaStream_t user) {
   const bool timed = h->timing.enabled, serial = timed && h->timing.serial;
-  const cudaStream_t s = timed ? user : h->stream_hi;
+  const cudaStream_t s = timed ? user : h->stream;
   h->launches = 0;
   tmark(h, 0, s);
   if (timed) {
@@ -984,7 +980,6 @@ int npme_gpu_destroy(npme_handle *h) {
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->stream2) cudaStreamSynchronize(h->stream2);
-  if (h->stream_hi) cudaStreamSynchronize(h->stream_hi);
   if (h->graph) cudaGraphExecDestroy(h->graph);
   release(h);
   pool_release(h);
@@ -994,7 +989,6 @@ int npme_gpu_destroy(npme_handle *h) {
   npme::pinned_return(&h->h_ktdesc, &h->ktdesc_cap);
   if (h->stream) cudaStreamDestroy(h->stream);
   if (h->stream2) cudaStreamDestroy(h->stream2);
-  if (h->stream_hi) cudaStreamDestroy(h->stream_hi);
   if (h->ev_chain) cudaEventDestroy(h->ev_chain);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
   if (h->ev_join) cudaEventDestroy(h->ev_join);
