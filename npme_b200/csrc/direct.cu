@@ -109,6 +109,27 @@ PairCoef<T> make_pair_coef(const npme_handle *h) {
         const cd g2 = -(2.0 * (i + 2) - 1.0) * g1 - kap * kap * g0;
         g0 = g1, g1 = g2, f = fn;
       }
+      // FP64: the polynomial that the smooth part carries (its coefficients of
+      // r^2n, rounded, magnify their rounding by their cancellation, 1e3 at |k0|
+      // Rdir = 8), expanded about u = 0, so that what one part adds the other
+      // takes away: otherwise the sum is off by 2e-14 at |k0| Rdir = 10.  The FP32
+      // kernels need the value at the cutoff to be zero and keep the exact c_n.
+      if (sizeof(T) == 8) {
+        typedef long double ld;
+        ld cr[kMaxDeriv + 1] = {}, ci[kMaxDeriv + 1] = {}, scale = R;  // R^(2n + 1)
+        for (int n = 0; n <= k.nder && n <= kMaxDeriv; n++, scale *= (ld)R * R) {
+          ld binom = 1;  // (-1)^m n over m
+          for (int m = 0; m <= n; m++) {
+            cr[m] += binom * scale * (ld)h->a_r[n];
+            ci[m] += binom * scale * (ld)h->a_i[n];
+            binom *= -(ld)(n - m) / (m + 1);
+          }
+        }
+        for (int m = 0; m <= k.nder && m <= kMaxDeriv; m++) {
+          k.hc[m].x = (T)-cr[m], k.hc[m].y = (T)-ci[m];
+          if (m > 0) k.hd[m - 1].x = (T)(2 * m * cr[m]), k.hd[m - 1].y = (T)(2 * m * ci[m]);
+        }
+      }
     }
     k.vscale = std::pow(R, al);
     k.gscale = (k.split == NPME_SPLIT_LAPLACE_ORIG ? 1.0 : -al) * std::pow(R, al - 1.0);

@@ -152,6 +152,21 @@ def test_fp64_helmholtz_wave_numbers(k0, nd, tol, monkeypatch):
         assert rel(one, Vo) < 10 * tol
 
 
+# The two parts of FP64 Helmholtz carry the same matching polynomial, also where
+# its coefficients cancel (1e3 times the sum at |k0| Rdir = 8 to 10): their
+# rounding, eps times that, must not show in the total.  Tolerances: twice and
+# more of what two orders of summation differ by, a half and less of that rounding.
+@pytest.mark.parametrize("k0,Rdir,nd,order,tol", [(0.5, 4.0, 6, 6, 4e-15), (2.0, 4.0, 8, 6, 1e-14),
+                                                  (0.85, 12.0, 8, 8, 2e-14),
+                                                  (0.85, 12.0, 10, 8, 4e-14)])
+def test_fp64_helmholtz_parts_match(k0, Rdir, nd, order, tol):
+    w = system(1500, "helmholtz", k0=k0, Rdir=Rdir, nDeriv=nd, order=order, grid=(64, 64, 64))
+    c, q = w.generate()
+    with npme_b200.Solver(api.params_from_workload(w, precision="fp64")) as s:
+        V = s.setup(c).calcv(q)
+    assert rel(V, ob.calcv(ob.params_from_workload(w), c, q)) < tol
+
+
 # The exact sum: partial groups, coincident points (whose gradients are not
 # finite) and target subsets, which divide the sources among several CTAs.
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
