@@ -153,12 +153,12 @@ def test_fp64_helmholtz_wave_numbers(k0, nd, tol, monkeypatch):
 
 
 # The two parts of FP64 Helmholtz carry the same matching polynomial, also where
-# its coefficients cancel (1e3 times the sum at |k0| Rdir = 8 to 10): their
-# rounding, eps times that, must not show in the total.  Tolerances: twice and
-# more of what two orders of summation differ by, a half and less of that rounding.
-@pytest.mark.parametrize("k0,Rdir,nd,order,tol", [(0.5, 4.0, 6, 6, 4e-15), (2.0, 4.0, 8, 6, 1e-14),
-                                                  (0.85, 12.0, 8, 8, 2e-14),
-                                                  (0.85, 12.0, 10, 8, 4e-14)])
+# its coefficients cancel (1e3 times the sum at |k0| Rdir = 10): their rounding,
+# eps times that (4e-14 at order 8, 1.6e-13 at 10), must not show in the total,
+# whose own rounding is 5e-15 and 1e-14.
+@pytest.mark.parametrize("k0,Rdir,nd,order,tol", [(0.5, 4.0, 6, 6, 1e-14),
+                                                  (0.85, 12.0, 8, 8, 2.5e-14),
+                                                  (0.85, 12.0, 10, 8, 6e-14)])
 def test_fp64_helmholtz_parts_match(k0, Rdir, nd, order, tol):
     w = system(1500, "helmholtz", k0=k0, Rdir=Rdir, nDeriv=nd, order=order, grid=(64, 64, 64))
     c, q = w.generate()
