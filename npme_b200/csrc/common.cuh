@@ -15,11 +15,13 @@ template <typename T> struct Vec2;
 template <> struct Vec2<float> { using type = float2; };
 template <> struct Vec2<double> { using type = double2; };
 
-// Pair-kernel constants, passed by value to the kernels.  Polynomial
-// coefficients are stored in the scaled variable s = r^2 / Rdir^2:
+// Pair-kernel constants, passed by value to the kernels.  ar, ai, br, bi: the
+// matched polynomial as the one-sided walks take it, for Helmholtz in the scaled
+// variable s = r^2 / Rdir^2:
 //   f_LR(r) = sum_n ar[n] s^n,   (1/r) d f_LR / dr = sum_n br[n] s^n
 // (the reference's a_n r^(2n) and b_n r^(2n), src/FunctionDerivMatch.cpp:379-402,
-// with a_n Rdir^(2n) folded in, which keeps the coefficients O(1/Rdir)).
+// with a_n Rdir^(2n) folded in, which keeps the coefficients O(1/Rdir)), for the
+// real kernels in u = 1 - s (dm_taylor).
 template <typename T>
 struct PairCoef {
   int func;   // 0 Laplace, 1 Ralpha, 2 Helmholtz
@@ -155,19 +157,19 @@ __device__ __forceinline__ void bspline_weights(T u, T (&w)[P], T (&dw)[P]) {
   for (int t = 0; t < P; t++) w[t] = c[t];
 }
 
-// Horner in s for the scaled derivative-match polynomial and its radial
-// derivative.  Returns f_LR, writes (1/r) d f_LR/dr.  ND > 0 is the degree
-// known at compile time (fully unrolled, coefficients read at fixed offsets
-// of the parameter bank); ND == 0 reads the degree from k.nder.
+// Horner for the derivative-match polynomial and its radial derivative, in u =
+// 1 - s (real kernels) or s (Helmholtz).  Returns f_LR, writes (1/r) d f_LR/dr.
+// ND > 0 is the degree known at compile time (fully unrolled, coefficients read
+// at fixed offsets of the parameter bank); ND == 0 reads the degree from k.nder.
 template <typename T, int ND>
-__device__ __forceinline__ T dm_poly_real(const PairCoef<T> &k, T s, T &f1) {
+__device__ __forceinline__ T dm_poly_real(const PairCoef<T> &k, T u, T &f1) {
   const int N = ND > 0 ? ND : k.nder;
   T p = k.ar[N];
 #pragma unroll
-  for (int n = N - 1; n >= 0; n--) p = fma(p, s, k.ar[n]);
+  for (int n = N - 1; n >= 0; n--) p = fma(p, u, k.ar[n]);
   T d = k.br[N - 1];
 #pragma unroll
-  for (int n = N - 2; n >= 0; n--) d = fma(d, s, k.br[n]);
+  for (int n = N - 2; n >= 0; n--) d = fma(d, u, k.br[n]);
   f1 = d;
   return p;
 }
@@ -208,7 +210,7 @@ __device__ __forceinline__ T pair_sr_real(const PairCoef<T> &k, T r2, T &f1) {
     return f0;
   }
   T g1;
-  const T g0 = dm_poly_real<T, ND>(k, r2 * k.invR2, g1);
+  const T g0 = dm_poly_real<T, ND>(k, fma(-r2, k.invR2, T(1)), g1);
   if (FUNC == 0) {
     const T rinv = rsqrt_t(r2);
     f1 = -rinv * rinv * rinv - g1;

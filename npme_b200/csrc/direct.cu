@@ -35,6 +35,16 @@ constexpr double kErfcxFit[10] = {
     3.7015627549e-02, 2.7656030148e-02, -8.1190085803e-02,
     3.0625252134e-02};
 
+double dm_taylor(const npme_params &p, double (&c)[kMaxDeriv + 1], double (&ca)[kMaxDeriv + 1]) {
+  const double al = p.funcType == NPME_FUNC_RALPHA ? p.alpha : -1.0, a = 0.5 * al;
+  for (int i = 0; i <= kMaxDeriv; i++) {
+    if (i < 2) ca[i] = i;
+    else ca[i] = i <= p.nDeriv ? ca[i - 1] * (i - 1 - a) / i : 0.0;
+    c[i] = i == 0 ? 1.0 : -a * ca[i];
+  }
+  return std::pow(p.Rdir, al);
+}
+
 template <typename T>
 PairCoef<T> make_pair_coef(const npme_handle *h) {
   PairCoef<T> k;
@@ -71,16 +81,18 @@ PairCoef<T> make_pair_coef(const npme_handle *h) {
   }
   {
     const double al = h->p.funcType == NPME_FUNC_RALPHA ? h->p.alpha : -1.0;
-    // Taylor coefficients of s^a, a = alpha/2, about s = 1 (zero above the
-    // order), and ca = c_n / -a from n = 1 (also defined for a = 0)
+    // the matched polynomial (zero above the order)
     const double a = 0.5 * al;
-    double c = 1.0, ca = 1.0;
+    double c[kMaxDeriv + 1], ca[kMaxDeriv + 1];
+    const double Ral = dm_taylor(h->p, c, ca);
     for (int i = 0; i <= k.nder && i <= kMaxDeriv; i++) {
-      if (i > 1) ca = ca * (i - 1 - a) / i;
-      if (i > 0) c = -a * ca;
-      k.nc2[i].x = k.nc2[i].y = (T)-c;
-      if (i > 0) k.nq2[i - 1].x = k.nq2[i - 1].y = (T)(-i * ca);
-      if (i == k.nder) k.kn2.x = k.kn2.y = (T)((k.nder - a) * ca);
+      k.nc2[i].x = k.nc2[i].y = (T)-c[i];
+      if (i > 0) k.nq2[i - 1].x = k.nq2[i - 1].y = (T)(-i * ca[i]);
+      if (i == k.nder) k.kn2.x = k.kn2.y = (T)((k.nder - a) * ca[i]);
+      if (h->p.funcType != NPME_FUNC_HELMHOLTZ) {
+        k.ar[i] = (T)(Ral * c[i]), k.ai[i] = (T)0;
+        if (i > 0) k.br[i - 1] = (T)(-2.0 * i * c[i] * Ral / R2), k.bi[i - 1] = (T)0;
+      }
     }
     if (k.split == NPME_SPLIT_LAPLACE_ORIG) {  // dm_eval2<2, 0>: coefficients and constants
       const double b = h->beta * R;
@@ -131,7 +143,7 @@ PairCoef<T> make_pair_coef(const npme_handle *h) {
         }
       }
     }
-    k.vscale = std::pow(R, al);
+    k.vscale = Ral;
     k.gscale = (k.split == NPME_SPLIT_LAPLACE_ORIG ? 1.0 : -al) * std::pow(R, al - 1.0);
   }
   return k;

@@ -299,6 +299,15 @@ int record_error(npme_handle *h, int code, const std::string &msg);
 // loads the static scratch of npme_gpu_direct_sum_device_noalloc onto the
 // current device (noalloc.cu)
 int noalloc_preload(std::string &err);
+// Real derivative-match kernels r^alpha (1/r: alpha = -1): with u = 1 - (r /
+// Rdir)^2, the matched polynomial is Rdir^alpha sum_{n <= nDeriv} c_n u^n, the
+// Taylor polynomial of s^(alpha/2) about s = 1; c_0 = 1, c_n = -(alpha/2) ca_n with
+// ca_1 = 1, ca_{n+1} = ca_n (n - alpha/2) / (n + 1) (also defined for alpha = 0;
+// ca_0 = 0).  The direct sum and the kernel transform both take it from here: the
+// rounding of what one subtracts and the other adds must be the same.  (As
+// coefficients of r^2n they are rounded after a cancellation that grows with the
+// order, 1e4 at order 15.)  Returns Rdir^alpha.
+double dm_taylor(const npme_params &p, double (&c)[kMaxDeriv + 1], double (&ca)[kMaxDeriv + 1]);
 // true when the direct sum takes the pair-once form (FP32 real DM kernels
 // with the half-shell lists built)
 bool pairs_once(const npme_handle *h);

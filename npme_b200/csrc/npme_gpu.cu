@@ -356,9 +356,16 @@ int apply_params(npme_handle *h) {
       h->a_r[i] = a[i].real(), h->a_i[i] = a[i].imag();
       h->b_r[i] = b[i].real(), h->b_i[i] = b[i].imag();
     }
-    // f_LR(0) = a[0] (src/Interface.cpp:1946-1952)
+    // f_LR(0) = a[0] (src/Interface.cpp:1946-1952); for the real kernels as the
+    // polynomial that the sums evaluate gives it
     h->fself_r = h->a_r[0];
     h->fself_i = h->a_i[0];
+    if (h->p.funcType != NPME_FUNC_HELMHOLTZ) {
+      double c[npme::kMaxDeriv + 1], ca[npme::kMaxDeriv + 1], f = 0;
+      const double Ral = npme::dm_taylor(h->p, c, ca);
+      for (int i = h->p.nDeriv; i >= 0; i--) f += c[i];
+      h->fself_r = Ral * f;
+    }
   } else {
     h->beta = orig_beta(h->p.Rdir, h->p.tol);
     if (h->beta <= 0) return fail(h, NPME_EINVAL, "original-Ewald beta did not converge");

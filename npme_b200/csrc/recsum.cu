@@ -33,7 +33,8 @@ namespace npme {
 struct LRKernel {
   int func, split, nder;
   double R2, alpha, beta, k0r, k0i;
-  double ar[32], ai[32];  // unscaled a_n (coefficients of r^(2n))
+  double ar[32], ai[32];  // Helmholtz: a_n (coefficients of r^(2n)); real: c_n (dm_taylor)
+  double invR2, scale;    // real kernels: 1 / Rdir^2, Rdir^alpha
 };
 
 __device__ double2 lr_eval(const LRKernel &k, double r2) {
@@ -56,6 +57,12 @@ __device__ double2 lr_eval(const LRKernel &k, double r2) {
     sincos(k.k0r * r, &s, &c);
     const double d = exp(-k.k0i * r) / r;
     return make_double2(c * d, s * d);
+  }
+  if (k.func != 2) {
+    const double u = fma(-r2, k.invR2, 1.0);
+    double p = k.ar[k.nder];
+    for (int n = k.nder - 1; n >= 0; n--) p = fma(p, u, k.ar[n]);
+    return make_double2(k.scale * p, 0.0);
   }
   double pr = k.ar[k.nder], pi = k.ai[k.nder];
   for (int n = k.nder - 1; n >= 0; n--) {
@@ -478,7 +485,14 @@ static int kt_prepare(npme_handle *h, cudaStream_t s, KtSys *d) {
   k.beta = h->beta;
   k.k0r = h->p.k0_r;
   k.k0i = h->p.k0_i;
-  for (int i = 0; i <= k.nder && i < 32; i++) k.ar[i] = h->a_r[i], k.ai[i] = h->a_i[i];
+  if (k.func == NPME_FUNC_HELMHOLTZ) {
+    for (int i = 0; i <= k.nder && i < 32; i++) k.ar[i] = h->a_r[i], k.ai[i] = h->a_i[i];
+  } else {
+    double c[kMaxDeriv + 1], ca[kMaxDeriv + 1];
+    k.scale = dm_taylor(h->p, c, ca);
+    k.invR2 = 1.0 / k.R2;
+    for (int i = 0; i <= k.nder && i <= kMaxDeriv; i++) k.ar[i] = c[i];
+  }
   // scratch kept by the handle, so a new geometry on the same handle reuses it
   int rc = NPME_OK;
   if ((rc = handle_buffer(h, (void **)&h->d_ft0, sizeof(double2) * MT)) ||

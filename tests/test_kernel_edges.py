@@ -167,6 +167,24 @@ def test_fp64_helmholtz_parts_match(k0, Rdir, nd, order, tol):
     assert rel(V, ob.calcv(ob.params_from_workload(w), c, q)) < tol
 
 
+# The same for 1/r and r^alpha, at cutoffs whose powers are not exact: were one part's
+# coefficients rounded in another form, the total would be off by 3e-14 to 1e-13 at
+# order 10, 2e-13 to 3e-13 at 12 and 3e-12 at 15.  The oracle's own rounding of its
+# coefficients of r^2n is 4e-15, 2e-14 and 1e-13; three times that is allowed.
+@pytest.mark.parametrize("once", ["1", "0"])
+@pytest.mark.parametrize("nd,tol", [(10, 1.4e-14), (12, 6e-14), (15, 3e-13)])
+@pytest.mark.parametrize("Rdir", [5.3, 7.123])
+@pytest.mark.parametrize("func", ["laplace", "ralpha"])
+def test_fp64_real_parts_match(func, Rdir, nd, tol, once, monkeypatch):
+    monkeypatch.setenv("NPME_PAIRS_ONCE", once)
+    w = system(3000, func, Rdir=Rdir, nDeriv=nd, order=8, grid=(64, 64, 64),
+               box=(16.0, 16.0, 16.0))
+    c, q = w.generate()
+    with npme_b200.Solver(api.params_from_workload(w, precision="fp64")) as s:
+        V = s.setup(c).calcv(q)
+    assert rel(V, ob.calcv(ob.params_from_workload(w), c, q)) < tol
+
+
 # The exact sum: partial groups, coincident points (whose gradients are not
 # finite) and target subsets, which divide the sources among several CTAs.
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
