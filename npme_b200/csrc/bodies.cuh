@@ -1996,8 +1996,8 @@ __device__ __forceinline__ double pow_n(double u) {
   }
 }
 
-// The real DM pair kernel of dm_eval2 in FP64 (coordinates in units of Rdir,
-// s = r^2 in (0, 1]; ND > 0 for alpha < 0, ND = 0 any order and alpha).
+// The real DM pair kernel of dm_eval2 in FP64 (s = (r / Rdir)^2 in (0, 1]; ND > 0
+// for alpha < 0, ND = 0 any order and alpha).
 template <int FUNC, int ND>
 __device__ __forceinline__ void dm_eval64(const PairCoef<double> &k, double s, double &f0,
                                           double &t) {
@@ -2020,12 +2020,15 @@ __device__ __forceinline__ void dm_eval64(const PairCoef<double> &k, double s, d
 }
 
 // FP64 real DM kernels with every unordered pair evaluated once: the walk of
-// direct_group_sym64 (below) in coordinates scaled by 1/Rdir, without
-// branches.  A pair is a hit when r^2 is a normal number below 1 (compared on
-// its high word, an integer operation: the FP64 pipe, at half the FP32 rate,
-// is what bounds the kernel); a miss gets s = 1 and charge 0 on both sides.
-// 35 FP64 operations per pair at order 6, 41 and a hit branch before.  The
-// group's work is shared by nsplit warps as in direct_group_sym.
+// direct_group_sym64 (below) without branches.  A pair is a hit when s = (r /
+// Rdir)^2 is a normal number below 1 (compared on its high word, an integer
+// operation: the FP64 pipe, at half the FP32 rate, is what bounds the kernel); a
+// miss gets s = 1 and charge 0 on both sides.  36 FP64 operations per pair at order
+// 6, 41 and a hit branch before.  (Scaling the coordinates instead of r^2 takes one
+// operation less, 1,186 against 1,200 us at 200,000 points, but rounds the
+// differences of near points; scaling by a power of two and expanding about (Rdir /
+// unit)^2 gave 1,274: its constants take registers.)  The group's work is shared by
+// nsplit warps as in direct_group_sym.
 template <int FUNC, int ND>
 __device__ __forceinline__ void direct_group_sym64_dm(
     const PairCoef<double> &k, const double4 *__restrict__ gpos,
@@ -2037,27 +2040,27 @@ __device__ __forceinline__ void direct_group_sym64_dm(
   const unsigned FULL = 0xffffffffu;
   const int ti = G.x + lane;
   const bool active = lane < G.y;
-  const double ir = k.invR, vs = k.vscale, gsc = k.gscale;
+  const double vs = k.vscale, gsc = k.gscale;
   double tx = 1e150, ty = 1e150, tz = 1e150, tq = 0.0;  // idle lanes: far away, no charge
   if (active) {
     const double4 p = gpos[ti];
-    tx = (p.x - c.x) * ir, ty = (p.y - c.y) * ir, tz = (p.z - c.z) * ir;
+    tx = p.x - c.x, ty = p.y - c.y, tz = p.z - c.z;
     tq = qcaller[perm[ti]];
   }
   tsm[lane] = make_double4(tx, ty, tz, tq);
   __syncwarp();
-  // r^2 in [2^-1022, 1): the high word in [0x00100000, 0x3ff00000)
-  auto inside = [](double r2) {
-    return (unsigned)__double2hiint(r2) - 0x00100000u < 0x3fe00000u;
+  // s in [2^-1022, 1): the high word in [0x00100000, 0x3ff00000)
+  auto inside = [](double s) {
+    return (unsigned)__double2hiint(s) - 0x00100000u < 0x3fe00000u;
   };
   // pairs inside the group, target side only (each is met from both ends)
   for (int s = part; s < G.y; s += nsplit) {
     const double4 S = tsm[s];
     const double x = tx - S.x, y = ty - S.y, z = tz - S.z;
-    const double r2 = fma(x, x, fma(y, y, z * z));
-    const bool hit = inside(r2);
+    const double d2 = fma(x, x, fma(y, y, z * z)) * k.invR2;
+    const bool hit = inside(d2);
     double f0, t;
-    dm_eval64<FUNC, ND>(k, hit ? r2 : 1.0, f0, t);
+    dm_eval64<FUNC, ND>(k, hit ? d2 : 1.0, f0, t);
     const double q = hit ? S.w : 0.0, gq = t * q;
     acc[0] = fma(f0, q, acc[0]);
     acc[1] = fma(-gq, x, acc[1]);
@@ -2086,8 +2089,7 @@ __device__ __forceinline__ void direct_group_sym64_dm(
       src[i] = make_double4(-1e150, -1e150, -1e150, 0.0);
       to[i] = walk.v[i] ? slot[i] : -1;
       if (walk.v[i])
-        src[i] = make_double4((p[i].x - c.x) * ir, (p[i].y - c.y) * ir, (p[i].z - c.z) * ir,
-                              p[i].w);
+        src[i] = make_double4(p[i].x - c.x, p[i].y - c.y, p[i].z - c.z, p[i].w);
     }
     walk.next();
 #pragma unroll
@@ -2107,10 +2109,10 @@ __device__ __forceinline__ void direct_group_sym64_dm(
 #pragma unroll
       for (int i = 0; i < 2; i++) {
         const double x = T.x - src[i].x, y = T.y - src[i].y, z = T.z - src[i].z;
-        const double r2 = fma(x, x, fma(y, y, z * z));
-        const bool hit = inside(r2);
+        const double d2 = fma(x, x, fma(y, y, z * z)) * k.invR2;
+        const bool hit = inside(d2);
         double f0, t;
-        dm_eval64<FUNC, ND>(k, hit ? r2 : 1.0, f0, t);
+        dm_eval64<FUNC, ND>(k, hit ? d2 : 1.0, f0, t);
         const double qm = hit ? src[i].w : 0.0, qt = hit ? T.w : 0.0;
         const double gm = t * qm, gt = t * qt;
         aV = fma(f0, qm, aV);
@@ -2183,14 +2185,14 @@ __device__ __forceinline__ void sincos_taylor(double x, double &sn, double &cs) 
   if ((q + 1) & 2) cs = -cs;
 }
 
-// Helmholtz DM pair kernel in FP64 (coordinates in units of Rdir, s = r^2 in
-// (0, 1]): F0 = exp(i kap r)/r - P and F1 = (1/r) dF0/dr, P the Taylor
-// polynomial in u = 1 - s (PairCoef; src/KernelFunctionHelmholtz.cpp:506-563).
+// Helmholtz DM pair kernel in FP64 (coordinates times k.invR, s = r^2 in (0, cut2]):
+// F0 = exp(i kap r)/r - P and F1 = (1/r) dF0/dr, P the matched polynomial in u =
+// cut2 - s (PairCoef; src/KernelFunctionHelmholtz.cpp:506-563).
 template <int ND>
 __device__ __forceinline__ void helm_eval64(const PairCoef<double> &k, double s, double2 &F0,
                                             double2 &F1) {
   constexpr int nd = dm_degree<ND>();  // ND = 0: zero-padded to kMaxDeriv
-  const double ri = rsqrt_iter(s), r = s * ri, u = 1.0 - s;
+  const double ri = rsqrt_iter(s), r = s * ri, u = k.cut2 - s;
   double sn, cs;
   sincos_taylor(k.kapr * r, sn, cs);
   const double damp = k.kapi != 0.0 ? exp(-k.kapi * r) * ri : ri;
@@ -2213,12 +2215,17 @@ __device__ __forceinline__ void cfma64(double2 a, double2 b, double &cr, double 
   ci = fma(a.x, b.y, fma(a.y, b.x, ci));
 }
 
+// 0 < r^2 < cut2 (r^2 a normal number) by its bits, in integer operations
+__device__ __forceinline__ bool inside64(const PairCoef<double> &k, double r2) {
+  return (unsigned long long)__double_as_longlong(r2) - kMinNormal64 < k.cut_bits;
+}
+
 // FP64 Helmholtz with every unordered pair evaluated once, the complex
-// counterpart of direct_group_sym64_dm: scaled coordinates, misses at s = 1
-// with charge 0, no branch.  One source per lane and chunks of 32 (two would
-// take 170-200 registers and halve the resident warps); the eight target sums
-// rotate one lane down per step, the source sums go to vsrc ([n][8] doubles:
-// V, x, y, z as re, im).  About 105 FP64 operations per pair at order 8; the
+// counterpart of direct_group_sym64_dm: coordinates scaled by a power of two,
+// misses at s = cut2 with charge 0, no branch.  One source per lane and chunks of
+// 32 (two would take 170-200 registers and halve the resident warps); the eight
+// target sums rotate one lane down per step, the source sums go to vsrc ([n][8]
+// doubles: V, x, y, z as re, im).  About 105 FP64 operations per pair at order 8; the
 // one-sided walk spends about 130 on each of the pair's two directions.
 // tsm: the targets' x, y, z, Re q, Im q.
 template <int ND>
@@ -2231,7 +2238,7 @@ __device__ __forceinline__ void direct_group_sym64_helm(
     double (&acc)[4], double (&acci)[4]) {
   const unsigned FULL = 0xffffffffu;
   const int ti = G.x + lane;
-  const double ir = k.invR, gsc = ir * ir;  // F0 / Rdir, F1 x / Rdir^2
+  const double ir = k.invR, gsc = ir * ir;  // F0 / unit, F1 x / unit^2
   double tx = 1e150, ty = 1e150, tz = 1e150;  // idle lanes: far away, no charge
   double2 tq = make_double2(0.0, 0.0);
   if (lane < G.y) {
@@ -2243,16 +2250,13 @@ __device__ __forceinline__ void direct_group_sym64_helm(
   tsm[0][lane] = tx, tsm[1][lane] = ty, tsm[2][lane] = tz;
   tsm[3][lane] = tq.x, tsm[4][lane] = tq.y;
   __syncwarp();
-  auto inside = [](double r2) {  // r^2 in [2^-1022, 1)
-    return (unsigned)__double2hiint(r2) - 0x00100000u < 0x3fe00000u;
-  };
   // pairs inside the group, target side only (each is met from both ends)
   for (int s = part; s < G.y; s += nsplit) {
     const double x = tx - tsm[0][s], y = ty - tsm[1][s], z = tz - tsm[2][s];
     const double r2 = fma(x, x, fma(y, y, z * z));
-    const bool hit = inside(r2);
+    const bool hit = inside64(k, r2);
     double2 F0, F1;
-    helm_eval64<ND>(k, hit ? r2 : 1.0, F0, F1);
+    helm_eval64<ND>(k, hit ? r2 : k.cut2, F0, F1);
     const double2 q = make_double2(hit ? tsm[3][s] : 0.0, hit ? tsm[4][s] : 0.0);
     double gr = 0, gi = 0;
     cfma64(F0, q, acc[0], acci[0]);
@@ -2293,9 +2297,9 @@ __device__ __forceinline__ void direct_group_sym64_helm(
       const int t = from + ((lane + kk) & mask);
       const double x = tsm[0][t] - sx, y = tsm[1][t] - sy, z = tsm[2][t] - sz;
       const double r2 = fma(x, x, fma(y, y, z * z));
-      const bool hit = inside(r2);
+      const bool hit = inside64(k, r2);
       double2 F0, F1;
-      helm_eval64<ND>(k, hit ? r2 : 1.0, F0, F1);
+      helm_eval64<ND>(k, hit ? r2 : k.cut2, F0, F1);
       const double2 qm = make_double2(hit ? sq.x : 0.0, hit ? sq.y : 0.0);
       const double2 qt = make_double2(hit ? tsm[3][t] : 0.0, hit ? tsm[4][t] : 0.0);
       const double gr = fma(F1.x, qm.x, -F1.y * qm.y), gi = fma(F1.x, qm.y, F1.y * qm.x);

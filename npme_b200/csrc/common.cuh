@@ -10,6 +10,7 @@
 namespace npme {
 
 constexpr int kMaxDeriv = 15;  // derivative-match order supported on device
+constexpr unsigned long long kMinNormal64 = 0x0010000000000000ull;  // bits of 2^-1022
 
 template <typename T> struct Vec2;
 template <> struct Vec2<float> { using type = float2; };
@@ -46,15 +47,19 @@ struct PairCoef {
   // -c_n, nq2[n] = (n + 1) c_{n+1} / a (those of -(dP/ds) / a), kn2 = K.  At s
   // = 1 both f0 and t are exactly zero, and the coefficients of 1/r are exact
   // in FP32.  (alpha = 0, a constant kernel with no short range: t as for a ->
-  // 0 and gscale = 0.)
+  // 0 and gscale = 0.)  FP64: the same functions of s, but coordinates as they are
+  // and s = r^2 invR2 (a coordinate scaled by 1/Rdir is rounded, and the difference
+  // of two near ones with it), so gscale = -alpha Rdir^(alpha-2).
   typename Vec2<T>::type nc2[kMaxDeriv + 1], nq2[kMaxDeriv + 1], kn2;
   double invR, vscale, gscale;
-  // Helmholtz in FP64, scaled frame (kap = k0 Rdir): with c_n the Taylor
-  // coefficients of exp(i kap sqrt(s))/sqrt(s) in u = 1 - s, (re, im) pairs
-  // hc[n] = -c_n and hd[n] = 2 (n + 1) c_{n+1}, the negated coefficients of
-  // 2 dP/ds
+  // Helmholtz in FP64, coordinates times invR, here the reciprocal of a power of
+  // two (the same reason; with Rdir in that unit in [1, 2) nothing overflows), kap =
+  // k0 in it: cut2 the squared cutoff, cut_bits its bits less kMinNormal64; with P =
+  // sum c_n u^n the matched polynomial, u = cut2 - s, (re, im) pairs hc[n] = -c_n
+  // and hd[n] = 2 (n + 1) c_{n+1}, the negated coefficients of 2 dP/ds
   typename Vec2<T>::type hc[kMaxDeriv + 1], hd[kMaxDeriv + 1];
-  T kapr, kapi;
+  T kapr, kapi, cut2;
+  unsigned long long cut_bits;
   // Helmholtz packed evaluation: (re, im) pairs of -ar/-ai and -br/-bi
   typename Vec2<T>::type nac2[kMaxDeriv + 1], nbc2[kMaxDeriv + 1];
 };

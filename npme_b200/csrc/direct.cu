@@ -18,6 +18,7 @@
 #include <cmath>
 #include <complex>
 #include <cstdlib>
+#include <cstring>
 
 #include "bodies.cuh"
 #include "internal.h"
@@ -106,7 +107,16 @@ PairCoef<T> make_pair_coef(const npme_handle *h) {
     // dm_coefficients with Rdir = 1), c_n = G_n (-1)^n / (2^n n!)
     if (h->p.funcType == NPME_FUNC_HELMHOLTZ) {
       typedef std::complex<double> cd;
-      const cd I(0, 1), kap(h->p.k0_r * R, h->p.k0_i * R);
+      // FP64: the unit of length is the greatest power of two <= Rdir, so that
+      // scaling by it rounds nothing and the cutoff is in [1, 2)
+      const double unit = sizeof(T) == 8 ? std::exp2(std::ilogb(R)) : R;
+      const double S2 = (R / unit) * (R / unit);
+      int64_t bits;
+      std::memcpy(&bits, &S2, sizeof(bits));
+      k.cut_bits = (unsigned long long)bits - kMinNormal64;
+      k.cut2 = (T)S2;
+      k.invR = 1.0 / unit;
+      const cd I(0, 1), kap(h->p.k0_r * unit, h->p.k0_i * unit);
       k.kapr = (T)kap.real(), k.kapi = (T)kap.imag();
       cd g0 = std::exp(I * kap), g1 = g0 * (I * kap - 1.0);  // G_n, G_{n+1}
       double f = 1.0;  // (-1)^n / (2^n n!)
@@ -123,18 +133,18 @@ PairCoef<T> make_pair_coef(const npme_handle *h) {
       }
       // FP64: the polynomial that the smooth part carries (its coefficients of
       // r^2n, rounded, magnify their rounding by their cancellation, 1e3 at |k0|
-      // Rdir = 8), expanded about u = 0, so that what one part adds the other
+      // Rdir = 8), expanded in u = S2 - s, so that what one part adds the other
       // takes away: otherwise the sum is off by 2e-14 at |k0| Rdir = 10.  The FP32
       // kernels need the value at the cutoff to be zero and keep the exact c_n.
       if (sizeof(T) == 8) {
         typedef long double ld;
-        ld cr[kMaxDeriv + 1] = {}, ci[kMaxDeriv + 1] = {}, scale = R;  // R^(2n + 1)
-        for (int n = 0; n <= k.nder && n <= kMaxDeriv; n++, scale *= (ld)R * R) {
-          ld binom = 1;  // (-1)^m n over m
+        ld cr[kMaxDeriv + 1] = {}, ci[kMaxDeriv + 1] = {}, scale = unit;  // unit^(2n + 1)
+        for (int n = 0; n <= k.nder && n <= kMaxDeriv; n++, scale *= (ld)unit * unit) {
+          ld binom = scale * std::pow((ld)S2, n);  // (-1)^m n over m, S2^(n - m)
           for (int m = 0; m <= n; m++) {
-            cr[m] += binom * scale * (ld)h->a_r[n];
-            ci[m] += binom * scale * (ld)h->a_i[n];
-            binom *= -(ld)(n - m) / (m + 1);
+            cr[m] += binom * (ld)h->a_r[n];
+            ci[m] += binom * (ld)h->a_i[n];
+            binom *= -(ld)(n - m) / ((m + 1) * (ld)S2);
           }
         }
         for (int m = 0; m <= k.nder && m <= kMaxDeriv; m++) {
@@ -144,7 +154,9 @@ PairCoef<T> make_pair_coef(const npme_handle *h) {
       }
     }
     k.vscale = Ral;
-    k.gscale = (k.split == NPME_SPLIT_LAPLACE_ORIG ? 1.0 : -al) * std::pow(R, al - 1.0);
+    // the real walks scale FP32 coordinates by 1/Rdir, those of FP64 not
+    k.gscale = (k.split == NPME_SPLIT_LAPLACE_ORIG ? 1.0 : -al) *
+               std::pow(R, al - (sizeof(T) == 4 ? 1.0 : 2.0));
   }
   return k;
 }

@@ -185,6 +185,25 @@ def test_fp64_real_parts_match(func, Rdir, nd, tol, once, monkeypatch):
     assert rel(V, ob.calcv(ob.params_from_workload(w), c, q)) < tol
 
 
+# Near pairs in FP64, 1e-5 apart, on coordinates of 35 bits: offsets from a group's
+# centre are exact, so the gradient, which is the sum here, has the rounding of its
+# formula (1e-15).  A coordinate scaled by 1/Rdir before the subtraction would leave
+# 1e-16 / 1e-5.
+@pytest.mark.parametrize("once", ["1", "0"])
+@pytest.mark.parametrize("n", [600, 20000])
+@pytest.mark.parametrize("func", ["laplace", "ralpha", "helmholtz"])
+def test_fp64_near_pairs(func, n, once, monkeypatch):
+    monkeypatch.setenv("NPME_PAIRS_ONCE", once)
+    w = system(n, func, Rdir=2.3, box=(n ** (1 / 3),) * 3)
+    c, q = w.generate()
+    d = np.random.default_rng(5).standard_normal((n // 2, 3))
+    c[1::2] = c[0::2] + 1e-5 * d / np.linalg.norm(d, axis=1)[:, None]
+    c = np.ldexp(np.round(np.ldexp(c, 30)), -30)
+    with npme_b200.Solver(api.params_from_workload(w, precision="fp64")) as s:
+        V = direct(s.setup(c), q)
+    assert rel(V, ob.direct(ob.params_from_workload(w), c, q)) < 1e-14
+
+
 # The exact sum: partial groups, coincident points (whose gradients are not
 # finite) and target subsets, which divide the sources among several CTAs.
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
