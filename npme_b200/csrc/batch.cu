@@ -67,7 +67,20 @@ __global__ void __launch_bounds__(256) batch_spread_kernel(const BatchSys *__res
   const int s = find_sys(off, count, u);
   const BatchSys &S = sys[s];
   spread_brick<float, P, CPLX>(S.brick_list[u - off[s]], S.brick_start, S.bpts, S.q, S.grid,
-                               S.nb2, S.nb3, S.g1, S.g2, S.g3, smem_raw);
+                               S.nb2, S.nb3, S.g1, S.g2, S.g3, smem_raw, S.apart != 0);
+}
+
+// the odd bricks
+template <int P, bool CPLX>
+__global__ void __launch_bounds__(256, kSpreadOddCtas<float, P, CPLX>)
+    batch_spread_odd_kernel(const BatchSys *__restrict__ sys, const long long *__restrict__ off,
+                            int count) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const long long u = blockIdx.x;
+  const int s = find_sys(off, count, u);
+  const BatchSys &S = sys[s];
+  spread_brick_shared<float, P, CPLX>(S.odd_list[u - off[s]], S.brick_start, S.bpts, S.q, S.grid,
+                                      S.nb2, S.nb3, S.g1, S.g2, S.g3, smem_raw);
 }
 
 // one warp per spectrum row of one system (units: rows)
@@ -100,7 +113,7 @@ __global__ void __launch_bounds__(256) batch_interp_kernel(const BatchSys *__res
   const long long u = blockIdx.x;
   const int s = find_sys(off, count, u);
   const BatchSys &S = sys[s];
-  interp_brick_body<float, P, CPLX>(S.brick_list[u - off[s]], S.brick_start, S.bpts, S.grid, S.V,
+  interp_brick_body<float, P, CPLX>(list_brick(S.brick_list[u - off[s]]), S.brick_start, S.bpts, S.grid, S.V,
                                     S.nb2, S.nb3, S.g1, S.g2, S.g3, S.c1, S.c2, S.c3,
                                     reinterpret_cast<float *>(smem_raw),
                                     S.fold ? (void *)S.vsrc : nullptr, S.vs, S.gs);
@@ -273,6 +286,8 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     S.dperm = h->d_dperm;
     S.qc = (float *)h->d_qc;
     S.brick_list = h->d_brick_list;
+    S.odd_list = h->d_odd_list;
+    S.apart = h->n_odd > 0;
     S.brick_start = h->d_brick_start;
     S.nb2 = (int)h->grid.nb[1];
     S.nb3 = (int)h->grid.nb[2];
@@ -312,7 +327,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   std::map<int, Class> clr;  // key: complex (members with the library's transforms)
   std::map<int, Class> gath, mult;                           // key: complex (mult: cuFFT members)
   std::map<int, FftClass> own;                               // key: complex
-  std::map<std::pair<int, int>, Class> spr;                  // (order, complex)
+  std::map<std::pair<int, int>, Class> spr, odd;             // (order, complex); odd bricks
   typedef std::tuple<int, int, int, int, double, double, double, double, double> DKey;
   std::map<DKey, Class> dir;  // direct sums
   for (int k = 0; k < m; k++) {
@@ -322,12 +337,14 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     if (h->own_fft) own[cx].members.push_back(k), clr[cx].members.push_back(k);
     else mult[cx].members.push_back(k);
     spr[{h->grid.order, cx}].members.push_back(k);
+    if (h->n_odd > 0) odd[{h->grid.order, cx}].members.push_back(k);
     const DKey key(pairs_once(h) ? 1 : 0, h->p.funcType, h->p.EwaldSplit, h->p.nDeriv,
                    h->p.Rdir, h->p.alpha, h->p.k0_r, h->p.k0_i, h->beta);
     dir[key].members.push_back(k);
   }
   auto units_gather = [&](int k) { return (long long)hs[f32[k]]->n; };
   auto units_spread = [&](int k) { return (long long)hs[f32[k]]->n_nonempty; };
+  auto units_odd = [&](int k) { return (long long)hs[f32[k]]->n_odd; };
   auto units_mult = [&](int k) {  // spectrum rows
     const long *N = hs[f32[k]]->grid.N;
     return (long long)N[0] * N[1];
@@ -358,6 +375,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   for (auto &kv : clr) lay(kv.second, units_clear);
   for (auto &kv : mult) lay(kv.second, units_mult);
   for (auto &kv : spr) lay(kv.second, units_spread);  // spread and interpolation: bricks
+  for (auto &kv : odd) lay(kv.second, units_odd);
   for (auto &kv : dir) lay(kv.second, units_dir);
   for (auto &kv : own) {  // transform descriptors, then the CTA prefixes of x, y and z
     FftClass &c = kv.second;
@@ -502,6 +520,26 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
 #undef NPME_BS_P
 #undef NPME_BS
     b->launches++;
+  }
+  for (auto &kv : odd) {
+    Class &c = kv.second;
+    const unsigned nb = (unsigned)c.off.back();
+    const int cnt = (int)c.members.size();
+    auto launch = [&](auto kern, size_t smem) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      kern<<<nb, 256, smem, s>>>(D(c), O(c), cnt);
+      b->launches++;
+    };
+    const int P = kv.first.first;  // the others take odd bricks with the rest (kSpreadApart)
+    static_assert(kSpreadApart<float, 6> && kSpreadApart<float, 8> && !kSpreadApart<float, 4>);
+    if (P == 6 && kv.first.second)
+      launch(batch_spread_odd_kernel<6, true>, SpreadOwner<float, 6, true>::kSharedBytes);
+    else if (P == 6)
+      launch(batch_spread_odd_kernel<6, false>, SpreadOwner<float, 6, false>::kSharedBytes);
+    else if (P == 8 && kv.first.second)
+      launch(batch_spread_odd_kernel<8, true>, SpreadOwner<float, 8, true>::kSharedBytes);
+    else if (P == 8)
+      launch(batch_spread_odd_kernel<8, false>, SpreadOwner<float, 8, false>::kSharedBytes);
   }
   {  // launch errors are checked before cuFFT runs
     const cudaError_t e = cudaGetLastError();

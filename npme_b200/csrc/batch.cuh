@@ -13,8 +13,9 @@ struct BatchSys {
   const uint32_t *cperm;  // targets: group order -> caller index
   const uint32_t *dperm;  // direct-sum sources: source order -> caller index
   float *qc;
-  const int *brick_list, *brick_start;
+  const int *brick_list, *odd_list, *brick_start;
   int nb2, nb3;
+  int apart;  // odd bricks go by themselves
   float *grid;    // real N1 N2 N3 (real kernels) or complex (Helmholtz)
   float2 *kgrid;  // R2C half spectrum (real kernels)
   const float *G;

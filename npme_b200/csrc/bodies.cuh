@@ -242,9 +242,129 @@ struct SpreadOwner {
   static constexpr int CC = (CPLX && sizeof(T) == 4) ? 2 : 1;
   static constexpr int kBatch = sizeof(T) == 4 ? 32 : 16;  // points per batch
   static constexpr int kRow = 20, kX = 12;  // padded rows: z and y weights; x weights and q
-  static constexpr size_t kWarpBytes = sizeof(T) * kBatch * (2 * kRow + kX) + sizeof(int) * 64;
-  static constexpr size_t kBytes = kBrick * kWarpBytes + sizeof(T) * C * TL * TL * TL;
+  static constexpr size_t kRowBytes = sizeof(T) * kBatch * (2 * kRow + kX);  // a warp's rows
+  static constexpr size_t kWarpBytes = kRowBytes + sizeof(int) * 64;
+  static constexpr size_t kTileBytes = sizeof(T) * C * TL * TL * TL;
+  static constexpr size_t kBytes = kBrick * kWarpBytes + kTileBytes;
+  // spread_brick_shared: the window's points by plane and their counters; the
+  // tile's second words
+  static constexpr int kChunks = kSpreadWindow / 32;
+  static constexpr size_t kSortBytes = 2 * kSpreadWindow + sizeof(int) * kBrick * kChunks;
+  static constexpr size_t kSharedBytes =
+      kBrick * kRowBytes + kSortBytes + (sizeof(T) == 4 ? 2 : 1) * kTileBytes;
 };
+
+// Points at(0) .. at(n - 1) (n <= kBatch) of a brick into the calling warp's sums, which
+// are the tile's planes from the points' own on; rows: the warp's shared rows.
+template <typename T, int P, bool CPLX, class At>
+__device__ __forceinline__ void spread_batch(
+    T (&acc)[SpreadOwner<T, P, CPLX>::CC][P][SpreadOwner<T, P, CPLX>::H], int n, const At &at,
+    const BrickPoint<T> *__restrict__ bp, const double *__restrict__ q, int pass, int b2, int b3,
+    T *rows, int lane) {
+  using S = SpreadOwner<T, P, CPLX>;
+  using V4 = typename Vec4<T>::type;
+  constexpr int H = S::H, C = S::C, CC = S::CC;
+  const int zl = lane & 15, half = lane >> 4;
+  T *wz = rows, *wy = wz + S::kBatch * S::kRow, *wx = wy + S::kBatch * S::kRow;
+  if (lane < n) {
+    const BrickPoint<T> pt = bp[at(lane)];
+    T a[P], dummy[P];
+    T *rz = wz + lane * S::kRow, *ry = wy + lane * S::kRow, *rx = wx + lane * S::kX;
+    V4 zero;
+    zero.x = zero.y = zero.z = zero.w = T(0);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      reinterpret_cast<V4 *>(rz)[i] = zero, reinterpret_cast<V4 *>(ry)[i] = zero;
+    const long o = pt.orig;
+    T qz = T(1);
+    if (CC == 2) {
+      rx[8] = (T)q[2 * o], rx[9] = (T)q[2 * o + 1];
+    } else {
+      qz = (T)q[C * o + pass];
+    }
+    bspline_weights<T, P, false>(pt.u[2], a, dummy);
+    const int l3 = (int)(pt.g0 & 1023u) - b3 * kBrick;
+#pragma unroll
+    for (int t = 0; t < P; t++) rz[l3 + t] = CC == 2 ? a[t] : qz * a[t];
+    bspline_weights<T, P, false>(pt.u[1], a, dummy);
+    const int l2 = (int)((pt.g0 >> 10) & 1023u) - b2 * kBrick;
+#pragma unroll
+    for (int t = 0; t < P; t++) {
+      const int y = l2 + t;
+      ry[y < H ? y : 8 + y - H] = a[t];
+    }
+    bspline_weights<T, P, false>(pt.u[0], a, dummy);
+#pragma unroll
+    for (int t = 0; t < P; t++) rx[t] = a[t];
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int p = 0; p < n; p++) {
+    const T z = wz[p * S::kRow + zl];
+    T y[8], x[8];
+    const V4 *vy = reinterpret_cast<const V4 *>(wy + p * S::kRow + 8 * half);
+    const V4 *vx = reinterpret_cast<const V4 *>(wx + p * S::kX);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const V4 ay = vy[i], ax = vx[i];
+      y[4 * i] = ay.x, y[4 * i + 1] = ay.y, y[4 * i + 2] = ay.z, y[4 * i + 3] = ay.w;
+      x[4 * i] = ax.x, x[4 * i + 1] = ax.y, x[4 * i + 2] = ax.z, x[4 * i + 3] = ax.w;
+    }
+#pragma unroll
+    for (int c = 0; c < CC; c++) {
+      const T s = CC == 2 ? z * wx[p * S::kX + 8 + c] : z;
+#pragma unroll
+      for (int h = 0; h < H; h++) {
+        const T v = s * y[h];
+#pragma unroll
+        for (int i = 0; i < P; i++) acc[c][i][h] = fma(x[i], v, acc[c][i][h]);
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// The tile's rows to the grid, FP32 in pieces of 16 bytes: one vector atomic
+// each (the atomic units count requests, and with 4 to 7 tile values per grid
+// point they, not the sums, would be the bound).  A row starts at a multiple
+// of 8 values; rows of the grid that are not 16-byte aligned, and pieces past
+// the end of a row, go value by value.  TWO: the tile's second words are added.
+template <typename T, int P, bool CPLX, bool TWO>
+__device__ __forceinline__ void spread_tile_out(const T *tile, T *__restrict__ grid, int b1, int b2,
+                                                int b3, long N1, long N2, long N3) {
+  using S = SpreadOwner<T, P, CPLX>;
+  constexpr int TL = S::TL, C = S::C;
+  constexpr int kPiece = sizeof(T) == 4 ? 4 / C : 1;  // grid points per piece
+  constexpr int kPieces = (TL + kPiece - 1) / kPiece;
+  const T *low = tile + TL * TL * TL * C;
+  const long g1 = (long)b1 * kBrick, g2 = (long)b2 * kBrick, g3 = (long)b3 * kBrick;
+  const bool aligned = (N3 * C) % 4 == 0;
+  for (int t = threadIdx.x; t < TL * TL * kPieces; t += blockDim.x) {
+    const int row = t / kPieces, i3 = (t - row * kPieces) * kPiece;
+    const int i1 = row / TL, i2 = row - i1 * TL;
+    if (g1 + i1 >= N1 || g2 + i2 >= N2) continue;  // always zero there
+    T *d = grid + C * (((g1 + i1) * N2 + (g2 + i2)) * N3 + (g3 + i3));
+    T v[kPiece * C];
+    bool any = false;
+#pragma unroll
+    for (int m = 0; m < kPiece * C; m++) {
+      const int at = C * (row * TL + i3) + m;
+      v[m] = i3 + m / C < TL ? tile[at] : T(0);
+      if (TWO && i3 + m / C < TL) v[m] += low[at];
+      any |= v[m] != T(0);
+    }
+    if (!any) continue;
+    if constexpr (sizeof(T) == 4) {
+      if (aligned && g3 + i3 + kPiece <= N3) {
+        atomicAdd(reinterpret_cast<float4 *>(d), make_float4(v[0], v[1], v[2], v[3]));
+        continue;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < kPiece * C; m++)
+      if (v[m] != T(0) && g3 + i3 + m / C < N3) atomicAdd(d + m, v[m]);
+  }
+}
 
 template <typename T, int P, bool CPLX>
 __device__ __forceinline__ void spread_brick_owner(int brick, const int *__restrict__ brick_start,
@@ -258,8 +378,7 @@ __device__ __forceinline__ void spread_brick_owner(int brick, const int *__restr
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, zl = lane & 15, half = lane >> 4;
   T *tile = reinterpret_cast<T *>(smem + kBrick * S::kWarpBytes);
   T *wz = reinterpret_cast<T *>(smem + w * S::kWarpBytes);
-  T *wy = wz + KB * S::kRow, *wx = wy + KB * S::kRow;
-  int *list = reinterpret_cast<int *>(wx + KB * S::kX);
+  int *list = reinterpret_cast<int *>(smem + w * S::kWarpBytes + S::kRowBytes);
   const int b3 = brick % nb3, b2 = (brick / nb3) % nb2, b1 = brick / (nb3 * nb2);
   const int beg = brick_start[brick], nbp = brick_start[brick + 1] - beg;
   for (int t = threadIdx.x; t < TV * C; t += blockDim.x) tile[t] = T(0);
@@ -272,64 +391,8 @@ __device__ __forceinline__ void spread_brick_owner(int brick, const int *__restr
 #pragma unroll
         for (int h = 0; h < H; h++) acc[c][x][h] = T(0);
     auto batch = [&](int n) {  // points list[0 .. n) into the sums
-      if (lane < n) {
-        const BrickPoint<T> pt = bp[beg + list[lane]];
-        T a[P], dummy[P];
-        T *rz = wz + lane * S::kRow, *ry = wy + lane * S::kRow, *rx = wx + lane * S::kX;
-        using V4 = typename Vec4<T>::type;
-        V4 zero;
-        zero.x = zero.y = zero.z = zero.w = T(0);
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-          reinterpret_cast<V4 *>(rz)[i] = zero, reinterpret_cast<V4 *>(ry)[i] = zero;
-        const long o = pt.orig;
-        T qz = T(1);
-        if (CC == 2) {
-          rx[8] = (T)q[2 * o], rx[9] = (T)q[2 * o + 1];
-        } else {
-          qz = (T)q[C * o + pass];
-        }
-        bspline_weights<T, P, false>(pt.u[2], a, dummy);
-        const int l3 = (int)(pt.g0 & 1023u) - b3 * kBrick;
-#pragma unroll
-        for (int t = 0; t < P; t++) rz[l3 + t] = CC == 2 ? a[t] : qz * a[t];
-        bspline_weights<T, P, false>(pt.u[1], a, dummy);
-        const int l2 = (int)((pt.g0 >> 10) & 1023u) - b2 * kBrick;
-#pragma unroll
-        for (int t = 0; t < P; t++) {
-          const int y = l2 + t;
-          ry[y < H ? y : 8 + y - H] = a[t];
-        }
-        bspline_weights<T, P, false>(pt.u[0], a, dummy);
-#pragma unroll
-        for (int t = 0; t < P; t++) rx[t] = a[t];
-      }
-      __syncwarp();
-#pragma unroll 1
-      for (int p = 0; p < n; p++) {
-        using V4 = typename Vec4<T>::type;
-        const T z = wz[p * S::kRow + zl];
-        T y[8], x[8];
-        const V4 *vy = reinterpret_cast<const V4 *>(wy + p * S::kRow + 8 * half);
-        const V4 *vx = reinterpret_cast<const V4 *>(wx + p * S::kX);
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-          const V4 ay = vy[i], ax = vx[i];
-          y[4 * i] = ay.x, y[4 * i + 1] = ay.y, y[4 * i + 2] = ay.z, y[4 * i + 3] = ay.w;
-          x[4 * i] = ax.x, x[4 * i + 1] = ax.y, x[4 * i + 2] = ax.z, x[4 * i + 3] = ax.w;
-        }
-#pragma unroll
-        for (int c = 0; c < CC; c++) {
-          const T s = CC == 2 ? z * wx[p * S::kX + 8 + c] : z;
-#pragma unroll
-          for (int h = 0; h < H; h++) {
-            const T v = s * y[h];
-#pragma unroll
-            for (int i = 0; i < P; i++) acc[c][i][h] = fma(x[i], v, acc[c][i][h]);
-          }
-        }
-      }
-      __syncwarp();
+      spread_batch<T, P, CPLX>(acc, n, [&](int i) { return list[i]; }, bp + beg, q, pass, b2, b3,
+                               wz, lane);
     };
     // the warp's points, in batches
     int cnt = 0;
@@ -375,50 +438,215 @@ __device__ __forceinline__ void spread_brick_owner(int brick, const int *__restr
     }
   }
   __syncthreads();
-  // the tile's rows to the grid, FP32 in pieces of 16 bytes: one vector atomic
-  // each (the atomic units count requests, and with 4 to 7 tile values per grid
-  // point they, not the sums, would be the bound).  A row starts at a multiple
-  // of 8 values; rows of the grid that are not 16-byte aligned, and pieces past
-  // the end of a row, go value by value.
-  constexpr int kPiece = sizeof(T) == 4 ? 4 / C : 1;  // grid points per piece
-  constexpr int kPieces = (TL + kPiece - 1) / kPiece;
-  const long g1 = (long)b1 * kBrick, g2 = (long)b2 * kBrick, g3 = (long)b3 * kBrick;
-  const bool aligned = (N3 * C) % 4 == 0;
-  for (int t = threadIdx.x; t < TL * TL * kPieces; t += blockDim.x) {
-    const int row = t / kPieces, i3 = (t - row * kPieces) * kPiece;
-    const int i1 = row / TL, i2 = row - i1 * TL;
-    if (g1 + i1 >= N1 || g2 + i2 >= N2) continue;  // always zero there
-    T *d = grid + C * (((g1 + i1) * N2 + (g2 + i2)) * N3 + (g3 + i3));
-    T v[kPiece * C];
-    bool any = false;
-#pragma unroll
-    for (int m = 0; m < kPiece * C; m++) {
-      v[m] = i3 + m / C < TL ? tile[C * (row * TL + i3) + m] : T(0);
-      any |= v[m] != T(0);
-    }
-    if (!any) continue;
-    if constexpr (sizeof(T) == 4) {
-      if (aligned && g3 + i3 + kPiece <= N3) {
-        atomicAdd(reinterpret_cast<float4 *>(d), make_float4(v[0], v[1], v[2], v[3]));
-        continue;
-      }
-    }
-#pragma unroll
-    for (int m = 0; m < kPiece * C; m++)
-      if (v[m] != T(0) && g3 + i3 + m / C < N3) atomicAdd(d + m, v[m]);
-  }
+  spread_tile_out<T, P, CPLX, false>(tile, grid, b1, b2, b3, N1, N2, N3);
 }
 
-// The spread body of an order and precision, and its shared memory.
+// The same for an odd brick (set-up, place_orders_kernel), one with many points in one
+// plane x.  Above, a warp would be alone with them, and their number would set the
+// error of FP32 sums: 200,000 points in a sheet normal to x (3,125 a brick), order 6,
+// took 307 us, 93 here and 104 in fixed point; in one to eight bricks, order 8,
+// they were off by 9e-5, 5e-7 here and 6e-7 in fixed point.
+// Here the points are taken kSpreadWindow at a time, sorted by plane; a plane with
+// more than a fifth of a window (and 32 points) is shared out over all warps, the
+// others go to their own warp.  FP32 runs in registers have at most a third of a
+// window's points, and the runs are collected in two floats per tile value.
 template <typename T, int P, bool CPLX>
-__device__ __forceinline__ void spread_brick(int brick, const int *__restrict__ brick_start,
+__device__ __forceinline__ void spread_brick_shared(int brick, const int *__restrict__ brick_start,
+                                                    const BrickPoint<T> *__restrict__ bp,
+                                                    const double *__restrict__ q,
+                                                    T *__restrict__ grid, int nb2, int nb3,
+                                                    long N1, long N2, long N3,
+                                                    unsigned char *smem) {
+  using S = SpreadOwner<T, P, CPLX>;
+  constexpr int TL = S::TL, TV = TL * TL * TL, H = S::H, C = S::C, CC = S::CC, KB = S::kBatch;
+  constexpr bool kTwo = sizeof(T) == 4;
+  constexpr int kLoads = kSpreadWindow / 256;
+  static_assert(kBrick == 8 && kLoads == 4, "8 warps, 8 counters a lane");
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, zl = lane & 15, half = lane >> 4;
+  T *rows = reinterpret_cast<T *>(smem + w * S::kRowBytes);
+  uint16_t *list = reinterpret_cast<uint16_t *>(smem + kBrick * S::kRowBytes);
+  int *count = reinterpret_cast<int *>(list + kSpreadWindow);  // [plane][chunk of 32 points]
+  T *tile = reinterpret_cast<T *>(smem + kBrick * S::kRowBytes + S::kSortBytes);
+  const int b3 = brick % nb3, b2 = (brick / nb3) % nb2, b1 = brick / (nb3 * nb2);
+  const int beg = brick_start[brick], nbp = brick_start[brick + 1] - beg;
+  for (int t = threadIdx.x; t < (kTwo ? 2 : 1) * TV * C; t += blockDim.x) tile[t] = T(0);
+  for (int pass = 0; pass < C / CC; pass++) {
+    T acc[CC][P][H];
+    auto clear = [&]() {
+#pragma unroll
+      for (int c = 0; c < CC; c++)
+#pragma unroll
+        for (int x = 0; x < P; x++)
+#pragma unroll
+          for (int h = 0; h < H; h++) acc[c][x][h] = T(0);
+    };
+    clear();
+    int run = 0;  // points in the fullest warp's sums at most
+    for (int w0 = 0; w0 < nbp; w0 += kSpreadWindow) {
+      const int nw = min(kSpreadWindow, nbp - w0);
+      // the window's points sorted by plane: chunk i is points 32 i .. of it
+      int plane[kLoads], rank[kLoads];
+#pragma unroll
+      for (int u = 0; u < kLoads; u++) {
+        const int i = 256 * u + threadIdx.x;
+        plane[u] = i < nw ? (int)(bp[beg + w0 + i].g0 >> 20) - b1 * kBrick : -1;
+      }
+      __syncthreads();  // the last window's list is done with
+#pragma unroll
+      for (int u = 0; u < kLoads; u++) {
+        int mine = 0;
+        rank[u] = 0;
+#pragma unroll
+        for (int p = 0; p < kBrick; p++) {
+          const unsigned m = __ballot_sync(FULL, plane[u] == p);
+          if (plane[u] == p) rank[u] = __popc(m & ((1u << lane) - 1u));
+          if (lane == p) mine = __popc(m);
+        }
+        if (lane < kBrick) count[lane * S::kChunks + 8 * u + w] = mine;
+      }
+      __syncthreads();
+      // every warp: the places of the counters; lane 4 p + u has those of chunks 8 u ..
+      const int4 n0 = reinterpret_cast<const int4 *>(count)[2 * lane];
+      const int4 n1 = reinterpret_cast<const int4 *>(count)[2 * lane + 1];
+      const int c[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
+      int sum = 0, before = 0;  // before: this warp's counter
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        if (i < w) before += c[i];
+        sum += c[i];
+      }
+      int first = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(FULL, first, o);
+        if (lane >= o) first += v;
+      }
+      first -= sum;
+#pragma unroll
+      for (int u = 0; u < kLoads; u++) {
+        const int p = __shfl_sync(FULL, first + before, 4 * max(plane[u], 0) + u);
+        if (plane[u] >= 0) list[p + rank[u]] = (uint16_t)(256 * u + threadIdx.x);
+      }
+      // start and points of plane lane (lanes 0 .. 7), the planes to share out
+      const int start = __shfl_sync(FULL, first, 4 * (lane & 7));
+      const int next = __shfl_sync(FULL, first, (4 * (lane & 7) + 4) & 31);
+      const int npl = ((lane & 7) < 7 ? next : nw) - start;
+      const bool many = npl > max(32, nw / 5);
+      unsigned over = __ballot_sync(FULL, many) & 0xffu;
+      const int most = __reduce_max_sync(FULL, many ? 0 : npl);
+      __syncthreads();
+      // rounds: the warps' own planes, then the shared ones; the sums go to the tile
+      // when the next points would not fit the run, before another plane's and at the
+      // end
+      const bool last = w0 + nw == nbp;
+      bool own = true;
+      do {
+        int pl = w, from = __shfl_sync(FULL, start, w), n = __shfl_sync(FULL, npl, w);
+        if (own) {
+          if (over >> w & 1) n = 0;
+          run += most;
+        } else {  // this warp's share of a plane of many
+          pl = __ffs(over) - 1;
+          over &= over - 1;
+          const int m = __shfl_sync(FULL, npl, pl), a = w * m >> 3, b = (w + 1) * m >> 3;
+          from = __shfl_sync(FULL, start, pl) + a, n = b - a;
+          run = 1;
+        }
+        for (; n > 0; from += KB, n -= KB)
+          spread_batch<T, P, CPLX>(acc, min(n, KB), [&](int i) { return (int)list[from + i]; },
+                                   bp + beg + w0, q, pass, b2, b3, rows, lane);
+        const bool flush = own ? run > 0 && (over != 0 || last || run > kSpreadWindow / 8) : true;
+        if (flush) {
+          // in step s plane w + s of every warp's own P, or, of one plane's P, number
+          // (w + s) mod 8
+          for (int s = 0; s < (own ? P : kBrick); s++) {
+            __syncthreads();
+            const int k = own ? s : (w + s) & (kBrick - 1);
+#pragma unroll
+            for (int i = 0; i < P; i++) {
+              if (i != k || zl >= TL) continue;
+              T *d = tile + C * (((pl + i) * TL + half * H) * TL + zl) + pass;
+              T v[CC][H];
+#pragma unroll
+              for (int c = 0; c < CC; c++)
+#pragma unroll
+                for (int h = 0; h < H; h++)
+                  v[c][h] = half * H + h < TL ? d[C * TL * h + c] : T(0);
+              if (kTwo) {  // what the additions round off (Knuth's two-sum)
+                T e[CC][H];
+#pragma unroll
+                for (int c = 0; c < CC; c++)
+#pragma unroll
+                  for (int h = 0; h < H; h++) {
+                    const T t = v[c][h], a = acc[c][i][h], x = t + a, b = x - t;
+                    e[c][h] = half * H + h < TL ? (d + TV * C)[C * TL * h + c] : T(0);
+                    e[c][h] += (t - (x - b)) + (a - b);
+                  }
+#pragma unroll
+                for (int c = 0; c < CC; c++)
+#pragma unroll
+                  for (int h = 0; h < H; h++)
+                    if (half * H + h < TL) (d + TV * C)[C * TL * h + c] = e[c][h];
+              }
+#pragma unroll
+              for (int c = 0; c < CC; c++)
+#pragma unroll
+                for (int h = 0; h < H; h++)
+                  if (half * H + h < TL) d[C * TL * h + c] = v[c][h] + acc[c][i][h];
+            }
+          }
+          clear();
+          run = 0;
+        }
+        own = false;
+      } while (over != 0);
+    }
+  }
+  __syncthreads();
+  spread_tile_out<T, P, CPLX, kTwo>(tile, grid, b1, b2, b3, N1, N2, N3);
+}
+
+// FP32 order 4: its stencil of 64 points is too small for the sweep over zero-padded
+// weights to pay in full bricks: odd ones, and for real kernels those of more than
+// kFixedFrom4 points, take the fixed-point form (uniform points, 390 a brick: 23.5 us
+// against 29.9; 78 a brick: 17.3 and 17.6; 8 a brick: 17.2 and 14.3).
+constexpr int kFixedFrom4 = 96;
+
+// Entries of the list of non-empty bricks: the brick, and whether it is odd.
+__device__ __forceinline__ int list_brick(int e) { return e & 0x7fffffff; }
+
+// resident CTAs of spread_brick_shared, by shared memory and registers for its sums
+template <typename T, int P, bool CPLX>
+constexpr int kSpreadOddCtas = sizeof(T) == 4 ? (P <= 6 && !CPLX ? 3 : P == 8 && CPLX ? 1 : 2)
+                                              : (P <= 6 ? 2 : 1);
+
+// true when odd bricks are left to a launch of their own (spread_brick_shared)
+template <typename T, int P>
+constexpr bool kSpreadApart = P <= 8 && !(P == 4 && sizeof(T) == 4);
+
+// The spread body of an order and precision for the brick of a list entry (apart: odd
+// ones are left out), and its shared memory.
+template <typename T, int P, bool CPLX>
+__device__ __forceinline__ void spread_brick(int entry, const int *__restrict__ brick_start,
                                              const BrickPoint<T> *__restrict__ bp,
                                              const double *__restrict__ q, T *__restrict__ grid,
                                              int nb2, int nb3, long N1, long N2, long N3,
-                                             unsigned char *smem) {
-  if constexpr (SpreadOwner<T, P, CPLX>::kUse)
+                                             unsigned char *smem, bool apart) {
+  const int brick = list_brick(entry);
+  if constexpr (SpreadOwner<T, P, CPLX>::kUse) {
+    if constexpr (kSpreadApart<T, P>) {
+      if (apart && entry < 0) return;
+    } else {
+      const int n = brick_start[brick + 1] - brick_start[brick];
+      if (entry < 0 || (!CPLX && n > kFixedFrom4)) {
+        spread_brick_fixed<P, CPLX>(brick, brick_start, bp, q, grid, nb2, nb3, N1, N2, N3,
+                                    reinterpret_cast<int *>(smem));
+        return;
+      }
+    }
     spread_brick_owner<T, P, CPLX>(brick, brick_start, bp, q, grid, nb2, nb3, N1, N2, N3, smem);
-  else if constexpr (std::is_same<T, float>::value)
+  } else if constexpr (std::is_same<T, float>::value)
     spread_brick_fixed<P, CPLX>(brick, brick_start, bp, q, grid, nb2, nb3, N1, N2, N3,
                                 reinterpret_cast<int *>(smem));
   else

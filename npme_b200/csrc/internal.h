@@ -19,6 +19,8 @@ namespace npme {
 
 // Brick edge (grid points) of the spread tiles.
 constexpr int kBrick = 8;
+// Points of an odd brick that the spread takes at a time.
+constexpr int kSpreadWindow = 1024;
 // Warps (one group of 32 targets each) per CTA of the direct sums.
 constexpr int kGroupWarps = 4;
 // Scratch buffers the device set-up keeps on a handle (setup.cu).
@@ -108,6 +110,7 @@ struct npme_handle {
   npme::GridGeom grid;
   npme::CellGeom cells;
   long n_bricks = 0, n_nonempty = 0;
+  long n_odd = 0;  // odd bricks that go by themselves (spread_brick_shared)
 
   // set-up, host entry points and the reciprocal chain, at high priority: the
   // chain's CTAs go before the direct sum's
@@ -127,7 +130,8 @@ struct npme_handle {
   double *d_coord = nullptr;     // original order, FP64 (exact sum, FP64 direct)
   void *d_bpts = nullptr;        // BrickPoint<T>[n]
   int *d_brick_start = nullptr;  // [n_bricks + 1]
-  int *d_brick_list = nullptr;   // non-empty brick ids
+  int *d_brick_list = nullptr;   // non-empty brick ids, odd ones with the sign bit set
+  int *d_odd_list = nullptr;     // odd ones
   uint32_t *d_cperm = nullptr;   // group order (direct-sum targets) -> caller index
   void *d_qc = nullptr;          // charges in the direct sum's source order (T or T2)
   void *d_grid = nullptr;        // spread grid, real N1 N2 N3 (or complex)

@@ -882,10 +882,21 @@ template <typename T, int P, bool CPLX>
 __global__ void __launch_bounds__(256) spread_kernel(
     const int *__restrict__ brick_list, const int *__restrict__ brick_start,
     const BrickPoint<T> *__restrict__ bp, const double *__restrict__ q, T *__restrict__ grid,
-    int nb2, int nb3, long N1, long N2, long N3) {
+    int nb2, int nb3, long N1, long N2, long N3, bool apart) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   spread_brick<T, P, CPLX>(brick_list[blockIdx.x], brick_start, bp, q, grid, nb2, nb3, N1, N2, N3,
-                           smem_raw);
+                           smem_raw, apart);
+}
+
+// The odd bricks (spread_brick_shared).
+template <typename T, int P, bool CPLX>
+__global__ void __launch_bounds__(256, kSpreadOddCtas<T, P, CPLX>) spread_odd_kernel(
+    const int *__restrict__ odd_list, const int *__restrict__ brick_start,
+    const BrickPoint<T> *__restrict__ bp, const double *__restrict__ q, T *__restrict__ grid,
+    int nb2, int nb3, long N1, long N2, long N3) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  spread_brick_shared<T, P, CPLX>(odd_list[blockIdx.x], brick_start, bp, q, grid, nb2, nb3, N1, N2,
+                                  N3, smem_raw);
 }
 
 template <typename T, bool CPLX, int P>
@@ -896,7 +907,17 @@ static void spread_dispatch(npme_handle *h, const double *d_q, cudaStream_t s) {
   kern<<<(unsigned)h->n_nonempty, 256, smem, s>>>(
       h->d_brick_list, h->d_brick_start, (const BrickPoint<T> *)h->d_bpts,
       d_q, (T *)h->d_grid, (int)h->grid.nb[1], (int)h->grid.nb[2], h->gd[0],
-      h->gd[1], h->gd[2]);
+      h->gd[1], h->gd[2], h->n_odd > 0);
+  if constexpr (kSpreadApart<T, P>) {
+    if (h->n_odd == 0) return;
+    constexpr size_t odd_smem = SpreadOwner<T, P, CPLX>::kSharedBytes;
+    auto odd = spread_odd_kernel<T, P, CPLX>;
+    cudaFuncSetAttribute(odd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)odd_smem);
+    odd<<<(unsigned)h->n_odd, 256, odd_smem, s>>>(
+        h->d_odd_list, h->d_brick_start, (const BrickPoint<T> *)h->d_bpts, d_q, (T *)h->d_grid,
+        (int)h->grid.nb[1], (int)h->grid.nb[2], h->gd[0], h->gd[1], h->gd[2]);
+    h->launches++;
+  }
 }
 
 template <typename T, bool CPLX>
@@ -992,7 +1013,7 @@ __global__ void __launch_bounds__(256) interp_kernel(
     int nb2, int nb3, long N1, long N2, long N3, T c1, T c2, T c3, void *vsrc, double vs,
     double gs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  interp_brick_body<T, P, CPLX>(brick_list[blockIdx.x], brick_start, bp, theta, V, nb2, nb3, N1,
+  interp_brick_body<T, P, CPLX>(list_brick(brick_list[blockIdx.x]), brick_start, bp, theta, V, nb2, nb3, N1,
                                 N2, N3, c1, c2, c3, reinterpret_cast<T *>(smem_raw), vsrc, vs,
                                 gs);
 }

@@ -163,6 +163,7 @@ struct SysDesc {
   void *bpts;        // BrickPoint<T>[n]
   int *brick_start;  // [nbt + 1]
   int *brick_list;   // [min(n, nbt)]
+  int *odd_list;     // [min(n, nbt)]
   uint32_t *cperm, *sperm, *bperm;
   double4 *gpos, *spos;
   int2 *segs, *hsegs;
@@ -176,6 +177,7 @@ constexpr int kWorkBins = 1024;
 struct SysStats {
   long long bad;                   // lowest index whose stencil leaves the octant
   unsigned long long cand, hcand;  // staged (target, source) candidates, both walks
+  int nodd, must;                  // odd bricks, whether some have to go by themselves
   // groups per work bin and the places handed out in each, full and half lists
   int bins[2][kWorkBins], taken[2][kWorkBins];
 };
@@ -184,7 +186,7 @@ struct SysStats {
 struct SetupCounts {
   long long bad;
   unsigned long long cand, hcand;
-  int ngroups, nnonempty;
+  int ngroups, nnonempty, nodd, must;
 };
 
 constexpr int kMaxZBits = 20;  // bits of the quantised z at most
@@ -206,6 +208,7 @@ __global__ void init_sys_stats_kernel(const SysDesc *__restrict__ d, SysStats *s
   if (threadIdx.x == 0) {
     S.bad = d[blockIdx.x].n;
     S.cand = S.hcand = 0;
+    S.nodd = S.must = 0;
   }
   for (int i = threadIdx.x; i < 2 * kWorkBins; i += blockDim.x)
     S.bins[i / kWorkBins][i % kWorkBins] = S.taken[i / kWorkBins][i % kWorkBins] = 0;
@@ -438,12 +441,44 @@ __global__ void place_bricks_kernel(const SysDesc *__restrict__ d, const long *_
 
 // The direct sum's two orders of every system: local permutations, FP64
 // positions (a source's w holds its brick-order position) and each point's
-// position in the target (group) order.
-__global__ void place_orders_kernel(const SysDesc *__restrict__ d, const long *__restrict__ poff,
-                                    int R, long P, const unsigned *__restrict__ corder,
-                                    const unsigned *__restrict__ sorder,
-                                    const unsigned *__restrict__ bpos,
-                                    unsigned *__restrict__ cpos) {
+// position in the target (group) order.  CTAs from nblocks on: the odd bricks, a warp
+// per brick slot, by the points of their fullest plane (one stencil start along x, of
+// eight): more than 256, where the error of FP32 sums by one warp shows (must), or
+// more than 96 and a third of the brick's, where the time of one warp does.  (Here
+// beside the orders they cost set-up nothing; in round_place_kernel, whose latency
+// they lengthen, 8 us.)
+template <typename T>
+__global__ void __launch_bounds__(256)
+    place_orders_kernel(const SysDesc *__restrict__ d, const long *__restrict__ poff, int R, long P,
+                        const unsigned *__restrict__ corder, const unsigned *__restrict__ sorder,
+                        const unsigned *__restrict__ bpos, unsigned *__restrict__ cpos,
+                        unsigned nblocks, const long *__restrict__ boff, long B,
+                        const int *__restrict__ start, const int *__restrict__ pos, SysStats *st) {
+  if (blockIdx.x >= nblocks) {
+    const long b = (long)(blockIdx.x - nblocks) * 8 + (threadIdx.x >> 5);
+    if (b >= B) return;  // warp-uniform
+    const int c = start[b + 1] - start[b], lane = threadIdx.x & 31;
+    if (c <= 96) return;
+    const int r = owner(boff, R, b);
+    const SysDesc &D = d[r];
+    const BrickPoint<T> *pts = static_cast<const BrickPoint<T> *>(D.bpts) + (start[b] - start[D.b_off]);
+    int mine = 0;  // lane p < 8: points of plane p
+    for (int i = lane; i - lane < c; i += 32) {
+      const int p = i < c ? (int)(pts[i].g0 >> 20) & (kBrick - 1) : -1;
+#pragma unroll
+      for (int v = 0; v < kBrick; v++) {
+        const unsigned m = __ballot_sync(0xffffffffu, p == v);
+        if (lane == v) mine += __popc(m);
+      }
+    }
+    const int most = __reduce_max_sync(0xffffffffu, mine);
+    if (lane == 0 && most > min(256, max(96, c / 3))) {
+      D.brick_list[pos[b] - pos[D.b_off]] = (int)(b - D.b_off) | (int)0x80000000;
+      D.odd_list[atomicAdd(&st[r].nodd, 1)] = (int)(b - D.b_off);
+      if (most > 256) st[r].must = 1;
+    }
+    return;
+  }
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= P) return;
   const int r = owner(poff, R, k);
@@ -737,6 +772,8 @@ __global__ void collect_counts_kernel(const SysDesc *__restrict__ d, int R,
   out[r].bad = st[r].bad;
   out[r].cand = st[r].cand;
   out[r].hcand = st[r].hcand;
+  out[r].nodd = st[r].nodd;
+  out[r].must = st[r].must;
   out[r].ngroups = (int)sys_groups(D, goff);
   out[r].nnonempty = pos[D.b_off + D.nbt] - pos[D.b_off];
 }
@@ -885,6 +922,8 @@ int describe(npme_handle *h, SysDesc &D) {
       (rc = handle_buffer(h, (void **)&h->d_brick_start, sizeof(int) * (D.nbt + 1))) ||
       (rc = handle_buffer(h, (void **)&h->d_brick_list,
                           sizeof(int) * std::max<long>(1, std::min(n, D.nbt)))) ||
+      (rc = handle_buffer(h, (void **)&h->d_odd_list,
+                          sizeof(int) * std::max<long>(1, std::min(n, D.nbt)))) ||
       (rc = handle_buffer(h, (void **)&h->d_cperm, sizeof(uint32_t) * n)) ||
       (rc = handle_buffer(h, (void **)&h->d_sperm, sizeof(uint32_t) * n)) ||
       (rc = handle_buffer(h, (void **)&h->d_bperm, sizeof(uint32_t) * n)) ||
@@ -934,7 +973,7 @@ int describe(npme_handle *h, SysDesc &D) {
   D.coord = h->d_coord;
   D.bpts = h->d_bpts;
   D.brick_start = h->d_brick_start;
-  D.brick_list = h->d_brick_list;
+  D.brick_list = h->d_brick_list, D.odd_list = h->d_odd_list;
   D.cperm = h->d_cperm, D.sperm = h->d_sperm, D.bperm = h->d_bperm;
   D.gpos = h->d_gpos, D.spos = h->d_spos;
   D.segs = h->d_segs, D.hsegs = h->d_hsegs;
@@ -1071,7 +1110,8 @@ int geometry_batch(npme_handle **hs, int R, cudaStream_t s, const std::function<
                                                                             bstart, B, border2);
   place_bricks_kernel<T><<<blocks_for(std::max(P, B)), 256, 0, s>>>(
       dd, poff, boff, R, P, B, border2, pts, bstart, pos, bpos);
-  place_orders_kernel<<<blocks_for(P), 256, 0, s>>>(dd, poff, R, P, corder, sorder, bpos, cpos);
+  place_orders_kernel<T><<<blocks_for(P) + blocks_for(B, 8), 256, 0, s>>>(
+      dd, poff, R, P, corder, sorder, bpos, cpos, blocks_for(P), boff, B, bstart, pos, st);
   SCK(cudaGetLastError());
 
   // --- warp groups and their source segments, heaviest groups first ---
@@ -1155,6 +1195,8 @@ int finish_setup(npme_handle *h, const npme_handle *owner, int r) {
                         "the charge octant (axis " + std::to_string(axis) + ")");
   }
   h->n_nonempty = c.nnonempty;
+  // odd bricks cost a launch of their own: not for a few that need not go (a system's edges)
+  h->n_odd = c.must || 2 * c.nodd > c.nnonempty ? c.nodd : 0;
   h->n_groups = h->n_hgroups = c.ngroups;
   h->cand_per_point = (double)c.cand / (double)n;
   h->hcand_per_point = (double)c.hcand / (double)n;

@@ -7,7 +7,6 @@ algorithm; sums of up to 1e4 terms in another order), the two FP64 walks of
 the same pairs 1e-13; FP32 against FP64 1e-5 for V and 3e-5 for the gradient
 (the stated bound of the FP32 mode), the two FP32 walks 1e-6.
 """
-import dataclasses
 
 import numpy as np
 import pytest
@@ -100,6 +99,38 @@ def test_spread_orders(shape, order, func, prec):
         assert np.abs(V - Vo).max() <= TOL[prec][0] * np.abs(q[0])
     else:
         check(V, Vo, prec)
+
+
+# The FP32 grid of bricks that are taken in many windows (1e5 points of one sign in a
+# few bricks), of sheets (one plane of each brick, shared out over the warps) and of
+# bricks on both sides of a window: the smooth part against FP64.  Sums in 64-bit
+# fixed point, rounded once, are off by up to 3e-7, 7e-7 and 6e-6 at orders 4, 6 and
+# 8 (sheets and clusters have a rough grid, whose rounding the division by the
+# splines' transform enlarges); FP32 registers without an end were by up to 5e-6,
+# 1.3e-5 and 9e-5.
+@pytest.mark.parametrize("func", ["laplace", "helmholtz"])
+@pytest.mark.parametrize("order,tol", [(4, 1e-6), (6, 1e-6), (8, 1e-5)])
+@pytest.mark.parametrize("shape", ["cluster", "sheet0", "sheet1", "sheet2", "window"])
+def test_spread_dense_bricks(shape, order, tol, func):
+    import torch
+    n = 100000 if shape == "cluster" else 60000
+    w = system(n, func, order=order, box=(60.0, 60.0, 60.0), grid=(96, 96, 96), Rdir=1.0)
+    c, q = w.generate()
+    q = np.abs(q.real) + 0.5 + (1j * np.abs(q.imag) if func == "helmholtz" else 0)
+    if shape == "cluster":
+        c = 31.0 + c / 12.0
+    elif shape == "window":  # points within one grid cell each
+        m = [1023, 1024, 1025, 2049]
+        c, q = c[:sum(m)] / 120.0, q[:sum(m)]
+        c += np.repeat([3.0, 20.0, 37.0, 50.0], m)[:, None]
+    else:
+        c[:, int(shape[5])] = 30.0 + 1e-3 * c[:, int(shape[5])]
+    c[:2] = [[0.0] * 3, [60.0] * 3]
+    smooth = {}
+    for prec in ("fp64", "fp32"):
+        with npme_b200.Solver(api.params_from_workload(w, precision=prec)) as s:
+            smooth[prec] = s.setup(c).calcv(q) - direct(s, q)
+    assert rel(smooth["fp32"], smooth["fp64"]) < tol
 
 
 # Warps per group of 32 targets: 16 up to 148 groups, 8 up to 592, 4 up to
