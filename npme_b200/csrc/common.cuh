@@ -106,6 +106,13 @@ __host__ __device__ constexpr double spline_scale(int P) {
   return s;
 }
 
+// The sum of the weights that spread charges in precision T: the scale itself, in
+// FP32 its rounding (they differ at order 16, whose scale takes 30 bits).
+template <typename T>
+__host__ __device__ constexpr double spread_scale(int P) {
+  return (double)(T)spline_scale(P);
+}
+
 // Cardinal B-spline weights of order P, times spline_scale(P), at the stencil
 // points u + t, t = 0..P-1, with u = w + mStart in [0, 1] (the reference
 // evaluates B_P(w + m) for m = mStart..mStart+P-1, src/RecSumQ.cpp:58-84).
@@ -113,10 +120,12 @@ __host__ __device__ constexpr double spline_scale(int P) {
 // uses dB_P/dw (x) = B_{P-1}(x) - B_{P-1}(x - 1) (src/Bspline.cpp:16766); dw is
 // times spline_scale(P - 1).
 // The weights that spread FP32 charges are multiples of 2^-24 (so that their sum
-// is exact) and add up to spline_scale(P) exactly: the net charge of a grid, which
-// a neutral system's long-range potential hangs on, was off by 1e-7 of each
-// charge.  With both, the error of r^-0.5 at 200k points went from 5e-07-1.2e-06
-// (by the charges drawn) to 2.2e-07-2.7e-07, at 0-3 us of 131 for spreading.
+// is exact) and add up to spread_scale<T>(P), spline_scale(P) in FP32: the net
+// charge of a grid, which a neutral system's long-range potential hangs on, was off
+// by 1e-7 of each charge.  With both, the error of r^-0.5 at 200k points went from
+// 5e-07-1.2e-06 (by the charges drawn) to 2.2e-07-2.7e-07, at 0-3 us of 131 for
+// spreading.  (c + 1/2) - 1/2 rounds to 2^-24 for c <= 1/2, which the central one or
+// two weights alone exceed, and by little.
 // Interpolation leaves its weights as they are: rounding them too gained less
 // and cost it 30 us of 100 at 1M points.
 template <typename T, int P, bool DERIV>
@@ -150,10 +159,10 @@ __device__ __forceinline__ void bspline_weights(T u, T (&w)[P], T (&dw)[P]) {
     }
   }
   if constexpr (sizeof(T) == 4 && !DERIV) {
-    T rest = T(spline_scale(P));
+    T rest = T(spread_scale<T>(P));
 #pragma unroll
     for (int t = 0; t < P; t++) {
-      c[t] = (c[t] + T(1)) - T(1);
+      c[t] = (c[t] + T(0.5)) - T(0.5);
       rest -= c[t];
     }
     c[P / 2] += rest;

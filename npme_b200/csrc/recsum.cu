@@ -15,6 +15,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <tuple>
 #include <type_traits>
 #include <vector>
 
@@ -312,13 +313,13 @@ static double bspline_host(int n, double w) {
 }
 
 // |1/sum_p B_n(p) exp(-2 pi i k p / N)|^2 for k = 0..N/2 (src/RecSumV.cpp:565-581),
-// over the square of the scale that spreading and interpolation leave in the
-// weights of an axis (spline_step)
-static void lambda2_host(long N, int order, std::vector<double> &out) {
+// over the scales that spreading and interpolation leave in the weights of an axis
+static void lambda2_host(long N, int order, bool fp32, std::vector<double> &out) {
   std::vector<double> b(order + 1);
   for (int p = 0; p <= order; p++) b[p] = bspline_host(order, p);
   out.resize(N / 2 + 1);
-  const double scale = spline_scale(order);
+  const double scale =
+      spline_scale(order) * (fp32 ? spread_scale<float>(order) : spread_scale<double>(order));
   for (long k = 0; k <= N / 2; k++) {
     const double z = (double)k / (double)N;
     double dr = 0, di = 0;
@@ -326,7 +327,7 @@ static void lambda2_host(long N, int order, std::vector<double> &out) {
       dr += b[p] * std::cos(2.0 * M_PI * z * p);
       di -= b[p] * std::sin(2.0 * M_PI * z * p);
     }
-    out[k] = 1.0 / ((dr * dr + di * di) * (scale * scale));
+    out[k] = 1.0 / ((dr * dr + di * di) * scale);
   }
 }
 
@@ -337,14 +338,14 @@ struct AxisTables {
   std::vector<double> lam, cosines;
 };
 static std::mutex g_axis_mu;
-static std::map<std::pair<long, int>, std::shared_ptr<const AxisTables>> g_axis_tables;
+static std::map<std::tuple<long, int, bool>, std::shared_ptr<const AxisTables>> g_axis_tables;
 
-static std::shared_ptr<const AxisTables> axis_tables(long N, int order) {
+static std::shared_ptr<const AxisTables> axis_tables(long N, int order, bool fp32) {
   std::lock_guard<std::mutex> lk(g_axis_mu);
-  auto &slot = g_axis_tables[std::make_pair(N, order)];
+  auto &slot = g_axis_tables[std::make_tuple(N, order, fp32)];
   if (!slot) {
     auto t = std::make_shared<AxisTables>();
-    lambda2_host(N, order, t->lam);
+    lambda2_host(N, order, fp32, t->lam);
     t->cosines.resize(N);
     for (long m = 0; m < N; m++) t->cosines[m] = std::cos(2.0 * M_PI * (double)m / (double)N);
     slot = t;
@@ -473,7 +474,7 @@ static int kt_prepare(npme_handle *h, cudaStream_t s, KtSys *d) {
   std::shared_ptr<const AxisTables> tab[3];
   for (int a = 0; a < 3; a++) {
     window_axis(N[a], h->box[a], dels[a], as[a], ax[a]);
-    tab[a] = axis_tables(N[a], h->grid.order);
+    tab[a] = axis_tables(N[a], h->grid.order, h->fp32);
   }
   LRKernel &k = d->k;
   k = LRKernel{};

@@ -7,11 +7,15 @@ algorithm; sums of up to 1e4 terms in another order), the two FP64 walks of
 the same pairs 1e-13; FP32 against FP64 1e-5 for V and 3e-5 for the gradient
 (the stated bound of the FP32 mode), the two FP32 walks 1e-6.
 """
+import ctypes
+import os
+import shutil
+import subprocess
 
 import numpy as np
 import pytest
 
-from conftest import rel
+from conftest import ROOT, rel
 import npme_b200
 from npme_b200 import api
 from npme_b200.workloads import Workload
@@ -99,6 +103,43 @@ def test_spread_orders(shape, order, func, prec):
         assert np.abs(V - Vo).max() <= TOL[prec][0] * np.abs(q[0])
     else:
         check(V, Vo, prec)
+
+
+def bspline(P, x):
+    """B_P(x) in 64 bits."""
+    if P == 1:
+        return ((x >= 0) & (x < 1)).astype(float)
+    return (x * bspline(P - 1, x) + (P - x) * bspline(P - 1, x - 1)) / (P - 1)
+
+
+# FP32 spreading weights: multiples of 2^-24 whose sum is the FP32 scale exactly; the
+# tails (below 2^-7) within half a quantum and a quarter for the rounding of the
+# recursion (0.15 in a restatement), so that they keep their digits.
+def test_fp32_spreading_weights(tmp_path):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not available")
+    lib = tmp_path / "libweights.so"
+    subprocess.run([nvcc, "-std=c++17", "-O3", "-Xcompiler", "-fPIC", "-shared", "-gencode",
+                    "arch=compute_100a,code=sm_100a", "--expt-relaxed-constexpr",
+                    "-I" + os.path.join(ROOT, "npme_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "user_kernel", "spline_weights.cu"),
+                    "-o", str(lib)], check=True)
+    run = ctypes.CDLL(str(lib)).spline_weights
+    u = np.linspace(0, 1, 20001).astype(np.float32)
+    halvings = {0: 0, 1: 0, 2: 1, 3: 2, 4: 2, 5: 2, 11: 4, 13: 4, 14: 4, 15: 4}  # else 3
+    for P in (4, 6, 8, 10, 12, 14, 16):
+        w = np.empty((P, len(u)), np.float32)
+        ptr = [a.ctypes.data_as(ctypes.POINTER(ctypes.c_float)) for a in (u, w)]
+        assert run(P, len(u), *ptr) == 0
+        w = w.astype(float)
+        scale = np.prod([j * 0.5 ** halvings.get(j, 3) for j in range(2, P)])
+        assert (np.ldexp(w, 24) % 1 == 0).all()
+        assert (w.sum(0) == np.float32(scale)).all()
+        exact = scale * np.stack([bspline(P, u.astype(float) + t) for t in range(P)])
+        tail = exact < 2.0 ** -7
+        tail[P // 2] = False  # takes the rest
+        assert (np.abs(w - exact)[tail] <= 1.25 * 2.0 ** -25).all()
 
 
 # The FP32 grid of bricks that are taken in many windows (1e5 points of one sign in a
