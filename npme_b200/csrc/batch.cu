@@ -202,6 +202,9 @@ int npme_gpu_batch_destroy(npme_batch *b) {
   cudaSetDevice(b->device);
   if (b->pending) cudaEventSynchronize(b->ev_done);
   if (b->stream2) cudaStreamSynchronize(b->stream2);
+  if (b->hi) cudaStreamSynchronize(b->hi);
+  for (int i = 0; i < npme_batch::kSide; i++)
+    if (b->side[i]) cudaStreamSynchronize(b->side[i]);
   if (b->stream2) cudaStreamDestroy(b->stream2);
   if (b->hi) cudaStreamDestroy(b->hi);
   for (int i = 0; i < npme_batch::kSide; i++) {
@@ -224,6 +227,9 @@ int npme_gpu_batch_sync(npme_batch *b) {
   cudaError_t e = cudaSuccess;
   if (b->pending) e = cudaEventSynchronize(b->ev_done);
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream2);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->hi);
+  for (int i = 0; i < npme_batch::kSide && e == cudaSuccess; i++)
+    e = cudaStreamSynchronize(b->side[i]);
   b->pending = false;
   if (e != cudaSuccess) return bfail(b, NPME_ECUDA, cudaGetErrorString(e));
   return NPME_OK;
@@ -442,6 +448,22 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
     return (unsigned)std::max<long long>(1, std::min<long long>((units + threads - 1) / threads, cap));
   };
 
+  // A failure from here on leaves with work of this call enqueued: all of its streams
+  // join the caller's, and the source-side sums that no interpolation takes are cleared.
+  auto leave = [&](const std::string &msg) {
+    for (int i = 0; i <= npme_batch::kSide; i++) {
+      cudaEvent_t ev = i < npme_batch::kSide ? b->ev_side[i] : b->ev_join;
+      cudaEventRecord(ev, i < npme_batch::kSide ? b->side[i] : b->stream2);
+      cudaStreamWaitEvent(b->hi, ev, 0);
+    }
+    for (int k = 0; k < m; k++) clear_source_sums(hs[f32[k]], b->hi);
+    cudaEventRecord(b->ev_done, b->hi);
+    cudaStreamWaitEvent(user, b->ev_done, 0);
+    b->pending = true;
+    cudaGetLastError();
+    return bfail(b, NPME_ECUDA, "batch: " + msg);
+  };
+
   // 1. gather, then 2. direct sums, on the second stream, beside the
   // reciprocal sums
   const cudaStream_t s = b->hi;  // the reciprocal chain
@@ -543,7 +565,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   }
   {  // launch errors are checked before cuFFT runs
     const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return bfail(b, NPME_ECUDA, std::string("batch: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) return leave(cudaGetErrorString(e));
   }
   // 4. transforms and kernel multiply of the members with the library's own
   // transforms: five launches for all of one kind
@@ -557,7 +579,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   // the others: forward transforms
   for (int k = 0; k < m; k++) {
     npme_handle *h = hs[f32[k]];
-    if (!h->own_fft && fft_forward(h, s)) return bfail(b, NPME_ECUDA, "batch: " + h->err);
+    if (!h->own_fft && fft_forward(h, s)) return leave(h->err);
   }
   // 5. kernel multiply
   for (auto &kv : mult) {
@@ -569,12 +591,12 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   }
   {  // launch errors are checked before cuFFT runs
     const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return bfail(b, NPME_ECUDA, std::string("batch: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) return leave(cudaGetErrorString(e));
   }
   // 6. inverse transforms
   for (int k = 0; k < m; k++) {
     npme_handle *h = hs[f32[k]];
-    if (!h->own_fft && fft_inverse(h, s)) return bfail(b, NPME_ECUDA, "batch: " + h->err);
+    if (!h->own_fft && fft_inverse(h, s)) return leave(h->err);
   }
   // 7. interpolation after the direct sums
   cudaStreamWaitEvent(s, b->ev_join, 0);
@@ -612,7 +634,7 @@ int npme_gpu_calcv_batch(npme_batch *b, npme_handle *const *hs, int count,
   cudaStreamWaitEvent(user, b->ev_done, 0);
   b->pending = true;
   const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return bfail(b, NPME_ECUDA, std::string("batch: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) return leave(cudaGetErrorString(e));
   return NPME_OK;
 }
 

@@ -554,6 +554,11 @@ void launch_merge_source(npme_handle *h, double *V, cudaStream_t s, double vs, d
     merge_source_kernel<<<blocks, 256, 0, s>>>(h->d_vsrc, h->d_bperm, n, vs, gs, V);
 }
 
+void clear_source_sums(npme_handle *h, cudaStream_t s) {
+  const size_t b = (h->fp32 ? sizeof(float) : sizeof(double)) * 4 * (h->complex_kernel ? 2 : 1) * h->n;
+  cudaMemsetAsync(h->fp32 ? (void *)h->d_vsrc : (void *)h->d_vsrc64, 0, b, s);
+}
+
 // The pair-once form applies to the built-in kernels: in FP32 the DM kernels
 // (1/r, r^alpha, Helmholtz; derivative orders 3, 6 and 8 compiled with the
 // order fixed, the others by one instance at degree kMaxDeriv with

@@ -321,6 +321,8 @@ bool needs_full_lists(const npme_handle *h);
 // the potential, gs for the gradient; FP32 real, FP32 complex or FP64 by the
 // handle), and zeroes them for the next call
 void launch_merge_source(npme_handle *h, double *V, cudaStream_t s, double vs, double gs);
+// zeroes them without taking them: after a call that failed before its merge
+void clear_source_sums(npme_handle *h, cudaStream_t s);
 // Both return NPME_OK, or the status a caller-defined kernel's launcher
 // reported (its launch error is not left pending for cudaGetLastError).
 int launch_direct(npme_handle *h, const double *d_q, double *d_V, cudaStream_t s);

@@ -1,8 +1,13 @@
 """Batched CalcV, the continuous-batching server and the autotuner."""
+import ctypes
+import os
+import shutil
+import subprocess
+
 import numpy as np
 import pytest
 
-from conftest import rel
+from conftest import ROOT, rel
 import npme_b200
 from npme_b200 import api, autotune, serving
 
@@ -331,3 +336,46 @@ def test_pool_keeps_handles_under_its_own_byte_budget():
     s = tiny.srv.stats()
     assert s["idle_handles"] == 0 and st["handles_dropped"] >= 1
     tiny.close()
+
+
+@pytest.mark.gpu
+def test_failed_batch_leaves_its_streams_joined(tmp_path):
+    """A batch call that fails after its first launches (a cuFFT call answers with an
+    error) leaves nothing running beside the caller's stream and no sums behind: what
+    the caller does next sees the buffers at rest, and the next call is right."""
+    import torch
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not available")
+    lib = str(tmp_path / "libbreak.so")
+    subprocess.run([nvcc, "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-gencode",
+                    "arch=compute_100a,code=sm_100a", "--expt-relaxed-constexpr",
+                    "-I" + os.path.join(ROOT, "npme_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "user_kernel", "break_plan.cu"), "-o", lib],
+                   check=True)
+    swap = ctypes.CDLL(lib).swap_forward_plan
+    n = 200000
+    g = np.random.default_rng(3)
+    c, q = 58.5 * g.random((n, 3)), g.uniform(-1, 1, n)
+    s = npme_b200.Solver(api.make_params("laplace", "dm", 8.0, 6, 6, (112, 112, 112))).setup(c)
+    want = s.calcv(q)
+    dq = torch.from_numpy(np.ascontiguousarray(q)).cuda()
+    V = torch.zeros((n, 4), dtype=torch.float64, device="cuda")
+    b = api.Batch()
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    plan = swap(s.h, 1 << 20)
+    try:
+        with torch.cuda.stream(st):
+            with pytest.raises(RuntimeError):
+                b.calcv([s], [V.data_ptr()], [dq.data_ptr()], st.cuda_stream)
+            seen = V.clone()
+    finally:
+        swap(s.h, plan)
+    torch.cuda.synchronize()
+    assert V.any(1).all() and torch.equal(seen, V)
+    b.calcv([s], [V.data_ptr()], [dq.data_ptr()])
+    b.sync()
+    assert rel(V.cpu().numpy(), want) < 1e-6
+    b.close()
+    s.close()
