@@ -647,7 +647,8 @@ static void tmark(npme_handle *h, int i, cudaStream_t s) {
 // and 261, complex 250k 1,406 and 1,388.  In the timing modes the chain runs on
 // the caller's stream, where its stages are timed; in the serial one the direct
 // sum starts after it, so that each stage's events time that stage alone.
-static int enqueue_calcv(npme_handle *h, double *d_V, const double *d_charge, cudaStream_t user) {
+static int enqueue_parts(npme_handle *h, double *d_V, const double *d_charge, cudaStream_t user,
+                         bool &forked) {
   const bool timed = h->timing.enabled, serial = timed && h->timing.serial;
   const cudaStream_t s = timed ? user : h->stream;
   h->launches = 0;
@@ -662,6 +663,7 @@ static int enqueue_calcv(npme_handle *h, double *d_V, const double *d_charge, cu
     if (timed) {
       CK(cudaEventRecord(h->ev_fork, s));
       CK(cudaStreamWaitEvent(h->stream2, h->ev_fork, 0));
+      forked = true;
     } else {
       npme::launch_gather_direct(h, d_charge, h->d_qc, h->stream2);
     }
@@ -678,6 +680,7 @@ static int enqueue_calcv(npme_handle *h, double *d_V, const double *d_charge, cu
     CK(cudaEventRecord(h->ev_fork, user));
     CK(cudaStreamWaitEvent(s, h->ev_fork, 0));
     CK(cudaStreamWaitEvent(h->stream2, h->ev_fork, 0));
+    forked = true;
   }
   if (timed && !serial && (frc = fork_direct())) return frc;
   if (npme::grid_clear(h, s)) return fail(h, NPME_ECUDA, "clearing the spread grid failed");
@@ -713,6 +716,26 @@ static int enqueue_calcv(npme_handle *h, double *d_V, const double *d_charge, cu
     CK(cudaStreamWaitEvent(user, h->ev_chain, 0));
   }
   return NPME_OK;
+}
+
+// The same; a failure after the fork leaves with the handle's streams joined to the
+// caller's (parts already enqueued read d_charge and write d_V) and without the
+// source-side sums that no interpolation takes.
+static int enqueue_calcv(npme_handle *h, double *d_V, const double *d_charge, cudaStream_t user) {
+  bool forked = false;
+  const int rc = enqueue_parts(h, d_V, d_charge, user, forked);
+  if (rc && forked) {
+    h->merge_pending = false;
+    npme::clear_source_sums(h, h->stream2);
+    cudaEventRecord(h->ev_join, h->stream2);
+    cudaStreamWaitEvent(user, h->ev_join, 0);
+    if (!h->timing.enabled) {
+      cudaEventRecord(h->ev_chain, h->stream);
+      cudaStreamWaitEvent(user, h->ev_chain, 0);
+    }
+    cudaGetLastError();
+  }
+  return rc;
 }
 
 namespace {

@@ -159,3 +159,42 @@ def test_complex_user_kernel_matches_its_exact_sum(user_lib, precision):
           "grad", rel(V[:, 1:], Ve[:, 1:]))
     assert rel(V[:, 0], Ve[:, 0]) < 1e-4
     assert rel(V[:, 1:], Ve[:, 1:]) < 1e-4
+
+
+@pytest.mark.gpu
+def test_failed_calcv_leaves_its_streams_joined(user_lib):
+    """A CalcV whose caller-defined direct sum reports a failure after it has enqueued
+    work: what the caller enqueues next waits for that work."""
+    import torch
+    from npme_b200 import api
+    import npme_b200
+    U = ctypes.CDLL(user_lib)
+    ops = api.UserOps()
+    U.screened_ops(ctypes.byref(ops))
+    n = 3000
+    g = np.random.default_rng(2)
+    c, q = 15.0 * g.random((n, 3)), g.uniform(-1, 1, n)
+    s = npme_b200.Solver(api.make_params("user", "dm", 4.0, 6, 6, (48, 48, 48)))
+    dq = torch.from_numpy(q).cuda()
+    V = torch.zeros((n, 4), dtype=torch.float64, device="cuda")
+
+    def late_failure(h, args, stream):
+        with torch.cuda.stream(torch.cuda.ExternalStream(stream)):
+            torch.cuda._sleep(40_000_000)  # 20 ms
+            V.fill_(7.0)
+        return 3
+
+    direct = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p,
+                              ctypes.c_void_p)(late_failure)
+    ops.direct = ctypes.cast(direct, ctypes.c_void_p)
+    s.set_user_kernel(ops)
+    s.setup(c)
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(st):
+        with pytest.raises(api.NPMEError):
+            s.calcv_device(V.data_ptr(), dq.data_ptr(), st.cuda_stream)
+        seen = V.clone()
+    torch.cuda.synchronize()
+    assert (seen == 7.0).all()
+    s.close()
