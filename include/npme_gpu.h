@@ -104,8 +104,8 @@ typedef struct {
   long nGroups;         /* direct sum: warp groups of <= 32 points */
   double candidatesPerPoint; /* direct sum: staged sources per target */
   int pairsOnce;        /* 1: the direct sum evaluates every pair once, for
-                           both of its points (0 for FP64 Helmholtz, whose
-                           walk does so as well) */
+                           both of its points, and adds the second one's with
+                           atomics; 0: one-sided, reproducible */
   double pairsOnceCandidatesPerPoint; /* half-shell sources per target */
 } npme_info;
 

@@ -559,13 +559,11 @@ void clear_source_sums(npme_handle *h, cudaStream_t s) {
   cudaMemsetAsync(h->fp32 ? (void *)h->d_vsrc : (void *)h->d_vsrc64, 0, b, s);
 }
 
-// The pair-once form applies to the built-in kernels: in FP32 the DM kernels
-// (1/r, r^alpha, Helmholtz; derivative orders 3, 6 and 8 compiled with the
-// order fixed, the others by one instance at degree kMaxDeriv with
-// zero-padded coefficients) and the original
-// Ewald split, in FP64 the real kernels (any order, original Ewald
-// included); FP64 Helmholtz and caller-defined complex kernels walk the full
-// segments.
+// The pair-once form applies to all built-in kernels (derivative orders 3, 6 and 8
+// compiled with the order fixed, the others by one instance at degree kMaxDeriv
+// with zero-padded coefficients) and to real caller-defined ones.  FP64 Helmholtz
+// with |k0| Rdir >= kMaxHelmArg, complex caller-defined kernels and handles set up
+// under NPME_PAIRS_ONCE=0 walk the full segments.
 bool needs_full_lists(const npme_handle *h) {
   if (!h->use_sym) return true;
   if (h->user_kernel) return h->complex_kernel;  // real: the functor's scalar pair kernel

@@ -986,8 +986,7 @@ int npme_gpu_get_info(const npme_handle *hc, npme_info *info) {
   info->launches = h->launches;
   info->nGroups = h->n_groups;
   info->candidatesPerPoint = h->cand_per_point;
-  // (FP64 Helmholtz evaluates every pair once too, but keeps reporting 0)
-  info->pairsOnce = npme::pairs_once(h) && (h->fp32 || !h->complex_kernel) ? 1 : 0;
+  info->pairsOnce = npme::pairs_once(h) ? 1 : 0;
   info->pairsOnceCandidatesPerPoint = h->hcand_per_point;
   return NPME_OK;
 }

@@ -274,19 +274,17 @@ def _direct(w, c, q, torch, prec="fp32"):
                                   "helmholtz_dm_small", "laplace_orig_small"])
 def test_pairs_once_matches_both_sides(name, prec, monkeypatch):
     # the built-in kernels evaluate every pair once, for both of its points
-    # (NPME_PAIRS_ONCE=0 selects the one-sided walk): all of them in FP32,
-    # the real ones in FP64; the two forms agree to rounding and both match
-    # the oracle
+    # (NPME_PAIRS_ONCE=0 selects the one-sided walk); the two forms agree to
+    # rounding and both match the oracle
     torch = pytest.importorskip("torch")
     w = SMALL[name]
     c, q = w.generate()
     Vo = ob.direct(ob.params_from_workload(w), c, q)
-    expect = prec == "fp32" or not np.iscomplexobj(q)
     got = {}
     for mode in ("0", "1"):
         monkeypatch.setenv("NPME_PAIRS_ONCE", mode)
         got[mode] = _direct(w, c, q, torch, prec)
-        assert _direct.pairs_once == (mode == "1" and expect)
+        assert _direct.pairs_once == (mode == "1")
     tol = (FP64_TOL, FP64_TOL) if prec == "fp64" else (FP32_V_TOL, FP32_G_TOL)
     assert rel(got["1"], got["0"]) < (1e-13 if prec == "fp64" else 1e-6)
     for V in got.values():

@@ -219,6 +219,8 @@ def test_fp64_helmholtz_wave_numbers(k0, nd, tol, monkeypatch):
     w = system(1500, "helmholtz", k0=k0, nDeriv=nd)
     c, q, two, one = both_walks(w, "fp64", monkeypatch)
     assert rel(one, two) < tol
+    with npme_b200.Solver(api.params_from_workload(w, precision="fp64")) as s:
+        assert s.setup(c).info()["pairsOnce"] == (abs(k0) < 25000)
     if abs(k0) < 100:
         Vo = ob.direct(ob.params_from_workload(w), c, q)
         assert rel(one, Vo) < 10 * tol
