@@ -912,11 +912,16 @@ int describe(npme_handle *h, SysDesc &D) {
   // 6,131 us, FP64 Helmholtz 62,500 1,088 -> 1,037, FP32 r^-0.5 500k 1,778 ->
   // 1,731, FP32 Helmholtz 250k 1,257 -> 1,239; FP32 1/r 1M 3,121 -> 3,168, and
   // with few groups, whose walks are split, 4,000 points 26 -> 41, 30,000 82 ->
-  // 98.  Not where three segments per column would exceed the offsets.
+  // 98.  Not for the walks that take all segments alike (one-sided, original Ewald in
+  // FP64, caller kernels), nor where three segments per column would exceed the
+  // offsets or the memory.
   const long min_points = sizeof(T) == 8 ? 32L * 4 * 148 : 32L * 20 * 148;
-  D.zones = n >= min_points && 3 * nsb < (1L << 31) &&
-            (sizeof(T) == 8 || h->p.funcType == NPME_FUNC_RALPHA ||
-             h->p.funcType == NPME_FUNC_HELMHOLTZ);
+  const bool zoned_walk = !D.full && h->p.EwaldSplit == NPME_SPLIT_DERIVMATCH &&
+                          (h->p.funcType == NPME_FUNC_RALPHA ||
+                           h->p.funcType == NPME_FUNC_HELMHOLTZ ||
+                           (sizeof(T) == 8 && h->p.funcType == NPME_FUNC_LAPLACE));
+  D.zones = zoned_walk && n >= min_points && 3 * nsb < (1L << 31);
+  if (D.zones && handle_buffer(h, (void **)&h->d_hsegs, sizeof(int2) * nsb * 3)) D.zones = false;
   const int C = h->complex_kernel ? 2 : 1;
   if ((rc = handle_buffer(h, &h->d_bpts, sizeof(BrickPoint<T>) * n)) ||
       (rc = handle_buffer(h, (void **)&h->d_brick_start, sizeof(int) * (D.nbt + 1))) ||

@@ -197,6 +197,20 @@ def test_group_splits_and_zones(func, split, prec, n, monkeypatch):
     assert rel(one[:, 1:], two[:, 1:]) < WALKS[prec]
 
 
+# Zones are built for the walks that use them alone: the others stage the same sources
+# whatever the precision (candidates per point), where FP64 1/r leaves some out.
+def test_zones_only_where_they_are_walked(monkeypatch):
+    def candidates(func, split, prec, once):
+        monkeypatch.setenv("NPME_PAIRS_ONCE", once)
+        w = system(20000, func, split, box=(27.0, 27.0, 27.0), Rdir=3.5)
+        with npme_b200.Solver(api.params_from_workload(w, precision=prec)) as s:
+            return s.setup(w.generate()[0]).info()["pairsOnceCandidatesPerPoint"]
+    plain = candidates("laplace", "dm", "fp32", "1")  # no zones at this size
+    assert candidates("laplace", "dm", "fp64", "1") < 0.97 * plain
+    assert candidates("laplace", "orig", "fp64", "1") == plain
+    assert candidates("laplace", "dm", "fp64", "0") == plain
+
+
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 @pytest.mark.parametrize("alpha,nd", [(1.0, 6), (3.0, 3), (0.5, 8), (-3.0, 6), (-2.5, 10),
                                       (-1.0, 3)])
