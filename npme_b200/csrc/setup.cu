@@ -892,15 +892,15 @@ int describe(npme_handle *h, SysDesc &D) {
   // Upper bounds (the kernels read the actual counts on the device; the
   // host reads them once the set-up has completed):
   //   groups   <= n / 32 + non-empty columns <= n / 32 + min(n, ncol)
-  //   segments <= groups x the fine columns of a group's window (a group lies
-  //               in one coarse column, so its window spans at most
-  //               (edge + 2 Rdir) / sedge + 4 fine columns per axis, one more
-  //               for rounding)
+  //   segments <= groups x the fine columns that can be within Rdir of a group: it
+  //               lies in one coarse column, so at most (edge + 2 Rdir) / sedge + 2
+  //               per axis (the window's margin columns are not), two more for
+  //               rounding
   //   non-empty bricks <= min(n, nbt)
   D.ngb = n / 32 + std::min(n, D.ncol) + 1;
   long wmax = 1;
   for (int a = 0; a < 2; a++)
-    wmax *= std::min<long>(g.ns[a], (long)std::floor((g.edge[a] + 2.0 * Rd) / g.sedge[a]) + 5);
+    wmax *= std::min<long>(g.ns[a], (long)std::floor((g.edge[a] + 2.0 * Rd) / g.sedge[a]) + 4);
   D.wmax = wmax;
   D.full = needs_full_lists(h);
   const long nsb = D.ngb * wmax;

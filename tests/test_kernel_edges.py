@@ -197,6 +197,29 @@ def test_group_splits_and_zones(func, split, prec, n, monkeypatch):
     assert rel(one[:, 1:], two[:, 1:]) < WALKS[prec]
 
 
+# The bound of the segment lists (2^31 in all): a set-up just within it, 2.4 million
+# points in a thin sheet with a cutoff of 38 column edges, and one beyond.
+def test_segment_bound():
+    import torch
+    if torch.cuda.mem_get_info()[0] < 60e9:
+        pytest.skip("needs 60 GB")
+    n = 2400000
+    c = np.random.default_rng(1).random((n, 3)) * [44.0, 44.0, 0.2]
+    c[:2] = [[0.0, 0.0, 0.0], [44.0, 44.0, 0.2]]
+    for Rdir, fits in ((19.05, True), (20.0, False)):
+        # segments: (n/32 + columns + 1) x the fine columns within reach of a group, squared
+        e = np.cbrt(32 * 44.0 * 44.0 * 0.25 * Rdir / n)
+        nc = int(np.ceil(44.0 / e))
+        bound = (n // 32 + nc * nc + 1) * (int((1 + 2 * Rdir * nc / 44.0) * 2) + 4) ** 2
+        assert (bound < 2 ** 31) == fits
+        with npme_b200.Solver(api.make_params("laplace", "dm", Rdir, 4, 3, (48, 48, 48))) as s:
+            if fits:
+                assert s.setup(c).info()["nGroups"] >= n // 32
+            else:
+                with pytest.raises(api.NPMEError, match="2\\^31"):
+                    s.setup(c)
+
+
 # Zones are built for the walks that use them alone: the others stage the same sources
 # whatever the precision (candidates per point), where FP64 1/r leaves some out.
 def test_zones_only_where_they_are_walked(monkeypatch):
