@@ -112,8 +112,10 @@ std::vector<int> radices(long N, int largest = 16) {
 std::mutex g_tw_mu;
 std::map<std::tuple<int, bool, long>, void *> g_tw;
 
+// (On a stream and waited for: cudaMemcpy from pageable memory may return before the
+// copy has arrived, and non-blocking streams do not wait for it.)
 template <typename C>
-cudaError_t make_table(long N, void **out) {
+cudaError_t make_table(long N, cudaStream_t s, void **out) {
   std::vector<C> t(N);
   for (long m = 0; m < N; m++) {
     const double a = -2.0 * M_PI * (double)m / (double)N;
@@ -121,7 +123,8 @@ cudaError_t make_table(long N, void **out) {
   }
   void *d = nullptr;
   cudaError_t e = cudaMalloc(&d, sizeof(C) * N);
-  if (e == cudaSuccess) e = cudaMemcpy(d, t.data(), sizeof(C) * N, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d, t.data(), sizeof(C) * N, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess && d) cudaFree(d), d = nullptr;
   *out = d;
   return e;
@@ -131,7 +134,8 @@ int twiddles(npme_handle *h, long N, const void **out) {
   std::lock_guard<std::mutex> lk(g_tw_mu);
   void *&d = g_tw[std::make_tuple(h->device, h->fp32, N)];
   if (!d) {
-    const cudaError_t e = h->fp32 ? make_table<float2>(N, &d) : make_table<double2>(N, &d);
+    const cudaError_t e = h->fp32 ? make_table<float2>(N, h->stream, &d)
+                                   : make_table<double2>(N, h->stream, &d);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return record_error(h, NPME_ECUDA, std::string("FFT tables: ") + cudaGetErrorString(e));
