@@ -9,9 +9,11 @@
 //                              coefficients stay in the parameter bank, as in
 //                              the single-system launch
 // Each class launch gets a device array of per-system descriptors and the
-// prefix sums of its work units (points, bricks, spectrum elements, warp
+// prefix sums of its work units (points, bricks, transform CTAs, warp
 // groups); a thread finds its system by binary search over the prefix.  The
-// FFTs run per system with each handle's cuFFT plans.  FP32-bulk handles use
+// library's own transforms take all members of one kind in five launches; boxes with
+// a length that has a prime factor above 5 run one by one with their handles' cuFFT
+// plans.  FP32-bulk handles use
 // the batch kernels; FP64 handles run their ordinary single-system path in
 // the same stream order.  Results equal the single-system path's: the same
 // bodies (bodies.cuh) run on the same data.

@@ -56,8 +56,10 @@ struct PairCoef {
   // two (the same reason; with Rdir in that unit in [1, 2) nothing overflows), kap =
   // k0 in it: cut2 the squared cutoff, cut_bits its bits less kMinNormal64; with P =
   // sum c_n u^n the matched polynomial, u = cut2 - s, (re, im) pairs hc[n] = -c_n
-  // and hd[n] = 2 (n + 1) c_{n+1}, the negated coefficients of 2 dP/ds
-  typename Vec2<T>::type hc[kMaxDeriv + 1], hd[kMaxDeriv + 1];
+  // and hd[n] = 2 (n + 1) c_{n+1}, the negated coefficients of 2 dP/ds.  (FP32
+  // Helmholtz takes nac2 and nbc2.)
+  static constexpr int kHelm64 = sizeof(T) == 8 ? kMaxDeriv + 1 : 1;
+  typename Vec2<T>::type hc[kHelm64], hd[kHelm64];
   T kapr, kapi, cut2;
   unsigned long long cut_bits;
   // Helmholtz packed evaluation: (re, im) pairs of -ar/-ai and -br/-bi

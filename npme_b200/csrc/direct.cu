@@ -16,7 +16,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <complex>
 #include <cstdlib>
 #include <cstring>
 
@@ -103,40 +102,22 @@ PairCoef<T> make_pair_coef(const npme_handle *h) {
       k.kn2.x = k.kn2.y = (T)(2.0 * b / std::sqrt(M_PI));
     }
     k.invR = 1.0 / R;
-    // Helmholtz: G_n = ((1/x) d/dx)^n exp(i kap x)/x at x = 1 (the recursion of
-    // dm_coefficients with Rdir = 1), c_n = G_n (-1)^n / (2^n n!)
-    if (h->p.funcType == NPME_FUNC_HELMHOLTZ) {
-      typedef std::complex<double> cd;
-      // FP64: the unit of length is the greatest power of two <= Rdir, so that
-      // scaling by it rounds nothing and the cutoff is in [1, 2)
-      const double unit = sizeof(T) == 8 ? std::exp2(std::ilogb(R)) : R;
-      const double S2 = (R / unit) * (R / unit);
-      int64_t bits;
-      std::memcpy(&bits, &S2, sizeof(bits));
-      k.cut_bits = (unsigned long long)bits - kMinNormal64;
-      k.cut2 = (T)S2;
-      k.invR = 1.0 / unit;
-      const cd I(0, 1), kap(h->p.k0_r * unit, h->p.k0_i * unit);
-      k.kapr = (T)kap.real(), k.kapi = (T)kap.imag();
-      cd g0 = std::exp(I * kap), g1 = g0 * (I * kap - 1.0);  // G_n, G_{n+1}
-      double f = 1.0;  // (-1)^n / (2^n n!)
-      for (int i = 0; i <= k.nder && i <= kMaxDeriv; i++) {
-        const cd c = g0 * f;
-        k.hc[i].x = (T)-c.real(), k.hc[i].y = (T)-c.imag();
-        const double fn = -f / (2.0 * (i + 1));
-        if (i < k.nder) {
-          const cd d = 2.0 * (i + 1) * fn * g1;
-          k.hd[i].x = (T)d.real(), k.hd[i].y = (T)d.imag();
-        }
-        const cd g2 = -(2.0 * (i + 2) - 1.0) * g1 - kap * kap * g0;
-        g0 = g1, g1 = g2, f = fn;
-      }
-      // FP64: the polynomial that the smooth part carries (its coefficients of
-      // r^2n, rounded, magnify their rounding by their cancellation, 1e3 at |k0|
-      // Rdir = 8), expanded in u = S2 - s, so that what one part adds the other
-      // takes away: otherwise the sum is off by 2e-14 at |k0| Rdir = 10.  The FP32
-      // kernels need the value at the cutoff to be zero and keep the exact c_n.
-      if (sizeof(T) == 8) {
+    if constexpr (sizeof(T) == 8) {
+      if (h->p.funcType == NPME_FUNC_HELMHOLTZ) {
+        // the unit of length is the greatest power of two <= Rdir, so that scaling by
+        // it rounds nothing and the cutoff is in [1, 2)
+        const double unit = std::exp2(std::ilogb(R));
+        const double S2 = (R / unit) * (R / unit);
+        int64_t bits;
+        std::memcpy(&bits, &S2, sizeof(bits));
+        k.cut_bits = (unsigned long long)bits - kMinNormal64;
+        k.cut2 = S2;
+        k.invR = 1.0 / unit;
+        k.kapr = h->p.k0_r * unit, k.kapi = h->p.k0_i * unit;
+        // the polynomial that the smooth part carries (its coefficients of r^2n,
+        // rounded, magnify their rounding by their cancellation, 1e3 at |k0| Rdir = 8),
+        // expanded in u = S2 - s, so that what one part adds the other takes away:
+        // with the exact coefficients the sum is off by 2e-14 at |k0| Rdir = 10
         typedef long double ld;
         ld cr[kMaxDeriv + 1] = {}, ci[kMaxDeriv + 1] = {}, scale = unit;  // unit^(2n + 1)
         for (int n = 0; n <= k.nder && n <= kMaxDeriv; n++, scale *= (ld)unit * unit) {
@@ -228,8 +209,8 @@ static void merge_or_defer(npme_handle *h, const DirectArgs &a, cudaStream_t s, 
 // serial walk of its half-shell list, so with few groups the launch lasts as
 // long as one walk with most of the chip idle, and with about one round of
 // them as long as the heaviest: the walk is split over the warps of a CTA.
-// Measured, whole against split walks: 170 groups (4,000 points) 92 / 26 us
-// with 16 warps, 28 with 8; 1,150 groups (30,000 points in a flat box) 110 /
+// Measured, whole against split walks: 141 groups (4,000 points) 92 / 26 us
+// with 16 warps, 28 with 8; 1,062 groups (30,000 points in a flat box) 110 /
 // 82 us with 4 warps, 96 with 2, 98 with 8; 2,000 groups (FP64 Helmholtz,
 // 62,500 points) 1,530 / 1,098 us with 4.  From about two rounds on the
 // splitting's own work (every warp stages the targets and walks all segments)

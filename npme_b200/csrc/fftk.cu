@@ -174,8 +174,8 @@ size_t own_fft_smem(const FftJob &j, int axis, size_t cbytes) {
   return cbytes * (a.twlen + 2 * (axis == 2 ? (size_t)(a.N + 1) * (B + 1) : (size_t)a.N * B));
 }
 
-// Shared memory of a CTA: at most about half of an SM's while 8 lines or more
-// fit that, so that two or more are resident.  Two lines of the greatest
+// Shared memory of a CTA: at most about half of an SM's, so that two or more are
+// resident, with 4 or 2 lines where 8 do not fit that; two lines of the greatest
 // length (2,048) fit a CTA in FP64 (229,472 bytes along z, complex).
 static constexpr size_t kFftSmem = 100 * 1024, kFftSmemMax = 226 * 1024;
 

@@ -312,8 +312,8 @@ int noalloc_preload(std::string &err);
 // coefficients of r^2n they are rounded after a cancellation that grows with the
 // order, 1e4 at order 15.)  Returns Rdir^alpha.
 double dm_taylor(const npme_params &p, double (&c)[kMaxDeriv + 1], double (&ca)[kMaxDeriv + 1]);
-// true when the direct sum takes the pair-once form (FP32 real DM kernels
-// with the half-shell lists built)
+// true when the direct sum takes the pair-once form (a handle that is set up and
+// does not need the full lists)
 bool pairs_once(const npme_handle *h);
 // true when it walks each target's sources instead (known before the set-up)
 bool needs_full_lists(const npme_handle *h);

@@ -1,6 +1,6 @@
 // Reciprocal sum on the B200: kernel transform (set-up), charge spreading,
-// Fourier-space multiply and potential interpolation.  The FFTs themselves
-// are cuFFT calls issued from npme_gpu.cu.
+// Fourier-space multiply and potential interpolation.  The transforms are in
+// fftk.cu (the library's own) and fft.cu (cuFFT, for other lengths).
 //
 // Grid convention: the charge octant of the reference's compact grid
 // (m in [-N/4, N/4), src/RecSumSupportFunctions.h:100-113) is stored at grid
@@ -870,11 +870,12 @@ void launch_gather_direct(npme_handle *h, const double *d_q, void *d_qdst, cudaS
 // ---------------------------------------------------------------------------
 // Spread (src/RecSumQ.cpp:184-314): Q[g] += q B1 B2 B3.  One CTA per
 // non-empty brick of kBrick^3 stencil origins.  The CTA accumulates its
-// points' stencils into a shared-memory tile of (kBrick + P - 1)^3 grid
-// points with shared atomics (FP32: 64-bit fixed point in two native
-// 32-bit integer atomics, spread_brick_fixed), then adds the tile to the
-// global grid (global atomics only where tiles of neighbouring bricks
-// overlap: one add per tile point instead of one per stencil point).  Complex charges are spread
+// points' stencils into a shared-memory tile of (kBrick + P - 1)^3 grid points, in
+// registers up to order 8 (spread_brick_owner, spread_brick_shared), with shared
+// atomics above (FP32: 64-bit fixed point in two native 32-bit integer atomics,
+// spread_brick_fixed), then adds the tile to the global grid with atomics, one add per
+// tile point instead of one per stencil point.
+// Complex charges are spread
 // without conjugation; with the cyclic convolution used here that gives the
 // reference's theta for conj(q) spreading (src/RecSumQ.cpp:337) because the
 // reference conjugates twice (src/RecSumV.cpp:672).
