@@ -279,6 +279,38 @@ def test_batched_setup_of_mixed_requests_equals_alone():
 
 
 @pytest.mark.gpu
+def test_odd_bricks_in_batches():
+    """Sheets and clusters, whose bricks the spread takes apart from the others, and
+    uniform systems in one set-up pass and in batched CalcVs: each as it is alone, in
+    FP64 (FP32 to its rounding)."""
+    g = np.random.default_rng(12)
+    srv = api.NativeServer(0, setup_threads=1, max_batch=64, pool_capacity=4, setup_batch=64)
+    jobs = []
+    for i, (shape, kernel, order) in enumerate(
+            [(sh, k, o) for sh in ("sheet", "uniform", "cluster")
+             for k in ("laplace", "helmholtz") for o in (4, 6, 8)]):
+        n = 3000 + 500 * i
+        c, q = 20.0 * g.random((n, 3)), g.uniform(0.5, 1.5, n)
+        if shape == "sheet":
+            c[:, 0] = 10.0 + 1e-3 * c[:, 0]
+        elif shape == "cluster":
+            c = 11.3 + 0.05 * c
+        c[:2] = [[0.0] * 3, [20.0] * 3]
+        if kernel == "helmholtz":
+            q = q * np.exp(1j * g.random(n))
+        p = {prec: api.make_params(kernel, "dm", 1.5, order, 6, (64, 64, 64),
+                                   k0=0.5 if kernel == "helmholtz" else 0.0, precision=prec)
+             for prec in ("fp32", "fp64")}
+        jobs.append((c, q, p, [srv.submit(p[prec], c, q) for prec in ("fp32", "fp64")]))
+    for c, q, p, tickets in jobs:
+        with npme_b200.Solver(p["fp64"]) as s:
+            alone = s.setup(c).calcv(q)
+        for t, tol in zip(tickets, (1e-5, 1e-12)):
+            assert rel(srv.result(t)[0], alone) < tol
+    srv.close()
+
+
+@pytest.mark.gpu
 def test_batch_sync_covers_plain_members():
     """npme_gpu_batch_sync waits for every member of the batch, also when all
     members are FP64 (plain) handles, which run their own CalcV on the batch's
