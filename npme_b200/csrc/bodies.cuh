@@ -2415,11 +2415,13 @@ __device__ __forceinline__ void sincos_taylor(double x, double &sn, double &cs) 
 
 // Helmholtz DM pair kernel in FP64 (coordinates times k.invR, s = r^2 in (0, cut2]):
 // F0 = exp(i kap r)/r - P and F1 = (1/r) dF0/dr, P the matched polynomial in u =
-// cut2 - s (PairCoef; src/KernelFunctionHelmholtz.cpp:506-563).
+// cut2 - s (PairCoef; src/KernelFunctionHelmholtz.cpp:506-563).  ND = 0: the order
+// at run time, in a loop.  (Zero-padded to kMaxDeriv as in FP32, the 62 coefficients
+// spilled 560 bytes a thread: 62,501 points 1,840 us at every order, in the loop
+// 1,206 at order 5, 1,423 at 10 and 1,616 at 15.)
 template <int ND>
 __device__ __forceinline__ void helm_eval64(const PairCoef<double> &k, double s, double2 &F0,
                                             double2 &F1) {
-  constexpr int nd = dm_degree<ND>();  // ND = 0: zero-padded to kMaxDeriv
   const double ri = rsqrt_iter(s), r = s * ri, u = k.cut2 - s;
   double sn, cs;
   sincos_taylor(k.kapr * r, sn, cs);
@@ -2427,12 +2429,23 @@ __device__ __forceinline__ void helm_eval64(const PairCoef<double> &k, double s,
   const double er = cs * damp, ei = sn * damp;  // exp(i kap r) / r
   // its radial derivative over r: E (i kap / r - 1 / r^2)
   const double A = fma(-k.kapi, ri, -ri * ri), B = k.kapr * ri;
-  double pr = k.hc[nd].x, pi = k.hc[nd].y;
+  double pr, pi, dr, di;
+  if constexpr (ND == 0) {
+    const int N = k.nder;  // 2 at least
+    pr = fma(k.hc[N].x, u, k.hc[N - 1].x), pi = fma(k.hc[N].y, u, k.hc[N - 1].y);
+    dr = k.hd[N - 1].x, di = k.hd[N - 1].y;
+#pragma unroll 2
+    for (int n = N - 2; n >= 0; n--) {
+      pr = fma(pr, u, k.hc[n].x), pi = fma(pi, u, k.hc[n].y);
+      dr = fma(dr, u, k.hd[n].x), di = fma(di, u, k.hd[n].y);
+    }
+  } else {
+    pr = k.hc[ND].x, pi = k.hc[ND].y, dr = k.hd[ND - 1].x, di = k.hd[ND - 1].y;
 #pragma unroll
-  for (int n = nd - 1; n >= 0; n--) pr = fma(pr, u, k.hc[n].x), pi = fma(pi, u, k.hc[n].y);
-  double dr = k.hd[nd - 1].x, di = k.hd[nd - 1].y;
+    for (int n = ND - 1; n >= 0; n--) pr = fma(pr, u, k.hc[n].x), pi = fma(pi, u, k.hc[n].y);
 #pragma unroll
-  for (int n = nd - 2; n >= 0; n--) dr = fma(dr, u, k.hd[n].x), di = fma(di, u, k.hd[n].y);
+    for (int n = ND - 2; n >= 0; n--) dr = fma(dr, u, k.hd[n].x), di = fma(di, u, k.hd[n].y);
+  }
   F0 = make_double2(er + pr, ei + pi);
   F1 = make_double2(fma(A, er, fma(-B, ei, dr)), fma(A, ei, fma(B, er, di)));
 }

@@ -536,7 +536,8 @@ void launch_merge_source(npme_handle *h, double *V, cudaStream_t s, double vs, d
 }
 
 void clear_source_sums(npme_handle *h, cudaStream_t s) {
-  const size_t b = (h->fp32 ? sizeof(float) : sizeof(double)) * 4 * (h->complex_kernel ? 2 : 1) * h->n;
+  const size_t b =
+      (h->fp32 ? sizeof(float) : sizeof(double)) * 4 * (h->complex_kernel ? 2 : 1) * h->n;
   cudaMemsetAsync(h->fp32 ? (void *)h->d_vsrc : (void *)h->d_vsrc64, 0, b, s);
 }
 

@@ -461,7 +461,8 @@ __global__ void __launch_bounds__(256)
     if (c <= 96) return;
     const int r = owner(boff, R, b);
     const SysDesc &D = d[r];
-    const BrickPoint<T> *pts = static_cast<const BrickPoint<T> *>(D.bpts) + (start[b] - start[D.b_off]);
+    const BrickPoint<T> *pts =
+        static_cast<const BrickPoint<T> *>(D.bpts) + (start[b] - start[D.b_off]);
     int mine = 0;  // lane p < 8: points of plane p
     for (int i = lane; i - lane < c; i += 32) {
       const int p = i < c ? (int)(pts[i].g0 >> 20) & (kBrick - 1) : -1;

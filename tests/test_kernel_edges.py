@@ -253,7 +253,8 @@ def test_exponents(alpha, nd, prec, monkeypatch):
 # the matched polynomial's terms reach (k0 Rdir)^2 times the sum, so the walks
 # differ by their rounding (eps 1e10 at most), relative to the polynomial.
 @pytest.mark.parametrize("k0,nd,tol", [(0.5, 6, 1e-13), (1.1 + 0.2j, 8, 1e-12),
-                                       (3.0 - 0.4j, 4, 1e-12), (24999.0, 2, 1e-9),
+                                       (3.0 - 0.4j, 4, 1e-12), (0.5, 3, 1e-13),
+                                       (0.5, 5, 1e-13), (0.5, 15, 1e-11), (24999.0, 2, 1e-9),
                                        (25001.0, 2, 1e-9)])
 def test_fp64_helmholtz_wave_numbers(k0, nd, tol, monkeypatch):
     w = system(1500, "helmholtz", k0=k0, nDeriv=nd)
