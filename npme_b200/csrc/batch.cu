@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(256) batch_interp_kernel(const BatchSys *__res
   const long long u = blockIdx.x;
   const int s = find_sys(off, count, u);
   const BatchSys &S = sys[s];
-  interp_brick_body<float, P, CPLX>(list_brick(S.brick_list[u - off[s]]), S.brick_start, S.bpts, S.grid, S.V,
-                                    S.nb2, S.nb3, S.g1, S.g2, S.g3, S.c1, S.c2, S.c3,
+  interp_brick_body<float, P, CPLX>(list_brick(S.brick_list[u - off[s]]), S.brick_start, S.bpts,
+                                    S.grid, S.V, S.nb2, S.nb3, S.g1, S.g2, S.g3, S.c1, S.c2, S.c3,
                                     reinterpret_cast<float *>(smem_raw),
                                     S.fold ? (void *)S.vsrc : nullptr, S.vs, S.gs);
 }

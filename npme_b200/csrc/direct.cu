@@ -150,9 +150,9 @@ template PairCoef<double> make_pair_coef<double>(const npme_handle *);
 // group's source segments in chunks of 32 that run across segment
 // boundaries: every lane loads one source (FP64 position), the warp stages
 // the chunk in shared memory as float coordinates relative to the group
-// centre and every lane then sweeps the staged chunk for its target.  The next chunk's loads are issued before the
-// sweep, so global latency hides behind the arithmetic.  Warps are
-// independent: only __syncwarp, no block barrier.
+// centre and every lane then sweeps the staged chunk for its target.  The next
+// chunk's loads are issued before the sweep, so global latency hides behind the
+// arithmetic.  Warps are independent: only __syncwarp, no block barrier.
 //
 // Coordinates: each FP64 offset from the group centre is split into a float
 // head and the float residual (hi + lo).  The distance test and the pair

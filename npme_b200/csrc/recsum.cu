@@ -1015,9 +1015,9 @@ __global__ void __launch_bounds__(256) interp_kernel(
     int nb2, int nb3, long N1, long N2, long N3, T c1, T c2, T c3, void *vsrc, double vs,
     double gs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  interp_brick_body<T, P, CPLX>(list_brick(brick_list[blockIdx.x]), brick_start, bp, theta, V, nb2, nb3, N1,
-                                N2, N3, c1, c2, c3, reinterpret_cast<T *>(smem_raw), vsrc, vs,
-                                gs);
+  interp_brick_body<T, P, CPLX>(list_brick(brick_list[blockIdx.x]), brick_start, bp, theta, V, nb2,
+                                nb3, N1, N2, N3, c1, c2, c3, reinterpret_cast<T *>(smem_raw), vsrc,
+                                vs, gs);
 }
 
 template <typename T, bool CPLX, int P>
